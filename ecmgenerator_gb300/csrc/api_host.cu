@@ -140,6 +140,7 @@ bool ecmg::knn_grid_of(float x0, float y0, float x1, float y1, float cell, Agent
     g.gw = (int)gw;
     g.gh = (int)gh;
     g.ncells = g.gw * g.gh;
+    g.slack = grid_slack(g.x0, g.y0, g.cell, g.gw, g.gh);
     *out = g;
     return true;
 }

@@ -133,10 +133,13 @@ struct ecmg_ctx {
     /* launch configuration (autotuned) */
     int block = 128;
     int tile = 32;
-    float cell_scale = 0.4f;
+    /* cells of a quarter of the k nearest agents' square: 0.25-0.3 is best from
+       25,000 to a million agents (neighbour kernel 56 us at 0.25 against 70 at
+       0.4 with 25,000 agents in 500 m, 324 against 330 at a million) */
+    float cell_scale = 0.25f;
     int lp_mode = 0; /* ECMG_LP_THREAD, ECMG_LP_WARP or ECMG_LP_THREAD_FUSED */
     int occ_div = 1; /* per-thread layout: resident blocks per SM divided by this */
-    int knn_wide = 0; /* neighbour kernel register budget (TickArgs::knn_wide) */
+    int knn_wide = 0; /* neighbour kernel: 8 resident blocks per SM at most, or 6 */
     int wgrab = 4;   /* agents per work grab in warp mode */
 
     /* host mirrors (Simulator bookkeeping, Simulator.h:164-171) */
@@ -1752,15 +1755,21 @@ static ecmg_status ensure_grids(ecmg_ctx* c)
                 cell = std::sqrt((float)c->prm.max_neighbors / dens) * c->cell_scale;
                 cell = std::min(std::max(cell, 0.3f), std::max(0.3f, c->prm.neighbor_dist));
             }
-            while ((double)(w / cell + 3) * (double)(h / cell + 3) > 32.0e6) cell *= 1.5f; /* <= 32M cells */
+            /* a dense crowd pushes agents out of the scene (some 8 m after 450
+               ticks of the 1M crossing, 3 % of it): cells of their own there
+               keep the border cells from filling up */
+            const float pad = std::min(2.0f * c->prm.neighbor_dist, 0.25f * std::max(w, h));
+            while ((double)((w + 2.0f * pad) / cell + 3) * (double)((h + 2.0f * pad) / cell + 3) > 32.0e6)
+                cell *= 1.5f; /* <= 32M cells */
             AgentGrid g;
             g.cell = cell;
             g.inv = 1.0f / cell;
-            g.x0 = s.bx0 - cell;
-            g.y0 = s.by0 - cell;
-            g.gw = (int)std::ceil(w / cell) + 3;
-            g.gh = (int)std::ceil(h / cell) + 3;
+            g.x0 = s.bx0 - pad - cell;
+            g.y0 = s.by0 - pad - cell;
+            g.gw = (int)std::ceil((w + 2.0f * pad) / cell) + 3;
+            g.gh = (int)std::ceil((h + 2.0f * pad) / cell) + 3;
             g.ncells = g.gw * g.gh;
+            g.slack = grid_slack(g.x0, g.y0, g.cell, g.gw, g.gh);
             sc->grid = g;
             sc->grid_ready = true;
             sc->grid_agents = std::max(1, sc->num_agents);
@@ -1774,7 +1783,7 @@ static ecmg_status ensure_grids(ecmg_ctx* c)
             SceneState* sc = c->scenes[i].get();
             HostScene& s = sc->hs;
             sc->bucket_base = base;
-            base += sc->grid.ncells + 1;
+            base += sc->grid.ncells;
             SceneDev& d = tab[i];
             d = SceneDev{};
             d.grid = sc->grid;
@@ -1877,7 +1886,7 @@ static void fill_args(ecmg_ctx* c, BinArgs& b, TickArgs& t, bool use_model)
     t.tile = c->lp_mode == ECMG_LP_WARP ? c->wgrab : c->tile;
     t.lp_mode = c->lp_mode;
     t.occ_div = c->occ_div;
-    t.knn_wide = c->knn_wide;
+    t.knn_blocks = c->knn_wide ? 6 : 8;
     const ecmg_params& p = c->prm;
     t.dt = p.dt;
     t.tau_a = p.tau_agent;
@@ -2032,8 +2041,6 @@ int ecmg_kernels_per_tick(const ecmg_ctx* c)
     if (c->nbr_mode == ECMG_NEIGHBORS_KDTREE) {
         const int L = c->kd.levels;
         n += -1 + 6 + 84 + 1 + 11 + (L - 1) + 5 * std::max(0, L - 2) + 2 + 4;
-    } else if (c->lp_mode == ECMG_LP_THREAD_FUSED && !c->model && !c->trace) {
-        n -= 1; /* the search runs inside the per-agent kernel */
     }
     return n;
 }

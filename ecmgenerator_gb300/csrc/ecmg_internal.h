@@ -58,13 +58,21 @@ enum {
     ECMG_DEV_ERR_MLP = 4, /* a bounded wait of the tensor-core inference gave up */
 };
 
-/* Uniform agent grid: cells [0, gw*gh) cover the scene rectangle; agents
-   outside it go to the overflow bucket gw*gh, which every query scans. */
+/* Uniform agent grid: cells [0, gw*gh) cover the scene rectangle; an agent
+   outside it belongs to the nearest border cell.  slack: the distance (m) by
+   which the rounding of a cell index may misplace an agent, generously. */
 struct AgentGrid {
-    float x0, y0, cell, inv;
+    float x0, y0, cell, inv, slack;
     int gw, gh;
-    int ncells; /* gw*gh, overflow bucket index */
+    int ncells; /* gw*gh */
 };
+/* slack of a grid: 1 cm, or more where a coordinate inside the grid has an
+   ulp (times the steps of the index computation) that is not small beside it */
+inline float grid_slack(float x0, float y0, float cell, int gw, int gh)
+{
+    const float reach = fmaxf(fmaxf(fabsf(x0), fabsf(y0)), fmaxf((float)gw, (float)gh) * cell);
+    return fmaxf(0.01f, 1.0e-6f * reach);
+}
 
 /* One independent scene of a batch: its agent grid, the first of its
    buckets in the global bucket array, and its static obstacle / ECM views
@@ -105,9 +113,9 @@ struct TickArgs {
     const SceneDev* scenes;
     const int* slot_scene; /* slot -> scene (null: one scene) */
     int tile;              /* agents a warp takes per work grab (per-thread mode: multiple of 32) */
-    int lp_mode;           /* 0: one thread per agent, 1: one warp per agent */
+    int lp_mode;           /* 1: one warp per agent, else one thread per agent */
     int occ_div;           /* per-thread layout: resident blocks per SM divided by this */
-    int knn_wide;          /* neighbour kernel: 0 = 8 blocks of 128 threads per SM (64 registers), 1 = 6 (80) */
+    int knn_blocks;        /* neighbour kernel: resident blocks of 128 threads per SM at most */
     /* parameters */
     float dt, tau_a, tau_o, rnb, rnb2, max_speed, mass_recip, arr_sq, del_sq;
     float inv_tau_a;       /* 1 / tau_a when tau_a is a power of two (exact), else 0 */

@@ -20,31 +20,12 @@
  * of separately rounded operations.
  */
 #include "ecmg_internal.h"
+#include "knn_rows.cuh"
 
 #include <cuda_bf16.h>
 #include <stdint.h>
 
 namespace ecmg {
-
-/* ---------------------------------------------------------------------- */
-/* grid cell of a position; cells outside [0,gw)x[0,gh) -> overflow bucket  */
-__device__ __forceinline__ void cell_of(const AgentGrid& g, V2 p, int* cx, int* cy)
-{
-    float fx = (p.x - g.x0) * g.inv;
-    float fy = (p.y - g.y0) * g.inv;
-    fx = fminf(fmaxf(fx, -1.0e6f), 1.0e6f); /* NaN -> -1e6 (fmaxf drops NaN) */
-    fy = fminf(fmaxf(fy, -1.0e6f), 1.0e6f);
-    *cx = (int)floorf(fx);
-    *cy = (int)floorf(fy);
-}
-
-__device__ __forceinline__ int bucket_of(const AgentGrid& g, V2 p)
-{
-    int cx, cy;
-    cell_of(g, p, &cx, &cy);
-    if (cx < 0 || cy < 0 || cx >= g.gw || cy >= g.gh) return g.ncells;
-    return cy * g.gw + cx;
-}
 
 __global__ void k_bin(BinArgs a)
 {
@@ -149,333 +130,6 @@ static cudaError_t scan(const int* in, int* out, int n, int* tmp, cudaStream_t s
     k_scan_top<<<1, kScanBlock, 0, s>>>(tmp, nb, out, n);
     k_scan_add<<<nb, kScanBlock, 0, s>>>(out, tmp, n);
     return cudaGetLastError();
-}
-
-/* ---------------------------------------------------------------------- */
-/* exact kNN on the grid: the k smallest (d2, slot) with EPS < d2 < r^2.
-   keys: d2 bits (non-negative floats order as unsigned ints) : slot.
-   The list holds the k nearest in key[K-k .. K-1], ascending; key[0 .. K-k)
-   hold 0 (below every real key, as d2 > EPS) and never move, unfilled
-   entries hold ~0 (above every real key), so the k-th key is key[K-1].  The
-   slot in the low half of a key identifies the neighbour; its grid-order
-   index is recovered once at the end (bucket start + rank of the slot). */
-template <int K>
-struct Knn {
-    unsigned long long key[K];
-    int cnt;
-};
-
-template <int K>
-__device__ __forceinline__ void knn_consider(Knn<K>& s, int k, int j, V2 p, const V2* s_pos, const int* s_slot,
-                                             float r2)
-{
-    V2 q = s_pos[j];
-    float dx = q.x - p.x, dy = q.y - p.y;
-    float d2 = dx * dx + dy * dy; /* KDTree.cpp:107-108 */
-    if (!(d2 > kEps) || !(d2 < r2)) return;
-    unsigned hi = __float_as_uint(d2);
-    if (hi > (unsigned)(s.key[K - 1] >> 32)) return;
-    unsigned long long kk = ((unsigned long long)hi << 32) | (unsigned)s_slot[j];
-    if (kk >= s.key[K - 1]) return;
-    /* drop key[K-1], shift the larger entries up, place kk */
-#pragma unroll
-    for (int q = K - 1; q >= 0; q--) {
-        unsigned long long nk;
-        if (q > 0 && s.key[q - 1] > kk) nk = s.key[q - 1];
-        else if (s.key[q] > kk) nk = kk;
-        else nk = s.key[q];
-        s.key[q] = nk;
-    }
-    if (s.cnt < k) s.cnt++;
-}
-
-template <int K>
-__device__ void knn_grid(Knn<K>& s, int k, V2 p, float rnb, float r2, const V2* s_pos, const int* s_slot,
-                         const int* cell_start, const AgentGrid& g)
-{
-#pragma unroll
-    for (int q = 0; q < K; q++) s.key[q] = q < K - k ? 0ull : ~0ull;
-    s.cnt = 0;
-    int cx, cy;
-    cell_of(g, p, &cx, &cy);
-    float x0 = g.x0 + (float)cx * g.cell, y0 = g.y0 + (float)cy * g.cell;
-    float m = fminf(fminf(p.x - x0, x0 + g.cell - p.x), fminf(p.y - y0, y0 + g.cell - p.y));
-    m = fmaxf(m, 0.0f);
-    const int rmax = (int)ceilf(rnb * g.inv) + 2;
-    /* ring R = -1 is the overflow bucket (agents outside the grid rectangle);
-       ring R >= 0 are the cells at Chebyshev distance R.  Every candidate range
-       funnels into one loop so that the insertion code exists once. */
-    for (int R = -1; R <= rmax; R++) {
-        if (R >= 1) {
-            /* lower bound of the distance to any agent in ring R or beyond;
-               1 cm absorbs the rounding of the bucket assignment */
-            float lb = (float)(R - 1) * g.cell + m - 0.01f;
-            if (lb >= rnb) break;
-            if (s.cnt == k && lb > 0.0f && lb * lb > __uint_as_float((unsigned)(s.key[K - 1] >> 32))) break;
-        }
-        const int ylo = R < 0 ? 0 : cy - R, yhi = R < 0 ? 0 : cy + R;
-        for (int y = ylo; y <= yhi; y++) {
-            /* cells whose distance from p (less 1 cm for the rounding of the
-               bucket assignment) exceeds the current k-th distance, or the
-               neighbour distance, cannot hold an accepted candidate */
-            const float kd2 = s.cnt == k ? __uint_as_float((unsigned)(s.key[K - 1] >> 32)) : r2;
-            float dy = 0.0f;
-            if (R >= 0) {
-                const float ry0 = g.y0 + (float)y * g.cell;
-                dy = fmaxf(fmaxf(ry0 - p.y, p.y - (ry0 + g.cell)) - 0.01f, 0.0f);
-                if (dy * dy > kd2) continue;
-            }
-            for (int side = 0; side < 2; side++) {
-                int j0 = 0, j1 = 0;
-                if (R < 0) {
-                    if (side == 0) { j0 = cell_start[g.ncells]; j1 = cell_start[g.ncells + 1]; }
-                } else if (y >= 0 && y < g.gh) {
-                    const int xa = cx - R, xb = cx + R;
-                    if (y == ylo || y == yhi) {
-                        const float dxm = sqrtf(kd2 - dy * dy) + 0.01f;
-                        const int xl = (int)floorf(fmaxf((p.x - dxm - g.x0) * g.inv, -1.0e6f));
-                        const int xr = (int)floorf(fminf((p.x + dxm - g.x0) * g.inv, 1.0e6f));
-                        int a = max(max(xa, 0), xl), b = min(min(xb, g.gw - 1), xr);
-                        if (side == 0 && a <= b) { j0 = cell_start[y * g.gw + a]; j1 = cell_start[y * g.gw + b + 1]; }
-                    } else {
-                        int x = side == 0 ? xa : xb;
-                        if (x >= 0 && x < g.gw && (side == 0 || xb != xa)) {
-                            const float rx0 = g.x0 + (float)x * g.cell;
-                            const float dx = fmaxf(fmaxf(rx0 - p.x, p.x - (rx0 + g.cell)) - 0.01f, 0.0f);
-                            if (!(dx * dx + dy * dy > kd2)) {
-                                j0 = cell_start[y * g.gw + x];
-                                j1 = cell_start[y * g.gw + x + 1];
-                            }
-                        }
-                    }
-                }
-                for (int j = j0; j < j1; j++) knn_consider<K>(s, k, j, p, s_pos, s_slot, r2);
-            }
-        }
-    }
-}
-
-/* ---------------------------------------------------------------------- */
-/* Fast path of the exact kNN: cells in ascending order of their distance.
-   The grid cells around an agent's cell (Chebyshev radius <= kTmplR) are
-   visited in ascending order of their smallest distance from the quarter of
-   the agent's cell that holds the agent (a table built at compile time for
-   the lower-left quarter and mirrored for the others), so the k nearest are
-   met early and few candidates enter the list only to be dropped again; the
-   walk stops at the first cell whose distance bound exceeds the current k-th
-   distance.
-   The list holds packed keys: a candidate's d2 with its 12 low mantissa bits
-   replaced by a code of where it came from (table step, offset in its
-   cell), so that one float min / max pair per list position inserts it --
-   the ALU pipe's work -- and the code gives its grid index back at the end.
-   Packed keys order candidates by d2 except within a relative 2^-11 of each
-   other ("near ties"); those groups are re-sorted by the exact (d2, slot)
-   key afterwards.  The list keeps two entries beyond the k-th so that a near
-   tie at the k-th is resolved inside the list; when it may reach beyond it
-   (a dropped candidate with the same leading bits), when a cell holds more
-   than 32 agents, when the table ends before the search could (sparse
-   crowds) or when the agent is outside the grid, the search returns false
-   and the caller runs the 64-bit (d2, slot) search (knn_grid). */
-constexpr int kTmplR = 5;
-/* bound per axis from the quarter [0, 1/2] of cell 0 to cell d, in half cells */
-constexpr int tmpl_half(int d) { return d >= 1 ? 2 * d - 1 : (d <= -1 ? 2 * (-d - 1) : 0); }
-/* the table holds the cells whose bound is at most kTmplR cells: every cell
-   outside it is at least kTmplR cells away, so a walk that stops inside the
-   table has passed every cell that can hold a closer agent */
-constexpr bool tmpl_in(int dx, int dy)
-{
-    return tmpl_half(dx) * tmpl_half(dx) + tmpl_half(dy) * tmpl_half(dy) <= 4 * kTmplR * kTmplR;
-}
-constexpr int tmpl_count()
-{
-    int n = 0;
-    for (int dy = -kTmplR; dy <= kTmplR; dy++)
-        for (int dx = -kTmplR; dx <= kTmplR; dx++) n += tmpl_in(dx, dy) ? 1 : 0;
-    return n;
-}
-constexpr int kTmplN = tmpl_count();
-struct KnnTemplate {
-    signed char dx[kTmplN], dy[kTmplN];
-    unsigned char hx[kTmplN], hy[kTmplN]; /* distance bound per axis in half cells */
-};
-constexpr KnnTemplate make_knn_template()
-{
-    KnnTemplate t{};
-    int key[kTmplN] = {};
-    int n = 0;
-    for (int dy = -kTmplR; dy <= kTmplR; dy++)
-        for (int dx = -kTmplR; dx <= kTmplR; dx++) {
-            if (!tmpl_in(dx, dy)) continue;
-            const int hx = tmpl_half(dx), hy = tmpl_half(dy);
-            /* squared bound, then the nearer cells first among equal bounds */
-            const int kk = (hx * hx + hy * hy) * 1024 + (dx < 0 ? -dx : dx) + (dy < 0 ? -dy : dy);
-            int i = n++;
-            while (i > 0 && key[i - 1] > kk) {
-                key[i] = key[i - 1];
-                t.dx[i] = t.dx[i - 1];
-                t.dy[i] = t.dy[i - 1];
-                t.hx[i] = t.hx[i - 1];
-                t.hy[i] = t.hy[i - 1];
-                i--;
-            }
-            key[i] = kk;
-            t.dx[i] = (signed char)dx;
-            t.dy[i] = (signed char)dy;
-            t.hx[i] = (unsigned char)hx;
-            t.hy[i] = (unsigned char)hy;
-        }
-    return t;
-}
-__constant__ KnnTemplate c_knn_tmpl = make_knn_template();
-
-constexpr unsigned kCodeMask = 0xFFFu;  /* low mantissa bits of a packed key */
-constexpr int kCodeOverflow = 127;       /* table step code of the overflow bucket */
-static_assert(kTmplN < kCodeOverflow, "table steps must fit 7 bits");
-
-__device__ __forceinline__ unsigned key_hi(float k) { return __float_as_uint(k) & ~kCodeMask; }
-
-/* one candidate (grid index j) into the packed list of KL entries; code =
-   table step << 5 | offset in the cell; a candidate not kept, or the entry
-   pushed out, lowers *rej */
-template <int KL>
-__device__ __forceinline__ void knn_pk_consider(float* key, float* rej, int j, unsigned code, V2 p, float r2,
-                                                const V2* s_pos)
-{
-    const V2 q = s_pos[j];
-    const float dx = q.x - p.x, dy = q.y - p.y;
-    const float d2 = dx * dx + dy * dy; /* KDTree.cpp:107-108 */
-    if (!(d2 > kEps) || !(d2 < r2)) return;
-    float nk = __uint_as_float((__float_as_uint(d2) & ~kCodeMask) | code);
-    if (nk < key[KL - 1]) {
-        /* every entry from the old list alone (no chain through the list):
-           entry q becomes min(old q, max(old q-1, nk)); the entry pushed out
-           is max(old last, nk) */
-        const float out = fmaxf(key[KL - 1], nk);
-#pragma unroll
-        for (int q2 = KL - 1; q2 > 0; q2--) key[q2] = fminf(key[q2], fmaxf(key[q2 - 1], nk));
-        key[0] = fminf(key[0], nk);
-        nk = out;
-    }
-    *rej = fminf(*rej, nk);
-}
-
-/* grid index of a packed key's candidate */
-__device__ __forceinline__ int knn_pk_index(float k, int cx, int cy, int sx, int sy, const int* cell_start,
-                                            const AgentGrid& g)
-{
-    const unsigned code = __float_as_uint(k) & kCodeMask;
-    const int i = (int)(code >> 5), off = (int)(code & 31u);
-    if (i == kCodeOverflow) return cell_start[g.ncells] + off;
-    const int x = cx + sx * (int)c_knn_tmpl.dx[i], y = cy + sy * (int)c_knn_tmpl.dy[i];
-    return cell_start[y * g.gw + x] + off;
-}
-
-/* where a packed list's codes point: the agent's cell and mirror signs */
-struct PkFrame {
-    int cx, cy, sx, sy;
-};
-
-/* the packed list of KL entries */
-template <int KL>
-struct PkList {
-    float key[KL];
-};
-
-/* near ties in the list (rare; out of line): the valid entries from lo on
-   decoded, re-sorted by the exact (d2, slot) key and the first k written to
-   o[0 .. k) (-1 beyond the count) */
-template <int KL>
-__device__ __noinline__ void knn_pk_write_exact(PkList<KL> L, int lo, int k, PkFrame f, V2 p, const V2* s_pos,
-                                                const int* s_slot, const int* cell_start, AgentGrid g, int* o)
-{
-    unsigned long long ek[KL];
-    int id[KL];
-    int n = 0;
-    for (int q = lo; q < KL; q++) {
-        if (!(L.key[q] < INFINITY)) break;
-        const int j = knn_pk_index(L.key[q], f.cx, f.cy, f.sx, f.sy, cell_start, g);
-        const V2 c = s_pos[j];
-        const float dx = c.x - p.x, dy = c.y - p.y;
-        const float d2 = dx * dx + dy * dy;
-        ek[n] = ((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)s_slot[j];
-        id[n] = j;
-        n++;
-    }
-    for (int q = 1; q < n; q++) {
-        for (int r = q; r > 0 && ek[r - 1] > ek[r]; r--) {
-            const unsigned long long t = ek[r];
-            ek[r] = ek[r - 1];
-            ek[r - 1] = t;
-            const int ti = id[r];
-            id[r] = id[r - 1];
-            id[r - 1] = ti;
-        }
-    }
-    for (int q = 0; q < k; q++) o[q] = q < n ? id[q] : -1;
-}
-
-/* 1: the packed list in *L is exact apart from near ties inside it (2: with
-   such ties); 0: the caller must run the 64-bit search.  *cnt = count. */
-template <int K>
-__device__ __forceinline__ int knn_fast(PkList<K + 2>* L, PkFrame* f, int k, V2 p, float r2, const V2* s_pos,
-                                        const int* cell_start, const AgentGrid& g, int* cnt)
-{
-    constexpr int KL = K + 2; /* two entries beyond the k-th */
-    float* key = L->key;
-#pragma unroll
-    for (int q = 0; q < KL; q++) key[q] = q < K - k ? 0.0f : INFINITY; /* 0: below every candidate */
-    float rej = INFINITY;
-    const int o0 = cell_start[g.ncells], o1 = cell_start[g.ncells + 1];
-    if (o1 - o0 > 32) return 0;
-    for (int j = o0; j < o1; j++)
-        knn_pk_consider<KL>(key, &rej, j, (unsigned)(kCodeOverflow << 5) | (unsigned)(j - o0), p, r2, s_pos);
-    const float fx = (p.x - g.x0) * g.inv, fy = (p.y - g.y0) * g.inv;
-    if (!(fx >= 0.0f && fy >= 0.0f && fx < (float)g.gw && fy < (float)g.gh)) return 0;
-    const int cx = (int)fx, cy = (int)fy;
-    const int sx = fx - (float)cx < 0.5f ? 1 : -1, sy = fy - (float)cy < 0.5f ? 1 : -1;
-    f->cx = cx;
-    f->cy = cy;
-    f->sx = sx;
-    f->sy = sy;
-    const float half = 0.5f * g.cell;
-    bool crowded = false;
-    int i = 0;
-    for (; i < kTmplN; i++) {
-        /* the largest d2 the k-th entry can stand for */
-        const float kd = fminf(r2, __uint_as_float(__float_as_uint(key[K - 1]) | kCodeMask));
-        /* every later cell is at least this far from the agent (1 cm for the
-           rounding of the bucket assignment) */
-        const float bx = fmaxf((float)c_knn_tmpl.hx[i] * half - 0.01f, 0.0f);
-        const float by = fmaxf((float)c_knn_tmpl.hy[i] * half - 0.01f, 0.0f);
-        if (bx * bx + by * by > kd) break;
-        const int x = cx + sx * (int)c_knn_tmpl.dx[i], y = cy + sy * (int)c_knn_tmpl.dy[i];
-        if (x < 0 || y < 0 || x >= g.gw || y >= g.gh) continue;
-        const float rx0 = g.x0 + (float)x * g.cell, ry0 = g.y0 + (float)y * g.cell;
-        const float ex = fmaxf(fmaxf(rx0 - p.x, p.x - (rx0 + g.cell)) - 0.01f, 0.0f);
-        const float ey = fmaxf(fmaxf(ry0 - p.y, p.y - (ry0 + g.cell)) - 0.01f, 0.0f);
-        if (ex * ex + ey * ey > kd) continue;
-        const int c = y * g.gw + x;
-        const int j0 = cell_start[c], j1 = cell_start[c + 1];
-        crowded |= j1 - j0 > 32;
-        const unsigned base = (unsigned)i << 5;
-        for (int j = j0; j < j1; j++) knn_pk_consider<KL>(key, &rej, j, base | (unsigned)(j - j0), p, r2, s_pos);
-    }
-    if (i == kTmplN || crowded) return 0;
-    int n = 0;
-    bool tie = false;
-#pragma unroll
-    for (int q = 0; q < KL; q++) {
-        if (q < K - k || !(key[q] < INFINITY)) continue;
-        if (q < K) n++;
-        if (q + 1 < KL && key[q + 1] < INFINITY && key_hi(key[q + 1]) == key_hi(key[q])) tie = true;
-    }
-    /* a dropped candidate may share the k-th entry's leading bits only when
-       the group reaches the list's last entry */
-    if (n == k && key[KL - 1] < INFINITY && key_hi(key[KL - 1]) == key_hi(key[K - 1]) &&
-        key_hi(rej) == key_hi(key[K - 1]))
-        return 0;
-    *cnt = n;
-    return tie ? 2 : 1;
 }
 
 /* ---------------------------------------------------------------------- */
@@ -812,61 +466,15 @@ __device__ void orca_tick(const TickArgs& a, int t)
     }
 }
 
-/* the 64-bit (d2, slot) search of grid-order agent t (rare: equal
-   distances, sparse crowds, agents outside the grid); out of line so that it
-   does not take registers from the fast path */
-template <int K>
-__device__ __noinline__ void knn_agent_exact(const TickArgs& a, int t, const SceneDev& sc)
-{
-    Knn<K> nn;
-    knn_grid<K>(nn, a.k, a.s_pos[t], a.rnb, a.rnb2, a.s_pos, a.s_slot, a.cell_start + sc.bucket_base, sc.grid);
-    a.ncnt[t] = nn.cnt;
-    int* o = a.nbr + (size_t)t * a.k;
-#pragma unroll
-    for (int q2 = 0; q2 < K; q2++) {
-        const int q = q2 - (K - a.k);
-        if (q >= 0) {
-            const int sl = (int)(unsigned)nn.key[q2];
-            o[q] = q < nn.cnt ? a.cell_start[a.slot_bucket[sl]] + a.slot_rank[sl] : -1;
-        }
-    }
-}
-
-/* neighbour lists of every grid-order agent of the tick (KNearestAgents,
-   KDTree.cpp:85-202, as the exact (d2, slot) query of the grid) */
-template <int K>
-__device__ __forceinline__ void knn_agent(const TickArgs& a, int t, int slot)
-{
-    const SceneDev& sc = a.scenes[a.slot_scene ? a.slot_scene[slot] : 0];
-    const int* cs = a.cell_start + sc.bucket_base;
-    const V2 p = a.s_pos[t];
-    PkList<K + 2> L;
-    PkFrame f;
-    int n = 0;
-    const int st = knn_fast<K>(&L, &f, a.k, p, a.rnb2, a.s_pos, cs, sc.grid, &n);
-    if (st != 0) {
-        a.ncnt[t] = n;
-        int* o = a.nbr + (size_t)t * a.k;
-        if (st == 1) {
-#pragma unroll
-            for (int q2 = 0; q2 < K; q2++) {
-                const int q = q2 - (K - a.k);
-                if (q >= 0) o[q] = q < n ? knn_pk_index(L.key[q2], f.cx, f.cy, f.sx, f.sy, cs, sc.grid) : -1;
-            }
-        } else {
-            knn_pk_write_exact<K + 2>(L, K - a.k, a.k, f, p, a.s_pos, a.s_slot, cs, sc.grid, o);
-        }
-        return;
-    }
-    knn_agent_exact<K>(a, t, sc);
-}
-
-/* persistent: a warp takes 32 consecutive grid-order agents per work grab
+/* neighbour lists of every grid-order agent of the tick (knn_rows.cuh).
+   Persistent: a warp takes 32 consecutive grid-order agents per work grab
    (neighbouring agents: their candidates share L1), so that warps whose
    agents have more candidates do not leave the SMs' last wave ragged */
-template <int K, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_neighbors(TickArgs a)
+constexpr int kNbrWarps = 4; /* per block */
+template <int K>
+__global__ void __launch_bounds__(32 * kNbrWarps, K <= 16 ? 8 : 4) k_neighbors(TickArgs a)
 {
+    __shared__ KnnSm<K> sm[kNbrWarps];
     const int n = a.counters[C_NSORTED];
     const int lane = threadIdx.x & 31;
     while (true) {
@@ -874,8 +482,12 @@ __global__ void __launch_bounds__(128, MINB) k_neighbors(TickArgs a)
         if (lane == 0) base = atomicAdd(&a.counters[C_NBR_WORK], 32);
         base = __shfl_sync(0xffffffffu, base, 0);
         if (base >= n) break;
-        const int t = base + lane;
-        if (t < n) knn_agent<K>(a, t, a.s_slot[t]);
+        const int t = min(base + lane, n - 1);
+        const bool in = base + lane < n;
+        const SceneDev& sc = a.scenes[a.slot_scene ? a.slot_scene[a.s_slot[t]] : 0];
+        const int c = knn_list<K, false>(sm[threadIdx.x >> 5], in, a.k, a.s_pos[t], a.rnb2, a.s_pos, a.s_slot,
+                                  a.cell_start + sc.bucket_base, sc.grid, a.nbr + (size_t)t * a.k);
+        if (in) a.ncnt[t] = c;
     }
 }
 
@@ -981,32 +593,6 @@ __global__ void __launch_bounds__(256, (K <= 16) ? 4 : 1) k_agents(TickArgs a)
         for (int o = 0; o < a.tile; o += 32) {
             int t = base + o + lane;
             if (t < n) orca_tick<K, FULL>(a, t);
-        }
-    }
-}
-
-/* the per-thread layout fused with the neighbour search (ECMG_LP_THREAD_FUSED):
-   each thread finds its agent's k nearest, then runs the agent's step, so
-   that warps in the ALU-bound search and warps in the issue-bound LPs share
-   every SM.  Agents destroyed by the attraction kernel get no list (no later
-   stage of a plain tick reads it). */
-template <int K, bool FULL>
-__global__ void __launch_bounds__(256) k_agents_knn(TickArgs a)
-{
-    const int n = a.counters[C_NSORTED];
-    const int lane = threadIdx.x & 31;
-    while (true) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(&a.counters[C_WORK], a.tile);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= n) break;
-        for (int o = 0; o < a.tile; o += 32) {
-            const int t = base + o + lane;
-            if (t >= n) continue;
-            const int slot = a.s_slot[t];
-            if (!a.active[slot]) continue;
-            knn_agent<K>(a, t, slot);
-            orca_tick<K, FULL>(a, t);
         }
     }
 }
@@ -1394,23 +980,22 @@ __global__ void __launch_bounds__(256) k_agents_warp(TickArgs a)
     }
 }
 
+/* the stand-alone query: lists of slots by slot */
 template <int K>
-__global__ void __launch_bounds__(128) k_knn(const V2* s_pos, const int* s_slot, const int* cell_start,
-                                             AgentGrid g, int k, float rnb, float r2, const int* counters,
-                                             int* out_ids, int* out_cnt)
+__global__ void __launch_bounds__(32 * kNbrWarps, K <= 16 ? 8 : 4)
+    k_knn(const V2* s_pos, const int* s_slot, const int* cell_start, AgentGrid g, int k, float r2, const int* counters,
+          int* out_ids, int* out_cnt)
 {
+    __shared__ KnnSm<K> sm[kNbrWarps];
     const int n = counters[C_NSORTED];
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        Knn<K> nn;
-        V2 p = s_pos[t];
-        knn_grid<K>(nn, k, p, rnb, r2, s_pos, s_slot, cell_start, g);
-        int slot = s_slot[t];
-        out_cnt[slot] = nn.cnt;
-#pragma unroll
-        for (int q2 = 0; q2 < K; q2++) {
-            const int q = q2 - (K - k);
-            if (q >= 0) out_ids[slot * k + q] = q < nn.cnt ? (int)(unsigned)nn.key[q2] : -1;
-        }
+    const int lane = threadIdx.x & 31;
+    for (int base = (blockIdx.x * kNbrWarps + (threadIdx.x >> 5)) * 32; base < n; base += gridDim.x * kNbrWarps * 32) {
+        const int t = min(base + lane, n - 1);
+        const bool in = base + lane < n;
+        const int slot = s_slot[t];
+        int* o = out_ids + (size_t)slot * k;
+        const int c = knn_list<K, true>(sm[threadIdx.x >> 5], in, k, s_pos[t], r2, s_pos, s_slot, cell_start, g, o);
+        if (in) out_cnt[slot] = c;
     }
 }
 
@@ -1458,41 +1043,26 @@ cudaError_t launch_tick(const BinArgs& b, const TickArgs& t, int max_slots, int*
         if (e != cudaSuccess) return e;
     }
     if (ev) cudaEventRecordWithFlags(ev[1], s2, evflags);
-    /* the fused layout runs the neighbour search inside the per-agent kernel
-       (not with a learned proposal, whose features need every list first) */
-    const bool fused = t.lp_mode == 2 && !kd && !t.feat;
     if (kd) {
         /* the reference's kd-tree: build and per-member query beside the
            attraction kernel, the cache composition after it */
         e = kd_build_and_query(*kd, s, sms);
         if (e != cudaSuccess) return e;
-    } else if (!fused) {
-        /* one resident wave of the persistent search */
-        /* two register budgets for k <= 16: 8 resident blocks per SM at
-           64 registers, or 6 at 80 (no spills); the autotuner picks */
-        int pn = 1;
-        if (t.k <= 8 && !t.knn_wide) {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pn, k_neighbors<8, 8>, 128, 0);
-            k_neighbors<8, 8><<<sms * (pn > 0 ? pn : 1), 128, 0, s>>>(t);
-        } else if (t.k <= 8) {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pn, k_neighbors<8, 6>, 128, 0);
-            k_neighbors<8, 6><<<sms * (pn > 0 ? pn : 1), 128, 0, s>>>(t);
-        } else if (t.k <= 16 && !t.knn_wide) {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pn, k_neighbors<16, 8>, 128, 0);
-            k_neighbors<16, 8><<<sms * (pn > 0 ? pn : 1), 128, 0, s>>>(t);
-        } else if (t.k <= 16) {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pn, k_neighbors<16, 6>, 128, 0);
-            k_neighbors<16, 6><<<sms * (pn > 0 ? pn : 1), 128, 0, s>>>(t);
-        } else {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pn, k_neighbors<32, 1>, 128, 0);
-            k_neighbors<32, 1><<<sms * (pn > 0 ? pn : 1), 128, 0, s>>>(t);
-        }
+    } else {
+        /* one resident wave of the persistent search at most */
+        auto go = [&](auto kern) {
+            int pn = 1;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pn, kern, 32 * kNbrWarps, 0);
+            kern<<<grid_for(max_slots, 32 * kNbrWarps, sms, std::max(1, std::min(pn, t.knn_blocks))), 32 * kNbrWarps, 0, s>>>(t);
+        };
+        if (t.k <= 8) go(k_neighbors<8>);
+        else if (t.k <= 16) go(k_neighbors<16>);
+        else go(k_neighbors<32>);
     }
-    if (ev && !kd && !fused) cudaEventRecordWithFlags(ev[2], s, evflags);
+    if (ev && !kd) cudaEventRecordWithFlags(ev[2], s, evflags);
     e = cudaEventRecord(ev_join, s2);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ev_join, 0);
     if (e != cudaSuccess) return e;
-    if (ev && fused) cudaEventRecordWithFlags(ev[2], s, evflags);
     if (kd) {
         e = kd_finish(*kd, s, sms);
         if (e != cudaSuccess) return e;
@@ -1517,16 +1087,6 @@ cudaError_t launch_tick(const BinArgs& b, const TickArgs& t, int max_slots, int*
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_agents_warp<32>, 256, 0);
             k_agents_warp<32><<<sms * (per_sm > 0 ? per_sm : 1), 256, 0, s>>>(t);
         }
-    } else if (fused) {
-        const int div = t.occ_div > 1 ? t.occ_div : 1;
-        const bool full = t.cls || t.cls_slot || t.label || t.rec_cnt;
-        auto go = [&](auto kern) {
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0);
-            kern<<<sms * (per_sm / div > 0 ? per_sm / div : 1), block, 0, s>>>(t);
-        };
-        if (t.k <= 8) full ? go(k_agents_knn<8, true>) : go(k_agents_knn<8, false>);
-        else if (t.k <= 16) full ? go(k_agents_knn<16, true>) : go(k_agents_knn<16, false>);
-        else full ? go(k_agents_knn<32, true>) : go(k_agents_knn<32, false>);
     } else {
         /* persistent grid: the resident blocks per SM, divided by occ_div
            (fewer resident warps leave each more L1 for its local arrays) */
@@ -1620,12 +1180,11 @@ cudaError_t launch_knn(const V2* pos, const unsigned char* active, int n, int k,
     e = scan(cell_count, cell_start, nb, scan_tmp, s);
     if (e != cudaSuccess) return e;
     k_scatter<<<gb, 256, 0, s>>>(b);
-    int ga = (n + 127) / 128;
-    if (ga < 1) ga = 1;
-    float r2 = r * r;
-    if (k <= 8) k_knn<8><<<ga, 128, 0, s>>>(s_pos, s_slot, cell_start, g, k, r, r2, counters, out_ids, out_cnt);
-    else if (k <= 16) k_knn<16><<<ga, 128, 0, s>>>(s_pos, s_slot, cell_start, g, k, r, r2, counters, out_ids, out_cnt);
-    else k_knn<32><<<ga, 128, 0, s>>>(s_pos, s_slot, cell_start, g, k, r, r2, counters, out_ids, out_cnt);
+    const int ga = (n + 32 * kNbrWarps - 1) / (32 * kNbrWarps);
+    const float r2 = r * r;
+    if (k <= 8) k_knn<8><<<ga, 32 * kNbrWarps, 0, s>>>(s_pos, s_slot, cell_start, g, k, r2, counters, out_ids, out_cnt);
+    else if (k <= 16) k_knn<16><<<ga, 32 * kNbrWarps, 0, s>>>(s_pos, s_slot, cell_start, g, k, r2, counters, out_ids, out_cnt);
+    else k_knn<32><<<ga, 32 * kNbrWarps, 0, s>>>(s_pos, s_slot, cell_start, g, k, r2, counters, out_ids, out_cnt);
     return cudaGetLastError();
 }
 

@@ -1,0 +1,362 @@
+/*
+ * knn_rows.cuh -- the exact kNN on the uniform agent grid: the k smallest
+ * (d2, slot) with EPS < d2 < r^2 (KNearestAgents, KDTree.cpp:85-202, as an
+ * exact query), one lane per agent, a warp at a time.
+ *
+ * The grid holds every agent: one outside the grid rectangle belongs to the
+ * nearest border cell, so the border cells stand for half-infinite strips
+ * and no agent needs a list of its own.
+ */
+#ifndef ECMG_KNN_ROWS_CUH
+#define ECMG_KNN_ROWS_CUH
+
+#include "ecmg_internal.h"
+
+namespace ecmg {
+
+/* cell index of a scaled coordinate, clamped to [0, n) (NaN: 0) */
+__device__ __forceinline__ int cell_clamp(float f, int n)
+{
+    f = fminf(fmaxf(f, 0.0f), (float)n);
+    return min((int)f, n - 1);
+}
+
+__device__ __forceinline__ int bucket_of(const AgentGrid& g, V2 p)
+{
+    return cell_clamp((p.y - g.y0) * g.inv, g.gh) * g.gw + cell_clamp((p.x - g.x0) * g.inv, g.gw);
+}
+
+/* ------------------------------------------------------------------------
+ * The search.  A lane scans the grid rows that its search disc meets, the
+ * nearest row first, from the disc's left to its right end: a row's cells are
+ * consecutive in grid order, so a row is one range of candidates.  The disc
+ * starts at the radius at which the local density (the 3 x 3 cells around the
+ * agent) promises about 1.8 (k + 2) agents, shrinks to the k-th distance once
+ * k are found, and grows (candidates below the old radius excluded) when it
+ * held fewer than k.
+ *
+ * Accepted candidates go to the lane's column of a shared-memory buffer; when
+ * a lane's buffer is full the whole warp sorts its buffers and merges them
+ * into the lanes' lists with min / max networks, so that the warp does not run
+ * a K-entry insertion for nearly every candidate because one of its lanes
+ * wants one.  Keys are d2 with its 6 low mantissa bits replaced by the entry
+ * of the lane's index column that holds the candidate's grid index: one float
+ * min / max pair per comparator, and the lists come out sorted by d2 except
+ * for keys within 2^-17 of each other ("near ties"), which are re-sorted by
+ * the exact (d2, slot); a near tie that may reach past the list (`rej` is the
+ * smallest key dropped) sends the lane to the 64-bit search.
+ * ---------------------------------------------------------------------- */
+constexpr unsigned kKnnCode = 63u; /* low key bits: entry of the index column */
+/* list capacity K: the k nearest in key[K-k .. K-1]; entries below hold 0.
+   Buffer entries: 8 merge into 16 at the cost per candidate of 16, with less
+   of the buffers empty (a flush takes the whole warp); for K = 32 the merge
+   weighs more.  Index column: the list's entries and the candidates since the
+   last renumbering. */
+template <int K>
+constexpr int kKnnBuf = K <= 16 ? 8 : 16;
+template <int K>
+constexpr int kKnnIdx = K <= 8 ? 32 : (K <= 16 ? 40 : 64);
+
+template <int K>
+struct KnnSm { /* of one warp */
+    float key[kKnnBuf<K>][32];
+    int idx[kKnnIdx<K>][32];
+    static_assert(kKnnIdx<K> <= (int)kKnnCode + 1, "index entries must fit the code");
+    static_assert(kKnnIdx<K> >= K + kKnnBuf<K>, "a renumbered list leaves room for a buffer");
+};
+
+__device__ __forceinline__ float knn_hi(float key) { return __uint_as_float(__float_as_uint(key) & ~kKnnCode); }
+
+/* Batcher's odd-even merge sort of N = 2^m floats, ascending */
+template <int N>
+__device__ __forceinline__ void sort_net(float (&v)[N])
+{
+#pragma unroll
+    for (int p = 1; p < N; p <<= 1)
+#pragma unroll
+        for (int q = p; q >= 1; q >>= 1)
+#pragma unroll
+            for (int j = q % p; j + q < N; j += 2 * q)
+#pragma unroll
+                for (int i = 0; i < q; i++)
+                    if (i + j + q < N && (i + j) / (2 * p) == (i + j + q) / (2 * p)) {
+                        const float a = v[i + j], b = v[i + j + q];
+                        v[i + j] = fminf(a, b);
+                        v[i + j + q] = fmaxf(a, b);
+                    }
+}
+
+/* sorts a bitonic sequence of N = 2^m floats, ascending */
+template <int N>
+__device__ __forceinline__ void bitonic_net(float (&v)[N])
+{
+#pragma unroll
+    for (int s = N / 2; s >= 1; s >>= 1)
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            if ((i & s) == 0) {
+                const float a = v[i], b = v[i + s];
+                v[i] = fminf(a, b);
+                v[i + s] = fmaxf(a, b);
+            }
+}
+
+/* the buffer's cnt entries into the list; *rej takes the smallest key dropped */
+template <int K>
+__device__ __forceinline__ void knn_flush(const KnnSm<K>& sm, int lane, int cnt, float (&key)[K], float* rej)
+{
+    constexpr int B = kKnnBuf<K>;
+    float b[B];
+#pragma unroll
+    for (int i = 0; i < B; i++) b[i] = i < cnt ? sm.key[i][lane] : INFINITY;
+    sort_net<B>(b);
+    float d = *rej;
+#pragma unroll
+    for (int i = 0; i < B; i++) {
+        const float o = key[K - B + i], n = b[B - 1 - i];
+        d = fminf(d, fmaxf(o, n));
+        key[K - B + i] = fminf(o, n);
+    }
+    *rej = d;
+    bitonic_net<K>(key);
+}
+
+/* dx*dx + dy*dy of KDTree.cpp:107-108 (np: the negated centre; adding it is
+   the subtraction), two components per instruction */
+__device__ __forceinline__ float dist2(V2 q, float2 np)
+{
+    const float2 d = __fadd2_rn(make_float2(q.x, q.y), np);
+    const float2 e = __fmul2_rn(d, d);
+    return e.x + e.y;
+}
+
+/* the list's indices move to the first K entries of the index column */
+template <int K>
+__device__ __forceinline__ int knn_renumber(KnnSm<K>& sm, int lane, int k, float (&key)[K])
+{
+    int id[K];
+#pragma unroll
+    for (int q = 0; q < K; q++) id[q] = sm.idx[__float_as_uint(key[q]) & kKnnCode][lane];
+#pragma unroll
+    for (int q = 0; q < K; q++)
+        if (q >= K - k && key[q] < INFINITY) {
+            sm.idx[q][lane] = id[q];
+            key[q] = __uint_as_float((__float_as_uint(key[q]) & ~kKnnCode) | (unsigned)q);
+        }
+    return K;
+}
+
+/* The k nearest of the agents at p (one per lane; `valid` false: none) into
+   the lanes' lists.  All 32 lanes must call.  Returns 1 when key[K-k .. K-1]
+   (INFINITY beyond the count) is the answer in order, 2 when it holds near
+   ties that must be re-sorted by the exact key, 0 when a near tie may reach
+   past the list.  cs: the scene's cell starts. */
+template <int K>
+__device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, float r2, const V2* s_pos,
+                                        const int* cs, const AgentGrid& g, float (&key)[K])
+{
+    constexpr int B = kKnnBuf<K>;
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < K; q++) key[q] = q < K - k ? 0.0f : INFINITY;
+    float rej = INFINITY;
+    float *const k0 = &sm.key[0][lane], *const kend = k0 + 32 * B;
+    float* kp = k0; /* next entry of the buffer column */
+    int ord = 0;    /* next entry of the index column */
+    valid = valid && p.x - p.x == 0.0f && p.y - p.y == 0.0f; /* no distance to a non-finite position is finite */
+    const float fy = (p.y - g.y0) * g.inv;
+    const int cx = cell_clamp((p.x - g.x0) * g.inv, g.gw), cy = cell_clamp(fy, g.gh);
+    /* distance to the nearer end of the own row (0 outside the grid) and the
+       side it lies on */
+    const float ry = p.y - (g.y0 + (float)cy * g.cell);
+    const int sy = ry + ry < g.cell ? -1 : 1;
+    const float edge = fmaxf(fminf(ry, g.cell - ry), 0.0f) - g.slack;
+    const float2 np = make_float2(-p.x, -p.y);
+    float lim = 0.0f, lo = kEps, disc = 0.0f, more_area = 3.0f;
+    if (valid) {
+        const int xa = max(cx - 1, 0), xb = min(cx + 1, g.gw - 1), ya = max(cy - 1, 0), yb = min(cy + 1, g.gh - 1);
+        int n9 = 0;
+        for (int y = ya; y <= yb; y++) n9 += cs[y * g.gw + xb + 1] - cs[y * g.gw + xa];
+        const float area = (float)((xb - xa + 1) * (yb - ya + 1)) * g.cell * g.cell;
+        /* pi disc n9 / area = 1.8 (k + 2) */
+        disc = fminf(r2, 0.573f * (float)(k + 2) * area / (float)max(n9, 1));
+        lim = disc;
+    }
+    while (true) {
+        const int far_row = max(cy, g.gh - 1 - cy);
+        for (int s = 0;; s++) {
+            const int m = (s + 1) >> 1;
+            const int y = cy + ((s & 1) ? sy * m : -sy * m);
+            /* every row from here on is at least this far */
+            const float at_least = (float)(m - 1) * g.cell + edge;
+            const bool more = s == 0 ? lim > 0.0f : (m <= far_row && !(at_least > 0.0f && at_least * at_least >= lim));
+            if (!__any_sync(kAll, more)) break;
+            int j = 0, left = 0;
+            if (more && y >= 0 && y < g.gh) {
+                float dy = 0.0f;
+                if (y > cy) dy = g.y0 + (float)y * g.cell - p.y;
+                else if (y < cy) dy = p.y - (g.y0 + (float)(y + 1) * g.cell);
+                dy = fmaxf(dy - g.slack, 0.0f);
+                const float w2 = lim - dy * dy;
+                if (w2 > 0.0f) {
+                    const float w = sqrtf(w2) * 1.000001f + g.slack;
+                    const int xa = cell_clamp((p.x - w - g.x0) * g.inv, g.gw);
+                    const int xb = cell_clamp((p.x + w - g.x0) * g.inv, g.gw);
+                    j = cs[y * g.gw + xa];
+                    left = cs[y * g.gw + xb + 1] - j;
+                }
+            }
+            const int longest = __reduce_max_sync(kAll, left);
+            /* the next candidate's position is loaded while this one is used */
+            V2 q = mk(0.0f, 0.0f);
+            if (left > 0) q = s_pos[j];
+            for (int it = 0; it < longest; it++) {
+                const float d2 = dist2(q, np);
+                if (it + 1 < left) q = s_pos[j + it + 1];
+                if (it < left && d2 > lo && d2 < lim) {
+                    *kp = __uint_as_float((__float_as_uint(d2) & ~kKnnCode) | (unsigned)ord);
+                    sm.idx[ord][lane] = j + it;
+                    kp += 32;
+                    ord++;
+                }
+                if (__any_sync(kAll, kp == kend)) {
+                    knn_flush<K>(sm, lane, (int)(kp - k0) >> 5, key, &rej);
+                    kp = k0;
+                    /* candidates beyond the k-th key (its code bits taken as
+                       ones) cannot enter any more; equal leading bits still
+                       count as near ties */
+                    if (key[K - 1] < INFINITY)
+                        lim = fminf(lim, __uint_as_float((__float_as_uint(key[K - 1]) | kKnnCode) + 1u));
+                    if (__any_sync(kAll, ord > kKnnIdx<K> - B)) ord = knn_renumber<K>(sm, lane, k, key);
+                }
+            }
+        }
+        if (__any_sync(kAll, kp != k0)) {
+            knn_flush<K>(sm, lane, (int)(kp - k0) >> 5, key, &rej);
+            kp = k0;
+        }
+        /* fewer than k inside the disc: a larger one, without what the last
+           one held (d2 >= disc is d2 > the float before it) */
+        const bool grow = valid && !(key[K - 1] < INFINITY) && disc < r2;
+        if (!__any_sync(kAll, grow)) break;
+        lim = 0.0f;
+        if (grow) {
+            lo = fmaxf(kEps, __uint_as_float(__float_as_uint(disc) - 1u));
+            disc = fminf(r2, more_area * disc);
+            more_area *= more_area;
+            lim = disc;
+        }
+        if (__any_sync(kAll, ord > kKnnIdx<K> - B)) ord = knn_renumber<K>(sm, lane, k, key);
+    }
+    bool tie = false;
+#pragma unroll
+    for (int q = 0; q + 1 < K; q++)
+        if (q >= K - k && key[q + 1] < INFINITY && knn_hi(key[q]) == knn_hi(key[q + 1])) tie = true;
+    if (key[K - 1] < INFINITY && knn_hi(rej) == knn_hi(key[K - 1])) return 0;
+    return tie ? 2 : 1;
+}
+
+/* near ties in the list (rare; out of line): the n indices in o[0 .. n)
+   re-sorted by the exact (d2, slot) key */
+__device__ __noinline__ void knn_resort(int n, V2 p, const V2* s_pos, const int* s_slot, int* o)
+{
+    for (int q = 1; q < n; q++) {
+        const int j = o[q];
+        const V2 c = s_pos[j];
+        float dx = c.x - p.x, dy = c.y - p.y;
+        const float d2 = dx * dx + dy * dy;
+        int r = q;
+        for (; r > 0; r--) {
+            const int i = o[r - 1];
+            const V2 b = s_pos[i];
+            dx = b.x - p.x;
+            dy = b.y - p.y;
+            const float e2 = dx * dx + dy * dy;
+            if (e2 < d2 || (e2 == d2 && s_slot[i] < s_slot[j])) break;
+            o[r] = i;
+        }
+        o[r] = j;
+    }
+}
+
+/* the search by 64-bit (d2, slot) keys (rare: a near tie at the k-th
+   distance that the list cannot settle; out of line): the rows of the disc of
+   squared radius `lim`, which holds at least k agents or is r^2; o[q] gets
+   the grid indices, the return value is the count */
+template <int K>
+__device__ __noinline__ int knn_exact(int k, V2 p, float lim, float r2, const V2* s_pos, const int* s_slot,
+                                      const int* cs, AgentGrid g, int* o)
+{
+    unsigned long long key[K];
+    int id[K];
+    for (int q = 0; q < k; q++) key[q] = ~0ull;
+    int n = 0;
+    const float w = sqrtf(lim) * 1.000001f + g.slack;
+    const int xa = cell_clamp((p.x - w - g.x0) * g.inv, g.gw), xb = cell_clamp((p.x + w - g.x0) * g.inv, g.gw);
+    const int ya = cell_clamp((p.y - w - g.y0) * g.inv, g.gh), yb = cell_clamp((p.y + w - g.y0) * g.inv, g.gh);
+    for (int y = ya; y <= yb; y++) {
+        for (int j = cs[y * g.gw + xa], e = cs[y * g.gw + xb + 1]; j < e; j++) {
+            const V2 c = s_pos[j];
+            const float dx = c.x - p.x, dy = c.y - p.y;
+            const float d2 = dx * dx + dy * dy;
+            if (!(d2 > kEps) || !(d2 < r2)) continue;
+            const unsigned long long kk = ((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)s_slot[j];
+            if (n == k && kk >= key[k - 1]) continue;
+            int q = n < k ? n++ : k - 1;
+            for (; q > 0 && key[q - 1] > kk; q--) {
+                key[q] = key[q - 1];
+                id[q] = id[q - 1];
+            }
+            key[q] = kk;
+            id[q] = j;
+        }
+    }
+    for (int q = 0; q < n; q++) o[q] = id[q];
+    return n;
+}
+
+/* the neighbour list of the agent at p: grid indices (SLOTS: slots) in
+   o[0 .. k), -1 beyond the count, which is returned.  All 32 lanes must call;
+   lanes with valid false write nothing. */
+template <int K, bool SLOTS>
+__device__ __forceinline__ int knn_list(KnnSm<K>& sm, bool valid, int k, V2 p, float r2, const V2* s_pos,
+                                        const int* s_slot, const int* cs, const AgentGrid& g, int* o)
+{
+    float key[K];
+    const int st = knn_rows<K>(sm, valid, k, p, r2, s_pos, cs, g, key);
+    if (!valid) return 0;
+    const int lane = threadIdx.x & 31;
+    int n = 0;
+    int id[K];
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+        const bool in = q >= K - k && key[q] < INFINITY;
+        id[q] = in ? sm.idx[__float_as_uint(key[q]) & kKnnCode][lane] : -1;
+        n += in ? 1 : 0;
+    }
+    if (SLOTS && st == 1) {
+#pragma unroll
+        for (int q = 0; q < K; q++)
+            if (id[q] >= 0) id[q] = s_slot[id[q]];
+    }
+    if (k == K && (reinterpret_cast<size_t>(o) & 15) == 0) {
+#pragma unroll
+        for (int q = 0; q < K; q += 4)
+            *reinterpret_cast<int4*>(o + q) = make_int4(id[q], id[q + 1], id[q + 2], id[q + 3]);
+    } else {
+#pragma unroll
+        for (int q = 0; q < K; q++)
+            if (q >= K - k) o[q - (K - k)] = id[q];
+    }
+    if (st == 2) knn_resort(n, p, s_pos, s_slot, o);
+    else if (st == 0)
+        n = knn_exact<K>(k, p, fminf(r2, __uint_as_float(__float_as_uint(key[K - 1]) | kKnnCode)), r2, s_pos, s_slot,
+                         cs, g, o);
+    if (SLOTS && st != 1)
+        for (int q = 0; q < n; q++) o[q] = s_slot[o[q]];
+    return n;
+}
+
+}  // namespace ecmg
+#endif
