@@ -137,10 +137,13 @@ struct ecmg_ctx {
        25,000 to a million agents (neighbour kernel 56 us at 0.25 against 70 at
        0.4 with 25,000 agents in 500 m, 324 against 330 at a million) */
     float cell_scale = 0.25f;
-    int lp_mode = 0; /* ECMG_LP_THREAD, ECMG_LP_WARP or ECMG_LP_THREAD_FUSED */
+    /* ECMG_LP_THREAD, ECMG_LP_WARP, ECMG_LP_THREAD_FUSED, or by the agent count */
+    static constexpr int kLpAuto = -1;
+    int lp_mode = kLpAuto;
+    int lanes_agents = 0; /* the agent count the automatic layout was chosen for */
     int occ_div = 1; /* per-thread layout: resident blocks per SM divided by this */
     int knn_wide = 0; /* neighbour kernel: 8 resident blocks per SM at most, or 6 */
-    int wgrab = 4;   /* agents per work grab in warp mode */
+    int wgrab = 4;   /* agents per warp in warp mode */
 
     /* host mirrors (Simulator bookkeeping, Simulator.h:164-171) */
     std::vector<unsigned char> active;
@@ -1841,6 +1844,34 @@ static ecmg_status ensure_grids(ecmg_ctx* c)
     return ECMG_OK;
 }
 
+/* lanes per agent of the per-agent kernel.  Sharing an agent among lanes
+   shortens its chain of half-planes and linear-program steps and costs
+   instructions: it wins while the agents leave the GPU waiting on that chain.
+   Measured (per-agent kernel, us; 1 / 4 / 8 / 16 / 32 lanes): 1,000 agents of
+   the box scene 42 / 23 / 20 / 19 / 18; 25,000 there 59 / 33 / 32 / 38 / 51;
+   crossing 30,000 93 / 45 / 45 / 50 / 64; 100,000 174 / 121 / 138 / 174 / 243;
+   300,000 249 / 264 / 322 / 434 / 672; 1,000,000 385 / 599 / ... -- so 4 lanes
+   up to 200,000 agents (8 where a handful of warps is all there is). */
+static int lanes_of(ecmg_ctx* c)
+{
+    if (c->lp_mode == ECMG_LP_WARP)
+        return c->wgrab >= 8 ? 4 : (c->wgrab >= 4 ? 8 : (c->wgrab >= 2 ? 16 : 32));
+    if (c->lp_mode != ecmg_ctx::kLpAuto) return 1;
+    return c->lanes_agents <= 8000 ? 8 : (c->lanes_agents <= 200000 ? 4 : 1);
+}
+
+/* the automatic layout follows the agent count; a count within a factor of
+   1.5 of the last choice's keeps it (a change re-captures the tick's graph) */
+static void choose_lanes(ecmg_ctx* c)
+{
+    if (c->lp_mode != ecmg_ctx::kLpAuto) return;
+    const long long n = c->num_agents, was = c->lanes_agents;
+    if (was > 0 && 2 * n <= 3 * was && 3 * n >= 2 * was) return;
+    const int before = lanes_of(c);
+    c->lanes_agents = (int)std::max<long long>(1, n);
+    if (lanes_of(c) != before) c->graph_dirty = true;
+}
+
 static void fill_args(ecmg_ctx* c, BinArgs& b, TickArgs& t, bool use_model)
 {
     b = BinArgs{};
@@ -1883,8 +1914,8 @@ static void fill_args(ecmg_ctx* c, BinArgs& b, TickArgs& t, bool use_model)
     t.slot_rank = c->rank.p;
     t.scenes = c->d_scenes.p;
     t.slot_scene = b.slot_scene;
-    t.tile = c->lp_mode == ECMG_LP_WARP ? c->wgrab : c->tile;
-    t.lp_mode = c->lp_mode;
+    t.tile = c->tile;
+    t.lanes = lanes_of(c);
     t.occ_div = c->occ_div;
     t.knn_blocks = c->knn_wide ? 6 : 8;
     const ecmg_params& p = c->prm;
@@ -2081,6 +2112,7 @@ static ecmg_status run_ticks(ecmg_ctx* c, int n_ticks, ecmg_tick_stats* stats)
         if (last < 0) continue;
         ecmg_status gs = ensure_grids(c);
         if (gs != ECMG_OK) return gs;
+        choose_lanes(c);
         std::memset(c->h_counters, 0, sizeof(int) * kCounters);
         c->h_counters[C_LAST] = last;
         const bool use_model = c->model && c->gate_left == 0;
@@ -2396,13 +2428,15 @@ ecmg_status ecmg_autotune(ecmg_ctx* c, int ticks_per_trial, ecmg_tune_result* ou
     const int divs[] = {1, 2, 3};
     const int wgrabs[] = {1, 2, 4, 8};
     const bool fixed_cell = c->prm.grid_cell > 0.0f;
+    const bool kdtree = c->nbr_mode == ECMG_NEIGHBORS_KDTREE;
+    const int base = kdtree ? ecmg_ctx::kLpAuto : ECMG_LP_THREAD;
     const int def_block = c->prm.block_size ? c->prm.block_size : 128;
     bool better = false;
     ecmg_status st = ECMG_OK;
     for (float sc : scales) {
         if (fixed_cell && sc != scales[0]) break;
         for (int kw = 0; kw < 2 && st == ECMG_OK; kw++)
-            st = trial(Launch{sc, 0, def_block, 32, 1, c->wgrab, kw}, &better);
+            st = trial(Launch{sc, base, def_block, 32, 1, c->wgrab, kw}, &better);
         if (st != ECMG_OK) break;
     }
     const float cell = bestL.scale;
@@ -2413,19 +2447,13 @@ ecmg_status ecmg_autotune(ecmg_ctx* c, int ticks_per_trial, ecmg_tune_result* ou
         for (int tl : tiles)
             for (int dv : divs) {
                 if (st != ECMG_OK) break;
-                st = trial(Launch{cell, 0, b, tl, dv, c->wgrab, kw}, &better);
+                st = trial(Launch{cell, base, b, tl, dv, c->wgrab, kw}, &better);
             }
     }
-    /* the per-thread layout fused with the neighbour search, at the best
-       per-thread launch (the kd-tree mode builds its lists separately) */
     const Launch thr = bestL;
-    for (int dv : divs) {
-        if (st != ECMG_OK || c->nbr_mode == ECMG_NEIGHBORS_KDTREE) break;
-        st = trial(Launch{cell, ECMG_LP_THREAD_FUSED, thr.block, thr.tile, dv, c->wgrab, kw}, &better);
-    }
     for (int w : wgrabs) {
-        if (st != ECMG_OK || c->nbr_mode == ECMG_NEIGHBORS_KDTREE) break; /* one thread per agent there */
-        st = trial(Launch{cell, 1, thr.block, thr.tile, 1, w, kw}, &better);
+        if (st != ECMG_OK || kdtree) break; /* the layout goes by the agent count there */
+        st = trial(Launch{cell, ECMG_LP_WARP, thr.block, thr.tile, 1, w, kw}, &better);
     }
     if (st != ECMG_OK) {
         c->replan_enabled = true;
@@ -2449,7 +2477,7 @@ ecmg_status ecmg_autotune(ecmg_ctx* c, int ticks_per_trial, ecmg_tune_result* ou
     if (out) {
         out->block_size = bb;
         out->agents_per_warp_grab = bmode == ECMG_LP_WARP ? bw : bt;
-        out->lp_mode = bmode;
+        out->lp_mode = bmode == ecmg_ctx::kLpAuto ? ECMG_LP_THREAD : bmode;
         out->grid_cell_scale = bs;
         out->best_tick_ms = best;
         out->trials = trials;
@@ -2491,7 +2519,7 @@ ecmg_status ecmg_set_neighbor_mode(ecmg_ctx* c, int mode)
         CK(K.keys.alloc(N)); CK(K.ktmp.alloc(N)); CK(K.flags.alloc(N));
         /* ORCA::m_NeighborCache starts as std::vector<Entity>(k): zeros */
         CK(cudaMemset(K.cache.p, 0, sizeof(int) * (size_t)k));
-        c->lp_mode = ECMG_LP_THREAD;
+        c->lp_mode = ecmg_ctx::kLpAuto;
     } else {
         c->kd.free_all();
     }
