@@ -97,8 +97,9 @@ struct SceneState {
     bool grid_ready = false;
     int grid_agents = 0;
     int bucket_base = 0;
-    DBuf<V2> d_ob_p, d_v_pos, d_he_left, d_he_right;
-    DBuf<int> d_ob_next, d_ob_prev, d_v_idx, d_he_target, d_ob_gstart, d_ob_gitems, d_ecm_gstart, d_ecm_gitems;
+    DBuf<V2> d_ob_p;
+    DBuf<EcmEdge> d_edges;
+    DBuf<int> d_ob_next, d_ob_prev, d_ob_gstart, d_ob_gitems, d_ecm_gstart, d_ecm_gitems;
     DBuf<unsigned char> d_ob_convex;
     DBuf<float> d_special_y;
     DBuf<int> d_sp_start, d_sp_items;
@@ -110,8 +111,8 @@ struct SceneState {
 
     void free_all()
     {
-        d_ob_p.free_(); d_v_pos.free_(); d_he_left.free_(); d_he_right.free_();
-        d_ob_next.free_(); d_ob_prev.free_(); d_v_idx.free_(); d_he_target.free_();
+        d_ob_p.free_(); d_edges.free_();
+        d_ob_next.free_(); d_ob_prev.free_();
         d_ob_gstart.free_(); d_ob_gitems.free_(); d_ecm_gstart.free_(); d_ecm_gitems.free_();
         d_ob_convex.free_(); d_special_y.free_(); d_sp_start.free_(); d_sp_items.free_(); d_sp_bloom.free_();
     }
@@ -599,9 +600,7 @@ ecmg_status ecmg_scene_set_ecm(ecmg_ctx* c, int scene, const ecmg_ecm* e)
     scene_bbox(*sc);
     build_ecm_grid(s);
     if (sc->has_obst) build_obst_grid(s, 0.0f, 4.0f, sc->vis_grid);
-    size_t nV = std::max<size_t>(1, V), nH = std::max<size_t>(1, 2 * (size_t)E);
-    CK(sc->d_v_pos.alloc(nV)); CK(sc->d_v_idx.alloc(nV)); CK(sc->d_he_target.alloc(nH));
-    CK(sc->d_he_left.alloc(nH)); CK(sc->d_he_right.alloc(nH));
+    CK(sc->d_edges.alloc(std::max<size_t>(1, (size_t)E)));
     CK(sc->d_ecm_gstart.alloc(s.ecm_grid.start.size()));
     CK(sc->d_ecm_gitems.alloc(std::max<size_t>(1, s.ecm_grid.items.size())));
     CK(sc->d_special_y.alloc(std::max<size_t>(1, s.special_y.size())));
@@ -614,15 +613,7 @@ ecmg_status ecmg_scene_set_ecm(ecmg_ctx* c, int scene, const ecmg_ecm* e)
     CK(sc->d_sp_bloom.alloc(std::max<size_t>(1, s.sp_bloom.size())));
     if (!s.sp_bloom.empty())
         CK(cudaMemcpy(sc->d_sp_bloom.p, s.sp_bloom.data(), sizeof(unsigned) * s.sp_bloom.size(), cudaMemcpyHostToDevice));
-    if (V) {
-        CK(cudaMemcpy(sc->d_v_pos.p, s.v_pos.data(), sizeof(V2) * V, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(sc->d_v_idx.p, s.v_idx.data(), sizeof(int) * V, cudaMemcpyHostToDevice));
-    }
-    if (E) {
-        CK(cudaMemcpy(sc->d_he_target.p, s.he_target.data(), sizeof(int) * 2 * E, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(sc->d_he_left.p, s.he_left.data(), sizeof(V2) * 2 * E, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(sc->d_he_right.p, s.he_right.data(), sizeof(V2) * 2 * E, cudaMemcpyHostToDevice));
-    }
+    if (E) CK(cudaMemcpy(sc->d_edges.p, s.edges.data(), sizeof(EcmEdge) * E, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(sc->d_ecm_gstart.p, s.ecm_grid.start.data(), sizeof(int) * s.ecm_grid.start.size(), cudaMemcpyHostToDevice));
     if (!s.ecm_grid.items.empty())
         CK(cudaMemcpy(sc->d_ecm_gitems.p, s.ecm_grid.items.data(), sizeof(int) * s.ecm_grid.items.size(), cudaMemcpyHostToDevice));
@@ -1804,11 +1795,7 @@ static ecmg_status ensure_grids(ecmg_ctx* c)
                 o.g_items = sc->d_ob_gitems.p;
             }
             EcmView& e = d.ecm;
-            e.v_pos = sc->d_v_pos.p;
-            e.v_idx = sc->d_v_idx.p;
-            e.he_target = sc->d_he_target.p;
-            e.he_left = sc->d_he_left.p;
-            e.he_right = sc->d_he_right.p;
+            e.edge = sc->d_edges.p;
             e.n_edges = (int)(s.he_target.size() / 2);
             e.gx0 = s.ecm_grid.x0; e.gy0 = s.ecm_grid.y0; e.ginv = s.ecm_grid.inv;
             e.gw = s.ecm_grid.gw; e.gh = s.ecm_grid.gh;
@@ -1824,6 +1811,7 @@ static ecmg_status ensure_grids(ecmg_ctx* c)
         CK(c->d_scenes.alloc(tab.size()));
         CK(cudaMemcpy(c->d_scenes.p, tab.data(), sizeof(SceneDev) * tab.size(), cudaMemcpyHostToDevice));
         CK(c->cell_count.alloc((size_t)base + 2));
+        CK(cudaMemsetAsync(c->cell_count.p, 0, sizeof(int) * ((size_t)base + 2), c->stream));
         CK(c->cell_start.alloc((size_t)base + 2));
         CK(c->scan_tmp.alloc((size_t)scan_tmp_ints(base)));
         c->table_dirty = false;
@@ -1882,6 +1870,7 @@ static void fill_args(ecmg_ctx* c, BinArgs& b, TickArgs& t, bool use_model)
     b.key = c->key.p;
     b.rank = c->rank.p;
     b.cell_count = c->cell_count.p;
+    b.block_sums = c->scan_tmp.p;
     b.s_slot = c->s_slot.p;
     b.s_pos = c->s_pos.p;
     b.s_vel = c->s_vel.p;
@@ -1908,6 +1897,8 @@ static void fill_args(ecmg_ctx* c, BinArgs& b, TickArgs& t, bool use_model)
     t.s_vel = c->s_vel.p;
     t.s_clear = c->s_clear.p;
     t.cell_start = c->cell_start.p;
+    t.cell_count = c->cell_count.p;
+    t.total_buckets = c->total_buckets;
     t.nbr = c->nbr.p;
     t.ncnt = c->ncnt.p;
     t.slot_bucket = c->key.p;
@@ -2049,7 +2040,7 @@ static cudaError_t enqueue_tick(ecmg_ctx* c, int launch_slots, bool use_model)
         kd.nbr = c->nbr.p;
         kd.ncnt = c->ncnt.p;
     }
-    e = launch_tick(b, t, launch_slots, c->scan_tmp.p, c->block, c->sms, c->stream, c->stream2, c->ev_fork,
+    e = launch_tick(b, t, launch_slots, c->block, c->sms, c->stream, c->stream2, c->ev_fork,
                     c->ev_join, c->ev_k,
                     use_model ? propose_cb : nullptr, &pc, after_attract_cb, c, c->nbr_mode == 1 ? &kd : nullptr);
     if (e != cudaSuccess) return e;
@@ -2061,11 +2052,11 @@ void* ecmg_stream(const ecmg_ctx* c) { return c ? (void*)c->stream : nullptr; }
 
 int ecmg_kernels_per_tick(const ecmg_ctx* c)
 {
-    /* k_bin, k_scan_local, k_scan_top, k_scan_add, k_scatter, k_attract,
-       k_neighbors, k_agents; k_features with a proposal model or a trace;
+    /* k_bin, k_scan, k_scatter, k_attract, k_neighbors, k_agents (or
+       k_agents_group); k_features with a proposal model or a trace;
        k_mlp_infer with a proposal model */
-    if (!c) return 8;
-    int n = 8 + ((c->model || c->trace) ? 1 : 0) + (c->model ? 1 : 0);
+    if (!c) return 6;
+    int n = 6 + ((c->model || c->trace) ? 1 : 0) + (c->model ? 1 : 0);
     /* kd-tree mode, instead of k_neighbors: members and slot-order list (6),
        four radix sorts of four passes (84), segment init (1), level 0 (11),
        levels 1.. (side + partition), the query (2) and the composition (4) */

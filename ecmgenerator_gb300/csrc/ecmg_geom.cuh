@@ -100,12 +100,19 @@ EG_HD V2 rotate(V2 v, float rad)
  * ECM (ECMGenerator/ECM.h), flattened.  Cell c: edge c>>1, left (even) or
  * right (odd) side (ECMCellCollection::Construct, ECMCellCollection.cpp:10-49).
  * ---------------------------------------------------------------------- */
+/* One ECM edge, gathered: a point-location test or a retraction is then two
+   dependent loads (cell list, record) instead of a chain through half-edge,
+   vertex index and vertex. */
+struct __align__(16) EcmEdge {
+    V2 p1, p2; /* positions of the targets of half-edges 1 and 0 */
+    V2 l0, r1; /* left boundary of half-edge 0, right of 1: with p1, p2 the quad of the even cell */
+    V2 r0, l1; /* right of 0, left of 1: the quad of the odd cell */
+    int to_p2; /* 0 when half-edge 0's target carries its own vertex index, else 1 (ECM.cpp:36) */
+    int pad[3];
+};
+
 struct EcmView {
-    const V2* v_pos;
-    const int* v_idx;
-    const int* he_target;
-    const V2* he_left;
-    const V2* he_right;
+    const EcmEdge* edge;
     int n_edges;
     /* point-location grid over the cell quads: cell g lists, in ascending
        order, every ECM cell whose bounding box (grown by a margin) meets g */
@@ -141,15 +148,12 @@ EG_HD unsigned sp_hash(float y)
    [v(he1.target), boundary.p0, boundary.p1, v(he0.target)] */
 EG_HD void cell_quad(const EcmView& e, int c, V2* q)
 {
-    int ed = c >> 1;
-    int h0 = 2 * ed, h1 = 2 * ed + 1;
-    V2 b0, b1;
-    if ((c & 1) == 0) { b0 = e.he_left[h0]; b1 = e.he_right[h1]; }
-    else { b0 = e.he_right[h0]; b1 = e.he_left[h1]; }
-    q[0] = e.v_pos[e.he_target[h1]];
-    q[1] = b0;
-    q[2] = b1;
-    q[3] = e.v_pos[e.he_target[h0]];
+    const EcmEdge& r = e.edge[c >> 1];
+    q[0] = r.p1;
+    q[3] = r.p2;
+    const V2* b = (c & 1) == 0 ? &r.l0 : &r.r0;
+    q[1] = b[0];
+    q[2] = b[1];
 }
 
 /* MathUtility::Contains(Point, vector<Segment>) (UtilityFunctions.cpp:54-86) */
@@ -210,12 +214,24 @@ EG_HD int point_location_inl(const EcmView& e, V2 p)
     float fx = (p.x - e.gx0) * e.ginv, fy = (p.y - e.gy0) * e.ginv;
     if (!(fx >= 0.0f && fy >= 0.0f && fx < (float)e.gw && fy < (float)e.gh)) return best;
     int g = (int)fy * e.gw + (int)fx;
-    int b = e.g_start[g], en = e.g_start[g + 1];
-    for (int i = b; i < en; i++) {
-        int c = e.g_items[i];
+    int i = e.g_start[g];
+    const int en = e.g_start[g + 1];
+    /* the next cell's number and quad are loaded while this one is tested */
+    int c = i < en ? e.g_items[i] : -1, cn = i + 1 < en ? e.g_items[i + 1] : -1;
+    if (c >= 0) cell_quad(e, c, q);
+    while (c >= 0) {
         if (best >= 0 && c >= best) break;
-        cell_quad(e, c, q);
+        V2 qn[4];
+        if (cn >= 0) cell_quad(e, cn, qn);
+        i++;
+        const int cnn = i + 1 < en ? e.g_items[i + 1] : -1;
         if (contains_quad(p, q)) return c;
+        c = cn;
+        cn = cnn;
+        if (c >= 0) {
+#pragma unroll
+            for (int s4 = 0; s4 < 4; s4++) q[s4] = qn[s4];
+        }
     }
     return best;
 }
@@ -249,20 +265,18 @@ EG_HD bool retract(const EcmView& e, V2 loc, V2* out, int* out_edge, int cell = 
     int c = cell == -2 ? point_location(e, loc) : cell;
     if (c < 0) return false;
     int ed = c >> 1;
-    int ip1 = e.he_target[2 * ed + 1], ip2 = e.he_target[2 * ed];
-    V2 p1 = e.v_pos[ip1], p2 = e.v_pos[ip2];
-    int toP2 = e.he_target[2 * ed] == e.v_idx[ip2] ? 0 : 1;
-    int toP1 = (toP2 + 1) % 2;
+    const EcmEdge r = e.edge[ed];
+    V2 p1 = r.p1, p2 = r.p2;
     V2 o1, o2, rd;
     bool isLeft = (p2.x - p1.x) * (loc.y - p1.y) - (p2.y - p1.y) * (loc.x - p1.x) > 0; /* IsLeftOfSegment */
     if (isLeft) {
-        o1 = e.he_left[2 * ed + toP2];
-        o2 = e.he_right[2 * ed + toP1];
+        o1 = r.to_p2 == 0 ? r.l0 : r.l1;
+        o2 = r.to_p2 == 0 ? r.r1 : r.r0;
         if (approx(o1, o2)) rd = (p1 - o1) + (p2 - o1);
         else { V2 v = o2 - o1; rd = mk(v.y, -v.x); }
     } else {
-        o1 = e.he_right[2 * ed + toP2];
-        o2 = e.he_left[2 * ed + toP1];
+        o1 = r.to_p2 == 0 ? r.r0 : r.r1;
+        o2 = r.to_p2 == 0 ? r.l1 : r.l0;
         if (approx(o1, o2)) rd = (p1 - o1) + (p2 - o1);
         else { V2 v = o2 - o1; rd = mk(-v.y, v.x); }
     }
@@ -284,15 +298,18 @@ EG_NI bool irm(const EcmView& e, V2 pos, const V2* path, int n, V2* out, bool* n
         return false;
     }
     if (edge) *edge = ed;
-    V2 co = closest_on_segment(r, e.he_left[2 * ed], e.he_right[2 * ed + 1]);
+    V2 co = closest_on_segment(r, e.edge[ed].l0, e.edge[ed].r1);
     float clr = len(r - co);
     float rcs = clr * clr;
     V2 goal = path[n - 1];
     if (len2(goal - r) < rcs) { *out = goal; return true; }
     bool success = false;
+    /* a point is loaded once, ahead of its segment */
+    V2 p2 = path[0] - r, ahead = n > 1 ? path[1] : path[0];
     for (int i = 0; i < n - 1; i++) {
-        V2 p1 = path[i] - r;
-        V2 p2 = path[i + 1] - r;
+        const V2 p1 = p2;
+        p2 = ahead - r;
+        if (i + 2 < n) ahead = path[i + 2];
         V2 ed2 = p2 - p1;
         float els = len2(ed2);
         float dd = det(p1, p2);

@@ -49,6 +49,7 @@ enum {
     C_ACCEPTED = 9,    /* proposals that passed the exact check */
     C_REPLAN_DEV = 10, /* re-plans that fail at the start retraction (not listed) */
     C_NBR_WORK = 11,   /* work counter of the persistent neighbour kernel */
+    C_SCANNED = 12,    /* blocks of the bucket scan that are done */
     kCounters = 16
 };
 
@@ -102,6 +103,8 @@ struct TickArgs {
     const V2* s_vel;
     const float* s_clear;
     const int* cell_start; /* total buckets + 1 */
+    int* cell_count;       /* bucket counts, cleared by k_attract for the next tick */
+    int total_buckets;
     int* nbr;              /* [n * k] neighbours of grid-order agent t, as grid-order indices */
     int* ncnt;             /* [n] neighbour count */
     const int* slot_bucket; /* slot -> bucket of this tick's binning */
@@ -145,17 +148,18 @@ struct BinArgs {
     const unsigned char* active;
     int* key;        /* slot -> bucket */
     int* rank;       /* slot -> rank inside the bucket */
-    int* cell_count; /* ncells + 1 buckets (+1 sentinel) */
+    int* cell_count; /* total_buckets counts, zero before the binning, scanned in place by it */
+    int* block_sums; /* scan_tmp_ints(total_buckets) */
     int* s_slot;
     V2* s_pos;
     V2* s_vel;
     float* s_clear;
-    const int* cell_start;
+    int* cell_start; /* total_buckets + 1 */
     int* counters;
     AgentGrid grid;           /* used when scenes is null */
     const SceneDev* scenes;   /* batch: per-scene grid and bucket base */
     const int* slot_scene;
-    int total_buckets;        /* sum over scenes of (cells + overflow) */
+    int total_buckets;        /* sum over scenes of their cells */
     int n_fixed;              /* > 0: bin slots [0, n_fixed) (stand-alone kNN); 0: [0, counters[C_LAST]] */
 };
 
@@ -172,7 +176,7 @@ typedef cudaError_t (*HookFn)(void* user, cudaStream_t s, unsigned evflags);
    the proposal (features + inference) and after the per-agent kernel. */
 struct KdArgs;
 /* kd (may be null): the kd-tree neighbour mode replaces the neighbour kernel */
-cudaError_t launch_tick(const BinArgs& b, const TickArgs& t, int max_slots, int* scan_tmp, int block, int sms,
+cudaError_t launch_tick(const BinArgs& b, const TickArgs& t, int max_slots, int block, int sms,
                         cudaStream_t s, cudaStream_t s2, cudaEvent_t ev_fork, cudaEvent_t ev_join,
                         const cudaEvent_t* ev, ProposeFn propose, void* propose_user,
                         HookFn after_attract, void* after_attract_user, const KdArgs* kd);

@@ -16,11 +16,7 @@ namespace ecmg {
 EcmView HostScene::ecm_view() const
 {
     EcmView e{};
-    e.v_pos = v_pos.data();
-    e.v_idx = v_idx.data();
-    e.he_target = he_target.data();
-    e.he_left = he_left.data();
-    e.he_right = he_right.data();
+    e.edge = edges.data();
     e.n_edges = (int)(he_target.size() / 2);
     e.gx0 = ecm_grid.x0;
     e.gy0 = ecm_grid.y0;
@@ -164,6 +160,18 @@ void build_ecm_grid(HostScene& s)
     build_landmarks(s);
     int E = (int)(s.he_target.size() / 2);
     int C = 2 * E;
+    s.edges.assign((size_t)E, EcmEdge{});
+    for (int ed = 0; ed < E; ed++) {
+        const int h0 = 2 * ed, h1 = 2 * ed + 1, t0 = s.he_target[h0];
+        EcmEdge& r = s.edges[ed];
+        r.p1 = s.v_pos[s.he_target[h1]];
+        r.p2 = s.v_pos[t0];
+        r.l0 = s.he_left[h0];
+        r.r0 = s.he_right[h0];
+        r.l1 = s.he_left[h1];
+        r.r1 = s.he_right[h1];
+        r.to_p2 = t0 == s.v_idx[t0] ? 0 : 1;
+    }
     EcmView ev = s.ecm_view();
     std::vector<V2> q(4 * (size_t)C);
     float x0 = std::numeric_limits<float>::max(), y0 = x0, x1 = -x0, y1 = -x0;

@@ -29,6 +29,7 @@ struct HostScene {
     std::vector<float> v_clear;
     std::vector<int> v_idx, v_halfedge, he_target, he_next;
     std::vector<V2> he_left, he_right;
+    std::vector<EcmEdge> edges; /* the device's and the planner's view of the edges (build_ecm_grid) */
     GridCSR ecm_grid;
     std::vector<float> special_y;
     std::vector<int> sp_start, sp_items; /* quads with a corner at special_y[s] */
