@@ -682,6 +682,26 @@ static int grid_for(int n, int block, int sms, int per_sm)
     return g < 1 ? 1 : (g > cap ? cap : g);
 }
 
+/* a launch with a given split of an SM's memory between L1 and shared memory
+   (per cent of shared memory).  Two kernels are resident on an SM together
+   only under one split: with the defaults -- the attraction kernel uses no
+   shared memory -- the search beside it waited for it to end on every SM that
+   it had reached (25,000 agents: 45 us from their common start, now 23). */
+template <class Kern>
+static cudaError_t launch_split(Kern kern, int blocks, int threads, int split, cudaStream_t s, const TickArgs& t)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at.val.sharedMemCarveout = split;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, t);
+}
+
 cudaError_t launch_tick(const BinArgs& b, const TickArgs& t, int max_slots, int block, int sms,
                         cudaStream_t s, cudaStream_t s2, cudaEvent_t ev_fork, cudaEvent_t ev_join,
                         const cudaEvent_t* ev, ProposeFn propose, void* propose_user,
@@ -704,10 +724,15 @@ cudaError_t launch_tick(const BinArgs& b, const TickArgs& t, int max_slots, int 
     e = cudaEventRecord(ev_fork, s);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s2, ev_fork, 0);
     if (e != cudaSuccess) return e;
+    /* one split for both: enough shared memory for the search's blocks that an
+       SM gets, the rest L1 for both (tick at 100,000 agents 218 us at 50 %, 220
+       at 75, 221 at 30; at a million 802, 791 and 831) */
+    const int split = max_slots <= sms * 2048 ? 50 : 75;
     int ao = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ao, k_attract, 128, 0);
     const int ga = ao > 0 && gk > sms * ao ? sms * ao : gk; /* one wave, grid-stride */
-    k_attract<<<ga, 128, 0, s2>>>(t);
+    e = launch_split(k_attract, ga, 128, split, s2, t);
+    if (e != cudaSuccess) return e;
     if (ev) cudaEventRecordWithFlags(ev[1], s2, evflags);
     /* the per-agent kernel waits for the attraction kernel, not for the
        copies of its lists behind it (joined at the end) */
@@ -727,11 +752,13 @@ cudaError_t launch_tick(const BinArgs& b, const TickArgs& t, int max_slots, int 
         auto go = [&](auto kern) {
             int pn = 1;
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pn, kern, 32 * kNbrWarps, 0);
-            kern<<<grid_for(max_slots, 32 * kNbrWarps, sms, std::max(1, std::min(pn, t.knn_blocks))), 32 * kNbrWarps, 0, s>>>(t);
+            e = launch_split(kern, grid_for(max_slots, 32 * kNbrWarps, sms, std::max(1, std::min(pn, t.knn_blocks))),
+                             32 * kNbrWarps, split, s, t);
         };
         if (t.k <= 8) go(k_neighbors<8>);
         else if (t.k <= 16) go(k_neighbors<16>);
         else go(k_neighbors<32>);
+        if (e != cudaSuccess) return e;
     }
     if (ev && !kd) cudaEventRecordWithFlags(ev[2], s, evflags);
     e = cudaStreamWaitEvent(s, ev_join, 0);

@@ -258,26 +258,33 @@ __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, f
 }
 
 /* near ties in the list (rare; out of line): the n indices in o[0 .. n)
-   re-sorted by the exact (d2, slot) key */
+   re-sorted by the exact (d2, slot) key.  The keys are gathered first, side by
+   side: a lone lane here is what the last warp waits for. */
+template <int K>
 __device__ __noinline__ void knn_resort(int n, V2 p, const V2* s_pos, const int* s_slot, int* o)
 {
-    for (int q = 1; q < n; q++) {
-        const int j = o[q];
+    unsigned long long key[K];
+    int id[K];
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+        const int j = q < n ? o[q] : o[0];
         const V2 c = s_pos[j];
-        float dx = c.x - p.x, dy = c.y - p.y;
-        const float d2 = dx * dx + dy * dy;
-        int r = q;
-        for (; r > 0; r--) {
-            const int i = o[r - 1];
-            const V2 b = s_pos[i];
-            dx = b.x - p.x;
-            dy = b.y - p.y;
-            const float e2 = dx * dx + dy * dy;
-            if (e2 < d2 || (e2 == d2 && s_slot[i] < s_slot[j])) break;
-            o[r] = i;
-        }
-        o[r] = j;
+        const float dx = c.x - p.x, dy = c.y - p.y;
+        key[q] = ((unsigned long long)__float_as_uint(dx * dx + dy * dy) << 32) | (unsigned)s_slot[j];
+        id[q] = j;
     }
+    for (int q = 1; q < n; q++) {
+        const unsigned long long kk = key[q];
+        const int j = id[q];
+        int r = q;
+        for (; r > 0 && key[r - 1] > kk; r--) {
+            key[r] = key[r - 1];
+            id[r] = id[r - 1];
+        }
+        key[r] = kk;
+        id[r] = j;
+    }
+    for (int q = 0; q < n; q++) o[q] = id[q];
 }
 
 /* the search by 64-bit (d2, slot) keys (rare: a near tie at the k-th
@@ -349,7 +356,7 @@ __device__ __forceinline__ int knn_list(KnnSm<K>& sm, bool valid, int k, V2 p, f
         for (int q = 0; q < K; q++)
             if (q >= K - k) o[q - (K - k)] = id[q];
     }
-    if (st == 2) knn_resort(n, p, s_pos, s_slot, o);
+    if (st == 2) knn_resort<K>(n, p, s_pos, s_slot, o);
     else if (st == 0)
         n = knn_exact<K>(k, p, fminf(r2, __uint_as_float(__float_as_uint(key[K - 1]) | kKnnCode)), r2, s_pos, s_slot,
                          cs, g, o);
