@@ -15,9 +15,9 @@
  * Inference: BF16 weights and activations on the 5th-generation tensor
  * cores (tcgen05.mma, FP32 accumulators in tensor memory), weights staged
  * once per CTA in shared memory in the MMA operand layout.  Training: FP32
- * master weights; every forward and backward GEMM on the tensor cores with
- * BF16 operands and FP32 accumulation (k_tc_gemm), the elementwise steps,
- * softmax cross-entropy and Adam in FP32.
+ * master weights; forward and backward pass of a row tile in one kernel, every
+ * contraction on the tensor cores with BF16 operands and FP32 accumulation
+ * (k_train), the elementwise steps, softmax cross-entropy and Adam in FP32.
  * This translation unit is not part of the parity-critical arithmetic.
  */
 #include "../../include/ecmg.h"
@@ -28,6 +28,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -38,19 +39,22 @@ using namespace ecmg;
 namespace {
 
 constexpr int IN = kMlpIn, HID = kMlpHid, OUT = kMlpOut;
-__device__ __forceinline__ float gelu(float x)
+/* GELU (tanh form) and its derivative of two values, in FP32 from one
+   accurate tanh each; products and sums two at a time, separately rounded:
+     y = x/2 (1 + th), th = tanh(k0 (x + k1 x^3)),
+     dy = (1 + th)/2 + x/2 (1 - th^2) k0 (1 + 3 k1 x^2) */
+__device__ __forceinline__ void gelu_both(float2 x, float2* y, float2* dy)
 {
     const float k0 = 0.7978845608028654f, k1 = 0.044715f; /* sqrt(2/pi), tanh approximation */
-    return 0.5f * x * (1.0f + tanhf(k0 * (x + k1 * x * x * x)));
-}
-
-__device__ __forceinline__ float gelu_grad(float x)
-{
-    const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-    float u = k0 * (x + k1 * x * x * x);
-    float th = tanhf(u);
-    float du = k0 * (1.0f + 3.0f * k1 * x * x);
-    return 0.5f * (1.0f + th) + 0.5f * x * (1.0f - th * th) * du;
+    auto c2 = [](float c) { return make_float2(c, c); };
+    const float2 x3 = __fmul2_rn(__fmul2_rn(__fmul2_rn(c2(k1), x), x), x);
+    const float2 u = __fmul2_rn(c2(k0), __fadd2_rn(x, x3));
+    const float2 th = make_float2(tanhf(u.x), tanhf(u.y));
+    const float2 hx = __fmul2_rn(c2(0.5f), x), t1 = __fadd2_rn(c2(1.0f), th);
+    *y = __fmul2_rn(hx, t1);
+    const float2 du = __fmul2_rn(c2(k0), __fadd2_rn(c2(1.0f), __fmul2_rn(__fmul2_rn(c2(3.0f * k1), x), x)));
+    const float2 sech2 = __fadd2_rn(c2(1.0f), __fmul2_rn(make_float2(-th.x, -th.y), th));
+    *dy = __fadd2_rn(__fmul2_rn(c2(0.5f), t1), __fmul2_rn(__fmul2_rn(hx, sech2), du));
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
@@ -455,302 +459,491 @@ __global__ void __launch_bounds__(kInferThreads, 1)
 }
 
 /* ------------------------------------------------------------------------
- * Training GEMMs on the tensor cores.  C[M x N] = A[M x K] * B[N x K]^T with
- * A and B BF16 row-major (K contiguous) in global memory, read by TMA in
- * stages of 64 K columns (8 boxes of 8 columns x 128 rows for A, 8 boxes of
- * 8 columns x N rows for B) into the canonical K-major layout, three stages
- * in flight; one thread issues the tcgen05.mma chain (M = 128, N <= 256,
- * K-steps of 16) into an FP32 accumulator in tensor memory; each warp reads
- * its 32 rows back for the epilogue: a plain FP32 store, or an atomic add
- * when the K range is split over CTAs (weight gradients, where K is the
- * batch).  Rows or columns beyond the tensors read as zeros.  Bounded waits
- * as in the inference kernel.
+ * Training: one kernel for the forward and backward pass of a minibatch, one
+ * that sums the gradients and takes the Adam step.
+ *
+ * k_train.  One CTA of sixteen warps per SM, persistent over tiles of 128
+ * rows; a tile's activations never leave the SM.  The weights (BF16, 96 KB)
+ * stay in shared memory as the B operands of the forward chains (K-major) and,
+ * read along the other axis (MN-major), of the backward ones; likewise an
+ * activation tile is the K-major A operand of the next layer and the MN-major
+ * operand of its weight gradient, so that nothing is transposed or stored
+ * twice.  Per tile, each chain issued by one thread and awaited by all:
+ *   Z1 = X W1, Z2 = A1 W2, Z3 = A2 W3 (outputs 0..127, then 128..159)
+ *   dW3 += A2^T dZ3, dA2 = dZ3 W3^T
+ *   dW2 += A1^T dZ2, dA1 = dZ2 W2^T
+ *   dW1^T += dZ1^T X
+ * with FP32 accumulators: tensor-memory columns 0..127 for the Z's and dA's,
+ * 128..511 for the three weight gradients, which stay there over all tiles of
+ * the CTA.  Between the chains a thread owns 32 columns of one row in
+ * registers: bias, GELU and its derivative (from one tanh; the derivative is
+ * kept in FP32 for the backward pass), softmax cross-entropy, and the FP32
+ * bias gradients, summed over a warp's rows by a transposing butterfly and
+ * over tiles in registers.  dZ2 overwrites A2, dZ1 overwrites A1.  A CTA
+ * writes its sums as one partial gradient.
+ *
+ * What bounds it: the elementwise work between the chains (accurate tanh, exp
+ * and divisions of 416 activations per row), about 80 % of its time; the
+ * chains take 2.3 us of a tile.  A step of 65,536 rows took 722 us as 24
+ * launches that passed every activation, its transpose and its BF16 copy
+ * through memory, with a two-block column sum for each bias gradient.
  * ---------------------------------------------------------------------- */
-constexpr int kGemmStages = 3;
-constexpr int kGemmKC = 64;                         /* K columns per stage */
-constexpr int kGemmAB = kTile * kGemmKC * 2;        /* A bytes per stage (16 KB) */
-constexpr int kGemmBB = 256 * kGemmKC * 2;          /* B bytes per stage, N <= 256 (32 KB) */
-constexpr int kGemmStageB = kGemmAB + kGemmBB;
-constexpr size_t kGemmSmem = (size_t)kGemmStages * kGemmStageB + 8 * (2 * kGemmStages + 1) + 16;
+constexpr int OW1 = 0, OB1 = OW1 + IN * HID, OW2 = OB1 + HID, OB2 = OW2 + HID * HID, OW3 = OB2 + HID,
+              OB3 = OW3 + HID * OUT, NPARAM = OB3 + OUT; /* W1 [IN x HID], b1, W2 [HID x HID], b2, W3 [HID x OUT], b3 */
+constexpr int kTrThreads = 512, kTrCols = 512; /* tensor memory: all of it */
+constexpr int kTrW3 = 128, kTrW2 = kTrW3 + OUT, kTrW1 = kTrW2 + HID; /* first columns of dW3, dW2, dW1^T */
+static_assert(kTrW1 + IN == kTrCols, "the weight gradients fill the tensor memory");
+constexpr int kZB = kTile * OUT * 2;
+constexpr size_t kTrainSmem = (size_t)kWB + kXB + 2 * kHB + kZB + sizeof(float) * (2 * HID + OUT) + 64;
+static_assert(kTrainSmem <= 232448, "shared memory of one CTA");
+static_assert(4 * 3 * kTile * 4 <= kZB, "the softmax's exchange fits the dZ3 tile before it is written");
 
-__device__ __forceinline__ void tma_box(const CUtensorMap* tm, uint32_t sdst, int x, int y, uint32_t mbar)
+/* instruction descriptor with the major axes of A and B (1: MN-major) */
+__host__ __device__ constexpr uint32_t tc_idesc_mn(int N, int amn, int bmn)
 {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
-            "r"(sdst), "l"(tm), "r"(x), "r"(y), "r"(mbar)
-        : "memory");
+    return tc_idesc(kTile, N) | ((uint32_t)amn << 15) | ((uint32_t)bmn << 16);
 }
 
-__global__ void __launch_bounds__(128, 1)
-    k_tc_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N, int K,
-              int kper, float* C, int ldc, int atomic, int* err, int spin)
+/* D[tmem] (+)= A B over `steps` K-steps of 16, one thread.  K-major operand of
+   R rows: chunks (8 columns) R x 16 bytes apart, a K-step is two chunks.
+   MN-major (the same storage read along the other axis): the 8-column groups
+   of the M or N axis are R x 16 bytes apart, the 8-row groups of the K axis
+   128 bytes, a K-step is two of those. */
+__device__ __forceinline__ void tc_chain(uint32_t tmem, uint32_t a, int ra, int amn, uint32_t b, int rb, int bmn,
+                                         int n, int steps, bool add)
+{
+    const uint32_t id = tc_idesc_mn(n, amn, bmn);
+    const uint32_t sa = amn ? 256u : 32u * (uint32_t)ra, sb = bmn ? 256u : 32u * (uint32_t)rb;
+    const uint64_t da = amn ? tc_sdesc(a, 128, 16u * ra) : tc_sdesc(a, 16u * ra, 128);
+    const uint64_t db = bmn ? tc_sdesc(b, 128, 16u * rb) : tc_sdesc(b, 16u * rb, 128);
+    for (int ks = 0; ks < steps; ks++) {
+        const uint32_t acc = add || ks > 0 ? 1u : 0u;
+        asm volatile(
+            "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+            "l"(da + (uint64_t)(ks * (sa >> 4))), "l"(db + (uint64_t)(ks * (sb >> 4))), "r"(id), "r"(acc));
+    }
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
+{
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+                 :
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
+}
+
+/* sum of v[c] over the warp's lanes, for column c in lane c: at each step a
+   lane keeps the half of the columns that its number points to */
+__device__ __forceinline__ float warp_colsum(float (&v)[32])
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; i++) {
+            const float keep = up ? v[i + o] : v[i], give = up ? v[i] : v[i + o];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    return v[0];
+}
+
+/* the row of X that row r of the minibatch is: r itself, or drawn by a hash
+   of the step's seed (splitmix64) */
+__device__ __forceinline__ int train_row(int r, int n, unsigned long long seed, int draw)
+{
+    if (!draw) return r;
+    unsigned long long z = seed + 0x9E3779B97F4A7C15ull * (unsigned long long)(r + 1);
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    z ^= z >> 31;
+    return (int)(z % (unsigned long long)n);
+}
+
+__global__ void __launch_bounds__(kTrThreads, 1)
+    k_train(const __nv_bfloat16* X, const unsigned char* y, int n, int B, unsigned long long seed, int draw,
+            const unsigned char* wpack, const float* P, float* part, float* part_loss, int* part_ok, int* err, int spin)
 {
     extern __shared__ __align__(128) unsigned char sm[];
-    __shared__ uint32_t s_tmem;
-    __shared__ int s_fail;
+    unsigned char *sW1 = sm, *sW2 = sW1 + kW1B, *sW3 = sW2 + kW2B;
+    unsigned char *sX = sW3 + kW3B, *sA1 = sX + kXB, *sA2 = sA1 + kHB, *sZ = sA2 + kHB;
+    float* sb = reinterpret_cast<float*>(sZ + kZB); /* biases; at the end the bias gradients */
+    uint64_t* s_mbar = reinterpret_cast<uint64_t*>(sb + 2 * HID + OUT);
+    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_mbar + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * kTile;
-    const int k0 = blockIdx.y * kper, k1 = min(K, k0 + kper);
-    const int nch = k1 > k0 ? (k1 - k0 + kGemmKC - 1) / kGemmKC : 0;
-    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
-    const uint32_t bar0 = sbase + (uint32_t)(kGemmStages * kGemmStageB);
-    auto full = [&](int st) { return bar0 + 8u * (uint32_t)st; };
-    auto empty = [&](int st) { return bar0 + 8u * (uint32_t)(kGemmStages + st); };
-    const uint32_t done = bar0 + 8u * (uint32_t)(2 * kGemmStages);
+    const int quad = warp & 3, cg = warp >> 2; /* tensor-memory lane quarter, column group */
+    const int row = quad * 32 + lane, c0 = cg * 32;
+
+    for (int i = tid; i < kWB / 16; i += kTrThreads)
+        reinterpret_cast<uint4*>(sm)[i] = reinterpret_cast<const uint4*>(wpack)[i];
+    for (int i = tid; i < 2 * HID + OUT; i += kTrThreads)
+        sb[i] = i < HID ? P[OB1 + i] : (i < 2 * HID ? P[OB2 + i - HID] : P[OB3 + i - 2 * HID]);
+    const uint32_t mb = (uint32_t)__cvta_generic_to_shared(s_mbar);
     if (tid == 0) {
-        for (int b = 0; b < 2 * kGemmStages + 1; b++)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8u * b) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        s_fail = 0;
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         (uint32_t)__cvta_generic_to_shared(&s_tmem)),
-                     "r"(256)
+                         (uint32_t)__cvta_generic_to_shared(s_tmem)),
+                     "r"(kTrCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem;
-    if (tid == 0 && nch > 0) {
-        uint32_t fph[kGemmStages] = {}, eph[kGemmStages] = {};
-        bool xpend[kGemmStages] = {};
-        const uint32_t bytes = (uint32_t)(kGemmAB + N * kGemmKC * 2);
-        const uint32_t id = tc_idesc(kTile, N);
-        auto load = [&](int c) {
-            const int st = c % kGemmStages;
-            const uint32_t a = sbase + (uint32_t)(st * kGemmStageB), b = a + (uint32_t)kGemmAB;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full(st)), "r"(bytes)
-                         : "memory");
-#pragma unroll 1
-            for (int kc = 0; kc < kGemmKC / 8; kc++) {
-                const int x = k0 + c * kGemmKC + kc * 8;
-                tma_box(&tmA, a + (uint32_t)(kc * kTile * 16), x, m0, full(st));
-                tma_box(&tmB, b + (uint32_t)(kc * N * 16), x, 0, full(st));
-            }
-            xpend[st] = true;
-        };
-        for (int c = 0; c < nch && c < kGemmStages; c++) load(c);
-        bool fail = false;
-        for (int c = 0; c < nch && !fail; c++) {
-            const int st = c % kGemmStages;
-            if (!mbar_wait(full(st), fph[st], spin)) { fail = true; break; }
-            fph[st] ^= 1u;
-            xpend[st] = false;
-            tc_fence_after();
-            const uint32_t a = sbase + (uint32_t)(st * kGemmStageB), b = a + (uint32_t)kGemmAB;
-#pragma unroll
-            for (int ks = 0; ks < kGemmKC / 16; ks++) {
-                const uint64_t ad = tc_sdesc(a + (uint32_t)(ks * 2 * kTile * 16), kTile * 16, 128);
-                const uint64_t bd = tc_sdesc(b + (uint32_t)(ks * 2 * N * 16), (uint32_t)N * 16, 128);
-                const uint32_t acc = (c > 0 || ks > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-                    "l"(ad), "l"(bd), "r"(id), "r"(acc));
-            }
-            tc_commit(empty(st));
-            /* refill the previous stage once its MMAs have read it */
-            const int pc = c - 1;
-            if (pc >= 0 && pc + kGemmStages < nch) {
-                const int ps = pc % kGemmStages;
-                if (!mbar_wait(empty(ps), eph[ps], spin)) { fail = true; break; }
-                eph[ps] ^= 1u;
-                load(pc + kGemmStages);
-            }
-        }
-        /* every MMA issued so far completes on `done` (also after a timeout:
-           nothing may be in flight when the CTA frees its tensor memory) */
-        tc_commit(done);
-        if (fail) {
-            for (int st = 0; st < kGemmStages; st++)
-                if (xpend[st]) (void)mbar_wait(full(st), fph[st]);
-            (void)mbar_wait(done, 0u);
-            s_fail = 1;
-        }
-    }
-    __syncthreads();
-    bool fail = s_fail != 0;
-    if (!fail && nch > 0) {
-        const bool ok = mbar_wait(done, 0u, spin);
+    const uint32_t tmem = *s_tmem;
+    const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
+    const uint32_t aW1 = (uint32_t)__cvta_generic_to_shared(sW1), aW2 = (uint32_t)__cvta_generic_to_shared(sW2),
+                   aW3 = (uint32_t)__cvta_generic_to_shared(sW3), aX = (uint32_t)__cvta_generic_to_shared(sX),
+                   aA1 = (uint32_t)__cvta_generic_to_shared(sA1), aA2 = (uint32_t)__cvta_generic_to_shared(sA2),
+                   aZ = (uint32_t)__cvta_generic_to_shared(sZ);
+    uint32_t ph = 0u;
+    bool pending = false, fail = false;
+    /* the tiles written and the accumulator read so far are visible to the
+       tensor core; then one thread issues */
+    auto ready = [&] {
+        fence_async_smem();
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        pending = true;
+        return tid == 0;
+    };
+    auto wait = [&] {
+        const bool ok = mbar_wait(mb, ph, spin);
         fail = __syncthreads_or(!ok) != 0;
-        if (fail && tid == 0) (void)mbar_wait(done, 0u);
-    }
-    tc_fence_after();
-    if (!fail && nch > 0) {
-        const int row = m0 + warp * 32 + lane;
-        const uint32_t lb = tmem + ((uint32_t)(warp * 32) << 16);
-#pragma unroll 1
-        for (int c = 0; c < N; c += 32) {
-            float v[32];
-            tmem_ld32(lb + (uint32_t)c, v);
-            if (row < M) {
-                float* out = C + (size_t)row * ldc + c;
-                if (atomic) {
+        if (!fail) {
+            ph ^= 1u;
+            pending = false;
+        }
+        tc_fence_after();
+        return !fail;
+    };
+    /* the 12 16-byte chunks of each of a tile's rows, three per thread */
+    const bool wide = (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+    uint4 xr[3];
+    auto load_x = [&](int tile) {
 #pragma unroll
-                    for (int i = 0; i < 32; i++) atomicAdd(out + i, v[i]);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(out + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-                }
+        for (int i = 0; i < 3; i++) {
+            const int e = tid + i * kTrThreads, r = tile * kTile + e / 12, c = e % 12;
+            xr[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (r >= B) continue;
+            const __nv_bfloat16* src = X + (size_t)train_row(r, n, seed, draw) * IN + c * 8;
+            if (wide) {
+                xr[i] = *reinterpret_cast<const uint4*>(src);
+            } else {
+                const unsigned short* h = reinterpret_cast<const unsigned short*>(src);
+                xr[i] = make_uint4(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16,
+                                   h[4] | (uint32_t)h[5] << 16, h[6] | (uint32_t)h[7] << 16);
             }
         }
+    };
+    auto store_x = [&] {
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const int e = tid + i * kTrThreads;
+            *reinterpret_cast<uint4*>(sX + tc_off(e / 12, (e % 12) * 8, kTile)) = xr[i];
+        }
+    };
+    auto pack8 = [](const float* v) {
+        return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+    };
+    auto store32 = [&](unsigned char* t, const float (&v)[32]) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) *reinterpret_cast<uint4*>(t + tc_off(row, c0 + 8 * q, kTile)) = pack8(v + 8 * q);
+    };
+    /* z -> gelu(z) as BF16 into the tile, v -> the derivative */
+    auto activate = [&](float (&v)[32], const float* bias, unsigned char* t) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            float a[8];
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) {
+                float* x = v + 8 * q + i;
+                float2 y2, d2;
+                gelu_both(__fadd2_rn(make_float2(x[0], x[1]), *reinterpret_cast<const float2*>(bias + c0 + 8 * q + i)),
+                          &y2, &d2);
+                a[i] = y2.x;
+                a[i + 1] = y2.y;
+                x[0] = d2.x;
+                x[1] = d2.y;
+            }
+            *reinterpret_cast<uint4*>(t + tc_off(row, c0 + 8 * q, kTile)) = pack8(a);
+        }
+    };
+
+    const int ntiles = (B + kTile - 1) / kTile;
+    /* 1 / B where that is exact: a product with it is the quotient */
+    const float inv_b = (B & (B - 1)) == 0 ? 1.0f / (float)B : 0.0f;
+    float db1 = 0.0f, db2 = 0.0f, db3 = 0.0f, db3b = 0.0f, loss = 0.0f;
+    int right = 0;
+    bool add = false;
+    int tile = (int)blockIdx.x;
+    load_x(tile);
+    for (; tile < ntiles; tile += (int)gridDim.x) {
+        const int r = tile * kTile + row;
+        store_x();
+        float g1[32], g2[32];
+        if (ready()) {
+            tc_chain(tmem, aX, kTile, 0, aW1, HID, 0, HID, IN / 16, false);
+            tc_commit(mb);
+        }
+        const int yy = r < B ? (int)y[train_row(r, n, seed, draw)] : 0;
+        if (!wait()) break;
+        tmem_ld32(lane_base + c0, g1);
+        activate(g1, sb, sA1);
+        if (ready()) {
+            tc_chain(tmem, aA1, kTile, 0, aW2, HID, 0, HID, HID / 16, false);
+            tc_commit(mb);
+        }
+        if (!wait()) break;
+        tmem_ld32(lane_base + c0, g2);
+        activate(g2, sb + HID, sA2);
+        if (ready()) {
+            tc_chain(tmem, aA2, kTile, 0, aW3, OUT, 0, kOutA, HID / 16, false);
+            tc_commit(mb);
+        }
+        if (!wait()) break;
+        float z[32], zb[8];
+        tmem_ld32(lane_base + c0, z);
+        if (ready()) { /* outputs 128..159, eight per column group */
+            tc_chain(tmem, aA2, kTile, 0, aW3 + (uint32_t)(kOutA / 8) * 128u, OUT, 0, OUT - kOutA, HID / 16, false);
+            tc_commit(mb);
+        }
+        if (!wait()) break;
+        tmem_ld8(lane_base + cg * 8, zb);
+        /* softmax cross-entropy of the row; its four column groups exchange
+           through the dZ3 tile's memory */
+        float* sx = reinterpret_cast<float*>(sZ);
+        int* sxi = reinterpret_cast<int*>(sx + 4 * kTile);
+        float mx = -INFINITY, zt = 0.0f;
+        int am = 0;
+#pragma unroll
+        for (int i = 0; i < 32; i++) {
+            z[i] += sb[2 * HID + c0 + i];
+            if (z[i] > mx) { mx = z[i]; am = c0 + i; }
+            if (c0 + i == yy) zt = z[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int c = kOutA + cg * 8 + i;
+            zb[i] += sb[2 * HID + c];
+            if (zb[i] > mx) { mx = zb[i]; am = c; }
+            if (c == yy) zt = zb[i];
+        }
+        sx[cg * kTile + row] = mx;
+        sxi[cg * kTile + row] = am;
+        group_sync(1 + quad);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const float m = sx[q * kTile + row];
+            const int a = sxi[q * kTile + row];
+            if (m > mx || (m == mx && a < am)) { mx = m; am = a; }
+        }
+        float se = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 32; i++) se += z[i] = expf(z[i] - mx);
+#pragma unroll
+        for (int i = 0; i < 8; i++) se += zb[i] = expf(zb[i] - mx);
+        float* sxs = reinterpret_cast<float*>(sxi + 4 * kTile);
+        sxs[cg * kTile + row] = se;
+        group_sync(1 + quad);
+        se = (sxs[row] + sxs[kTile + row]) + (sxs[2 * kTile + row] + sxs[3 * kTile + row]);
+        /* the column group that holds the label counts the row */
+        const int own = yy < kOutA ? yy >> 5 : (yy - kOutA) >> 3;
+        if (r < B && own == cg) loss += -(zt - mx - logf(se));
+        if (r < B && cg == 0 && am == yy) right++;
+        /* e / se, correctly rounded from the row's reciprocal by one residual
+           step (Markstein): the divisor is shared, 1 <= se <= 160 */
+        const float rse = 1.0f / se;
+        auto dz = [&](float e, int c) {
+            const float q0 = e * rse, quo = __fmaf_rn(__fmaf_rn(-q0, se, e), rse, q0);
+            const float d = quo - (c == yy ? 1.0f : 0.0f);
+            return r < B ? (inv_b != 0.0f ? d * inv_b : d / (float)B) : 0.0f;
+        };
+#pragma unroll
+        for (int i = 0; i < 32; i++) z[i] = dz(z[i], c0 + i);
+#pragma unroll
+        for (int i = 0; i < 8; i++) zb[i] = dz(zb[i], kOutA + cg * 8 + i);
+        group_sync(1 + quad); /* the quarter's exchange has been read */
+        __syncthreads();      /* and the other quarters': the tile may be written */
+        store32(sZ, z);
+        *reinterpret_cast<uint4*>(sZ + tc_off(row, kOutA + cg * 8, kTile)) = pack8(zb);
+        if (ready()) {
+            tc_chain(tmem + kTrW3, aA2, kTile, 1, aZ, kTile, 1, OUT, kTile / 16, add);
+            tc_chain(tmem, aZ, kTile, 0, aW3, OUT, 1, HID, OUT / 16, false);
+            tc_commit(mb);
+        }
+        db3 += warp_colsum(z);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+#pragma unroll
+            for (int o = 16; o; o >>= 1) zb[i] += __shfl_xor_sync(0xffffffffu, zb[i], o);
+            if (lane == i) db3b += zb[i];
+        }
+        if (!wait()) break;
+        float d[32];
+        tmem_ld32(lane_base + c0, d);
+#pragma unroll
+        for (int i = 0; i < 32; i++) d[i] *= g2[i];
+        store32(sA2, d);
+        if (ready()) {
+            tc_chain(tmem + kTrW2, aA1, kTile, 1, aA2, kTile, 1, HID, kTile / 16, add);
+            tc_chain(tmem, aA2, kTile, 0, aW2, HID, 1, HID, HID / 16, false);
+            tc_commit(mb);
+        }
+        db2 += warp_colsum(d);
+        load_x(tile + (int)gridDim.x); /* rows beyond the batch: zeros, not used */
+        if (!wait()) break;
+        tmem_ld32(lane_base + c0, d);
+#pragma unroll
+        for (int i = 0; i < 32; i++) d[i] *= g1[i];
+        store32(sA1, d);
+        if (ready()) {
+            tc_chain(tmem + kTrW1, aA1, kTile, 1, aX, kTile, 1, IN, kTile / 16, add);
+            tc_commit(mb);
+        }
+        db1 += warp_colsum(d);
+        if (!wait()) break;
+        add = true;
     }
     if (fail && tid == 0) atomicOr(err, 1);
+    if (pending) (void)mbar_wait(mb, ph);
+    if (!fail) {
+        /* the CTA's partial gradient: dW3 and dW2 by rows of the lane's input
+           unit, dW1^T by the lane's output unit */
+        float* G = part + (size_t)blockIdx.x * NPARAM;
+        float v[32];
+        for (int b = cg; b < (OUT + HID + IN) / 32; b += 4) {
+            tmem_ld32(lane_base + kTrW3 + b * 32, v);
+            if (b < OUT / 32 + HID / 32) {
+                float* o = b < OUT / 32 ? G + OW3 + row * OUT + b * 32 : G + OW2 + row * HID + (b - OUT / 32) * 32;
+#pragma unroll
+                for (int i = 0; i < 32; i += 4)
+                    *reinterpret_cast<float4*>(o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 32; i++) G[OW1 + ((b - (OUT + HID) / 32) * 32 + i) * HID + row] = v[i];
+            }
+        }
+        /* bias gradients: the four row quarters in order, through the dZ3 tile */
+        float* sg = reinterpret_cast<float*>(sZ) + quad * (2 * HID + OUT);
+        sg[c0 + lane] = db1;
+        sg[HID + c0 + lane] = db2;
+        sg[2 * HID + c0 + lane] = db3;
+        if (lane < 8) sg[2 * HID + kOutA + cg * 8 + lane] = db3b;
+        float* sl = reinterpret_cast<float*>(sA1);
+        int* sr = reinterpret_cast<int*>(sA2);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+        right = __reduce_add_sync(0xffffffffu, right);
+        if (lane == 0) {
+            sl[warp] = loss;
+            sr[warp] = right;
+        }
+        __syncthreads();
+        const float* s4 = reinterpret_cast<const float*>(sZ);
+        constexpr int NB = 2 * HID + OUT;
+        for (int i = tid; i < NB; i += kTrThreads)
+            G[i < HID ? OB1 + i : (i < 2 * HID ? OB2 + i - HID : OB3 + i - 2 * HID)] =
+                (s4[i] + s4[NB + i]) + (s4[2 * NB + i] + s4[3 * NB + i]);
+        if (tid == 0) {
+            float l = 0.0f;
+            int k = 0;
+            for (int w = 0; w < kTrThreads / 32; w++) {
+                l += sl[w];
+                k += sr[w];
+            }
+            part_loss[blockIdx.x] = l;
+            part_ok[blockIdx.x] = k;
+        }
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTrCols) : "memory");
 }
 
-/* the minibatch: rows of X (BF16) gathered by idx or by a seeded hash */
-__global__ void k_gather(const __nv_bfloat16* X, const unsigned char* y, int n, int B, unsigned long long seed,
-                         const int* idx, __nv_bfloat16* xb, int* yb)
+/* place of parameter i of the flat array in the packed weights (-1: a bias) */
+__device__ __forceinline__ int pack_off(int i)
 {
-    int r = blockIdx.x;
-    if (r >= B) return;
-    int src;
-    if (idx) src = idx[r];
-    else {
-        unsigned long long z = seed + 0x9E3779B97F4A7C15ull * (unsigned long long)(r + 1);
-        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-        z ^= z >> 31;
-        src = (int)(z % (unsigned long long)n);
-    }
-    for (int c = threadIdx.x; c < IN; c += blockDim.x) xb[(size_t)r * IN + c] = X[(size_t)src * IN + c];
-    if (threadIdx.x == 0) yb[r] = y[src];
+    if (i < OB1) return tc_off(i % HID, i / HID, HID);
+    if (i < OW2) return -1;
+    if (i < OB2) return kW1B + tc_off((i - OW2) % HID, (i - OW2) / HID, HID);
+    if (i < OW3) return -1;
+    if (i < OB3) return kW1B + kW2B + tc_off((i - OW3) % OUT, (i - OW3) / OUT, OUT);
+    return -1;
 }
 
-/* elementwise steps between the GEMMs, in 32 x 32 tiles so that the
-   transposed BF16 copy (the operand of a weight-gradient GEMM, [cols][ldT])
-   is written coalesced as well:
-     kPostGelu  Z += bias (kept for the backward pass), out = gelu(Z)
-     kPostBack  D *= gelu'(Zs) (kept in place for the bias gradient), out = D
-     kPostCopy  out = D (FP32 or BF16 input)
-   out (BF16 row-major) and outT (BF16 transposed) may be null */
-enum { kPostGelu = 0, kPostBack = 1, kPostCopy = 2 };
-template <class TIn>
-__global__ void k_post(TIn* D, const float* Zs, const float* bias, int rows, int cols, int mode, __nv_bfloat16* out,
-                       __nv_bfloat16* outT, int ldT)
+__global__ void k_pack_all(const float* p, unsigned char* pack)
 {
-    __shared__ float tile[32][33];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int r = r0 + ty + 8 * i, c = c0 + tx;
-        float v = 0.0f;
-        if (r < rows && c < cols) {
-            const size_t o = (size_t)r * cols + c;
-            v = (float)D[o];
-            if (mode == kPostGelu) {
-                v += bias[c];
-                D[o] = (TIn)v;
-                v = gelu(v);
-            } else if (mode == kPostBack) {
-                v *= gelu_grad(Zs[o]);
-                D[o] = (TIn)v;
-            }
-            if (out) out[o] = __float2bfloat16_rn(v);
-        }
-        tile[ty + 8 * i][tx] = v;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= NPARAM) return;
+    const int o = pack_off(i);
+    if (o >= 0) *reinterpret_cast<__nv_bfloat16*>(pack + o) = __float2bfloat16_rn(p[i]);
+}
+
+/* gradient = sum of the partial gradients (the same order on every run), then
+   the Adam step on it (lr > 0) with the BF16 copy of the new weights.  A warp
+   sums an eighth of the partials of 32 parameters; block 0 adds up the loss. */
+__global__ void __launch_bounds__(256) k_reduce_adam(const float* part, int nparts, float* g, float* p, float* m,
+                                                     float* v, unsigned char* pack, float lr, float b1, float b2,
+                                                     float eps, float c1, float c2, const float* part_loss,
+                                                     const int* part_ok, float* loss, int* right)
+{
+    __shared__ float s[8][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    float a = 0.0f;
+    if (i < NPARAM) {
+#pragma unroll 10
+        for (int q = w; q < nparts; q += 8) a += part[(size_t)q * NPARAM + i];
     }
-    if (!outT) return;
+    s[w][lane] = a;
     __syncthreads();
+    if (blockIdx.x == 0 && w == 1) {
+        float l = 0.0f;
+        int k = 0;
+        for (int q = lane; q < nparts; q += 32) {
+            l += part_loss[q];
+            k += part_ok[q];
+        }
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int c = c0 + ty + 8 * i, r = r0 + tx;
-        if (r < rows && c < cols) outT[(size_t)c * ldT + r] = __float2bfloat16_rn(tile[tx][ty + 8 * i]);
+        for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        k = __reduce_add_sync(0xffffffffu, k);
+        if (lane == 0) {
+            *loss = l;
+            *right = k;
+        }
     }
-}
-
-/* BF16 copies of the master weights for the GEMM operands: W^T ([N][K],
-   forward) and W as stored ([K][N] = the backward B operand) */
-__global__ void k_wconv(const float* W, int K, int N, __nv_bfloat16* WT, __nv_bfloat16* Wn)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < K * N; i += gridDim.x * blockDim.x) {
-        const int k = i / N, n = i % N;
-        const __nv_bfloat16 v = __float2bfloat16_rn(W[i]);
-        if (WT) WT[(size_t)n * K + k] = v;
-        if (Wn) Wn[i] = v;
-    }
-}
-
-__global__ void k_bias_act(float* Z, float* Aout, const float* b, int rows, int cols, int act)
-{
-    size_t total = (size_t)rows * cols;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        float z = Z[i] + b[i % cols];
-        Z[i] = z;
-        if (Aout) Aout[i] = act ? gelu(z) : z;
-    }
-}
-
-/* softmax cross-entropy: dZ = (softmax - onehot) / B, loss summed in *loss */
-__global__ void k_softmax_ce(const float* Z, const int* y, int B, float* dZ, float* loss, int* correct)
-{
-    int r = blockIdx.x * blockDim.y + threadIdx.y;
-    if (r >= B) return;
-    const float* z = Z + (size_t)r * OUT;
-    int lane = threadIdx.x;
-    float mx = -INFINITY;
-    int am = 0;
-    for (int c = lane; c < OUT; c += 32)
-        if (z[c] > mx) { mx = z[c]; am = c; }
-    for (int o = 16; o; o >>= 1) {
-        float om = __shfl_xor_sync(0xffffffffu, mx, o);
-        int oa = __shfl_xor_sync(0xffffffffu, am, o);
-        if (om > mx || (om == mx && oa < am)) { mx = om; am = oa; }
-    }
-    float se = 0.0f;
-    for (int c = lane; c < OUT; c += 32) se += expf(z[c] - mx);
-    for (int o = 16; o; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
-    int yy = y[r];
-    for (int c = lane; c < OUT; c += 32) {
-        float p = expf(z[c] - mx) / se;
-        dZ[(size_t)r * OUT + c] = (p - (c == yy ? 1.0f : 0.0f)) / (float)B;
-    }
-    if (lane == 0) {
-        atomicAdd(loss, -(z[yy] - mx - logf(se)));
-        if (correct && am == yy) atomicAdd(correct, 1);
-    }
-}
-
-/* db[c] += sum over a chunk of rows of dZ[r][c] (db zeroed by the caller;
-   grid.y chunks of rows) */
-__global__ void k_colsum(const float* dZ, int rows, int cols, float* db)
-{
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    int chunk = (rows + gridDim.y - 1) / gridDim.y;
-    int r0 = blockIdx.y * chunk, r1 = min(rows, r0 + chunk);
-    float s = 0.0f;
-    for (int r = r0; r < r1; r++) s += dZ[(size_t)r * cols + c];
-    atomicAdd(&db[c], s);
-}
-
-__global__ void k_adam(float* w, const float* g, float* m, float* v, int n, float lr, float b1, float b2, float eps,
-                       float c1, float c2)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float gi = g[i];
-    float mi = b1 * m[i] + (1.0f - b1) * gi;
-    float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+    if (w != 0 || i >= NPARAM) return;
+    float gi = s[0][lane];
+#pragma unroll
+    for (int q = 1; q < 8; q++) gi += s[q][lane];
+    g[i] = gi;
+    if (!(lr > 0.0f)) return;
+    const float mi = b1 * m[i] + (1.0f - b1) * gi;
+    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    const float pn = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    p[i] = pn;
+    const int o = pack_off(i);
+    if (o >= 0) *reinterpret_cast<__nv_bfloat16*>(pack + o) = __float2bfloat16_rn(pn);
 }
 
 }  // namespace
-
-/* parameter layout in one FP32 array: W1 [IN x HID], b1, W2 [HID x HID], b2, W3 [HID x OUT], b3 */
-constexpr int OW1 = 0, OB1 = OW1 + IN * HID, OW2 = OB1 + HID, OB2 = OW2 + HID * HID, OW3 = OB2 + HID,
-              OB3 = OW3 + HID * OUT, NPARAM = OB3 + OUT;
 
 struct ecmg_mlp {
     float* p = nullptr;     /* FP32 master parameters */
@@ -763,14 +956,16 @@ struct ecmg_mlp {
     float* bias = nullptr;  /* b1 | b2 | b3 */
     int step = 0;
     bool packed = false;
-    /* training scratch for batch B (transposed copies have rows of capT) */
-    int cap = 0, capT = 0;
-    float *z1 = nullptr, *z2 = nullptr, *z3 = nullptr, *dz3 = nullptr, *d2 = nullptr, *d1 = nullptr, *loss = nullptr;
-    __nv_bfloat16 *xb = nullptr, *xT = nullptr, *a1 = nullptr, *a1T = nullptr, *a2 = nullptr, *a2T = nullptr,
-                  *dz3h = nullptr, *dz3T = nullptr, *d2h = nullptr, *d2T = nullptr, *d1T = nullptr;
-    /* BF16 operand copies of the weights: W^T for the forward GEMMs, W for the backward ones */
-    __nv_bfloat16 *w1T = nullptr, *w2T = nullptr, *w3T = nullptr, *w2n = nullptr, *w3n = nullptr;
-    int *yb = nullptr, *correct = nullptr, *gerr = nullptr;
+    /* training (allocated by its first use): the partial gradients of up to
+       one CTA per SM with their losses and hits, the BF16 operand copy of the
+       weights, and per-step losses and hits; page-locked staging of what
+       loss_grad and train read back */
+    int parts = 0;
+    float *part = nullptr, *part_loss = nullptr, *hist_loss = nullptr;
+    int *part_ok = nullptr, *hist_ok = nullptr, *gerr = nullptr;
+    unsigned char* tpack = nullptr;
+    float* h_grad = nullptr;
+    int hist = 0;
     cudaStream_t s = nullptr;
 };
 
@@ -797,6 +992,8 @@ cudaError_t ecmg::mlp_pack(ecmg_mlp* mm)
     if (e == cudaSuccess) mm->packed = true;
     return e;
 }
+
+constexpr float kBeta1 = 0.9f, kBeta2 = 0.999f; /* Adam */
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -869,8 +1066,7 @@ ecmg_status ecmg_mlp_create(unsigned long long seed, ecmg_mlp** out)
               cudaMalloc(&mm->v, sizeof(float) * NPARAM) == cudaSuccess &&
               cudaMalloc(&mm->pack, (size_t)kWB) == cudaSuccess &&
               cudaMalloc(&mm->derr, sizeof(int)) == cudaSuccess &&
-              cudaMalloc(&mm->bias, sizeof(float) * (2 * HID + OUT)) == cudaSuccess &&
-              cudaMalloc(&mm->loss, sizeof(float)) == cudaSuccess && cudaMalloc(&mm->correct, sizeof(int)) == cudaSuccess;
+              cudaMalloc(&mm->bias, sizeof(float) * (2 * HID + OUT)) == cudaSuccess;
     if (!ok) {
         ecmg_mlp_destroy(mm);
         return ECMG_ERR_CUDA;
@@ -904,18 +1100,11 @@ ecmg_status ecmg_mlp_destroy(ecmg_mlp* mm)
 {
     if (!mm) return ECMG_ERR_INVALID_ARG;
     if (mm->s) cudaStreamSynchronize(mm->s);
-    float* fs[] = {mm->p, mm->g, mm->m, mm->v, mm->bias, mm->z1, mm->z2, mm->z3, mm->dz3, mm->d2, mm->d1, mm->loss};
-    for (float* f : fs)
-        if (f) cudaFree(f);
-    __nv_bfloat16* hs[] = {mm->xb, mm->xT, mm->a1, mm->a1T, mm->a2, mm->a2T, mm->dz3h, mm->dz3T, mm->d2h, mm->d2T,
-                           mm->d1T, mm->w1T, mm->w2T, mm->w3T, mm->w2n, mm->w3n};
-    for (__nv_bfloat16* h : hs)
-        if (h) cudaFree(h);
-    if (mm->gerr) cudaFree(mm->gerr);
-    if (mm->pack) cudaFree(mm->pack);
-    if (mm->derr) cudaFree(mm->derr);
-    if (mm->yb) cudaFree(mm->yb);
-    if (mm->correct) cudaFree(mm->correct);
+    void* ds[] = {mm->p, mm->g, mm->m, mm->v, mm->bias, mm->pack, mm->derr, mm->part, mm->part_loss, mm->hist_loss,
+                  mm->part_ok, mm->hist_ok, mm->gerr, mm->tpack};
+    for (void* d : ds)
+        if (d) cudaFree(d);
+    if (mm->h_grad) cudaFreeHost(mm->h_grad);
     if (mm->s) cudaStreamDestroy(mm->s);
     delete mm;
     return ECMG_OK;
@@ -942,148 +1131,82 @@ ecmg_status ecmg_mlp_set_params(ecmg_mlp* mm, const float* host_in)
     return ECMG_OK;
 }
 
-static ecmg_status ensure_batch(ecmg_mlp* mm, int B)
+/* training scratch, and room for the losses of `steps` steps */
+static ecmg_status ensure_train(ecmg_mlp* mm, int steps)
 {
-    if (B <= mm->cap) return ECMG_OK;
-    float** fs[] = {&mm->z1, &mm->z2, &mm->z3, &mm->dz3, &mm->d2, &mm->d1};
-    for (float** f : fs)
-        if (*f) { cudaFree(*f); *f = nullptr; }
-    __nv_bfloat16** hs[] = {&mm->xb, &mm->xT, &mm->a1, &mm->a1T, &mm->a2, &mm->a2T, &mm->dz3h, &mm->dz3T, &mm->d2h,
-                            &mm->d2T, &mm->d1T};
-    for (__nv_bfloat16** h : hs)
-        if (*h) { cudaFree(*h); *h = nullptr; }
-    if (mm->yb) { cudaFree(mm->yb); mm->yb = nullptr; }
-    const size_t b = (size_t)B, bt = (size_t)((B + 7) & ~7); /* 16-byte rows of the transposed copies */
-    auto fa = [](float** p, size_t n) { return cudaMalloc(p, sizeof(float) * n) == cudaSuccess; };
-    auto ha = [](__nv_bfloat16** p, size_t n) { return cudaMalloc(p, 2 * n) == cudaSuccess; };
-    bool ok = fa(&mm->z1, b * HID) && fa(&mm->z2, b * HID) && fa(&mm->z3, b * OUT) && fa(&mm->dz3, b * OUT) &&
-              fa(&mm->d2, b * HID) && fa(&mm->d1, b * HID) && ha(&mm->xb, b * IN) && ha(&mm->xT, bt * IN) &&
-              ha(&mm->a1, b * HID) && ha(&mm->a1T, bt * HID) && ha(&mm->a2, b * HID) && ha(&mm->a2T, bt * HID) &&
-              ha(&mm->dz3h, b * OUT) && ha(&mm->dz3T, bt * OUT) && ha(&mm->d2h, b * HID) && ha(&mm->d2T, bt * HID) &&
-              ha(&mm->d1T, bt * HID) && cudaMalloc(&mm->yb, sizeof(int) * b) == cudaSuccess;
-    if (ok && !mm->w1T)
-        ok = ha(&mm->w1T, (size_t)IN * HID) && ha(&mm->w2T, (size_t)HID * HID) && ha(&mm->w3T, (size_t)HID * OUT) &&
-             ha(&mm->w2n, (size_t)HID * HID) && ha(&mm->w3n, (size_t)HID * OUT) &&
-             cudaMalloc(&mm->gerr, sizeof(int)) == cudaSuccess && cudaMemset(mm->gerr, 0, sizeof(int)) == cudaSuccess;
-    /* outside any stream capture: the GEMM kernel's shared memory limit */
-    if (ok) ok = cudaFuncSetAttribute(k_tc_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem) ==
-                 cudaSuccess;
-    if (!ok) return ECMG_ERR_CUDA;
-    mm->cap = B;
-    mm->capT = (int)bt;
+    if (!mm->part) {
+        int dev = 0, sms = 1;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const size_t np = (size_t)sms;
+        bool ok = cudaMalloc(&mm->part_loss, sizeof(float) * np) == cudaSuccess &&
+                  cudaMalloc(&mm->part_ok, sizeof(int) * np) == cudaSuccess &&
+                  cudaMalloc(&mm->tpack, (size_t)kWB) == cudaSuccess &&
+                  cudaMalloc(&mm->gerr, sizeof(int)) == cudaSuccess &&
+                  cudaMemset(mm->gerr, 0, sizeof(int)) == cudaSuccess &&
+                  cudaMallocHost(&mm->h_grad, sizeof(float) * (NPARAM + 2)) == cudaSuccess &&
+                  /* outside any stream capture: the kernel's shared memory limit */
+                  cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem) ==
+                      cudaSuccess &&
+                  cudaMalloc(&mm->part, sizeof(float) * np * NPARAM) == cudaSuccess;
+        if (!ok) return ECMG_ERR_CUDA;
+        mm->parts = sms;
+    }
+    if (steps > mm->hist) {
+        if (mm->hist_loss) cudaFree(mm->hist_loss);
+        if (mm->hist_ok) cudaFree(mm->hist_ok);
+        mm->hist_loss = nullptr;
+        mm->hist_ok = nullptr;
+        mm->hist = 0;
+        if (cudaMalloc(&mm->hist_loss, sizeof(float) * (size_t)steps) != cudaSuccess ||
+            cudaMalloc(&mm->hist_ok, sizeof(int) * (size_t)steps) != cudaSuccess)
+            return ECMG_ERR_CUDA;
+        mm->hist = steps;
+    }
     return ECMG_OK;
 }
 
-/* [rows x cols] BF16 row-major with `ld` elements per row as a 2D tensor;
-   boxes of 8 columns x box_rows rows, reads beyond the tensor give zeros */
-static cudaError_t bf16_map(CUtensorMap* tm, const void* p, int rows, int cols, int ld, int box_rows)
+/* forward and backward on B rows (the rows of X in order, or drawn with the
+   seed), the gradient in mm->g and, for lr > 0, the Adam step; the summed
+   loss and the hits go to entry `at` of the history.  Every contraction takes
+   BF16 operands on the tensor cores and accumulates in FP32; the elementwise
+   steps and the master weights are FP32. */
+static cudaError_t train_step(ecmg_mlp* mm, const void* X, const unsigned char* y, int n, int B,
+                              unsigned long long seed, int draw, int at, float lr, float c1, float c2)
 {
-    EncodeTiledFn enc = tensor_map_encoder();
-    if (!enc) return cudaErrorNotSupported;
-    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {8, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
-}
-
-/* C[M x N] (+)= A[M x K] B[N x K]^T on the tensor cores (k_tc_gemm); A has
-   lda, B ldb elements per row; split > 1 cuts K over CTAs, added atomically
-   into C (which must hold the initial value) */
-static cudaError_t tc_gemm(ecmg_mlp* mm, int M, int N, int K, const __nv_bfloat16* A, int lda,
-                           const __nv_bfloat16* B, int ldb, float* C, int ldc, int split)
-{
-    CUtensorMap ta, tb;
-    cudaError_t e = bf16_map(&ta, A, M, K, lda, kTile);
-    if (e == cudaSuccess) e = bf16_map(&tb, B, N, K, ldb, N);
-    if (e != cudaSuccess) return e;
-    int kper = (K + split - 1) / split;
-    kper = (kper + kGemmKC - 1) / kGemmKC * kGemmKC;
-    const dim3 grid((M + kTile - 1) / kTile, (K + kper - 1) / kper);
-    k_tc_gemm<<<grid, 128, kGemmSmem, mm->s>>>(ta, tb, M, N, K, kper, C, ldc, split > 1 ? 1 : 0, mm->gerr, mm->spin);
+    const int grid = std::min(mm->parts, (B + kTile - 1) / kTile);
+    k_train<<<grid, kTrThreads, kTrainSmem, mm->s>>>((const __nv_bfloat16*)X, y, n, B, seed, draw, mm->tpack, mm->p,
+                                                     mm->part, mm->part_loss, mm->part_ok, mm->gerr, mm->spin);
+    k_reduce_adam<<<(NPARAM + 31) / 32, 256, 0, mm->s>>>(mm->part, grid, mm->g, mm->p, mm->m, mm->v, mm->tpack, lr,
+                                                         kBeta1, kBeta2, 1e-8f, c1, c2, mm->part_loss, mm->part_ok,
+                                                         mm->hist_loss + at, mm->hist_ok + at);
     return cudaGetLastError();
-}
-
-/* forward + backward on B rows (gathered by idx, or sampled with seed);
-   leaves gradients in mm->g and the summed loss in mm->loss.  Every GEMM
-   takes BF16 operands on the tensor cores and accumulates in FP32; the
-   elementwise steps and the master weights stay FP32. */
-static cudaError_t fwd_bwd(ecmg_mlp* mm, const void* X, const unsigned char* y, int n, int B, unsigned long long seed,
-                           const int* idx)
-{
-    cudaStream_t s = mm->s;
-    const float* P = mm->p;
-    float* G = mm->g;
-    const int T = mm->capT;
-    const dim3 pb(32, 8);
-    auto pg = [](int rows, int cols) { return dim3((cols + 31) / 32, (rows + 31) / 32); };
-    cudaMemsetAsync(mm->loss, 0, sizeof(float), s);
-    cudaMemsetAsync(mm->correct, 0, sizeof(int), s);
-    k_wconv<<<64, 256, 0, s>>>(P + OW1, IN, HID, mm->w1T, nullptr);
-    k_wconv<<<64, 256, 0, s>>>(P + OW2, HID, HID, mm->w2T, mm->w2n);
-    k_wconv<<<64, 256, 0, s>>>(P + OW3, HID, OUT, mm->w3T, mm->w3n);
-    k_gather<<<B, 96, 0, s>>>((const __nv_bfloat16*)X, y, n, B, seed, idx, mm->xb, mm->yb);
-    k_post<__nv_bfloat16><<<pg(B, IN), pb, 0, s>>>(mm->xb, nullptr, nullptr, B, IN, kPostCopy, nullptr, mm->xT, T);
-    cudaError_t e;
-    /* forward */
-    if ((e = tc_gemm(mm, B, HID, IN, mm->xb, IN, mm->w1T, IN, mm->z1, HID, 1)) != cudaSuccess) return e;
-    k_post<float><<<pg(B, HID), pb, 0, s>>>(mm->z1, nullptr, P + OB1, B, HID, kPostGelu, mm->a1, mm->a1T, T);
-    if ((e = tc_gemm(mm, B, HID, HID, mm->a1, HID, mm->w2T, HID, mm->z2, HID, 1)) != cudaSuccess) return e;
-    k_post<float><<<pg(B, HID), pb, 0, s>>>(mm->z2, nullptr, P + OB2, B, HID, kPostGelu, mm->a2, mm->a2T, T);
-    if ((e = tc_gemm(mm, B, OUT, HID, mm->a2, HID, mm->w3T, HID, mm->z3, OUT, 1)) != cudaSuccess) return e;
-    k_bias_act<<<1024, 256, 0, s>>>(mm->z3, nullptr, P + OB3, B, OUT, 0);
-    k_softmax_ce<<<(B + 3) / 4, dim3(32, 4), 0, s>>>(mm->z3, mm->yb, B, mm->dz3, mm->loss, mm->correct);
-    k_post<float><<<pg(B, OUT), pb, 0, s>>>(mm->dz3, nullptr, nullptr, B, OUT, kPostCopy, mm->dz3h, mm->dz3T, T);
-    /* backward: weight gradients reduce over the batch, split over CTAs */
-    const int split = std::max(1, std::min(128, B / 512));
-    const int csplit = B >= 4096 ? 256 : 1;
-    cudaMemsetAsync(G, 0, sizeof(float) * NPARAM, s);
-    if ((e = tc_gemm(mm, HID, OUT, B, mm->a2T, T, mm->dz3T, T, G + OW3, OUT, split)) != cudaSuccess) return e;
-    k_colsum<<<dim3((OUT + 127) / 128, csplit), 128, 0, s>>>(mm->dz3, B, OUT, G + OB3);
-    if ((e = tc_gemm(mm, B, HID, OUT, mm->dz3h, OUT, mm->w3n, OUT, mm->d2, HID, 1)) != cudaSuccess) return e;
-    k_post<float><<<pg(B, HID), pb, 0, s>>>(mm->d2, mm->z2, nullptr, B, HID, kPostBack, mm->d2h, mm->d2T, T);
-    if ((e = tc_gemm(mm, HID, HID, B, mm->a1T, T, mm->d2T, T, G + OW2, HID, split)) != cudaSuccess) return e;
-    k_colsum<<<dim3((HID + 127) / 128, csplit), 128, 0, s>>>(mm->d2, B, HID, G + OB2);
-    if ((e = tc_gemm(mm, B, HID, HID, mm->d2h, HID, mm->w2n, HID, mm->d1, HID, 1)) != cudaSuccess) return e;
-    k_post<float><<<pg(B, HID), pb, 0, s>>>(mm->d1, mm->z1, nullptr, B, HID, kPostBack, nullptr, mm->d1T, T);
-    if ((e = tc_gemm(mm, IN, HID, B, mm->xT, T, mm->d1T, T, G + OW1, HID, split)) != cudaSuccess) return e;
-    k_colsum<<<dim3((HID + 127) / 128, csplit), 128, 0, s>>>(mm->d1, B, HID, G + OB1);
-    return cudaGetLastError();
-}
-
-/* a tensor-core wait of the training GEMMs timed out (flag cleared) */
-static bool gemm_timed_out(ecmg_mlp* mm)
-{
-    int h = 0;
-    if (cudaMemcpyAsync(&h, mm->gerr, sizeof(int), cudaMemcpyDeviceToHost, mm->s) != cudaSuccess ||
-        cudaStreamSynchronize(mm->s) != cudaSuccess)
-        return true;
-    if (h) cudaMemsetAsync(mm->gerr, 0, sizeof(int), mm->s);
-    return h != 0;
 }
 
 ecmg_status ecmg_mlp_loss_grad(ecmg_mlp* mm, const void* dev_x, const unsigned char* dev_y, int n, float* loss,
                                float* host_grad)
 {
     if (!mm || !dev_x || !dev_y || n < 1) return ECMG_ERR_INVALID_ARG;
-    if (ensure_batch(mm, n) != ECMG_OK) return ECMG_ERR_CUDA;
-    std::vector<int> idx(n);
-    for (int i = 0; i < n; i++) idx[i] = i;
-    int* didx = nullptr;
-    if (cudaMalloc(&didx, sizeof(int) * n) != cudaSuccess) return ECMG_ERR_CUDA;
-    cudaMemcpy(didx, idx.data(), sizeof(int) * n, cudaMemcpyHostToDevice);
-    cudaError_t e = fwd_bwd(mm, dev_x, dev_y, n, n, 0, didx);
+    if (ensure_train(mm, 1) != ECMG_OK) return ECMG_ERR_CUDA;
+    k_pack_all<<<(NPARAM + 255) / 256, 256, 0, mm->s>>>(mm->p, mm->tpack);
+    cudaError_t e = train_step(mm, dev_x, dev_y, n, n, 0, 0, 0, 0.0f, 1.0f, 1.0f);
+    /* one wait for everything that is read back */
+    float* h = mm->h_grad;
+    int* herr = (int*)(h + NPARAM + 1);
+    auto get = [&](void* dst, const void* src, size_t bytes) {
+        if (e == cudaSuccess) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, mm->s);
+    };
+    if (host_grad) get(h, mm->g, sizeof(float) * NPARAM);
+    get(h + NPARAM, mm->hist_loss, sizeof(float));
+    get(herr, mm->gerr, sizeof(int));
     if (e == cudaSuccess) e = cudaStreamSynchronize(mm->s);
-    cudaFree(didx);
     if (e != cudaSuccess) return ECMG_ERR_CUDA;
-    if (gemm_timed_out(mm)) return ECMG_ERR_BOUND;
-    float l = 0;
-    cudaMemcpy(&l, mm->loss, sizeof(float), cudaMemcpyDeviceToHost);
-    if (loss) *loss = l / (float)n;
-    if (host_grad) cudaMemcpy(host_grad, mm->g, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost);
+    if (*herr) {
+        cudaMemsetAsync(mm->gerr, 0, sizeof(int), mm->s);
+        return ECMG_ERR_BOUND;
+    }
+    if (loss) *loss = h[NPARAM] / (float)n;
+    if (host_grad) std::memcpy(host_grad, h, sizeof(float) * NPARAM);
     return ECMG_OK;
 }
 
@@ -1091,28 +1214,32 @@ ecmg_status ecmg_mlp_train(ecmg_mlp* mm, const void* dev_x, const unsigned char*
                            float lr, unsigned long long seed, float* host_loss, float* host_acc)
 {
     if (!mm || !dev_x || !dev_y || n < 1 || steps < 0 || batch < 1 || !(lr > 0.0f)) return ECMG_ERR_INVALID_ARG;
-    if (ensure_batch(mm, batch) != ECMG_OK) return ECMG_ERR_CUDA;
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    if (ensure_train(mm, std::max(1, steps)) != ECMG_OK) return ECMG_ERR_CUDA;
+    k_pack_all<<<(NPARAM + 255) / 256, 256, 0, mm->s>>>(mm->p, mm->tpack);
     for (int it = 0; it < steps; it++) {
-        if (fwd_bwd(mm, dev_x, dev_y, n, batch, seed + 0x51ED27ull * (unsigned long long)(mm->step + 1), nullptr) !=
-            cudaSuccess)
-            return ECMG_ERR_CUDA;
+        const unsigned long long sd = seed + 0x51ED27ull * (unsigned long long)(mm->step + 1);
         mm->step++;
-        float c1 = 1.0f - powf(b1, (float)mm->step), c2 = 1.0f - powf(b2, (float)mm->step);
-        k_adam<<<(NPARAM + 255) / 256, 256, 0, mm->s>>>(mm->p, mm->g, mm->m, mm->v, NPARAM, lr, b1, b2, eps, c1, c2);
-        if (host_loss || host_acc) {
-            float l = 0;
-            int cc = 0;
-            cudaMemcpyAsync(&l, mm->loss, sizeof(float), cudaMemcpyDeviceToHost, mm->s);
-            cudaMemcpyAsync(&cc, mm->correct, sizeof(int), cudaMemcpyDeviceToHost, mm->s);
-            if (cudaStreamSynchronize(mm->s) != cudaSuccess) return ECMG_ERR_CUDA;
-            if (host_loss) host_loss[it] = l / (float)batch;
-            if (host_acc) host_acc[it] = (float)cc / (float)batch;
-        }
+        const float c1 = 1.0f - powf(kBeta1, (float)mm->step), c2 = 1.0f - powf(kBeta2, (float)mm->step);
+        if (train_step(mm, dev_x, dev_y, n, batch, sd, 1, it, lr, c1, c2) != cudaSuccess) return ECMG_ERR_CUDA;
     }
     mm->packed = false;
-    if (cudaStreamSynchronize(mm->s) != cudaSuccess) return ECMG_ERR_CUDA;
-    return gemm_timed_out(mm) ? ECMG_ERR_BOUND : ECMG_OK;
+    /* the steps' losses and hits are read back together at the end */
+    std::vector<int> ok(host_acc ? (size_t)steps : 0);
+    int herr = 0;
+    cudaError_t e = cudaSuccess;
+    if (host_loss && steps)
+        e = cudaMemcpyAsync(host_loss, mm->hist_loss, sizeof(float) * (size_t)steps, cudaMemcpyDeviceToHost, mm->s);
+    if (e == cudaSuccess && host_acc && steps)
+        e = cudaMemcpyAsync(ok.data(), mm->hist_ok, sizeof(int) * (size_t)steps, cudaMemcpyDeviceToHost, mm->s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, mm->gerr, sizeof(int), cudaMemcpyDeviceToHost, mm->s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(mm->s);
+    if (e != cudaSuccess) return ECMG_ERR_CUDA;
+    for (int it = 0; it < steps; it++) {
+        if (host_loss) host_loss[it] /= (float)batch;
+        if (host_acc) host_acc[it] = (float)ok[it] / (float)batch;
+    }
+    if (herr) cudaMemsetAsync(mm->gerr, 0, sizeof(int), mm->s);
+    return herr ? ECMG_ERR_BOUND : ECMG_OK;
 }
 
 ecmg_status ecmg_mlp_set_wait_limit(ecmg_mlp* mm, int polls)
