@@ -267,17 +267,17 @@ struct ecmg_ctx {
     int nbr_mode = 0;
     struct KdBufs {
         DBuf<unsigned char> mark, side;
-        DBuf<int> n_dev, iscan, ids0, vtmp, X0, X[2], Y[2], seg_lo, seg_hi, seg_node, scan_tmp32, hist, tree, map,
-            kfound, agg, prev_in, cache;
+        DBuf<int> n_dev, iscan, ids0, vtmp, X0, X[2], Y[2], seg_lo, seg_hi, seg_node, scan_tmp32, hist, tree, gidx,
+            agg, cache;
         DBuf<unsigned> keys, ktmp;
         DBuf<unsigned long long> flags, scan_tmp64;
-        DBuf<V2> tree_pos;
+        DBuf<float4> tree_pos;
         int levels = 0, tree_cap = 0;
         void free_all()
         {
             mark.free_(); side.free_();
             DBuf<int>* is[] = {&n_dev, &iscan, &ids0, &vtmp, &X0, &X[0], &X[1], &Y[0], &Y[1], &seg_lo, &seg_hi,
-                               &seg_node, &scan_tmp32, &hist, &tree, &map, &kfound, &agg, &prev_in, &cache};
+                               &seg_node, &scan_tmp32, &hist, &tree, &gidx, &agg, &cache};
             for (auto* b : is) b->free_();
             keys.free_(); ktmp.free_(); flags.free_(); scan_tmp64.free_(); tree_pos.free_();
         }
@@ -2011,9 +2011,6 @@ static cudaError_t enqueue_tick(ecmg_ctx* c, int launch_slots, bool use_model)
         kd.s_slot = c->s_slot.p;
         kd.counters = c->counters.p;
         kd.active = c->d_active.p;
-        kd.cell_start = c->cell_start.p;
-        kd.slot_bucket = c->key.p;
-        kd.slot_rank = c->rank.p;
         kd.mark = K.mark.p;
         kd.n_dev = K.n_dev.p;
         kd.iscan = K.iscan.p;
@@ -2032,10 +2029,9 @@ static cudaError_t enqueue_tick(ecmg_ctx* c, int launch_slots, bool use_model)
         kd.hist = K.hist.p;
         kd.tree = K.tree.p;
         kd.tree_pos = K.tree_pos.p;
-        kd.map = K.map.p;
-        kd.kfound = K.kfound.p;
+        kd.gidx = K.gidx.p;
+        kd.open = K.side.p; /* free once the tree is built */
         kd.agg = K.agg.p;
-        kd.prev_in = K.prev_in.p;
         kd.cache = K.cache.p;
         kd.nbr = c->nbr.p;
         kd.ncnt = c->ncnt.p;
@@ -2057,13 +2053,8 @@ int ecmg_kernels_per_tick(const ecmg_ctx* c)
        k_mlp_infer with a proposal model */
     if (!c) return 6;
     int n = 6 + ((c->model || c->trace) ? 1 : 0) + (c->model ? 1 : 0);
-    /* kd-tree mode, instead of k_neighbors: members and slot-order list (6),
-       four radix sorts of four passes (84), segment init (1), level 0 (11),
-       levels 1.. (side + partition), the query (2) and the composition (4) */
-    if (c->nbr_mode == ECMG_NEIGHBORS_KDTREE) {
-        const int L = c->kd.levels;
-        n += -1 + 6 + 84 + 1 + 11 + (L - 1) + 5 * std::max(0, L - 2) + 2 + 4;
-    }
+    /* kd-tree mode, instead of k_neighbors */
+    if (c->nbr_mode == ECMG_NEIGHBORS_KDTREE) n += -1 + kd_kernels(c->max_agents);
     return n;
 }
 
@@ -2503,9 +2494,8 @@ ecmg_status ecmg_set_neighbor_mode(ecmg_ctx* c, int mode)
         CK(K.scan_tmp64.alloc((size_t)kd_scan_tmp(c->max_agents)));
         CK(K.hist.alloc((size_t)hist)); CK(K.tree.alloc((size_t)K.tree_cap));
         CK(K.tree_pos.alloc((size_t)K.tree_cap));
-        CK(K.map.alloc(N * (size_t)k)); CK(K.kfound.alloc(N));
-        CK(K.agg.alloc((size_t)kd_compose_blocks(c->max_agents) * k));
-        CK(K.prev_in.alloc((size_t)kd_compose_blocks(c->max_agents) * k));
+        CK(K.gidx.alloc(N));
+        CK(K.agg.alloc((size_t)kd_compose_rows(c->max_agents) * k));
         CK(K.cache.alloc((size_t)k));
         CK(K.keys.alloc(N)); CK(K.ktmp.alloc(N)); CK(K.flags.alloc(N));
         /* ORCA::m_NeighborCache starts as std::vector<Entity>(k): zeros */

@@ -233,16 +233,12 @@ cudaError_t launch_spawn_place(const SpawnRec* rec, int n, const SpawnTargets& t
 /* kdtree.cu: the reference's kd-tree neighbour query (neighbour mode
    ECMG_NEIGHBORS_KDTREE).  Members = agents in this tick's grid (active at
    the start of the tick); lists hold slots. */
-constexpr int kKdMaxDepth = 30;
 struct KdArgs {
     int max_slots, cap, k, levels, tree_cap;
     const V2* pos;              /* slot-indexed positions at the start of the tick */
     const int* s_slot;          /* grid order -> slot */
     const int* counters;        /* C_NSORTED (members), C_LAST */
     const unsigned char* active; /* after the attraction kernel (kd_finish) */
-    const int* cell_start;
-    const int* slot_bucket;
-    const int* slot_rank;
     unsigned char* mark;        /* [max_slots] member flags */
     int* n_dev;                 /* [2] members, max depth */
     int* iscan;                 /* [max_slots] */
@@ -262,16 +258,16 @@ struct KdArgs {
     unsigned long long* scan_tmp64;
     int* hist;                  /* [kd_hist_ints(cap)] */
     int* tree;                  /* [tree_cap] KDTree::m_Tree */
-    V2* tree_pos;               /* [tree_cap] position of each node's agent */
-    int* map;                   /* [max_slots * k] per-member cache maps, then local prefixes */
-    int* kfound;                /* [max_slots] */
-    int* agg;
-    int* prev_in;               /* [kd_compose_blocks * k] */
+    float4* tree_pos;           /* [tree_cap] position and slot (bits) of each node's agent */
+    int* gidx;                  /* [max_slots] members' grid indices */
+    unsigned char* open;        /* [cap] by grid index: the row refers to the list before it */
+    int* agg;                   /* [kd_compose_rows * k] */
     int* cache;                 /* [k] ORCA::m_NeighborCache, kept across ticks */
-    int* nbr;                   /* [cap * k] per-agent kernel input, grid order */
+    int* nbr;                   /* [cap * k] grid order: the members' cache maps, in the end the per-agent kernel's input */
     int* ncnt;                  /* [cap] */
 };
-int kd_compose_blocks(int max_slots);
+int kd_compose_rows(int max_slots);
+int kd_kernels(int max_slots);
 int kd_hist_ints(int cap);
 int kd_scan_tmp(int n);
 cudaError_t kd_build_and_query(const KdArgs& a, cudaStream_t s, int sms);

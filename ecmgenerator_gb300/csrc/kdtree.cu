@@ -25,9 +25,9 @@
  * (-1, -2, ..., -k) = "previous agent's slot q" and ends with a map: each
  * slot either an agent or a previous slot.  Maps compose associatively; the
  * composition over the querying agents in index order (members still active
- * after the attraction stage) runs as a warp per block of 1024 slots, one
- * warp over the block results, and a resolving pass -- the last agent's list
- * is the cache the next tick starts from.
+ * after the attraction stage) folds 64 maps at a time, level by level, and the
+ * lists that refer to an earlier one look it up -- the last agent's list is
+ * the cache the next tick starts from.
  */
 #include "ecmg_internal.h"
 
@@ -37,9 +37,9 @@ namespace ecmg {
 
 namespace {
 
-constexpr int kRsThreads = 256, kRsItems = 16, kRsTile = kRsThreads * kRsItems;
+constexpr int kRsThreads = 256, kRsItems = 8, kRsTile = kRsThreads * kRsItems;
 constexpr int kScanThreads = 256, kScanItems = 8, kScanTile = kScanThreads * kScanItems;
-constexpr int kComposeSlots = 1024;
+constexpr int kFold = 64;
 
 __device__ __forceinline__ unsigned order_key(float f)
 {
@@ -163,22 +163,67 @@ cudaError_t scan_excl(T* data, int n, T* tmp, cudaStream_t s)
     return cudaGetLastError();
 }
 
-/* ---- stable LSD radix sort of (key, value) pairs, 8-bit digits ---------- */
+/* ---- stable LSD radix sort of (key, value) pairs, 8-bit digits ----------
+   Tiles of 2,048 keys: a quarter of a million agents fill the GPU (with 4,096
+   they were 62 blocks). */
 __global__ void __launch_bounds__(kRsThreads) k_rs_hist(const unsigned* __restrict__ keys, const int* __restrict__ n_ptr,
-                                                        int shift, int* __restrict__ hist, int nblk)
+                                                        int shift, int* __restrict__ hist)
 {
     __shared__ int h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
     const int n = *n_ptr;
     const int base = blockIdx.x * kRsTile;
-#pragma unroll 4
+#pragma unroll
     for (int i = 0; i < kRsItems; i++) {
         const int idx = base + i * kRsThreads + threadIdx.x;
         if (idx < n) atomicAdd(&h[(keys[idx] >> shift) & 255u], 1);
     }
     __syncthreads();
-    hist[threadIdx.x * nblk + blockIdx.x] = h[threadIdx.x];
+    hist[blockIdx.x * 256 + threadIdx.x] = h[threadIdx.x];
+}
+
+/* hist [nblk][256] -> where each tile's keys of each digit go, in place: one
+   block, four threads per digit over a quarter of the tiles each */
+__global__ void __launch_bounds__(1024) k_rs_scan(int* __restrict__ hist, int nblk)
+{
+    __shared__ int part[4][256];
+    __shared__ int ws[8];
+    const int d = threadIdx.x & 255, g = threadIdx.x >> 8;
+    const int per = (nblk + 3) / 4, b0 = g * per, b1 = min(nblk, b0 + per);
+    int s = 0;
+#pragma unroll 8
+    for (int b = b0; b < b1; b++) s += hist[b * 256 + d];
+    part[g][d] = s;
+    __syncthreads();
+    int run = 0;
+    if (g == 0) {
+        const int p0 = part[0][d], p1 = part[1][d], p2 = part[2][d], p3 = part[3][d];
+        const int lane = d & 31, w = d >> 5;
+        int x = p0 + p1 + p2 + p3;
+        const int tot = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) ws[w] = x;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        for (int q = 0; q < w; q++) x += ws[q];
+        run = x - tot;
+        part[0][d] = run;
+        part[1][d] = run + p0;
+        part[2][d] = run + p0 + p1;
+        part[3][d] = run + p0 + p1 + p2;
+    }
+    __syncthreads();
+    run = part[g][d];
+#pragma unroll 8
+    for (int b = b0; b < b1; b++) {
+        const int c = hist[b * 256 + d];
+        hist[b * 256 + d] = run;
+        run += c;
+    }
 }
 
 /* elements of a tile are placed in tile order, round by round (256 per
@@ -187,22 +232,30 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_hist(const unsigned* __restri
 __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const unsigned* __restrict__ kin, const int* __restrict__ vin,
                                                            unsigned* __restrict__ kout, int* __restrict__ vout,
                                                            const int* __restrict__ n_ptr, int shift,
-                                                           const int* __restrict__ offs, int nblk)
+                                                           const int* __restrict__ offs)
 {
     __shared__ int base[256];
     __shared__ int wc[kRsThreads / 32][256];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int n = *n_ptr;
-    base[threadIdx.x] = offs[threadIdx.x * nblk + blockIdx.x];
+    base[threadIdx.x] = offs[blockIdx.x * 256 + threadIdx.x];
     const int t0 = blockIdx.x * kRsTile;
+    if (t0 >= n) return;
+    unsigned keys[kRsItems];
+    int vals[kRsItems];
+#pragma unroll
+    for (int r = 0; r < kRsItems; r++) {
+        const int idx = t0 + r * kRsThreads + threadIdx.x;
+        keys[r] = idx < n ? kin[idx] : 0u;
+        vals[r] = idx < n ? vin[idx] : 0;
+    }
+#pragma unroll
     for (int r = 0; r < kRsItems; r++) {
 #pragma unroll
         for (int q = 0; q < kRsThreads / 32; q++) wc[q][threadIdx.x] = 0;
         __syncthreads();
-        const int idx = t0 + r * kRsThreads + threadIdx.x;
-        const bool valid = idx < n;
-        const unsigned key = valid ? kin[idx] : 0u;
-        const int d = valid ? (int)((key >> shift) & 255u) : 256 + lane;
+        const bool valid = t0 + r * kRsThreads + (int)threadIdx.x < n;
+        const int d = valid ? (int)((keys[r] >> shift) & 255u) : 256 + lane;
         const unsigned peers = __match_any_sync(0xffffffffu, d);
         const int rank = __popc(peers & ((1u << lane) - 1u));
         if (valid && rank == 0) wc[w][d] = __popc(peers);
@@ -220,8 +273,8 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const unsigned* __res
         __syncthreads();
         if (valid) {
             const int pos = wc[w][d] + rank;
-            kout[pos] = key;
-            vout[pos] = vin[idx];
+            kout[pos] = keys[r];
+            vout[pos] = vals[r];
         }
         __syncthreads();
     }
@@ -230,7 +283,7 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const unsigned* __res
 /* sorts keys[0, n) with their values; n is read on the device; the result
    ends in (keys, vals) after the four passes */
 cudaError_t radix_sort(unsigned* keys, int* vals, unsigned* ktmp, int* vtmp, const int* n_ptr, int cap, int* hist,
-                       int* scan_tmp, cudaStream_t s)
+                       cudaStream_t s)
 {
     const int nblk = (cap + kRsTile - 1) / kRsTile;
     unsigned* ka = keys;
@@ -238,10 +291,9 @@ cudaError_t radix_sort(unsigned* keys, int* vals, unsigned* ktmp, int* vtmp, con
     unsigned* kb = ktmp;
     int* vb = vtmp;
     for (int shift = 0; shift < 32; shift += 8) {
-        k_rs_hist<<<nblk, kRsThreads, 0, s>>>(ka, n_ptr, shift, hist, nblk);
-        cudaError_t e = scan_excl<int>(hist, 256 * nblk, scan_tmp, s);
-        if (e != cudaSuccess) return e;
-        k_rs_scatter<<<nblk, kRsThreads, 0, s>>>(ka, va, kb, vb, n_ptr, shift, hist, nblk);
+        k_rs_hist<<<nblk, kRsThreads, 0, s>>>(ka, n_ptr, shift, hist);
+        k_rs_scan<<<1, 1024, 0, s>>>(hist, nblk);
+        k_rs_scatter<<<nblk, kRsThreads, 0, s>>>(ka, va, kb, vb, n_ptr, shift, hist);
         unsigned* tk = ka; ka = kb; kb = tk;
         int* tv = va; va = vb; vb = tv;
     }
@@ -252,7 +304,11 @@ cudaError_t radix_sort(unsigned* keys, int* vals, unsigned* ktmp, int* vtmp, con
 __global__ void k_kd_mark(KdArgs a)
 {
     const int n = a.counters[C_NSORTED];
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) a.mark[a.s_slot[t]] = 1;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const int slot = a.s_slot[t];
+        a.mark[slot] = 1;
+        a.gidx[slot] = t;
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         a.n_dev[0] = n;
         /* KDTree.cpp:47: ceil(log2(size + 1) - 1) = bit length of size - 1 */
@@ -293,7 +349,7 @@ __global__ void k_kd_seg_init(KdArgs a)
     }
 }
 
-/* ---- one level of ConstructRecursive ------------------------------------ */
+/* ---- one level of ConstructRecursive over the whole lists ---------------- */
 __global__ void k_kd_side(KdArgs a, const int* A)
 {
     const int n = a.n_dev[0];
@@ -307,16 +363,42 @@ __global__ void k_kd_side(KdArgs a, const int* A)
     }
 }
 
-__global__ void k_kd_lrflags(KdArgs a, const int* B)
+/* left | right << 32 of position i of list B */
+__device__ __forceinline__ unsigned long long kd_flag(const KdArgs& a, const int* B, int i, int n)
+{
+    if (i >= n || a.seg_lo[i] >= a.seg_hi[i]) return 0ull;
+    const int s = a.side[B[i]];
+    return (s == 0 ? 1ull : 0ull) | (s == 2 ? (1ull << 32) : 0ull);
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_kd_count(KdArgs a, const int* B)
 {
     const int n = a.n_dev[0];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.cap; i += gridDim.x * blockDim.x) {
-        unsigned long long f = 0;
-        if (i < n && a.seg_lo[i] < a.seg_hi[i]) {
-            const int s = a.side[B[i]];
-            f = (s == 0 ? 1ull : 0ull) | (s == 2 ? (1ull << 32) : 0ull);
-        }
-        a.flags[i] = f;
+    const int base = blockIdx.x * kScanTile + threadIdx.x;
+    unsigned long long s = 0;
+#pragma unroll
+    for (int i = 0; i < kScanItems; i++) s += kd_flag(a, B, base + i * kScanThreads, n);
+    unsigned long long tot;
+    block_excl_scan<unsigned long long>(s, &tot);
+    if (threadIdx.x == 0) a.scan_tmp64[blockIdx.x] = tot;
+}
+
+/* exclusive left / right counts of every position (the tiles' sums scanned) */
+__global__ void __launch_bounds__(kScanThreads) k_kd_prefix(KdArgs a, const int* B)
+{
+    const int n = a.n_dev[0];
+    const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+    unsigned long long v[kScanItems], s = 0;
+#pragma unroll
+    for (int i = 0; i < kScanItems; i++) {
+        v[i] = kd_flag(a, B, base + i, n);
+        s += v[i];
+    }
+    unsigned long long run = block_excl_scan<unsigned long long>(s, nullptr) + a.scan_tmp64[blockIdx.x];
+#pragma unroll
+    for (int i = 0; i < kScanItems; i++) {
+        if (base + i < n) a.flags[base + i] = run;
+        run += v[i];
     }
 }
 
@@ -341,151 +423,313 @@ __global__ void k_kd_partition(KdArgs a, const int* B, int* Bout, int update_seg
         else if (s == 1) pos = mid;
         else pos = mid + 1 + (int)((unsigned)(f >> 32) - (unsigned)(f0 >> 32));
         Bout[pos] = id;
-        if (update_seg) {
-            const int node = a.seg_node[i];
-            if (i < mid) {
-                a.seg_hi[i] = mid;
-                a.seg_node[i] = 2 * node + 1;
-            } else if (i > mid) {
-                a.seg_lo[i] = mid + 1;
-                a.seg_node[i] = 2 * node + 2;
-            } else {
-                a.seg_lo[i] = hi;
-            }
+        if (!update_seg) continue;
+        const int node = a.seg_node[i];
+        if (i < mid) {
+            a.seg_hi[i] = mid;
+            a.seg_node[i] = 2 * node + 1;
+        } else if (i > mid) {
+            a.seg_lo[i] = mid + 1;
+            a.seg_node[i] = 2 * node + 2;
+        } else {
+            a.seg_lo[i] = hi;
         }
     }
 }
 
-/* positions in tree order (one dependent load per visit in the query) */
+cudaError_t kd_partition(const KdArgs& a, const int* B, int* Bout, int update_seg, int gc, cudaStream_t s)
+{
+    const int nb = (a.cap + kScanTile - 1) / kScanTile;
+    if (nb > 8192) return cudaErrorInvalidValue;
+    k_kd_count<<<nb, kScanThreads, 0, s>>>(a, B);
+    k_scan_top<unsigned long long><<<1, 1024, 0, s>>>(a.scan_tmp64, nb);
+    k_kd_prefix<<<nb, kScanThreads, 0, s>>>(a, B);
+    k_kd_partition<<<gc, 256, 0, s>>>(a, B, Bout, update_seg);
+    return cudaGetLastError();
+}
+
+/* ---- all remaining levels of one segment of up to kKdSmall members, by one
+   block in shared memory.  A level over the whole lists is six launches bound
+   by their latency (29 us each level at 250,000 agents); a segment of 4,096
+   has as many levels left as the ones above it have, and they cost it a few
+   block scans each.  Members are numbered by their place in the segment's X
+   list. */
+constexpr int kKdSmall = 4096, kSmallThreads = 1024, kSmallPer = kKdSmall / kSmallThreads;
+struct KdSmallSm {
+    int id[kKdSmall];             /* slot of each member */
+    unsigned count[kKdSmall + 1]; /* left | right << 16 before each position */
+    unsigned short list[3][kKdSmall]; /* X, Y and the list being written */
+    unsigned short lo[kKdSmall], hi[kKdSmall], node[kKdSmall]; /* of each position; node: place in its level */
+    unsigned char side[kKdSmall];
+    unsigned warp[32];
+};
+
+__global__ void __launch_bounds__(kSmallThreads) k_kd_small(KdArgs a, const int* X, const int* Y, int top, int* place)
+{
+    extern __shared__ __align__(16) unsigned char raw[];
+    KdSmallSm& m = *reinterpret_cast<KdSmallSm*>(raw);
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    /* the segment: the block's path of left / right turns from the root */
+    int lo0 = 0, hi0 = a.n_dev[0];
+    for (int b = top - 1; b >= 0 && lo0 < hi0; b--) {
+        const int mid = lo0 + (hi0 - 1 - lo0) / 2;
+        if ((blockIdx.x >> b) & 1) lo0 = mid + 1;
+        else hi0 = mid;
+    }
+    const int n = hi0 - lo0;
+    if (n <= 0) return;
+    for (int i = tid; i < n; i += kSmallThreads) {
+        const int id = X[lo0 + i];
+        m.id[i] = id;
+        m.list[0][i] = (unsigned short)i;
+        m.lo[i] = 0;
+        m.hi[i] = (unsigned short)n;
+        m.node[i] = 0;
+        place[id] = i;
+    }
+    __syncthreads();
+    for (int i = tid; i < n; i += kSmallThreads) m.list[1][i] = (unsigned short)place[Y[lo0 + i]];
+    __syncthreads();
+    int lx = 0, ly = 1, spare = 2;
+    for (int lv = top; lv < a.levels; lv++) {
+        const bool on_y = (lv & 1) != 0;
+        const unsigned short* A = m.list[on_y ? ly : lx];
+        const unsigned short* B = m.list[on_y ? lx : ly];
+        unsigned short* out = m.list[spare];
+        const int depth = lv - top;
+        bool any = false;
+        for (int i = tid; i < n; i += kSmallThreads) {
+            const int lo = m.lo[i], hi = m.hi[i];
+            if (lo >= hi) continue;
+            any = true;
+            const int mid = lo + (hi - 1 - lo) / 2;
+            const int q = A[i];
+            m.side[q] = i < mid ? 0 : (i == mid ? 1 : 2);
+            /* heap index: node `place` of depth lv under the segment's root */
+            if (i == mid) a.tree[((((1 << top) + (int)blockIdx.x) << depth) - 1) + m.node[i]] = m.id[q];
+        }
+        if (!__syncthreads_or(any)) return;
+        /* exclusive left / right counts over the segment's positions */
+        unsigned v[kSmallPer], sum = 0;
+#pragma unroll
+        for (int r = 0; r < kSmallPer; r++) {
+            const int i = tid * kSmallPer + r;
+            v[r] = 0;
+            if (i < n && m.lo[i] < m.hi[i]) {
+                const int sd = m.side[B[i]];
+                v[r] = (sd == 0 ? 1u : 0u) | (sd == 2 ? 0x10000u : 0u);
+            }
+            sum += v[r];
+        }
+        unsigned x = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) m.warp[w] = x;
+        __syncthreads();
+        if (w == 0) {
+            unsigned y = m.warp[lane];
+            const unsigned own = y;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned z = __shfl_up_sync(0xffffffffu, y, o);
+                if (lane >= o) y += z;
+            }
+            m.warp[lane] = y - own;
+        }
+        __syncthreads();
+        unsigned run = m.warp[w] + x - sum;
+#pragma unroll
+        for (int r = 0; r < kSmallPer; r++) {
+            m.count[tid * kSmallPer + r] = run;
+            run += v[r];
+        }
+        __syncthreads();
+        for (int i = tid; i < n; i += kSmallThreads) {
+            const int lo = m.lo[i], hi = m.hi[i];
+            const int q = B[i];
+            int pos = i;
+            if (lo < hi) {
+                const int mid = lo + (hi - 1 - lo) / 2;
+                const unsigned f = m.count[i], f0 = m.count[lo];
+                const int sd = m.side[q];
+                if (sd == 0) pos = lo + (int)((f & 0xffffu) - (f0 & 0xffffu));
+                else if (sd == 1) pos = mid;
+                else pos = mid + 1 + (int)((f >> 16) - (f0 >> 16));
+                if (i < mid) {
+                    m.hi[i] = (unsigned short)mid;
+                    m.node[i] = (unsigned short)(2 * m.node[i]);
+                } else if (i > mid) {
+                    m.lo[i] = (unsigned short)(mid + 1);
+                    m.node[i] = (unsigned short)(2 * m.node[i] + 1);
+                } else {
+                    m.lo[i] = (unsigned short)hi;
+                }
+            }
+            out[pos] = (unsigned short)q;
+        }
+        __syncthreads();
+        const int freed = on_y ? lx : ly;
+        if (on_y) lx = spare;
+        else ly = spare;
+        spare = freed;
+    }
+}
+
+/* position and grid index of each node's agent (-1: none) in tree order: one
+   load per visit in the query */
 __global__ void k_kd_tree_pos(KdArgs a)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.tree_cap; i += gridDim.x * blockDim.x) {
         const int id = a.tree[i];
-        a.tree_pos[i] = id >= 0 ? a.pos[id] : mk(0.0f, 0.0f);
+        const V2 p = id >= 0 ? a.pos[id] : mk(0.0f, 0.0f);
+        a.tree_pos[i] = make_float4(p.x, p.y, __int_as_float(id >= 0 ? a.gidx[id] : -1), 0.0f);
     }
 }
 
-/* ---- KNearestAgents_R (KDTree.cpp:98-202) with a symbolic cache ---------- */
-__global__ void __launch_bounds__(128) k_kd_query(KdArgs a, const int* members)
+/* ---- KNearestAgents_R (KDTree.cpp:98-202) with a symbolic cache ----------
+   A lane walks down the near children and keeps, by depth, each far child's
+   split distance and a lower bound of its region's distance (the far child is
+   the sibling of the path's node at that depth); one visit per lane and round, the lanes together (left
+   to itself a lane that goes on down never meets the others again: 5 of 32
+   lanes active).  The lists are columns in shared memory: their positions are
+   written by index.  Bound by issue and divergence: about 115 rounds a warp
+   for about 50 visits an agent, an update in nearly every round. */
+constexpr int kQueryWarps = 4;
+template <int K>
+__global__ void __launch_bounds__(32 * kQueryWarps, K <= 16 ? 8 : 4) k_kd_query(KdArgs a, const int* members)
 {
+    __shared__ float s_nd[kQueryWarps][K][33];
+    __shared__ int s_ni[kQueryWarps][K][33];
+    extern __shared__ float2 s_far[]; /* [warp][depth][lane]: distance to the split line, bounds (two upper halves) */
     const int n = a.n_dev[0];
     const int max_depth = a.n_dev[1];
     const int k = a.k;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int agent = members[i];
-        const V2 target = a.pos[agent];
-        int ni[kMaxK];
-        float nd[kMaxK];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    float (*nd)[33] = s_nd[wp];
+    int (*ni)[33] = s_ni[wp];
+    float2* far = s_far + wp * a.levels * 32 + lane;
+    for (int i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < n; i0 += gridDim.x * blockDim.x) {
+        const int i = i0 + lane;
+        const V2 target = a.pos[members[min(i, n - 1)]];
         for (int q = 0; q < k; q++) {
-            ni[q] = -(q + 1); /* the previous agent's slot q */
-            nd[q] = FLT_MAX;  /* Utility::MAX_FLOAT */
+            ni[q][lane] = -(q + 1); /* the previous agent's slot q */
+            nd[q][lane] = FLT_MAX;  /* Utility::MAX_FLOAT */
         }
+        float first = FLT_MAX, last = FLT_MAX; /* nd[0], nd[k - 1] */
         int kfound = 0;
-        /* frames: node and stage (0 visit, 1 first child done, 2 both),
-           and the least |x - target.x|, |y - target.y| of the subtree's
-           region known from the split planes above it */
-        /* frame j holds a node of depth j: node | stage << 28 */
-        int st[kKdMaxDepth + 2];
-        float2 stb[kKdMaxDepth + 2];
-        st[0] = 0;
-        stb[0] = make_float2(0.0f, 0.0f);
-        int sp = 1;
-        while (sp > 0) {
-            const int node = st[sp - 1] & 0x0fffffff;
-            const int depth = sp - 1;
-            const int stage = st[sp - 1] >> 28;
-            if (stage == 0) {
-                if (depth > max_depth) {
-                    sp--;
-                    continue;
-                }
-                /* the node's slot and its position (tree order, loaded
-                   side by side) */
-                const int cur = a.tree[node];
-                const V2 cp = a.tree_pos[node];
-                if (cur == -1) {
-                    sp--;
-                    continue;
-                }
-                /* Once k are found, visiting a node changes nothing unless
-                   d < nd[0]; every node of this subtree has
-                   d >= bx^2 + by^2 (rounding is monotonic), so when that
-                   bound reaches nd[0] the whole subtree is visited by the
-                   reference without effect and is skipped here. */
-                if (kfound == k) {
-                    const float bx = stb[sp - 1].x, by = stb[sp - 1].y;
-                    if (bx * bx + by * by >= nd[0]) {
-                        sp--;
-                        continue;
-                    }
-                }
-                const float dx = cp.x - target.x, dy = cp.y - target.y;
-                const float d = dx * dx + dy * dy;
+        unsigned todo = 0u; /* depths of the far children to come back to */
+        int node = 0;
+        /* the least |x - target.x|, |y - target.y| of the node's region known
+           from the split lines above it */
+        float bx = 0.0f, by = 0.0f;
+        bool run = i < n;
+        while (__any_sync(0xffffffffu, run)) {
+            const int depth = 31 - __clz(node + 1);
+            float4 rec = make_float4(0.0f, 0.0f, __int_as_float(-1), 0.0f);
+            if (run && depth <= max_depth) rec = a.tree_pos[node];
+            const int cur = __float_as_int(rec.z);
+            /* Once k are found, visiting a node changes nothing unless
+               d < nd[0]; every node of this subtree has d >= bx^2 + by^2
+               (rounding is monotonic), so when that bound reaches nd[0] the
+               whole subtree is visited by the reference without effect and
+               is skipped here. */
+            const bool visit = cur != -1 && !(kfound == k && bx * bx + by * by >= first);
+            const float dx = rec.x - target.x, dy = rec.y - target.y;
+            const float d = dx * dx + dy * dy;
+            /* fill slot kfound, or replace slot 0; then the largest entry (the
+               first one, if above d) moves to slot 0 and d takes its place */
+            bool full = false;
+            int li = 0; /* where d is going */
+            if (visit) {
                 if (kfound < k && d > 1e-4f) {
-                    ni[kfound] = cur;
-                    nd[kfound] = d;
-                    kfound++;
-                    if (kfound == k) {
-                        float largest = d;
-                        int li = k - 1;
-                        for (int q = 0; q < k - 1; q++)
-                            if (nd[q] > largest) {
-                                largest = nd[q];
-                                li = q;
-                            }
-                        nd[0] = largest;
-                        ni[0] = ni[li];
-                        nd[li] = d;
-                        ni[li] = cur;
-                    }
+                    li = kfound++;
+                    nd[li][lane] = d;
+                    ni[li][lane] = cur;
+                    if (li == 0) first = d;
+                    if (li == k - 1) last = d;
+                    full = kfound == k;
                 } else {
                     kfound = k;
-                    if (d < nd[0] && d > 1e-4f) {
-                        nd[0] = d;
-                        ni[0] = cur;
-                        float largest = d;
-                        int li = 0;
-                        for (int q = 1; q < k; q++)
-                            if (nd[q] > largest) {
-                                largest = nd[q];
-                                li = q;
-                            }
-                        nd[0] = largest;
-                        ni[0] = ni[li];
-                        nd[li] = d;
-                        ni[li] = cur;
+                    full = d < first && d > 1e-4f;
+                }
+            }
+            if (full) {
+                float lg = d;
+                /* a replaced slot 0 is out of the search, a filled slot k - 1
+                   is not above d */
+                const int q0 = li == 0 ? 1 : 0;
+                if (K <= 16) {
+#pragma unroll
+                    for (int q = 0; q < K; q++) {
+                        const float x = q >= q0 && q < k ? nd[q][lane] : 0.0f;
+                        if (x > lg) {
+                            lg = x;
+                            li = q;
+                        }
+                    }
+                } else {
+                    for (int q = q0; q < k; q++) {
+                        const float x = nd[q][lane];
+                        if (x > lg) {
+                            lg = x;
+                            li = q;
+                        }
                     }
                 }
-                const float cv = (depth & 1) == 0 ? cp.x : cp.y;
-                const float tv = (depth & 1) == 0 ? target.x : target.y;
-                st[sp - 1] = node | (1 << 28);
-                st[sp] = tv < cv ? 2 * node + 1 : 2 * node + 2;
-                stb[sp] = stb[sp - 1]; /* the near side: no new bound */
-                sp++;
-            } else if (stage == 1) {
-                const V2 cp = a.tree_pos[node];
-                const float cv = (depth & 1) == 0 ? cp.x : cp.y;
-                const float tv = (depth & 1) == 0 ? target.x : target.y;
-                const float db = tv - cv;
-                if (db * db < nd[k - 1]) {
-                    st[sp - 1] = node | (2 << 28);
-                    st[sp] = tv < cv ? 2 * node + 2 : 2 * node + 1;
-                    /* the far side: at least |db| away along this axis */
-                    float2 b = stb[sp - 1];
-                    if ((depth & 1) == 0) b.x = fmaxf(b.x, fabsf(db));
-                    else b.y = fmaxf(b.y, fabsf(db));
-                    stb[sp] = b;
-                    sp++;
-                } else {
-                    sp--;
-                }
-            } else {
-                sp--;
+                const int ln = lg > d ? ni[li][lane] : cur;
+                nd[0][lane] = lg;
+                ni[0][lane] = ln;
+                first = lg;
+                nd[li][lane] = d;
+                ni[li][lane] = cur;
+                if (li == 0) first = d;
+                if (li == k - 1) last = d;
             }
+            __syncwarp();
+            if (visit) {
+                const bool x_axis = (depth & 1) == 0;
+                const float db = x_axis ? target.x - rec.x : target.y - rec.y;
+                if (depth < max_depth) { /* a child on each side at most */
+                    /* the far side: at least |db| away along the axis; the
+                       bounds rounded down to 16 bits */
+                    const float fx = x_axis ? fmaxf(bx, fabsf(db)) : bx, fy = x_axis ? by : fmaxf(by, fabsf(db));
+                    far[(depth + 1) * 32] = make_float2(
+                        db, __uint_as_float((__float_as_uint(fx) & 0xffff0000u) | (__float_as_uint(fy) >> 16)));
+                    todo |= 2u << depth;
+                }
+                node = db < 0.0f ? 2 * node + 1 : 2 * node + 2; /* the near side: no new bound */
+            } else if (run) {
+                /* back to the last far child that is still within reach */
+                run = false;
+                while (todo && !run) {
+                    const int at = 31 - __clz(todo);
+                    todo ^= 1u << at;
+                    const float2 e = far[at * 32];
+                    if (e.x * e.x < last) {
+                        run = true;
+                        node = (((node + 1) >> (depth - at)) ^ 1) - 1;
+                        bx = __uint_as_float(__float_as_uint(e.y) & 0xffff0000u);
+                        by = __uint_as_float(__float_as_uint(e.y) << 16);
+                    }
+                }
+            }
+            __syncwarp();
         }
-        int* m = a.map + (size_t)agent * k;
-        for (int q = 0; q < k; q++) m[q] = ni[q];
-        a.kfound[agent] = kfound;
+        /* rows of the warp's 32 agents, coalesced; a row with a reference to
+           the list before it is open */
+        bool open = false;
+        for (int q = 0; q < k; q++) open |= ni[q][lane] < 0;
+        if (i < n) {
+            a.ncnt[i] = kfound;
+            a.open[i] = open ? 1 : 0;
+        }
+        int* out = a.nbr + (size_t)i0 * k;
+        const int cnt = min(32, n - i0) * k;
+        for (int e = lane; e < cnt; e += 32) out[e] = ni[e % k][e / k];
+        __syncwarp();
     }
 }
 
@@ -495,99 +739,134 @@ __device__ __forceinline__ bool querying(const KdArgs& a, int s)
     return a.mark[s] && a.active[s];
 }
 
-/* one warp per block of kComposeSlots slots, lane q = cache slot q: local
-   prefix maps (in place) and the block's map.  The rows of 32 slots at a
-   time are staged in shared memory, so that the sequential chain runs on
-   shared memory. */
-__global__ void __launch_bounds__(32) k_kd_compose_local(KdArgs a)
+/* rows of level 0 (slots) in use, and of the levels above it: a row of level
+   l + 1 is the composition of kFold rows of level l */
+__device__ __forceinline__ int fold_rows(const KdArgs& a, int level)
 {
-    __shared__ int rows[32][kMaxK];
-    __shared__ int use[32];
-    const int q = threadIdx.x;
-    const int k = a.k;
-    const int last = a.counters[C_LAST];
-    const int s0 = blockIdx.x * kComposeSlots;
-    const int s1 = min(s0 + kComposeSlots, last + 1);
-    int cur = -(q + 1);
-    for (int c0 = s0; c0 < s1; c0 += 32) {
-        const int cn = min(32, s1 - c0);
-        use[q] = q < cn && querying(a, c0 + q);
-        __syncwarp();
+    int n = a.counters[C_LAST] + 1;
+    for (int l = 0; l < level; l++) n = (n + kFold - 1) / kFold;
+    return n;
+}
+
+/* the rows of a level (level 0: the slots' maps, kept in grid order): in groups
+   of kFold, each row becomes the composition of its group up to it, the
+   group's the row of the next level.  A warp per group, lane q = cache slot q;
+   the sequential chain runs on shared memory and is only kFold long (one warp
+   per 1,024 rows and one over the blocks took 504 us at 250,000 agents). */
+constexpr int kFoldWarps = 4;
+__global__ void __launch_bounds__(32 * kFoldWarps) k_kd_fold(KdArgs a, int level, int* rows, int* out)
+{
+    __shared__ int sm[kFoldWarps][32 * kMaxK];
+    const int q = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int k = a.k, n = fold_rows(a, level);
+    int* row = sm[w];
+    for (int g = blockIdx.x * kFoldWarps + w; g * kFold < n; g += gridDim.x * kFoldWarps) {
+        const int s1 = min((g + 1) * kFold, n);
+        int cur = -(q + 1);
+        for (int c0 = g * kFold; c0 < s1; c0 += 32) {
+            const int cn = min(32, s1 - c0);
+            bool mine = q < cn, mine_open = true;
+            int at = c0 + q; /* the lane's row */
+            if (level == 0) {
+                mine = mine && querying(a, c0 + q);
+                at = mine ? a.gidx[c0 + q] : 0;
+                mine_open = mine && a.open[at];
+            }
+            const unsigned use = __ballot_sync(0xffffffffu, mine);
+            const unsigned refers = __ballot_sync(0xffffffffu, mine && mine_open);
+            /* 32 rows of k entries, 32 entries at a time */
+            int j = q / k, x = q - j * k;
+            const int dj = 32 / k, dx = 32 - dj * k;
 #pragma unroll 8
-        for (int j = 0; j < cn; j++)
-            if (use[j] && q < k) rows[j][q] = a.map[(size_t)(c0 + j) * k + q];
-        __syncwarp();
-        for (int j = 0; j < cn; j++) {
-            if (!use[j]) continue;
-            int v = q < k ? rows[j][q] : -(q + 1);
-            const int src = v < 0 ? -v - 1 : q;
-            const int got = __shfl_sync(0xffffffffu, cur, src);
-            if (v < 0) v = got;
-            cur = v;
-            if (q < k) rows[j][q] = v;
+            for (int i = 0; i < k; i++) {
+                const int t = __shfl_sync(0xffffffffu, at, j);
+                if ((use >> j) & 1u) row[i * 32 + q] = rows[(size_t)t * k + x];
+                j += dj;
+                x += dx;
+                if (x >= k) {
+                    x -= k;
+                    j++;
+                }
+            }
+            __syncwarp();
+            for (unsigned left = use; left; left &= left - 1u) {
+                const int r = __ffs(left) - 1;
+                int v = q < k ? row[r * k + q] : 0;
+                if ((refers >> r) & 1u) {
+                    const int got = __shfl_sync(0xffffffffu, cur, v < 0 ? -v - 1 : q);
+                    if (v < 0) v = got;
+                    if (q < k) row[r * k + q] = v;
+                }
+                cur = v;
+            }
+            __syncwarp();
+            j = q / k;
+            x = q - j * k;
+#pragma unroll 4
+            for (int i = 0; i < k; i++) {
+                const int t = __shfl_sync(0xffffffffu, at, j);
+                if ((refers >> j) & 1u) rows[(size_t)t * k + x] = row[i * 32 + q];
+                j += dj;
+                x += dx;
+                if (x >= k) {
+                    x -= k;
+                    j++;
+                }
+            }
+            __syncwarp();
         }
-        __syncwarp();
-#pragma unroll 8
-        for (int j = 0; j < cn; j++)
-            if (use[j] && q < k) a.map[(size_t)(c0 + j) * k + q] = rows[j][q];
-        __syncwarp();
+        if (q < k) out[(size_t)g * k + q] = cur;
     }
-    if (q < k) a.agg[(size_t)blockIdx.x * k + q] = cur;
 }
 
-/* one warp: the list each block starts from, and the cache the next tick
-   starts from (block maps staged 32 at a time) */
-__global__ void __launch_bounds__(32) k_kd_compose_top(KdArgs a, int nblk)
+/* entry -v - 1 of the list that slot group b starts from: the rows before b in
+   its group of the next level, then of the level above that, ..., then the
+   cache the tick started with (a slot: its grid index, or -(slot + 1) for one
+   that is not in this tick's grid) */
+__device__ __forceinline__ int fold_resolve(const KdArgs& a, int v, int b)
 {
-    __shared__ int rows[32][kMaxK];
+    const int* rows = a.agg;
+    int n = (a.max_slots + kFold - 1) / kFold;
+    while (v < 0) {
+        if (b == 0) {
+            const int c = a.cache[-v - 1];
+            return a.mark[c] ? a.gidx[c] : -(c + 1);
+        }
+        if (b % kFold) v = rows[(size_t)(b - 1) * a.k + (-v - 1)];
+        rows += (size_t)n * a.k;
+        n = (n + kFold - 1) / kFold;
+        b /= kFold;
+    }
+    return v;
+}
+
+/* the cache the next tick starts from: the composition of all rows (`total`)
+   on this tick's */
+__global__ void k_kd_cache(KdArgs a, const int* total)
+{
     const int q = threadIdx.x;
-    const int k = a.k;
-    const int last = a.counters[C_LAST];
-    const int used = last < 0 ? 0 : min(nblk, last / kComposeSlots + 1);
-    int prev = q < k ? a.cache[q] : 0;
-    for (int c0 = 0; c0 < used; c0 += 32) {
-        const int cn = min(32, used - c0);
-        for (int j = 0; j < cn; j++)
-            if (q < k) rows[j][q] = a.agg[(size_t)(c0 + j) * k + q];
-        __syncwarp();
-        for (int j = 0; j < cn; j++) {
-            if (q < k) a.prev_in[(size_t)(c0 + j) * k + q] = prev;
-            const int v = q < k ? rows[j][q] : -(q + 1);
-            const int src = v < 0 ? -v - 1 : q;
-            const int got = __shfl_sync(0xffffffffu, prev, src);
-            prev = v < 0 ? got : v;
-        }
-        __syncwarp();
-    }
-    if (q < k) a.cache[q] = prev;
+    if (q >= a.k || a.counters[C_LAST] < 0) return;
+    const int v = total[q];
+    const int c = v < 0 ? a.cache[-v - 1] : a.s_slot[v];
+    __syncwarp(__activemask());
+    a.cache[q] = c;
 }
 
-/* grid index of every slot (members), -(slot + 1) for the others */
-__global__ void k_kd_gidx(KdArgs a)
-{
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < a.max_slots; s += gridDim.x * blockDim.x)
-        a.iscan[s] = a.mark[s] ? a.cell_start[a.slot_bucket[s]] + a.slot_rank[s] : -(s + 1);
-}
-
-/* final lists -> the per-agent kernel's inputs (grid order): a neighbour in
-   this tick's grid by its grid index, any other slot as -(slot + 1) */
+/* the open rows' references, looked up: the per-agent kernel's inputs (grid
+   order; a neighbour in this tick's grid by its grid index, any other slot as
+   -(slot + 1)) */
 __global__ void k_kd_emit(KdArgs a)
 {
-    const int k = a.k;
-    const int last = a.counters[C_LAST];
-    const int* gidx = a.iscan;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s <= last; s += gridDim.x * blockDim.x) {
-        if (!querying(a, s)) continue;
-        const int t = gidx[s];
-        const int b = s / kComposeSlots;
-        const int cnt = a.kfound[s];
-        int* out = a.nbr + (size_t)t * k;
-        for (int q = 0; q < cnt; q++) {
-            int v = a.map[(size_t)s * k + q];
-            if (v < 0) v = a.prev_in[(size_t)b * k + (-v - 1)];
-            out[q] = gidx[v];
+    const int k = a.k, n = a.counters[C_NSORTED];
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        if (!a.open[t]) continue;
+        const int slot = a.s_slot[t];
+        if (!a.active[slot]) continue;
+        int* row = a.nbr + (size_t)t * k;
+        for (int q = 0; q < k; q++) {
+            const int v = row[q];
+            if (v < 0) row[q] = fold_resolve(a, v, slot / kFold);
         }
-        a.ncnt[t] = cnt;
     }
 }
 
@@ -600,7 +879,31 @@ int grid_n(int n, int threads, int sms)
 
 }  // namespace
 
-int kd_compose_blocks(int max_slots) { return (max_slots + kComposeSlots - 1) / kComposeSlots; }
+/* rows of the composition's levels above the slots, together */
+int kd_compose_rows(int max_slots)
+{
+    int n = max_slots, total = 0;
+    do {
+        n = (n + kFold - 1) / kFold;
+        total += n;
+    } while (n > 1);
+    return total;
+}
+/* levels over the whole lists: at least the first (its own order), then until a
+   segment fits a block */
+static int kd_top(int cap)
+{
+    int top = 1;
+    while ((cap >> top) > kKdSmall) top++;
+    return top;
+}
+/* launches of the build, the query and the composition */
+int kd_kernels(int max_slots)
+{
+    int fold = 0;
+    for (int n = max_slots; fold == 0 || n > 1; fold++) n = (n + kFold - 1) / kFold;
+    return 6 + 3 * 13 + 1 + 5 * kd_top(max_slots) + 4 + 1 + 2 + fold + 2;
+}
 int kd_hist_ints(int cap) { return 256 * ((cap + kRsTile - 1) / kRsTile); }
 int kd_scan_tmp(int n) { return (n + kScanTile - 1) / kScanTile + 1; }
 
@@ -617,56 +920,52 @@ cudaError_t kd_build_and_query(const KdArgs& a, cudaStream_t s, int sms)
     e = scan_excl<int>(a.iscan, a.max_slots, a.scan_tmp32, s);
     if (e != cudaSuccess) return e;
     k_kd_compact<<<gs, 256, 0, s>>>(a, a.iscan, a.ids0);
-    /* X0 = (x, index); Y = (y, x, index) sorted from X0 */
+    /* X0 = (x, index); Y = (y, x, index) sorted from X0; X = (x, y, index)
+       sorted from Y (equal x keep Y's order, and equal x and y the index's) */
     k_kd_keys<<<gc, 256, 0, s>>>(a, a.ids0, 0, a.keys, a.X0);
-    e = radix_sort(a.keys, a.X0, a.ktmp, a.vtmp, a.n_dev, a.cap, a.hist, a.scan_tmp32, s);
+    e = radix_sort(a.keys, a.X0, a.ktmp, a.vtmp, a.n_dev, a.cap, a.hist, s);
     if (e != cudaSuccess) return e;
     k_kd_keys<<<gc, 256, 0, s>>>(a, a.X0, 1, a.keys, a.Y[0]);
-    e = radix_sort(a.keys, a.Y[0], a.ktmp, a.vtmp, a.n_dev, a.cap, a.hist, a.scan_tmp32, s);
+    e = radix_sort(a.keys, a.Y[0], a.ktmp, a.vtmp, a.n_dev, a.cap, a.hist, s);
     if (e != cudaSuccess) return e;
-    /* X = (x, y, index) sorted from (y, index) */
-    k_kd_keys<<<gc, 256, 0, s>>>(a, a.ids0, 1, a.keys, a.X[1]);
-    e = radix_sort(a.keys, a.X[1], a.ktmp, a.vtmp, a.n_dev, a.cap, a.hist, a.scan_tmp32, s);
-    if (e != cudaSuccess) return e;
-    k_kd_keys<<<gc, 256, 0, s>>>(a, a.X[1], 0, a.keys, a.X[0]);
-    e = radix_sort(a.keys, a.X[0], a.ktmp, a.vtmp, a.n_dev, a.cap, a.hist, a.scan_tmp32, s);
+    k_kd_keys<<<gc, 256, 0, s>>>(a, a.Y[0], 0, a.keys, a.X[0]);
+    e = radix_sort(a.keys, a.X[0], a.ktmp, a.vtmp, a.n_dev, a.cap, a.hist, s);
     if (e != cudaSuccess) return e;
     k_kd_seg_init<<<gc, 256, 0, s>>>(a);
-    /* level 0 splits on X0 and partitions X and Y; then Y / X alternate */
+    /* level 0 splits on X0 and partitions X and Y; then Y / X alternate; from
+       level `top` on a segment is one block's */
     int xi = 0, yi = 0;
-    for (int lv = 0; lv < a.levels; lv++) {
-        if (lv == 0) {
-            k_kd_side<<<gc, 256, 0, s>>>(a, a.X0);
-            k_kd_lrflags<<<gc, 256, 0, s>>>(a, a.X[xi]);
-            e = scan_excl<unsigned long long>(a.flags, a.cap, a.scan_tmp64, s);
-            if (e != cudaSuccess) return e;
-            k_kd_partition<<<gc, 256, 0, s>>>(a, a.X[xi], a.X[xi ^ 1], 0);
+    const int top = kd_top(a.cap);
+    for (int lv = 0; lv < top; lv++) {
+        const bool on_y = (lv & 1) != 0;
+        k_kd_side<<<gc, 256, 0, s>>>(a, lv == 0 ? a.X0 : (on_y ? a.Y[yi] : a.X[xi]));
+        if (lv == 0 || on_y) {
+            e = kd_partition(a, a.X[xi], a.X[xi ^ 1], lv == 0 ? 0 : 1, gc, s);
             xi ^= 1;
-            k_kd_lrflags<<<gc, 256, 0, s>>>(a, a.Y[yi]);
-            e = scan_excl<unsigned long long>(a.flags, a.cap, a.scan_tmp64, s);
-            if (e != cudaSuccess) return e;
-            k_kd_partition<<<gc, 256, 0, s>>>(a, a.Y[yi], a.Y[yi ^ 1], 1);
-            yi ^= 1;
-        } else {
-            const bool on_y = (lv & 1) != 0;
-            const int* A = on_y ? a.Y[yi] : a.X[xi];
-            k_kd_side<<<gc, 256, 0, s>>>(a, A);
-            if (lv + 1 < a.levels) {
-                const int* B = on_y ? a.X[xi] : a.Y[yi];
-                int* Bout = on_y ? a.X[xi ^ 1] : a.Y[yi ^ 1];
-                k_kd_lrflags<<<gc, 256, 0, s>>>(a, B);
-                e = scan_excl<unsigned long long>(a.flags, a.cap, a.scan_tmp64, s);
-                if (e != cudaSuccess) return e;
-                k_kd_partition<<<gc, 256, 0, s>>>(a, B, Bout, 1);
-                if (on_y) xi ^= 1;
-                else yi ^= 1;
-            }
         }
+        if (e == cudaSuccess && !on_y) {
+            e = kd_partition(a, a.Y[yi], a.Y[yi ^ 1], 1, gc, s);
+            yi ^= 1;
+        }
+        if (e != cudaSuccess) return e;
     }
+    e = cudaFuncSetAttribute(k_kd_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KdSmallSm));
+    if (e != cudaSuccess) return e;
+    k_kd_small<<<1 << top, kSmallThreads, sizeof(KdSmallSm), s>>>(a, a.X[xi], a.Y[yi], top, a.iscan);
     /* queries in grid order: the agents of a warp are neighbours, so their
        traversals share nodes in cache */
     k_kd_tree_pos<<<grid_n(a.tree_cap, 256, sms), 256, 0, s>>>(a);
-    k_kd_query<<<grid_n(a.cap, 128, sms), 128, 0, s>>>(a, a.s_slot);
+    const int gq = grid_n(a.cap, 128, sms);
+    /* at most 25 levels (2^24 slots): 25.6 KB beside the lists' 33.8 KB at
+       K = 32, above the default limit of 48 KB only there */
+    const size_t far = sizeof(float2) * 32 * kQueryWarps * (size_t)a.levels;
+    if (a.k <= 8) k_kd_query<8><<<gq, 32 * kQueryWarps, far, s>>>(a, a.s_slot);
+    else if (a.k <= 16) k_kd_query<16><<<gq, 32 * kQueryWarps, far, s>>>(a, a.s_slot);
+    else {
+        e = cudaFuncSetAttribute(k_kd_query<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * 1024);
+        if (e != cudaSuccess) return e;
+        k_kd_query<32><<<gq, 32 * kQueryWarps, far, s>>>(a, a.s_slot);
+    }
     return cudaGetLastError();
 }
 
@@ -674,11 +973,19 @@ cudaError_t kd_build_and_query(const KdArgs& a, cudaStream_t s, int sms)
    of the per-agent kernel */
 cudaError_t kd_finish(const KdArgs& a, cudaStream_t s, int sms)
 {
-    const int nblk = kd_compose_blocks(a.max_slots);
-    k_kd_compose_local<<<nblk, 32, 0, s>>>(a);
-    k_kd_compose_top<<<1, 32, 0, s>>>(a, nblk);
-    k_kd_gidx<<<grid_n(a.max_slots, 256, sms), 256, 0, s>>>(a);
-    k_kd_emit<<<grid_n(a.max_slots, 256, sms), 256, 0, s>>>(a);
+    int* rows = a.nbr;
+    int* out = a.agg;
+    int n = a.max_slots, level = 0;
+    do {
+        const int m = (n + kFold - 1) / kFold;
+        k_kd_fold<<<grid_n(m, kFoldWarps, sms), 32 * kFoldWarps, 0, s>>>(a, level, rows, out);
+        rows = out;
+        out += (size_t)m * a.k;
+        n = m;
+        level++;
+    } while (n > 1);
+    k_kd_emit<<<grid_n(a.cap, 256, sms), 256, 0, s>>>(a);
+    k_kd_cache<<<1, 32, 0, s>>>(a, rows);
     return cudaGetLastError();
 }
 
