@@ -1838,14 +1838,19 @@ static ecmg_status ensure_grids(ecmg_ctx* c)
    Measured (per-agent kernel, us; 1 / 4 / 8 / 16 / 32 lanes): 1,000 agents of
    the box scene 42 / 23 / 20 / 19 / 18; 25,000 there 59 / 33 / 32 / 38 / 51;
    crossing 30,000 93 / 45 / 45 / 50 / 64; 100,000 174 / 121 / 138 / 174 / 243;
-   300,000 249 / 264 / 322 / 434 / 672; 1,000,000 385 / 599 / ... -- so 4 lanes
-   up to 200,000 agents (8 where a handful of warps is all there is). */
+   300,000 249 / 264 / 322 / 434 / 672; 1,000,000 385 / 599 / ... .  The line
+   between 1 and 4 lies at 230,000 agents in the 400 m crossing (200,000: 227
+   and 218) and at 160,000 at the density of its million (125,000 in 200 m: 176
+   and 156; 180,000: 173 and 192).  The kd-tree mode's lists are not in order
+   of distance, which costs a thread's constraint loop its coherence: 4 lanes
+   there (250,000 agents: 422 and 347). */
 static int lanes_of(ecmg_ctx* c)
 {
     if (c->lp_mode == ECMG_LP_WARP)
         return c->wgrab >= 8 ? 4 : (c->wgrab >= 4 ? 8 : (c->wgrab >= 2 ? 16 : 32));
     if (c->lp_mode != ecmg_ctx::kLpAuto) return 1;
-    return c->lanes_agents <= 8000 ? 8 : (c->lanes_agents <= 200000 ? 4 : 1);
+    if (c->lanes_agents <= 8000) return 8;
+    return c->lanes_agents <= 160000 || c->nbr_mode == ECMG_NEIGHBORS_KDTREE ? 4 : 1;
 }
 
 /* the automatic layout follows the agent count; a count within a factor of
@@ -2048,11 +2053,11 @@ void* ecmg_stream(const ecmg_ctx* c) { return c ? (void*)c->stream : nullptr; }
 
 int ecmg_kernels_per_tick(const ecmg_ctx* c)
 {
-    /* k_bin, k_scan, k_scatter, k_attract, k_neighbors, k_agents (or
-       k_agents_group); k_features with a proposal model or a trace;
-       k_mlp_infer with a proposal model */
+    /* the binning (k_bin, k_scan, k_scatter, or k_bin_small), k_attract,
+       k_neighbors, k_agents (or k_agents_group); k_features with a proposal
+       model or a trace; k_mlp_infer with a proposal model */
     if (!c) return 6;
-    int n = 6 + ((c->model || c->trace) ? 1 : 0) + (c->model ? 1 : 0);
+    int n = bin_kernels(c->total_buckets, c->max_agents) + 3 + ((c->model || c->trace) ? 1 : 0) + (c->model ? 1 : 0);
     /* kd-tree mode, instead of k_neighbors */
     if (c->nbr_mode == ECMG_NEIGHBORS_KDTREE) n += -1 + kd_kernels(c->max_agents);
     return n;

@@ -160,6 +160,7 @@ struct BinArgs {
     const SceneDev* scenes;   /* batch: per-scene grid and bucket base */
     const int* slot_scene;
     int total_buckets;        /* sum over scenes of their cells */
+    int* out_cnt;             /* stand-alone kNN: its counts (the inactive slots' are zeroed), else null */
     int n_fixed;              /* > 0: bin slots [0, n_fixed) (stand-alone kNN); 0: [0, counters[C_LAST]] */
 };
 
@@ -189,6 +190,7 @@ cudaError_t launch_knn(const V2* pos, const unsigned char* active, int n, int k,
                        int* key, int* rank, int* cell_count, int* cell_start, int* s_slot, V2* s_pos,
                        int* scan_tmp, int scan_blocks, int* out_ids, int* out_cnt, cudaStream_t s);
 int scan_tmp_ints(int n);
+int bin_kernels(int total_buckets, int slots); /* launches of the binning */
 /* kernels.cu: mark the agents of `list` pending (before the tick's graph);
    after the graph and the upload of their paths, their attraction and ORCA
    step of the tick (k_fixup) */

@@ -32,7 +32,10 @@ __global__ void k_bin(BinArgs a)
 {
     const int last = a.n_fixed > 0 ? a.n_fixed - 1 : a.counters[C_LAST];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= last; i += gridDim.x * blockDim.x) {
-        if (!a.active[i]) continue;
+        if (!a.active[i]) {
+            if (a.out_cnt) a.out_cnt[i] = 0;
+            continue;
+        }
         int b;
         if (a.scenes) {
             const SceneDev& sc = a.scenes[a.slot_scene ? a.slot_scene[i] : 0];
@@ -138,9 +141,87 @@ __global__ void k_scatter(BinArgs a)
     if (t0 == 0) a.cell_start[a.total_buckets] = a.counters[C_NSORTED];
 }
 
-/* counts (zero) -> bins, starts and snapshot */
-static cudaError_t launch_bin(const BinArgs& b, int blocks, cudaStream_t s)
+/* the whole binning of up to kSmallSlots slots by one block, the counts in
+   shared memory: below that size the three launches' latency is all there is
+   (1,000 agents: three launches 12 us of the tick, this 5) */
+constexpr int kSmallSlots = 8192, kSmallCells = 11264, kSmallBlock = 1024;
+__global__ void __launch_bounds__(kSmallBlock) k_bin_small(BinArgs a)
 {
+    constexpr int R = kSmallSlots / kSmallBlock, C = kSmallCells / kSmallBlock;
+    __shared__ int count[kSmallCells];
+    __shared__ int sh[32];
+    const int last = a.n_fixed > 0 ? a.n_fixed - 1 : a.counters[C_LAST];
+    for (int c = threadIdx.x; c < kSmallCells; c += kSmallBlock) count[c] = 0;
+    __syncthreads();
+    int bucket[R], rank[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int i = r * kSmallBlock + threadIdx.x;
+        bucket[r] = -1;
+        rank[r] = 0;
+        if (i > last) continue;
+        if (!a.active[i]) {
+            if (a.out_cnt) a.out_cnt[i] = 0;
+            continue;
+        }
+        if (a.scenes) {
+            const SceneDev& sc = a.scenes[a.slot_scene ? a.slot_scene[i] : 0];
+            bucket[r] = sc.bucket_base + bucket_of(sc.grid, a.pos[i]);
+        } else {
+            bucket[r] = bucket_of(a.grid, a.pos[i]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (bucket[r] >= 0) rank[r] = atomicAdd(&count[bucket[r]], 1);
+    __syncthreads();
+    int v[C], sum = 0, tot;
+#pragma unroll
+    for (int q = 0; q < C; q++) {
+        v[q] = count[threadIdx.x * C + q]; /* an odd stride: no bank conflicts */
+        sum += v[q];
+    }
+    int run = block_exclusive_scan(sum, sh, &tot);
+#pragma unroll
+    for (int q = 0; q < C; q++) {
+        count[threadIdx.x * C + q] = run;
+        run += v[q];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        if (bucket[r] < 0) continue;
+        const int i = r * kSmallBlock + threadIdx.x;
+        const int d = count[bucket[r]] + rank[r];
+        a.key[i] = bucket[r];
+        a.rank[i] = rank[r];
+        a.s_slot[d] = i;
+        a.s_pos[d] = a.pos[i];
+        if (a.s_vel) a.s_vel[d] = a.vel[i];
+        if (a.s_clear) a.s_clear[d] = a.clear[i];
+    }
+    for (int c = threadIdx.x; c < a.total_buckets; c += kSmallBlock) a.cell_start[c] = count[c];
+    if (threadIdx.x == 0) {
+        a.cell_start[a.total_buckets] = tot;
+        a.counters[C_NSORTED] = tot;
+    }
+}
+
+static bool bins_small(const BinArgs& b, int slots) { return slots <= kSmallSlots && b.total_buckets <= kSmallCells; }
+int bin_kernels(int total_buckets, int slots)
+{
+    BinArgs b{};
+    b.total_buckets = total_buckets;
+    return bins_small(b, slots) ? 1 : 3;
+}
+
+/* counts (zero) -> bins, starts and snapshot */
+static cudaError_t launch_bin(const BinArgs& b, int slots, int blocks, cudaStream_t s)
+{
+    if (bins_small(b, slots)) {
+        k_bin_small<<<1, kSmallBlock, 0, s>>>(b);
+        return cudaGetLastError();
+    }
     k_bin<<<blocks, 256, 0, s>>>(b);
     k_scan<<<(b.total_buckets + kScanTile - 1) / kScanTile, kScanBlock, 0, s>>>(b.cell_count, b.total_buckets,
                                                                               b.block_sums, b.counters);
@@ -711,7 +792,7 @@ cudaError_t launch_tick(const BinArgs& b, const TickArgs& t, int max_slots, int 
     cudaStreamIsCapturing(s, &cap);
     const unsigned evflags = cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : 0u;
     int gb = grid_for(max_slots, 256, sms, 8);
-    cudaError_t e = launch_bin(b, gb, s);
+    cudaError_t e = launch_bin(b, max_slots, gb, s);
     if (e != cudaSuccess) return e;
     /* external event nodes when captured, so that the kernel can be timed */
     if (ev) cudaEventRecordWithFlags(ev[0], s, evflags);
@@ -865,10 +946,6 @@ cudaError_t launch_knn(const V2* pos, const unsigned char* active, int n, int k,
     /* the counters live behind the bucket counts: [nb+1 .. nb+1+kCounters) */
     int nb = g.ncells + 1;
     int* counters = cell_count + nb + 1;
-    cudaError_t e = cudaMemsetAsync(cell_count, 0, sizeof(int) * (size_t)(nb + 1 + kCounters), s);
-    if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(out_cnt, 0, sizeof(int) * (size_t)n, s);
-    if (e != cudaSuccess) return e;
     /* the slot range is passed by value: the query queues no host-to-device copy */
     BinArgs b{};
     b.n_fixed = n;
@@ -884,7 +961,10 @@ cudaError_t launch_knn(const V2* pos, const unsigned char* active, int n, int k,
     b.grid = g;
     b.total_buckets = g.ncells;
     b.block_sums = scan_tmp;
-    e = launch_bin(b, (n + 255) / 256, s);
+    b.out_cnt = out_cnt; /* zero for the inactive */
+    cudaError_t e = cudaSuccess;
+    if (!bins_small(b, n)) e = cudaMemsetAsync(cell_count, 0, sizeof(int) * (size_t)(nb + 1 + kCounters), s);
+    if (e == cudaSuccess) e = launch_bin(b, n, (n + 255) / 256, s);
     if (e != cudaSuccess) return e;
     const int ga = (n + 32 * kNbrWarps - 1) / (32 * kNbrWarps);
     const float r2 = r * r;
