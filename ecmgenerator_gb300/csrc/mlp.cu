@@ -253,14 +253,19 @@ __device__ __forceinline__ float tanh_approx(float x)
     return y;
 }
 
-/* GELU (tanh form) for inference: the hardware tanh approximation (relative
-   error about 2^-11, below the BF16 rounding of the activations) */
-__device__ __forceinline__ float gelu_fast(float x)
+/* GELU (tanh form) for inference of two values plus their biases: the
+   hardware tanh approximation (relative error about 2^-11, below the BF16
+   rounding of the activations); everything else two values per instruction,
+   the epilogues being bound by their instruction count */
+__device__ __forceinline__ uint32_t gelu_fast2(uint32_t z0, uint32_t z1, float b0, float b1)
 {
     const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-    const float u = k0 * __fmaf_rn(k1 * (x * x), x, x);
-    const float hx = 0.5f * x;
-    return __fmaf_rn(hx, tanh_approx(u), hx);
+    const float2 x = __fadd2_rn(make_float2(__uint_as_float(z0), __uint_as_float(z1)), make_float2(b0, b1));
+    const float2 c = __fmul2_rn(make_float2(k1, k1), __fmul2_rn(x, x));
+    const float2 u = __fmul2_rn(make_float2(k0, k0), __ffma2_rn(c, x, x));
+    const float2 hx = __fmul2_rn(make_float2(0.5f, 0.5f), x);
+    const float2 y = __ffma2_rn(hx, make_float2(tanh_approx(u.x), tanh_approx(u.y)), hx);
+    return pack_bf16(y.x, y.y);
 }
 
 /* 32 consecutive fp32 columns of this thread's lane, one wait */
@@ -387,12 +392,12 @@ __global__ void __launch_bounds__(kInferThreads, 1)
 #pragma unroll
             for (int q = 0; q < 2; q++) {
                 const float4 ba = b4[2 * q], bb = b4[2 * q + 1];
-                const float* v = reinterpret_cast<const float*>(r) + 8 * q;
+                const uint32_t* v = r + 8 * q;
                 uint4 u;
-                u.x = pack_bf16(gelu_fast(v[0] + ba.x), gelu_fast(v[1] + ba.y));
-                u.y = pack_bf16(gelu_fast(v[2] + ba.z), gelu_fast(v[3] + ba.w));
-                u.z = pack_bf16(gelu_fast(v[4] + bb.x), gelu_fast(v[5] + bb.y));
-                u.w = pack_bf16(gelu_fast(v[6] + bb.z), gelu_fast(v[7] + bb.w));
+                u.x = gelu_fast2(v[0], v[1], ba.x, ba.y);
+                u.y = gelu_fast2(v[2], v[3], ba.z, ba.w);
+                u.z = gelu_fast2(v[4], v[5], bb.x, bb.y);
+                u.w = gelu_fast2(v[6], v[7], bb.z, bb.w);
                 *reinterpret_cast<uint4*>(tbuf + tc_off(row, c + 8 * q, kTile)) = u;
             }
         });
@@ -405,12 +410,14 @@ __global__ void __launch_bounds__(kInferThreads, 1)
 #pragma unroll
             for (int i = 0; i < 16; i += 4) {
                 const float4 b = b4[i / 4];
-                const float z0 = __uint_as_float(r[i]) + b.x, z1 = __uint_as_float(r[i + 1]) + b.y;
-                const float z2 = __uint_as_float(r[i + 2]) + b.z, z3 = __uint_as_float(r[i + 3]) + b.w;
-                if (z0 > best) { best = z0; bi = o0 + c + i; }
-                if (z1 > best) { best = z1; bi = o0 + c + i + 1; }
-                if (z2 > best) { best = z2; bi = o0 + c + i + 2; }
-                if (z3 > best) { best = z3; bi = o0 + c + i + 3; }
+                const float2 za = __fadd2_rn(make_float2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])),
+                                             make_float2(b.x, b.y));
+                const float2 zb = __fadd2_rn(make_float2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])),
+                                             make_float2(b.z, b.w));
+                if (za.x > best) { best = za.x; bi = o0 + c + i; }
+                if (za.y > best) { best = za.y; bi = o0 + c + i + 1; }
+                if (zb.x > best) { best = zb.x; bi = o0 + c + i + 2; }
+                if (zb.y > best) { best = zb.y; bi = o0 + c + i + 3; }
             }
         });
     };
@@ -951,7 +958,9 @@ struct ecmg_mlp {
     float* m = nullptr;     /* Adam first moment */
     float* v = nullptr;     /* Adam second moment */
     unsigned char* pack = nullptr; /* BF16 weights in the tensor-core operand layout (inference) */
-    int* derr = nullptr;           /* inference error flag (ecmg_mlp_predict) */
+    int* derr = nullptr;           /* inference error flag (ecmg_mlp_predict), and its page-locked copy */
+    int* h_err = nullptr;
+    int sms = 1;
     int spin = kSpinDefault;       /* polls of an mbarrier before the inference gives up */
     float* bias = nullptr;  /* b1 | b2 | b3 */
     int step = 0;
@@ -1059,13 +1068,17 @@ ecmg_status ecmg_mlp_create(unsigned long long seed, ecmg_mlp** out)
         return ECMG_ERR_NO_DEVICE;
     }
     ecmg_mlp* mm = new ecmg_mlp();
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&mm->sms, cudaDevAttrMultiProcessorCount, dev);
     bool ok = cudaStreamCreateWithFlags(&mm->s, cudaStreamNonBlocking) == cudaSuccess &&
               cudaMalloc(&mm->p, sizeof(float) * NPARAM) == cudaSuccess &&
               cudaMalloc(&mm->g, sizeof(float) * NPARAM) == cudaSuccess &&
               cudaMalloc(&mm->m, sizeof(float) * NPARAM) == cudaSuccess &&
               cudaMalloc(&mm->v, sizeof(float) * NPARAM) == cudaSuccess &&
               cudaMalloc(&mm->pack, (size_t)kWB) == cudaSuccess &&
-              cudaMalloc(&mm->derr, sizeof(int)) == cudaSuccess &&
+              cudaMalloc(&mm->derr, sizeof(int)) == cudaSuccess && cudaMemset(mm->derr, 0, sizeof(int)) == cudaSuccess &&
+              cudaMallocHost(&mm->h_err, sizeof(int)) == cudaSuccess &&
               cudaMalloc(&mm->bias, sizeof(float) * (2 * HID + OUT)) == cudaSuccess;
     if (!ok) {
         ecmg_mlp_destroy(mm);
@@ -1105,6 +1118,7 @@ ecmg_status ecmg_mlp_destroy(ecmg_mlp* mm)
     for (void* d : ds)
         if (d) cudaFree(d);
     if (mm->h_grad) cudaFreeHost(mm->h_grad);
+    if (mm->h_err) cudaFreeHost(mm->h_err);
     if (mm->s) cudaStreamDestroy(mm->s);
     delete mm;
     return ECMG_OK;
@@ -1135,10 +1149,7 @@ ecmg_status ecmg_mlp_set_params(ecmg_mlp* mm, const float* host_in)
 static ecmg_status ensure_train(ecmg_mlp* mm, int steps)
 {
     if (!mm->part) {
-        int dev = 0, sms = 1;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const size_t np = (size_t)sms;
+        const size_t np = (size_t)mm->sms;
         bool ok = cudaMalloc(&mm->part_loss, sizeof(float) * np) == cudaSuccess &&
                   cudaMalloc(&mm->part_ok, sizeof(int) * np) == cudaSuccess &&
                   cudaMalloc(&mm->tpack, (size_t)kWB) == cudaSuccess &&
@@ -1150,7 +1161,7 @@ static ecmg_status ensure_train(ecmg_mlp* mm, int steps)
                       cudaSuccess &&
                   cudaMalloc(&mm->part, sizeof(float) * np * NPARAM) == cudaSuccess;
         if (!ok) return ECMG_ERR_CUDA;
-        mm->parts = sms;
+        mm->parts = mm->sms;
     }
     if (steps > mm->hist) {
         if (mm->hist_loss) cudaFree(mm->hist_loss);
@@ -1254,16 +1265,14 @@ ecmg_status ecmg_mlp_predict(ecmg_mlp* mm, const void* dev_x, int n, unsigned ch
     if (!mm || !dev_x || !dev_cls || n < 0) return ECMG_ERR_INVALID_ARG;
     if (n == 0) return ECMG_OK;
     if (ecmg::mlp_pack(mm) != cudaSuccess) return ECMG_ERR_CUDA;
-    int dev = 0, sms = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaMemsetAsync(mm->derr, 0, sizeof(int), mm->s) != cudaSuccess) return ECMG_ERR_CUDA;
-    if (ecmg::mlp_infer(mm, dev_x, nullptr, n, dev_cls, mm->s, sms, mm->derr, 1) != cudaSuccess) return ECMG_ERR_CUDA;
-    int herr = 0;
-    if (cudaMemcpyAsync(&herr, mm->derr, sizeof(int), cudaMemcpyDeviceToHost, mm->s) != cudaSuccess ||
+    if (ecmg::mlp_infer(mm, dev_x, nullptr, n, dev_cls, mm->s, mm->sms, mm->derr, 1) != cudaSuccess)
+        return ECMG_ERR_CUDA;
+    if (cudaMemcpyAsync(mm->h_err, mm->derr, sizeof(int), cudaMemcpyDeviceToHost, mm->s) != cudaSuccess ||
         cudaStreamSynchronize(mm->s) != cudaSuccess)
         return ECMG_ERR_CUDA;
-    return herr ? ECMG_ERR_BOUND : ECMG_OK;
+    if (*mm->h_err == 0) return ECMG_OK;
+    cudaMemsetAsync(mm->derr, 0, sizeof(int), mm->s); /* the flag is zero between calls */
+    return ECMG_ERR_BOUND;
 }
 
 }  // extern "C"
