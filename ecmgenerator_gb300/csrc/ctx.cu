@@ -230,7 +230,9 @@ struct ecmg_ctx {
     int trace_rows = 0;
     DBuf<unsigned char> feat, cls, label;
     /* pinned staging */
-    int* h_counters = nullptr; /* [3 * kCounters]: in, out, after k_attract */
+    int* h_counters = nullptr; /* [3 * kCounters]: (unused), out, after k_attract */
+    DBuf<int> d_last;          /* the last slot index of the tick's binning, uploaded when it changes */
+    int dev_last = -1;
     void* hview[4] = {nullptr, nullptr, nullptr, nullptr}; /* ecmg_host_view of the float2 fields */
     /* ecmg_set_host_mirror: every tick ends with a copy of the slots it may
        have moved into hview[position] and hview[velocity] (device addresses
@@ -430,6 +432,7 @@ ecmg_status ecmg_create_batch(const ecmg_params* p, int n_scenes, const int* max
     CKC(cudaMemset(c->d_active.p, 0, N)); CKC(cudaMemset(c->path_len.p, 0, sizeof(int) * N));
     CKC(cudaMemset(c->path_off.p, 0, sizeof(int) * N));
     CKC(cudaMemset(c->d_clear.p, 0, sizeof(float) * N)); CKC(cudaMemset(c->d_speed.p, 0, sizeof(float) * N));
+    CKC(c->d_last.alloc(1));
     CKC(cudaHostAlloc((void**)&c->h_counters, sizeof(int) * 3 * kCounters, cudaHostAllocDefault));
     CKC(cudaHostAlloc((void**)&c->h_lists, sizeof(int) * 4 * ecmg_ctx::kListStage, cudaHostAllocDefault));
     c->active.assign(N, 0);
@@ -487,6 +490,7 @@ ecmg_status ecmg_destroy(ecmg_ctx* c)
     c->label.free_();
     c->d_scenes.free_();
     for (auto& s : c->scenes) s->free_all();
+    c->d_last.free_();
     if (c->h_counters) cudaFreeHost(c->h_counters);
     if (c->h_lists) cudaFreeHost(c->h_lists);
     if (c->h_up) cudaFreeHost(c->h_up);
@@ -1882,6 +1886,7 @@ static void fill_args(ecmg_ctx* c, BinArgs& b, TickArgs& t, bool use_model)
     b.s_clear = c->s_clear.p;
     b.cell_start = c->cell_start.p;
     b.counters = c->counters.p;
+    b.last = c->d_last.p;
     b.scenes = c->d_scenes.p;
     b.slot_scene = c->scenes.size() > 1 ? c->d_slot_scene.p : nullptr;
     b.total_buckets = c->total_buckets;
@@ -1996,8 +2001,7 @@ static cudaError_t enqueue_tick(ecmg_ctx* c, int launch_slots, bool use_model)
     TickArgs t;
     fill_args(c, b, t, use_model);
     cudaGetLastError(); /* launch errors below must not be confused with older ones */
-    cudaError_t e = cudaMemcpyAsync(c->counters.p, c->h_counters, sizeof(int) * kCounters, cudaMemcpyHostToDevice, c->stream);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
     if (c->trace) {
         e = cudaMemsetAsync(c->label.p, kClsOther, (size_t)launch_slots, c->stream);
         if (e != cudaSuccess) return e;
@@ -2100,8 +2104,11 @@ static ecmg_status run_ticks(ecmg_ctx* c, int n_ticks, ecmg_tick_stats* stats)
         ecmg_status gs = ensure_grids(c);
         if (gs != ECMG_OK) return gs;
         choose_lanes(c);
-        std::memset(c->h_counters, 0, sizeof(int) * kCounters);
-        c->h_counters[C_LAST] = last;
+        if (last != c->dev_last) { /* the counters themselves start on the device */
+            ecmg_status ls = stage_copy(c, c->d_last.p, &last, sizeof(int));
+            if (ls != ECMG_OK) return ls;
+            c->dev_last = last;
+        }
         const bool use_model = c->model && c->gate_left == 0;
         if (c->model && !use_model) {
             c->gate_left--;
@@ -2273,8 +2280,12 @@ static ecmg_status run_ticks(ecmg_ctx* c, int n_ticks, ecmg_tick_stats* stats)
         if (cudaEventElapsedTime(&tot, c->ev_k[0], c->ev_k[4]) != cudaSuccess) tot = 0;
         if (cudaEventElapsedTime(&att, c->ev_k[0], c->ev_k[1]) != cudaSuccess) att = 0;
         if (cudaEventElapsedTime(&nbr, c->ev_k[0], c->ev_k[2]) != cudaSuccess) nbr = 0;
-        if (cudaEventElapsedTime(&prop, c->ev_k[2], c->ev_k[3]) != cudaSuccess) prop = 0;
-        if (cudaEventElapsedTime(&orca, c->ev_k[3], c->ev_k[4]) != cudaSuccess) orca = 0;
+        if (use_model || c->trace) {
+            if (cudaEventElapsedTime(&prop, c->ev_k[2], c->ev_k[3]) != cudaSuccess) prop = 0;
+            if (cudaEventElapsedTime(&orca, c->ev_k[3], c->ev_k[4]) != cudaSuccess) orca = 0;
+        } else { /* the per-agent kernel starts when both have ended */
+            orca = std::max(0.0f, tot - std::max(att, nbr));
+        }
         cudaGetLastError();
         st.device_ms += ms;
         st.agent_kernel_ms += tot;

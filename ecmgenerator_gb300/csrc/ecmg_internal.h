@@ -35,7 +35,7 @@ constexpr unsigned char kActivePending = 2;
 constexpr int kMlpIn = 96, kMlpHid = 128, kMlpOut = 160, kMlpNbrs = 16;
 constexpr int kClsPref = 0, kClsSingle = 1, kClsPair = 17, kClsCircle = 137, kClsOther = 153;
 
-/* device counters (int[kCounters]) */
+/* device counters (int[kCounters]); the binning starts a tick's at zero */
 enum {
     C_DESTROYED = 0,
     C_REPLAN = 1,
@@ -43,7 +43,7 @@ enum {
     C_ERROR = 3,       /* bitmask of ECMG_DEV_ERR_* */
     C_PROCESSED = 4,   /* agents processed by the per-agent kernel */
     C_WORK = 5,        /* work counter of the persistent agent kernel */
-    C_LAST = 6,        /* last slot index to scan (host-written before the tick) */
+    C_LAST = 6,        /* last slot index of the tick */
     C_NSORTED = 7,     /* agents in the neighbour grid */
     C_PROPOSED = 8,    /* LPs that received a learned proposal */
     C_ACCEPTED = 9,    /* proposals that passed the exact check */
@@ -161,7 +161,8 @@ struct BinArgs {
     const int* slot_scene;
     int total_buckets;        /* sum over scenes of their cells */
     int* out_cnt;             /* stand-alone kNN: its counts (the inactive slots' are zeroed), else null */
-    int n_fixed;              /* > 0: bin slots [0, n_fixed) (stand-alone kNN); 0: [0, counters[C_LAST]] */
+    const int* last;          /* the last slot to bin (n_fixed 0) */
+    int n_fixed;              /* > 0: bin slots [0, n_fixed) (stand-alone kNN); 0: [0, *last] */
 };
 
 /* kernels.cu; propose (may be null) runs between the feature kernel and the
@@ -174,7 +175,8 @@ typedef cudaError_t (*HookFn)(void* user, cudaStream_t s, unsigned evflags);
 /* The attraction kernel runs on s2 beside the neighbour kernel on s (fork and
    join through ev_fork / ev_join).  ev (may be null): five events -- before
    both, after the attraction kernel (on s2), after the neighbour kernel, after
-   the proposal (features + inference) and after the per-agent kernel. */
+   the proposal (features + inference; only where TickArgs::feat is set) and
+   after the per-agent kernel. */
 struct KdArgs;
 /* kd (may be null): the kd-tree neighbour mode replaces the neighbour kernel */
 cudaError_t launch_tick(const BinArgs& b, const TickArgs& t, int max_slots, int block, int sms,

@@ -28,9 +28,18 @@
 
 namespace ecmg {
 
+/* the counters of a tick: zero but for the last slot (the other kernels of
+   the tick start after the binning) */
+__device__ __forceinline__ int start_counters(const BinArgs& a)
+{
+    const int last = a.n_fixed > 0 ? a.n_fixed - 1 : *a.last;
+    if (blockIdx.x == 0 && threadIdx.x < kCounters) a.counters[threadIdx.x] = threadIdx.x == C_LAST ? last : 0;
+    return last;
+}
+
 __global__ void k_bin(BinArgs a)
 {
-    const int last = a.n_fixed > 0 ? a.n_fixed - 1 : a.counters[C_LAST];
+    const int last = start_counters(a);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= last; i += gridDim.x * blockDim.x) {
         if (!a.active[i]) {
             if (a.out_cnt) a.out_cnt[i] = 0;
@@ -126,7 +135,7 @@ int scan_tmp_ints(int n) { return (n + 1023) / 1024 + 32; }
 /* tick-start snapshot in grid order, and the final bucket starts */
 __global__ void k_scatter(BinArgs a)
 {
-    const int last = a.n_fixed > 0 ? a.n_fixed - 1 : a.counters[C_LAST];
+    const int last = a.counters[C_LAST];
     const int t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
     for (int i = t0; i <= last; i += step) {
         if (!a.active[i]) continue;
@@ -150,7 +159,7 @@ __global__ void __launch_bounds__(kSmallBlock) k_bin_small(BinArgs a)
     constexpr int R = kSmallSlots / kSmallBlock, C = kSmallCells / kSmallBlock;
     __shared__ int count[kSmallCells];
     __shared__ int sh[32];
-    const int last = a.n_fixed > 0 ? a.n_fixed - 1 : a.counters[C_LAST];
+    const int last = start_counters(a);
     for (int c = threadIdx.x; c < kSmallCells; c += kSmallBlock) count[c] = 0;
     __syncthreads();
     int bucket[R], rank[R];
@@ -856,7 +865,7 @@ cudaError_t launch_tick(const BinArgs& b, const TickArgs& t, int max_slots, int 
             if (e2 != cudaSuccess) return e2;
         }
     }
-    if (ev) cudaEventRecordWithFlags(ev[3], s, evflags);
+    if (ev && t.feat) cudaEventRecordWithFlags(ev[3], s, evflags);
     if (t.lanes > 1) {
         const bool full = t.cls || t.cls_slot || t.label || t.rec_cnt;
         auto go = [&](auto kern) {
@@ -963,7 +972,7 @@ cudaError_t launch_knn(const V2* pos, const unsigned char* active, int n, int k,
     b.block_sums = scan_tmp;
     b.out_cnt = out_cnt; /* zero for the inactive */
     cudaError_t e = cudaSuccess;
-    if (!bins_small(b, n)) e = cudaMemsetAsync(cell_count, 0, sizeof(int) * (size_t)(nb + 1 + kCounters), s);
+    if (!bins_small(b, n)) e = cudaMemsetAsync(cell_count, 0, sizeof(int) * (size_t)nb, s);
     if (e == cudaSuccess) e = launch_bin(b, n, (n + 255) / 256, s);
     if (e != cudaSuccess) return e;
     const int ga = (n + 32 * kNbrWarps - 1) / (32 * kNbrWarps);
