@@ -163,8 +163,8 @@ struct ecmg_ctx {
     size_t path_used = 0;
     /* snapshot */
     DBuf<int> s_slot;
-    DBuf<V2> s_pos, s_vel;
-    DBuf<float> s_clear;
+    DBuf<V2> s_pos;
+    DBuf<float4> s_rec;
     /* buckets of all scenes */
     int total_buckets = 0;
     bool table_dirty = true;
@@ -419,7 +419,7 @@ ecmg_status ecmg_create_batch(const ecmg_params* p, int n_scenes, const int* max
     CKC(c->path_off.alloc(N)); CKC(c->path_len.alloc(N)); CKC(c->key.alloc(N)); CKC(c->rank.alloc(N));
     CKC(c->destroyed_list.alloc(N)); CKC(c->replan_list.alloc(N)); CKC(c->replan_pos.alloc(N));
     CKC(c->d_pend.alloc(N));
-    CKC(c->s_slot.alloc(N)); CKC(c->s_pos.alloc(N)); CKC(c->s_vel.alloc(N)); CKC(c->s_clear.alloc(N));
+    CKC(c->s_slot.alloc(N)); CKC(c->s_pos.alloc(N)); CKC(c->s_rec.alloc(N));
     CKC(c->d_slot_scene.alloc(N));
     CKC(c->nbr.alloc(N * (size_t)prm.max_neighbors));
     CKC(c->ncnt.alloc(N));
@@ -474,7 +474,7 @@ ecmg_status ecmg_destroy(ecmg_ctx* c)
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (auto& g : c->graph)
         if (g) cudaGraphExecDestroy(g);
-    DBuf<V2>* v2s[] = {&c->pos, &c->vel, &c->attr, &c->pref_vel, &c->replan_pos, &c->path_xy, &c->s_pos, &c->s_vel,
+    DBuf<V2>* v2s[] = {&c->pos, &c->vel, &c->attr, &c->pref_vel, &c->replan_pos, &c->path_xy, &c->s_pos,
                        &c->rec_vorca};
     for (auto* b : v2s) b->free_();
     DBuf<int>* is[] = {&c->d_pend, &c->path_off, &c->path_len, &c->key, &c->rank, &c->destroyed_list, &c->replan_list,
@@ -483,7 +483,7 @@ ecmg_status ecmg_destroy(ecmg_ctx* c)
     for (auto* b : is) b->free_();
     c->d_clear.free_();
     c->d_speed.free_();
-    c->s_clear.free_();
+    c->s_rec.free_();
     c->d_active.free_();
     c->feat.free_();
     c->cls.free_();
@@ -1875,6 +1875,7 @@ static void fill_args(ecmg_ctx* c, BinArgs& b, TickArgs& t, bool use_model)
     b.pos = c->pos.p;
     b.vel = c->vel.p;
     b.clear = c->d_clear.p;
+    b.speed = c->d_speed.p;
     b.active = c->d_active.p;
     b.key = c->key.p;
     b.rank = c->rank.p;
@@ -1882,8 +1883,7 @@ static void fill_args(ecmg_ctx* c, BinArgs& b, TickArgs& t, bool use_model)
     b.block_sums = c->scan_tmp.p;
     b.s_slot = c->s_slot.p;
     b.s_pos = c->s_pos.p;
-    b.s_vel = c->s_vel.p;
-    b.s_clear = c->s_clear.p;
+    b.s_rec = c->s_rec.p;
     b.cell_start = c->cell_start.p;
     b.counters = c->counters.p;
     b.last = c->d_last.p;
@@ -1904,8 +1904,7 @@ static void fill_args(ecmg_ctx* c, BinArgs& b, TickArgs& t, bool use_model)
     t.path_xy = c->path_xy.p;
     t.s_slot = c->s_slot.p;
     t.s_pos = c->s_pos.p;
-    t.s_vel = c->s_vel.p;
-    t.s_clear = c->s_clear.p;
+    t.s_rec = c->s_rec.p;
     t.cell_start = c->cell_start.p;
     t.cell_count = c->cell_count.p;
     t.total_buckets = c->total_buckets;

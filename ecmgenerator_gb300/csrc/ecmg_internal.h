@@ -100,8 +100,7 @@ struct TickArgs {
     /* tick-start snapshot in grid order */
     const int* s_slot;
     const V2* s_pos;
-    const V2* s_vel;
-    const float* s_clear;
+    const float4* s_rec; /* velocity, radius, preferred speed */
     const int* cell_start; /* total buckets + 1 */
     int* cell_count;       /* bucket counts, cleared by k_attract for the next tick */
     int total_buckets;
@@ -144,6 +143,7 @@ struct TickArgs {
 struct BinArgs {
     const V2* pos;
     const float* clear;
+    const float* speed;
     const V2* vel;
     const unsigned char* active;
     int* key;        /* slot -> bucket */
@@ -152,8 +152,7 @@ struct BinArgs {
     int* block_sums; /* scan_tmp_ints(total_buckets) */
     int* s_slot;
     V2* s_pos;
-    V2* s_vel;
-    float* s_clear;
+    float4* s_rec; /* null: not wanted (stand-alone kNN) */
     int* cell_start; /* total_buckets + 1 */
     int* counters;
     AgentGrid grid;           /* used when scenes is null */

@@ -143,8 +143,7 @@ __global__ void k_scatter(BinArgs a)
         const int d = a.cell_count[b] + a.block_sums[b / kScanTile] + a.rank[i];
         a.s_slot[d] = i;
         a.s_pos[d] = a.pos[i];
-        if (a.s_vel) a.s_vel[d] = a.vel[i];
-        if (a.s_clear) a.s_clear[d] = a.clear[i];
+        if (a.s_rec) a.s_rec[d] = make_float4(a.vel[i].x, a.vel[i].y, a.clear[i], a.speed[i]);
     }
     for (int c = t0; c < a.total_buckets; c += step) a.cell_start[c] = a.cell_count[c] + a.block_sums[c / kScanTile];
     if (t0 == 0) a.cell_start[a.total_buckets] = a.counters[C_NSORTED];
@@ -206,8 +205,7 @@ __global__ void __launch_bounds__(kSmallBlock) k_bin_small(BinArgs a)
         a.rank[i] = rank[r];
         a.s_slot[d] = i;
         a.s_pos[d] = a.pos[i];
-        if (a.s_vel) a.s_vel[d] = a.vel[i];
-        if (a.s_clear) a.s_clear[d] = a.clear[i];
+        if (a.s_rec) a.s_rec[d] = make_float4(a.vel[i].x, a.vel[i].y, a.clear[i], a.speed[i]);
     }
     for (int c = threadIdx.x; c < a.total_buckets; c += kSmallBlock) a.cell_start[c] = count[c];
     if (threadIdx.x == 0) {
@@ -399,6 +397,7 @@ __device__ void attract_tick(const TickArgs& a, int t)
     const int slot = a.s_slot[t];
     if (a.active[slot] & kActivePending) return; /* done by k_fixup once its new path is in */
     const V2 pos = a.s_pos[t];
+    const float speed = a.s_rec[t].w;
     const SceneDev& sc = a.scenes[a.slot_scene ? a.slot_scene[slot] : 0];
     /* the point location of the retraction, issued before the path loads
        (independent chains of dependent loads); unused when the agent arrives */
@@ -447,7 +446,6 @@ __device__ void attract_tick(const TickArgs& a, int t)
     }
 
     /* ApplySteeringForce (Simulator.cpp:638-657) */
-    const float speed = a.speed[slot];
     V2 pv = normalize(attr - pos) * speed;
     a.pref_vel[slot] = pv;
 }
@@ -463,10 +461,10 @@ __device__ void orca_tick(const TickArgs& a, int t)
     const int slot = a.s_slot[t];
     if (a.active[slot] != 1) return; /* inactive, or waiting for its re-plan (k_fixup) */
     const V2 pos = a.s_pos[t];
-    const V2 vel = a.s_vel[t];
-    const float clr = a.s_clear[t];
+    const float4 rec = a.s_rec[t];
+    const V2 vel = mk(rec.x, rec.y);
+    const float clr = rec.z, speed = rec.w;
     const SceneDev& sc = a.scenes[a.slot_scene ? a.slot_scene[slot] : 0];
-    const float speed = a.speed[slot];
     const V2 pv = a.pref_vel[slot];
 
     /* ORCA::GetVelocity (ORCA.cpp:14-57) with maxSpeed = preferred speed
@@ -519,8 +517,8 @@ __device__ void orca_tick(const TickArgs& a, int t)
         if (j >= 0) {
             /* inline in the plain kernel (no other callers compete for the
                instruction cache there), out of line in the full one */
-            cons[m] = agent_constraint(pos, vel, clr, a.s_pos[j], a.s_vel[j], a.s_clear[j], a.tau_a, a.dt,
-                                       a.inv_tau_a);
+            const float4 r = a.s_rec[j];
+            cons[m] = agent_constraint(pos, vel, clr, a.s_pos[j], mk(r.x, r.y), r.z, a.tau_a, a.dt, a.inv_tau_a);
         } else {
             /* kd-tree mode: a cache entry left by an earlier agent that is
                not in this tick's grid; its slot is not written this tick */
@@ -662,9 +660,9 @@ __global__ void __launch_bounds__(128) k_features(TickArgs a)
         for (int i = 0; i < kMlpIn; i++) f[i] = 0.0f;
         const int slot = a.s_slot[t];
         if (a.active[slot]) {
-            const V2 pos = a.s_pos[t], vel = a.s_vel[t];
-            const float clr = a.s_clear[t];
-            const float speed = a.speed[slot];
+            const float4 rec = a.s_rec[t];
+            const V2 pos = a.s_pos[t], vel = mk(rec.x, rec.y);
+            const float clr = rec.z, speed = rec.w;
             const float maxSpeed = a.max_speed > 0.0f ? a.max_speed : speed;
             const int ncnt = a.ncnt[t];
             const int* nbr = a.nbr + (size_t)t * a.k;
@@ -673,12 +671,13 @@ __global__ void __launch_bounds__(128) k_features(TickArgs a)
             for (int q = 0; q < kMlpNbrs; q++) {
                 if (q < ncnt) {
                     int j = nbr[q];
-                    V2 pj = a.s_pos[j], vj = a.s_vel[j];
+                    const float4 rj = a.s_rec[j];
+                    V2 pj = a.s_pos[j], vj = mk(rj.x, rj.y);
                     f[5 * q + 0] = (pj.x - pos.x) * inv_r;
                     f[5 * q + 1] = (pj.y - pos.y) * inv_r;
                     f[5 * q + 2] = (vel.x - vj.x) * 0.5f;
                     f[5 * q + 3] = (vel.y - vj.y) * 0.5f;
-                    f[5 * q + 4] = a.s_clear[j] + clr;
+                    f[5 * q + 4] = rj.z + clr;
                 }
             }
             V2 pv = a.pref_vel[slot];

@@ -373,9 +373,10 @@ __device__ __forceinline__ void orca_group(const TickArgs& a, int t, bool in, fl
     const SceneDev& sc = a.scenes[on && a.slot_scene ? a.slot_scene[slot] : 0];
     if (on) {
         pos = a.s_pos[t];
-        vel = a.s_vel[t];
-        clr = a.s_clear[t];
-        speed = a.speed[slot];
+        const float4 rec = a.s_rec[t];
+        vel = mk(rec.x, rec.y);
+        clr = rec.z;
+        speed = rec.w;
         pv = a.pref_vel[slot];
         ncnt = a.ncnt[t];
     }
@@ -419,8 +420,9 @@ __device__ __forceinline__ void orca_group(const TickArgs& a, int t, bool in, fl
         float nc;
         if (j >= 0) {
             np = a.s_pos[j];
-            nv = a.s_vel[j];
-            nc = a.s_clear[j];
+            const float4 rec = a.s_rec[j];
+            nv = mk(rec.x, rec.y);
+            nc = rec.z;
         } else {
             /* kd-tree mode: a cache entry left by an earlier agent that is
                not in this tick's grid; its slot is not written this tick */
