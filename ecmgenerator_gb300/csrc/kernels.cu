@@ -601,8 +601,11 @@ __global__ void __launch_bounds__(32 * kNbrWarps, K <= 16 ? 8 : 4) k_neighbors(T
     }
 }
 
-/* UpdateAttractionPointSystem + ApplySteeringForce for every agent */
-__global__ void __launch_bounds__(128) k_attract(TickArgs a)
+/* UpdateAttractionPointSystem + ApplySteeringForce for every agent.  Bound by
+   its dependent loads; 8 resident blocks at 64 registers (24 bytes of spills)
+   against 6 at 80: 158 and 191 us beside the search at a million agents, no
+   difference at 25,000; 10 blocks spill 92 bytes and take 247 */
+__global__ void __launch_bounds__(128, 8) k_attract(TickArgs a)
 {
     const int n = a.counters[C_NSORTED];
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) attract_tick(a, t);
