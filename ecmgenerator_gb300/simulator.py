@@ -104,6 +104,7 @@ class Simulator:
             raise EcmgError(rc, "ecmg_create failed (is a CUDA device visible?)")
         self.h = h
         self.max_agents = int(max_agents)
+        self._views = {}
         self.k = int(max_neighbors)
         self.scene = scene
         self._keep, o, e = _scene_structs(scene)
@@ -329,15 +330,20 @@ class Simulator:
         velocities while set_host_mirror is on)."""
         p = C.c_void_p()
         self._ck(self.L.ecmg_host_view(self.h, FIELD[field], C.byref(p)))
-        n = self.max_agents
-        if field == "active":
-            arr = np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_uint8)), shape=(n,))
-        elif field in ("clearance", "speed"):
-            arr = np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_float)), shape=(n,))
-        else:
-            arr = np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_float)), shape=(n, 2))
-        arr.flags.writeable = False
-        return arr
+        # the array of a field stays where it is: one numpy array is built per
+        # field and every call returns a view of it (building one takes 5 us)
+        kept = self._views.get(field)
+        if kept is None or kept[0] != p.value:
+            n = self.max_agents
+            if field == "active":
+                arr = np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_uint8)), shape=(n,))
+            elif field in ("clearance", "speed"):
+                arr = np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_float)), shape=(n,))
+            else:
+                arr = np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_float)), shape=(n, 2))
+            arr.flags.writeable = False
+            kept = self._views[field] = (p.value, arr)
+        return kept[1].view()
 
     def get_num_agents(self) -> int:
         n = C.c_int()
@@ -451,6 +457,7 @@ class BatchSimulator(Simulator):
             raise EcmgError(rc, "ecmg_create_batch failed (is a CUDA device visible?)")
         self.h = h
         self.max_agents = int(caps.sum())
+        self._views = {}
         self.k = int(p.max_neighbors)
         self.scenes = scenes
         self._keep = []
