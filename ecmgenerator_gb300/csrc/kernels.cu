@@ -382,13 +382,13 @@ __device__ __noinline__ Con agent_constraint_ni(V2 position, V2 velocity, float 
     return agent_constraint(position, velocity, clr, np, nv, nclr, tau, dt, inv_tau);
 }
 
-template <int MC>
+template <int MC, bool FULL>
 __device__ __noinline__ void lp3d_local(const Con* cons, int m, int nObst, float maxSpeed, int failed, V2* v,
                                         bool fp64)
 {
     Con proj[MC - kMaxObstCons]; /* bisectors: at most the neighbour constraints */
     LocalGet get{cons};
-    lp3d(get, m, nObst, maxSpeed, failed, v, proj, fp64);
+    lp3d(get, m, nObst, maxSpeed, failed, v, proj, FULL && fp64);
 }
 
 /* attraction point and preferred velocity of grid-order agent t */
@@ -452,9 +452,10 @@ __device__ void attract_tick(const TickArgs& a, int t)
 
 /* ApplyObstacleAvoidanceForce + UpdateVelocitySystem + UpdatePositionSystem
    of grid-order agent t (agents destroyed this tick are skipped).  FULL
-   keeps the learned proposal's check, the trace labels and the recording of
-   the step; the plain tick's kernel is compiled without them (smaller code,
-   the same arithmetic). */
+   keeps the learned proposal's check, the trace labels, the recording of the
+   step, the FP64 bisectors and the kd-tree mode's entries outside the grid;
+   the plain tick's kernel is compiled without them (a fifth of its stalls are
+   for instructions; the same arithmetic). */
 template <int K, bool FULL = true>
 __device__ void orca_tick(const TickArgs& a, int t)
 {
@@ -514,7 +515,7 @@ __device__ void orca_tick(const TickArgs& a, int t)
     const int nObst = m;
     for (int q = 0; q < ncnt; q++) {
         const int j = nbr[q];
-        if (j >= 0) {
+        if (!FULL || j >= 0) {
             /* inline in the plain kernel (no other callers compete for the
                instruction cache there), out of line in the full one */
             const float4 r = a.s_rec[j];
@@ -551,7 +552,7 @@ __device__ void orca_tick(const TickArgs& a, int t)
             failed = failed2 < 0 ? m : failed2;
         }
         if (failed < m) {
-            lp3d_local<MC>(cons, m, nObst, maxSpeed, failed, &v, a.lp3d_fp64 != 0);
+            lp3d_local<MC, FULL>(cons, m, nObst, maxSpeed, failed, &v, a.lp3d_fp64 != 0);
             need3d = true;
         }
     }
@@ -869,7 +870,7 @@ cudaError_t launch_tick(const BinArgs& b, const TickArgs& t, int max_slots, int 
     }
     if (ev && t.feat) cudaEventRecordWithFlags(ev[3], s, evflags);
     if (t.lanes > 1) {
-        const bool full = t.cls || t.cls_slot || t.label || t.rec_cnt;
+        const bool full = t.cls || t.cls_slot || t.label || t.rec_cnt || t.lp3d_fp64;
         auto go = [&](auto kern) {
             /* one agent set per warp, so that the block scheduler evens out
                their unequal work; a slot range far above the agents in it
@@ -890,7 +891,7 @@ cudaError_t launch_tick(const BinArgs& b, const TickArgs& t, int max_slots, int 
         /* persistent grid: the resident blocks per SM, divided by occ_div
            (fewer resident warps leave each more L1 for its local arrays) */
         const int div = t.occ_div > 1 ? t.occ_div : 1;
-        const bool full = t.cls || t.cls_slot || t.label || t.rec_cnt;
+        const bool full = t.cls || t.cls_slot || t.label || t.rec_cnt || t.lp3d_fp64 || kd;
         auto go = [&](auto kern) {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, 0);
             kern<<<sms * (per_sm / div > 0 ? per_sm / div : 1), block, 0, s>>>(t);
@@ -942,7 +943,7 @@ cudaError_t launch_mirror(const V2* pos, const V2* vel, V2* h_pos, V2* h_vel, in
 cudaError_t launch_fixup(const TickArgs& t, const int* list, int n, cudaStream_t s)
 {
     if (n <= 0) return cudaSuccess;
-    const bool full = t.cls || t.cls_slot || t.label || t.rec_cnt;
+    const bool full = t.cls || t.cls_slot || t.label || t.rec_cnt || t.lp3d_fp64;
     if (t.k <= 8) full ? k_fixup<8, true><<<n, 32, 0, s>>>(t, list) : k_fixup<8, false><<<n, 32, 0, s>>>(t, list);
     else if (t.k <= 16) full ? k_fixup<16, true><<<n, 32, 0, s>>>(t, list) : k_fixup<16, false><<<n, 32, 0, s>>>(t, list);
     else full ? k_fixup<32, true><<<n, 32, 0, s>>>(t, list) : k_fixup<32, false><<<n, 32, 0, s>>>(t, list);

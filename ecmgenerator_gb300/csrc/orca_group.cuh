@@ -457,7 +457,7 @@ __device__ __forceinline__ void orca_group(const TickArgs& a, int t, bool in, fl
     }
     const bool need3d = solve && failed < m;
     if (__any_sync(kFull, need3d)) {
-        lp3d_group<G>(s, s + kGroupLines<K>, need3d, m, nObst, maxSpeed, failed, a.lp3d_fp64 != 0, sub, &v);
+        lp3d_group<G>(s, s + kGroupLines<K>, need3d, m, nObst, maxSpeed, failed, FULL && a.lp3d_fp64, sub, &v);
         if (need3d && sub == 0) gc.lp3d++;
     }
 
