@@ -50,19 +50,22 @@ constexpr unsigned kKnnCode = 63u; /* low key bits: entry of the index column */
 /* list capacity K: the k nearest in key[K-k .. K-1]; entries below hold 0.
    Buffer entries: 8 merge into 16 at the cost per candidate of 16, with less
    of the buffers empty (a flush takes the whole warp); for K = 32 the merge
-   weighs more.  Index column: the list's entries and the candidates since the
-   last renumbering. */
+   weighs more.  Index column: every candidate accepted (24 on average at
+   k = 16); 46 entries keep eight blocks on an SM, a lane that needs more (9 %
+   of the warps have one in the 1M crossing) searches again (renumbering the
+   column instead cost every warp 15 % of its instructions, run or not; sent to
+   the 64-bit search these lanes took the kernel from 318 to 369 us). */
 template <int K>
 constexpr int kKnnBuf = K <= 16 ? 8 : 16;
 template <int K>
-constexpr int kKnnIdx = K <= 8 ? 32 : (K <= 16 ? 40 : 64);
+constexpr int kKnnIdx = K <= 8 ? 32 : (K <= 16 ? 46 : 64);
 
 template <int K>
 struct KnnSm { /* of one warp */
     float key[kKnnBuf<K>][32];
     int idx[kKnnIdx<K>][32];
     static_assert(kKnnIdx<K> <= (int)kKnnCode + 1, "index entries must fit the code");
-    static_assert(kKnnIdx<K> >= K + kKnnBuf<K>, "a renumbered list leaves room for a buffer");
+    static_assert(kKnnIdx<K> - kKnnBuf<K> >= K, "a column without room for a buffer has filled the list");
 };
 
 __device__ __forceinline__ float knn_hi(float key) { return __uint_as_float(__float_as_uint(key) & ~kKnnCode); }
@@ -110,14 +113,18 @@ __device__ __forceinline__ void knn_flush(const KnnSm<K>& sm, int lane, int cnt,
 #pragma unroll
     for (int i = 0; i < B; i++) b[i] = i < cnt ? sm.key[i][lane] : INFINITY;
     sort_net<B>(b);
-    float d = *rej;
+    float d[B]; /* the dropped ones; their minimum as a tree, not a chain */
 #pragma unroll
     for (int i = 0; i < B; i++) {
         const float o = key[K - B + i], n = b[B - 1 - i];
-        d = fminf(d, fmaxf(o, n));
+        d[i] = fmaxf(o, n);
         key[K - B + i] = fminf(o, n);
     }
-    *rej = d;
+#pragma unroll
+    for (int w = B / 2; w >= 1; w >>= 1)
+#pragma unroll
+        for (int i = 0; i < w; i++) d[i] = fminf(d[i], d[i + w]);
+    *rej = fminf(*rej, d[0]);
     bitonic_net<K>(key);
 }
 
@@ -128,22 +135,6 @@ __device__ __forceinline__ float dist2(V2 q, float2 np)
     const float2 d = __fadd2_rn(make_float2(q.x, q.y), np);
     const float2 e = __fmul2_rn(d, d);
     return e.x + e.y;
-}
-
-/* the list's indices move to the first K entries of the index column */
-template <int K>
-__device__ __forceinline__ int knn_renumber(KnnSm<K>& sm, int lane, int k, float (&key)[K])
-{
-    int id[K];
-#pragma unroll
-    for (int q = 0; q < K; q++) id[q] = sm.idx[__float_as_uint(key[q]) & kKnnCode][lane];
-#pragma unroll
-    for (int q = 0; q < K; q++)
-        if (q >= K - k && key[q] < INFINITY) {
-            sm.idx[q][lane] = id[q];
-            key[q] = __uint_as_float((__float_as_uint(key[q]) & ~kKnnCode) | (unsigned)q);
-        }
-    return K;
 }
 
 /* The k nearest of the agents at p (one per lane; `valid` false: none) into
@@ -161,9 +152,9 @@ __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, f
 #pragma unroll
     for (int q = 0; q < K; q++) key[q] = q < K - k ? 0.0f : INFINITY;
     float rej = INFINITY;
-    float *const k0 = &sm.key[0][lane], *const kend = k0 + 32 * B;
-    float* kp = k0; /* next entry of the buffer column */
-    int ord = 0;    /* next entry of the index column */
+    int ord = 0, ord0 = 0; /* next entry of the index column; that of the buffer's first candidate */
+    bool over = false;     /* the index column is full */
+    int tries = 0;         /* searches begun again for that */
     valid = valid && p.x - p.x == 0.0f && p.y - p.y == 0.0f; /* no distance to a non-finite position is finite */
     const float fy = (p.y - g.y0) * g.inv;
     const int cx = cell_clamp((p.x - g.x0) * g.inv, g.gw), cy = cell_clamp(fy, g.gh);
@@ -209,37 +200,45 @@ __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, f
             }
             const int longest = __reduce_max_sync(kAll, left);
             /* the next candidate's position is loaded while this one is used */
+            const int end = j + left;
             V2 q = mk(0.0f, 0.0f);
             if (left > 0) q = s_pos[j];
-            for (int it = 0; it < longest; it++) {
+            for (int it = longest; it > 0; it--) {
                 const float d2 = dist2(q, np);
-                if (it + 1 < left) q = s_pos[j + it + 1];
-                if (it < left && d2 > lo && d2 < lim) {
-                    *kp = __uint_as_float((__float_as_uint(d2) & ~kKnnCode) | (unsigned)ord);
-                    sm.idx[ord][lane] = j + it;
-                    kp += 32;
+                const bool in = j < end && d2 > lo && d2 < lim;
+                if (j + 1 < end) q = s_pos[j + 1];
+                if (in) {
+                    sm.key[ord - ord0][lane] = __uint_as_float((__float_as_uint(d2) & ~kKnnCode) | (unsigned)ord);
+                    sm.idx[ord][lane] = j;
                     ord++;
                 }
-                if (__any_sync(kAll, kp == kend)) {
-                    knn_flush<K>(sm, lane, (int)(kp - k0) >> 5, key, &rej);
-                    kp = k0;
+                j++;
+                if (__any_sync(kAll, ord == ord0 + B)) {
+                    knn_flush<K>(sm, lane, ord - ord0, key, &rej);
+                    ord0 = ord;
                     /* candidates beyond the k-th key (its code bits taken as
                        ones) cannot enter any more; equal leading bits still
                        count as near ties */
                     if (key[K - 1] < INFINITY)
                         lim = fminf(lim, __uint_as_float((__float_as_uint(key[K - 1]) | kKnnCode) + 1u));
-                    if (__any_sync(kAll, ord > kKnnIdx<K> - B)) ord = knn_renumber<K>(sm, lane, k, key);
+                    if (ord > kKnnIdx<K> - B) { /* no room for another buffer */
+                        over = true;
+                        lim = 0.0f;
+                    }
                 }
             }
         }
-        if (__any_sync(kAll, kp != k0)) {
-            knn_flush<K>(sm, lane, (int)(kp - k0) >> 5, key, &rej);
-            kp = k0;
+        if (__any_sync(kAll, ord != ord0)) {
+            knn_flush<K>(sm, lane, ord - ord0, key, &rej);
+            ord0 = ord;
         }
         /* fewer than k inside the disc: a larger one, without what the last
            one held (d2 >= disc is d2 > the float before it) */
         const bool grow = valid && !(key[K - 1] < INFINITY) && disc < r2;
-        if (!__any_sync(kAll, grow)) break;
+        /* a full index column: once more from the start, with the k-th
+           distance known by now (a disc of little more than k agents) */
+        const bool again = over && tries < 2;
+        if (!__any_sync(kAll, grow || again)) break;
         lim = 0.0f;
         if (grow) {
             lo = fmaxf(kEps, __uint_as_float(__float_as_uint(disc) - 1u));
@@ -247,13 +246,23 @@ __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, f
             more_area *= more_area;
             lim = disc;
         }
-        if (__any_sync(kAll, ord > kKnnIdx<K> - B)) ord = knn_renumber<K>(sm, lane, k, key);
+        if (again) {
+            disc = fminf(r2, __uint_as_float((__float_as_uint(key[K - 1]) | kKnnCode) + 1u));
+            lim = disc;
+            lo = kEps;
+            rej = INFINITY;
+            ord = ord0 = 0;
+            over = false;
+            tries++;
+#pragma unroll
+            for (int q = 0; q < K; q++) key[q] = q < K - k ? 0.0f : INFINITY;
+        }
     }
     bool tie = false;
 #pragma unroll
     for (int q = 0; q + 1 < K; q++)
         if (q >= K - k && key[q + 1] < INFINITY && knn_hi(key[q]) == knn_hi(key[q + 1])) tie = true;
-    if (key[K - 1] < INFINITY && knn_hi(rej) == knn_hi(key[K - 1])) return 0;
+    if (over || (key[K - 1] < INFINITY && knn_hi(rej) == knn_hi(key[K - 1]))) return 0;
     return tie ? 2 : 1;
 }
 
@@ -288,7 +297,7 @@ __device__ __noinline__ void knn_resort(int n, V2 p, const V2* s_pos, const int*
 }
 
 /* the search by 64-bit (d2, slot) keys (rare: a near tie at the k-th
-   distance that the list cannot settle; out of line): the rows of the disc of
+   distance that the list cannot settle, a full index column; out of line): the rows of the disc of
    squared radius `lim`, which holds at least k agents or is r^2; o[q] gets
    the grid indices, the return value is the count */
 template <int K>
