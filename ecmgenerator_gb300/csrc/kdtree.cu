@@ -183,47 +183,34 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_hist(const unsigned* __restri
     hist[blockIdx.x * 256 + threadIdx.x] = h[threadIdx.x];
 }
 
-/* hist [nblk][256] -> where each tile's keys of each digit go, in place: one
-   block, four threads per digit over a quarter of the tiles each */
-__global__ void __launch_bounds__(1024) k_rs_scan(int* __restrict__ hist, int nblk)
+/* hist [nblk][256] -> the keys of each digit in the tiles before each tile, in
+   place, and the digits' totals: a warp per digit.  (One block over all
+   digits took 9.6 us a pass at 123 tiles, as long as the scatter.) */
+__global__ void __launch_bounds__(256) k_rs_scan(int* __restrict__ hist, int nblk, int* __restrict__ total)
 {
-    __shared__ int part[4][256];
-    __shared__ int ws[8];
-    const int d = threadIdx.x & 255, g = threadIdx.x >> 8;
-    const int per = (nblk + 3) / 4, b0 = g * per, b1 = min(nblk, b0 + per);
-    int s = 0;
-#pragma unroll 8
-    for (int b = b0; b < b1; b++) s += hist[b * 256 + d];
-    part[g][d] = s;
-    __syncthreads();
-    int run = 0;
-    if (g == 0) {
-        const int p0 = part[0][d], p1 = part[1][d], p2 = part[2][d], p3 = part[3][d];
-        const int lane = d & 31, w = d >> 5;
-        int x = p0 + p1 + p2 + p3;
-        const int tot = x;
+    const int lane = threadIdx.x & 31, d = blockIdx.x * 8 + (threadIdx.x >> 5);
+    int carry = 0;
+    for (int b0 = 0; b0 < nblk; b0 += 128) {
+        int v[4];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
+        for (int q = 0; q < 4; q++) {
+            const int b = b0 + q * 32 + lane;
+            v[q] = b < nblk ? hist[b * 256 + d] : 0;
         }
-        if (lane == 31) ws[w] = x;
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        for (int q = 0; q < w; q++) x += ws[q];
-        run = x - tot;
-        part[0][d] = run;
-        part[1][d] = run + p0;
-        part[2][d] = run + p0 + p1;
-        part[3][d] = run + p0 + p1 + p2;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            int x = v[q];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            const int b = b0 + q * 32 + lane;
+            if (b < nblk) hist[b * 256 + d] = carry + x - v[q];
+            carry += __shfl_sync(0xffffffffu, x, 31);
+        }
     }
-    __syncthreads();
-    run = part[g][d];
-#pragma unroll 8
-    for (int b = b0; b < b1; b++) {
-        const int c = hist[b * 256 + d];
-        hist[b * 256 + d] = run;
-        run += c;
-    }
+    if (lane == 0) total[d] = carry;
 }
 
 /* elements of a tile are placed in tile order, round by round (256 per
@@ -232,15 +219,17 @@ __global__ void __launch_bounds__(1024) k_rs_scan(int* __restrict__ hist, int nb
 __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const unsigned* __restrict__ kin, const int* __restrict__ vin,
                                                            unsigned* __restrict__ kout, int* __restrict__ vout,
                                                            const int* __restrict__ n_ptr, int shift,
-                                                           const int* __restrict__ offs)
+                                                           const int* __restrict__ offs,
+                                                           const int* __restrict__ total)
 {
     __shared__ int base[256];
     __shared__ int wc[kRsThreads / 32][256];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int n = *n_ptr;
-    base[threadIdx.x] = offs[blockIdx.x * 256 + threadIdx.x];
     const int t0 = blockIdx.x * kRsTile;
     if (t0 >= n) return;
+    /* the keys of smaller digits, then those of this digit in earlier tiles */
+    base[threadIdx.x] = block_excl_scan<int>(total[threadIdx.x], nullptr) + offs[blockIdx.x * 256 + threadIdx.x];
     unsigned keys[kRsItems];
     int vals[kRsItems];
 #pragma unroll
@@ -292,8 +281,8 @@ cudaError_t radix_sort(unsigned* keys, int* vals, unsigned* ktmp, int* vtmp, con
     int* vb = vtmp;
     for (int shift = 0; shift < 32; shift += 8) {
         k_rs_hist<<<nblk, kRsThreads, 0, s>>>(ka, n_ptr, shift, hist);
-        k_rs_scan<<<1, 1024, 0, s>>>(hist, nblk);
-        k_rs_scatter<<<nblk, kRsThreads, 0, s>>>(ka, va, kb, vb, n_ptr, shift, hist);
+        k_rs_scan<<<32, 256, 0, s>>>(hist, nblk, hist + nblk * 256);
+        k_rs_scatter<<<nblk, kRsThreads, 0, s>>>(ka, va, kb, vb, n_ptr, shift, hist, hist + nblk * 256);
         unsigned* tk = ka; ka = kb; kb = tk;
         int* tv = va; va = vb; vb = tv;
     }
@@ -363,21 +352,36 @@ __global__ void k_kd_side(KdArgs a, const int* A)
     }
 }
 
-/* left | right << 32 of position i of list B */
-__device__ __forceinline__ unsigned long long kd_flag(const KdArgs& a, const int* B, int i, int n)
+/* left | right << 32 of the positions first, first + step, ... of list B: the
+   loads of all of them in flight together */
+__device__ __forceinline__ void kd_flags(const KdArgs& a, const int* B, int first, int step, int n,
+                                         unsigned long long (&f)[kScanItems])
 {
-    if (i >= n || a.seg_lo[i] >= a.seg_hi[i]) return 0ull;
-    const int s = a.side[B[i]];
-    return (s == 0 ? 1ull : 0ull) | (s == 2 ? (1ull << 32) : 0ull);
+    int id[kScanItems];
+#pragma unroll
+    for (int q = 0; q < kScanItems; q++) {
+        const int i = first + q * step;
+        id[q] = -1;
+        if (i < n) {
+            const int lo = a.seg_lo[i], hi = a.seg_hi[i], b = B[i];
+            id[q] = lo < hi ? b : -1;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kScanItems; q++) {
+        const int s = id[q] >= 0 ? a.side[id[q]] : 1;
+        f[q] = (s == 0 ? 1ull : 0ull) | (s == 2 ? (1ull << 32) : 0ull);
+    }
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_kd_count(KdArgs a, const int* B)
 {
     const int n = a.n_dev[0];
     const int base = blockIdx.x * kScanTile + threadIdx.x;
-    unsigned long long s = 0;
+    unsigned long long f[kScanItems], s = 0;
+    kd_flags(a, B, base, kScanThreads, n, f);
 #pragma unroll
-    for (int i = 0; i < kScanItems; i++) s += kd_flag(a, B, base + i * kScanThreads, n);
+    for (int i = 0; i < kScanItems; i++) s += f[i];
     unsigned long long tot;
     block_excl_scan<unsigned long long>(s, &tot);
     if (threadIdx.x == 0) a.scan_tmp64[blockIdx.x] = tot;
@@ -389,11 +393,9 @@ __global__ void __launch_bounds__(kScanThreads) k_kd_prefix(KdArgs a, const int*
     const int n = a.n_dev[0];
     const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     unsigned long long v[kScanItems], s = 0;
+    kd_flags(a, B, base, 1, n, v);
 #pragma unroll
-    for (int i = 0; i < kScanItems; i++) {
-        v[i] = kd_flag(a, B, base + i, n);
-        s += v[i];
-    }
+    for (int i = 0; i < kScanItems; i++) s += v[i];
     unsigned long long run = block_excl_scan<unsigned long long>(s, nullptr) + a.scan_tmp64[blockIdx.x];
 #pragma unroll
     for (int i = 0; i < kScanItems; i++) {
@@ -773,14 +775,18 @@ __global__ void __launch_bounds__(32 * kFoldWarps) k_kd_fold(KdArgs a, int level
                 mine_open = mine && a.open[at];
             }
             const unsigned use = __ballot_sync(0xffffffffu, mine);
-            const unsigned refers = __ballot_sync(0xffffffffu, mine && mine_open);
+            unsigned refers = __ballot_sync(0xffffffffu, mine && mine_open), negative = 0u;
             /* 32 rows of k entries, 32 entries at a time */
             int j = q / k, x = q - j * k;
             const int dj = 32 / k, dx = 32 - dj * k;
 #pragma unroll 8
             for (int i = 0; i < k; i++) {
                 const int t = __shfl_sync(0xffffffffu, at, j);
-                if ((use >> j) & 1u) row[i * 32 + q] = rows[(size_t)t * k + x];
+                if ((use >> j) & 1u) {
+                    const int v = rows[(size_t)t * k + x];
+                    row[i * 32 + q] = v;
+                    if (v < 0) negative |= 1u << j;
+                }
                 j += dj;
                 x += dx;
                 if (x >= k) {
@@ -788,17 +794,20 @@ __global__ void __launch_bounds__(32 * kFoldWarps) k_kd_fold(KdArgs a, int level
                     j++;
                 }
             }
+            refers &= __reduce_or_sync(0xffffffffu, negative);
             __syncwarp();
-            for (unsigned left = use; left; left &= left - 1u) {
+            /* the open rows in order, each after the row in use before it */
+            for (unsigned left = refers; left; left &= left - 1u) {
                 const int r = __ffs(left) - 1;
+                const unsigned before = use & ((1u << r) - 1u);
+                if (before && q < k) cur = row[(31 - __clz(before)) * k + q];
                 int v = q < k ? row[r * k + q] : 0;
-                if ((refers >> r) & 1u) {
-                    const int got = __shfl_sync(0xffffffffu, cur, v < 0 ? -v - 1 : q);
-                    if (v < 0) v = got;
-                    if (q < k) row[r * k + q] = v;
-                }
-                cur = v;
+                const int got = __shfl_sync(0xffffffffu, cur, v < 0 ? -v - 1 : q);
+                if (v < 0) v = got;
+                if (q < k) row[r * k + q] = v;
+                __syncwarp();
             }
+            if (use && q < k) cur = row[(31 - __clz(use)) * k + q];
             __syncwarp();
             j = q / k;
             x = q - j * k;
@@ -904,7 +913,7 @@ int kd_kernels(int max_slots)
     for (int n = max_slots; fold == 0 || n > 1; fold++) n = (n + kFold - 1) / kFold;
     return 6 + 3 * 13 + 1 + 5 * kd_top(max_slots) + 4 + 1 + 2 + fold + 2;
 }
-int kd_hist_ints(int cap) { return 256 * ((cap + kRsTile - 1) / kRsTile); }
+int kd_hist_ints(int cap) { return 256 * ((cap + kRsTile - 1) / kRsTile + 1); } /* tiles, totals */
 int kd_scan_tmp(int n) { return (n + kScanTile - 1) / kScanTile + 1; }
 
 /* the build and the per-member maps, on s (beside the attraction kernel) */
