@@ -141,7 +141,7 @@ struct ecmg_ctx {
     /* ECMG_LP_THREAD, ECMG_LP_WARP, ECMG_LP_THREAD_FUSED, or by the agent count */
     static constexpr int kLpAuto = -1;
     int lp_mode = kLpAuto;
-    int lanes_agents = 0; /* the agent count the automatic layout was chosen for */
+    int lanes_agents = 0; /* the agent count the automatic layouts were chosen for */
     int occ_div = 1; /* per-thread layout: resident blocks per SM divided by this */
     int knn_wide = 0; /* neighbour kernel: 8 resident blocks per SM at most, or 6 */
     int wgrab = 4;   /* agents per warp in warp mode */
@@ -1857,16 +1857,24 @@ static int lanes_of(ecmg_ctx* c)
     return c->lanes_agents <= 160000 || c->nbr_mode == ECMG_NEIGHBORS_KDTREE ? 4 : 1;
 }
 
-/* the automatic layout follows the agent count; a count within a factor of
-   1.5 of the last choice's keeps it (a change re-captures the tick's graph) */
+/* the attraction kernel with several lanes per agent: its chain is the point
+   location and the path, which 8 lanes share (kernel, us, one thread / 8 lanes
+   per agent, box scene: 1,000 agents 20.5 / 12.3; 8,000 of 500 m 27.3 / 17.9;
+   16,000 28.5 / 20.0).  It costs instructions, and the neighbour search
+   beside it feels them: at 25,000 agents attraction 30.4 / 24.0, search 25.8 /
+   32.1, the tick 87.3 / 87.7; crossing 100,000 35.6 / 45.1 and 58.9 / 78.3. */
+static bool attract_lanes_of(ecmg_ctx* c) { return c->lanes_agents <= 16000; }
+
+/* the automatic layouts follow the agent count; a count within a factor of
+   1.5 of the last choice's keeps them (a change re-captures the tick's graph) */
 static void choose_lanes(ecmg_ctx* c)
 {
-    if (c->lp_mode != ecmg_ctx::kLpAuto) return;
     const long long n = c->num_agents, was = c->lanes_agents;
     if (was > 0 && 2 * n <= 3 * was && 3 * n >= 2 * was) return;
     const int before = lanes_of(c);
+    const bool attract = attract_lanes_of(c);
     c->lanes_agents = (int)std::max<long long>(1, n);
-    if (lanes_of(c) != before) c->graph_dirty = true;
+    if (lanes_of(c) != before || attract_lanes_of(c) != attract) c->graph_dirty = true;
 }
 
 static void fill_args(ecmg_ctx* c, BinArgs& b, TickArgs& t, bool use_model)
@@ -1916,6 +1924,7 @@ static void fill_args(ecmg_ctx* c, BinArgs& b, TickArgs& t, bool use_model)
     t.slot_scene = b.slot_scene;
     t.tile = c->tile;
     t.lanes = lanes_of(c);
+    t.attract_lanes = attract_lanes_of(c);
     t.occ_div = c->occ_div;
     t.knn_blocks = c->knn_wide ? 6 : 8;
     const ecmg_params& p = c->prm;

@@ -285,6 +285,30 @@ EG_HD bool retract(const EcmView& e, V2 loc, V2* out, int* out_edge, int cell = 
     return ray_segment(loc, rd, p1, p2, out);
 }
 
+/* one path segment of FindAttractionPoint (IRMPathFollower.cpp:62-108), p1 and
+   p2 relative to the retraction point r: its intersections with the circle
+   of squared radius rcs and their places on the segment; false when the
+   line misses it */
+EG_HD bool irm_segment(V2 p1, V2 p2, V2 r, float rcs, V2* gi1, V2* gi2, float* t1, float* t2)
+{
+    V2 ed2 = p2 - p1;
+    float els = len2(ed2);
+    float dd = det(p1, p2);
+    float disc = rcs * els - dd * dd;
+    if (disc < kEps) return false;
+    float dySign = ed2.y < 0.0f ? -1.0f : 1.0f;
+    float sd = sqrtf(disc);
+    V2 i1 = mk((dd * ed2.y + dySign * ed2.x * sd) / els, (-dd * ed2.x + fabsf(ed2.y) * sd) / els);
+    V2 i2 = mk((dd * ed2.y - dySign * ed2.x * sd) / els, (-dd * ed2.x - fabsf(ed2.y) * sd) / els);
+    V2 g1 = p1 + r, g2 = p2 + r;
+    *gi1 = i1 + r;
+    *gi2 = i2 + r;
+    V2 edge = g2 - g1;
+    *t1 = dot(*gi1 - g1, edge) / els;
+    *t2 = dot(*gi2 - g1, edge) / els;
+    return true;
+}
+
 /* IRMPathFollower::FindAttractionPoint (IRMPathFollower.cpp:14-115).
    *out is written only where the reference writes outPoint; *no_retract is
    set when the failure is the retraction of pos itself. */
@@ -310,21 +334,10 @@ EG_NI bool irm(const EcmView& e, V2 pos, const V2* path, int n, V2* out, bool* n
         const V2 p1 = p2;
         p2 = ahead - r;
         if (i + 2 < n) ahead = path[i + 2];
-        V2 ed2 = p2 - p1;
-        float els = len2(ed2);
-        float dd = det(p1, p2);
-        float disc = rcs * els - dd * dd;
-        if (disc < kEps) continue;
+        V2 gi1, gi2;
+        float t1, t2;
+        if (!irm_segment(p1, p2, r, rcs, &gi1, &gi2, &t1, &t2)) continue;
         success = true;
-        float dySign = ed2.y < 0.0f ? -1.0f : 1.0f;
-        float sd = sqrtf(disc);
-        V2 i1 = mk((dd * ed2.y + dySign * ed2.x * sd) / els, (-dd * ed2.x + fabsf(ed2.y) * sd) / els);
-        V2 i2 = mk((dd * ed2.y - dySign * ed2.x * sd) / els, (-dd * ed2.x - fabsf(ed2.y) * sd) / els);
-        V2 g1 = p1 + r, g2 = p2 + r;
-        V2 gi1 = i1 + r, gi2 = i2 + r;
-        V2 edge = g2 - g1;
-        float t1 = dot(gi1 - g1, edge) / els;
-        float t2 = dot(gi2 - g1, edge) / els;
         float maxT = -1.0f;
         if (t1 >= 0.0f && t1 <= 1.0f) { *out = gi1; maxT = t1; }
         if (t2 >= 0.0f && t2 <= 1.0f) {

@@ -115,6 +115,7 @@ struct TickArgs {
     const SceneDev* scenes;
     const int* slot_scene; /* slot -> scene (null: one scene) */
     int tile;              /* agents a warp takes per work grab (per-thread mode: multiple of 32) */
+    int attract_lanes;     /* the attraction kernel with several lanes per agent */
     int lanes;             /* lanes per agent of the per-agent kernel: 1, 4, 8, 16 or 32 */
     int occ_div;           /* per-thread layout: resident blocks per SM divided by this */
     int knn_blocks;        /* neighbour kernel: resident blocks of 128 threads per SM at most */
