@@ -39,22 +39,16 @@ using namespace ecmg;
 namespace {
 
 constexpr int IN = kMlpIn, HID = kMlpHid, OUT = kMlpOut;
-/* GELU (tanh form) and its derivative of two values, in FP32 from one
-   accurate tanh each; products and sums two at a time, separately rounded:
-     y = x/2 (1 + th), th = tanh(k0 (x + k1 x^3)),
-     dy = (1 + th)/2 + x/2 (1 - th^2) k0 (1 + 3 k1 x^2) */
-__device__ __forceinline__ void gelu_both(float2 x, float2* y, float2* dy)
+/* GELU (tanh form) and its derivative from one tanh.  Scalar operations: as
+   pairs of products and sums the derivative came out an ulp apart here and
+   there, which moves its BF16 product over a rounding line once in 70,000. */
+__device__ __forceinline__ void gelu_both(float x, float* y, float* dy)
 {
     const float k0 = 0.7978845608028654f, k1 = 0.044715f; /* sqrt(2/pi), tanh approximation */
-    auto c2 = [](float c) { return make_float2(c, c); };
-    const float2 x3 = __fmul2_rn(__fmul2_rn(__fmul2_rn(c2(k1), x), x), x);
-    const float2 u = __fmul2_rn(c2(k0), __fadd2_rn(x, x3));
-    const float2 th = make_float2(tanhf(u.x), tanhf(u.y));
-    const float2 hx = __fmul2_rn(c2(0.5f), x), t1 = __fadd2_rn(c2(1.0f), th);
-    *y = __fmul2_rn(hx, t1);
-    const float2 du = __fmul2_rn(c2(k0), __fadd2_rn(c2(1.0f), __fmul2_rn(__fmul2_rn(c2(3.0f * k1), x), x)));
-    const float2 sech2 = __fadd2_rn(c2(1.0f), __fmul2_rn(make_float2(-th.x, -th.y), th));
-    *dy = __fadd2_rn(__fmul2_rn(c2(0.5f), t1), __fmul2_rn(__fmul2_rn(hx, sech2), du));
+    const float th = tanhf(k0 * (x + k1 * x * x * x));
+    const float du = k0 * (1.0f + 3.0f * k1 * x * x);
+    *y = 0.5f * x * (1.0f + th);
+    *dy = 0.5f * (1.0f + th) + 0.5f * x * (1.0f - th * th) * du;
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
@@ -477,8 +471,8 @@ __global__ void __launch_bounds__(kInferThreads, 1)
  * operand of its weight gradient, so that nothing is transposed or stored
  * twice.  Per tile, each chain issued by one thread and awaited by all:
  *   Z1 = X W1, Z2 = A1 W2, Z3 = A2 W3 (outputs 0..127, then 128..159)
- *   dW3 += A2^T dZ3, dA2 = dZ3 W3^T
- *   dW2 += A1^T dZ2, dA1 = dZ2 W2^T
+ *   dA2 = dZ3 W3^T, then dW3 += A2^T dZ3
+ *   dA1 = dZ2 W2^T, then dW2 += A1^T dZ2
  *   dW1^T += dZ1^T X
  * with FP32 accumulators: tensor-memory columns 0..127 for the Z's and dA's,
  * 128..511 for the three weight gradients, which stay there over all tiles of
@@ -486,24 +480,32 @@ __global__ void __launch_bounds__(kInferThreads, 1)
  * registers: bias, GELU and its derivative (from one tanh; the derivative is
  * kept in FP32 for the backward pass), softmax cross-entropy, and the FP32
  * bias gradients, summed over a warp's rows by a transposing butterfly and
- * over tiles in registers.  dZ2 overwrites A2, dZ1 overwrites A1.  A CTA
- * writes its sums as one partial gradient.
+ * over tiles in registers.  dZ2 overwrites A2 and dZ1 overwrites A1 once
+ * dW3 and dW2 have read them (a second mbarrier: the next stage's loads and
+ * products run beside these chains).  A CTA writes its sums as one partial
+ * gradient.
  *
- * What bounds it: the elementwise work between the chains (accurate tanh, exp
- * and divisions of 416 activations per row), about 80 % of its time; the
- * chains take 2.3 us of a tile.  A step of 65,536 rows took 722 us as 24
- * launches that passed every activation, its transpose and its BF16 copy
- * through memory, with a two-block column sum for each bias gradient.
+ * What bounds it: the latency of the elementwise work between the chains
+ * (accurate tanh, exp and quotients of 416 activations per row) at the four
+ * warps per scheduler that the registers leave: of a tile's 35,000 cycles the
+ * two activations take 8,700, the softmax 8,500, waiting for chains and
+ * barriers 9,000; the scheduler issues in 44 % of them.  65,536 rows: 85 us
+ * (107 us with a 64-bit remainder per loaded chunk, a divide per output and
+ * weights loaded through registers) and 14 us for k_reduce_adam; a step took
+ * 722 us as 24 launches that passed every activation, its transpose and its
+ * BF16 copy through memory, with a two-block column sum for each bias
+ * gradient.
  * ---------------------------------------------------------------------- */
 constexpr int OW1 = 0, OB1 = OW1 + IN * HID, OW2 = OB1 + HID, OB2 = OW2 + HID * HID, OW3 = OB2 + HID,
-              OB3 = OW3 + HID * OUT, NPARAM = OB3 + OUT; /* W1 [IN x HID], b1, W2 [HID x HID], b2, W3 [HID x OUT], b3 */
+              OB3 = OW3 + HID * OUT, NPARAM = OB3 + OUT, NWEIGHT = HID * (IN + HID + OUT); /* W1 [IN x HID], b1, W2 [HID x HID], b2, W3 [HID x OUT], b3 */
 constexpr int kTrThreads = 512, kTrCols = 512; /* tensor memory: all of it */
 constexpr int kTrW3 = 128, kTrW2 = kTrW3 + OUT, kTrW1 = kTrW2 + HID; /* first columns of dW3, dW2, dW1^T */
 static_assert(kTrW1 + IN == kTrCols, "the weight gradients fill the tensor memory");
 constexpr int kZB = kTile * OUT * 2;
-constexpr size_t kTrainSmem = (size_t)kWB + kXB + 2 * kHB + kZB + sizeof(float) * (2 * HID + OUT) + 64;
+constexpr size_t kTrainSmem =
+    (size_t)kWB + kXB + 2 * kHB + kZB + sizeof(float) * (2 * HID + OUT) + sizeof(int) * 2 * kTile + 64;
 static_assert(kTrainSmem <= 232448, "shared memory of one CTA");
-static_assert(4 * 3 * kTile * 4 <= kZB, "the softmax's exchange fits the dZ3 tile before it is written");
+static_assert((4 * 2 + 4 * 8) * kTile * 4 <= kZB, "the softmax's exchange fits the dZ3 tile before it is written");
 
 /* instruction descriptor with the major axes of A and B (1: MN-major) */
 __host__ __device__ constexpr uint32_t tc_idesc_mn(int N, int amn, int bmn)
@@ -530,6 +532,31 @@ __device__ __forceinline__ void tc_chain(uint32_t tmem, uint32_t a, int ra, int 
             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
             "l"(da + (uint64_t)(ks * (sa >> 4))), "l"(db + (uint64_t)(ks * (sb >> 4))), "r"(id), "r"(acc));
     }
+}
+
+/* eight columns each from taddr, taddr + 32, + 64 and + 96 */
+__device__ __forceinline__ void tmem_ld8x4(uint32_t taddr, float (&v)[32])
+{
+    uint32_t r[32];
+#pragma unroll
+    for (int g = 0; g < 4; g++)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                     : "=r"(r[8 * g]), "=r"(r[8 * g + 1]), "=r"(r[8 * g + 2]), "=r"(r[8 * g + 3]), "=r"(r[8 * g + 4]),
+                       "=r"(r[8 * g + 5]), "=r"(r[8 * g + 6]), "=r"(r[8 * g + 7])
+                     : "r"(taddr + 32u * (uint32_t)g));
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
+                   "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]),
+                   "+r"(r[23])
+                 :
+                 : "memory");
+    asm volatile("" : "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]),
+                 "+r"(r[31])
+                 :
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
@@ -563,39 +590,78 @@ __device__ __forceinline__ float warp_colsum(float (&v)[32])
     return v[0];
 }
 
-/* the row of X that row r of the minibatch is: r itself, or drawn by a hash
-   of the step's seed (splitmix64) */
-__device__ __forceinline__ int train_row(int r, int n, unsigned long long seed, int draw)
+/* the same of 8 columns, for column c in the lanes c, c + 8, c + 16, c + 24 */
+__device__ __forceinline__ float warp_colsum8(float (&v)[8])
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 4; o; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; i++) {
+            const float keep = up ? v[i + o] : v[i], give = up ? v[i] : v[i + o];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 8);
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+}
+
+/* the row of X that row r of the minibatch is: r itself, or (draw) a hash of
+   the step's seed (splitmix64) modulo n, by the quotient's estimate with inv =
+   floor((2^64 - 1) / n), which is short by two at most */
+__device__ __forceinline__ int train_row(int r, int n, unsigned long long inv, unsigned long long seed, int draw)
 {
     if (!draw) return r;
     unsigned long long z = seed + 0x9E3779B97F4A7C15ull * (unsigned long long)(r + 1);
     z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
     z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
     z ^= z >> 31;
-    return (int)(z % (unsigned long long)n);
+    unsigned long long m = z - __umul64hi(z, inv) * (unsigned long long)n;
+    if (m >= (unsigned long long)n) m -= (unsigned long long)n;
+    if (m >= (unsigned long long)n) m -= (unsigned long long)n;
+    return (int)m;
 }
 
 __global__ void __launch_bounds__(kTrThreads, 1)
-    k_train(const __nv_bfloat16* X, const unsigned char* y, int n, int B, unsigned long long seed, int draw,
-            const unsigned char* wpack, const float* P, float* part, float* part_loss, int* part_ok, int* err, int spin)
+    k_train(const __nv_bfloat16* X, const unsigned char* y, int n, int B, unsigned long long inv,
+            unsigned long long seed, int draw, const unsigned char* wpack, const float* P, float* part, float* part_loss, int* part_ok, int* err, int spin)
 {
     extern __shared__ __align__(128) unsigned char sm[];
     unsigned char *sW1 = sm, *sW2 = sW1 + kW1B, *sW3 = sW2 + kW2B;
     unsigned char *sX = sW3 + kW3B, *sA1 = sX + kXB, *sA2 = sA1 + kHB, *sZ = sA2 + kHB;
     float* sb = reinterpret_cast<float*>(sZ + kZB); /* biases; at the end the bias gradients */
-    uint64_t* s_mbar = reinterpret_cast<uint64_t*>(sb + 2 * HID + OUT);
-    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_mbar + 1);
+    int* s_row = reinterpret_cast<int*>(sb + 2 * HID + OUT); /* this tile's and the next one's rows of X */
+    uint64_t* s_mbar = reinterpret_cast<uint64_t*>(s_row + 2 * kTile);
+    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_mbar + 2);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int quad = warp & 3, cg = warp >> 2; /* tensor-memory lane quarter, column group */
     const int row = quad * 32 + lane, c0 = cg * 32;
 
-    for (int i = tid; i < kWB / 16; i += kTrThreads)
-        reinterpret_cast<uint4*>(sm)[i] = reinterpret_cast<const uint4*>(wpack)[i];
+    static_assert(kWB % (16 * kTrThreads) == 0, "whole 16-byte pieces per thread");
+#pragma unroll
+    for (int i = 0; i < kWB / (16 * kTrThreads); i++) {
+        const int o = (i * kTrThreads + tid) * 16;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(sm + o)),
+                     "l"(wpack + o)
+                     : "memory");
+    }
+    /* the rows of a tile, by the last four warps (-1: beyond the batch) */
+    const int ntiles = (B + kTile - 1) / kTile;
+    auto set_rows = [&](int tile, int buf) {
+        const int i = tid - (kTrThreads - kTile), r = tile * kTile + i;
+        if (i < 0) return;
+        const int x = tile < ntiles && r < B ? train_row(r, n, inv, seed, draw) : -1;
+        s_row[buf * kTile + i] = x;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(y + max(x, 0)));
+    };
+    set_rows((int)blockIdx.x, 0);
     for (int i = tid; i < 2 * HID + OUT; i += kTrThreads)
         sb[i] = i < HID ? P[OB1 + i] : (i < 2 * HID ? P[OB2 + i - HID] : P[OB3 + i - 2 * HID]);
-    const uint32_t mb = (uint32_t)__cvta_generic_to_shared(s_mbar);
+    const uint32_t mb = (uint32_t)__cvta_generic_to_shared(s_mbar), mbw = mb + 8;
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbw) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -614,8 +680,8 @@ __global__ void __launch_bounds__(kTrThreads, 1)
                    aW3 = (uint32_t)__cvta_generic_to_shared(sW3), aX = (uint32_t)__cvta_generic_to_shared(sX),
                    aA1 = (uint32_t)__cvta_generic_to_shared(sA1), aA2 = (uint32_t)__cvta_generic_to_shared(sA2),
                    aZ = (uint32_t)__cvta_generic_to_shared(sZ);
-    uint32_t ph = 0u;
-    bool pending = false, fail = false;
+    uint32_t ph = 0u, phw = 0u;
+    bool pending = false, pending_w = false, fail = false;
     /* the tiles written and the accumulator read so far are visible to the
        tensor core; then one thread issues */
     auto ready = [&] {
@@ -626,9 +692,22 @@ __global__ void __launch_bounds__(kTrThreads, 1)
         pending = true;
         return tid == 0;
     };
+    /* the weight-gradient chain: its operands may be overwritten.  A wait that
+       runs out is reported by the next wait() */
+    bool late = false;
+    auto wait_w = [&] {
+        if (!pending_w) return;
+        if (mbar_wait(mbw, phw, spin)) {
+            phw ^= 1u;
+            pending_w = false;
+        } else {
+            late = true;
+        }
+        tc_fence_after();
+    };
     auto wait = [&] {
         const bool ok = mbar_wait(mb, ph, spin);
-        fail = __syncthreads_or(!ok) != 0;
+        fail = __syncthreads_or(!ok || late) != 0;
         if (!fail) {
             ph ^= 1u;
             pending = false;
@@ -636,30 +715,34 @@ __global__ void __launch_bounds__(kTrThreads, 1)
         tc_fence_after();
         return !fail;
     };
-    /* the 12 16-byte chunks of each of a tile's rows, three per thread */
+    /* the 12 16-byte chunks of each of a tile's rows, three per thread.  They
+       are loaded where the backward pass leaves registers, and take no branch,
+       so that nothing waits for them before store_x (loaded earlier they were
+       spilled, which waits); rows beyond the batch load the first row and are
+       stored as zeros. */
     const bool wide = (reinterpret_cast<uintptr_t>(X) & 15) == 0;
     uint4 xr[3];
-    auto load_x = [&](int tile) {
+    auto load_x = [&](int buf) {
+        if (!wide) return;
 #pragma unroll
         for (int i = 0; i < 3; i++) {
-            const int e = tid + i * kTrThreads, r = tile * kTile + e / 12, c = e % 12;
-            xr[i] = make_uint4(0u, 0u, 0u, 0u);
-            if (r >= B) continue;
-            const __nv_bfloat16* src = X + (size_t)train_row(r, n, seed, draw) * IN + c * 8;
-            if (wide) {
-                xr[i] = *reinterpret_cast<const uint4*>(src);
-            } else {
-                const unsigned short* h = reinterpret_cast<const unsigned short*>(src);
-                xr[i] = make_uint4(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16,
-                                   h[4] | (uint32_t)h[5] << 16, h[6] | (uint32_t)h[7] << 16);
-            }
+            const int e = tid + i * kTrThreads, r = max(s_row[buf * kTile + e / 12], 0);
+            xr[i] = __ldg(reinterpret_cast<const uint4*>(X + (size_t)r * IN + e % 12 * 8));
         }
     };
-    auto store_x = [&] {
+    auto store_x = [&](int buf) {
 #pragma unroll
         for (int i = 0; i < 3; i++) {
-            const int e = tid + i * kTrThreads;
-            *reinterpret_cast<uint4*>(sX + tc_off(e / 12, (e % 12) * 8, kTile)) = xr[i];
+            const int e = tid + i * kTrThreads, r = s_row[buf * kTile + e / 12];
+            uint4 x = make_uint4(0u, 0u, 0u, 0u);
+            if (wide) {
+                if (r >= 0) x = xr[i];
+            } else if (r >= 0) {
+                const unsigned short* h = reinterpret_cast<const unsigned short*>(X + (size_t)r * IN + e % 12 * 8);
+                x = make_uint4(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16, h[4] | (uint32_t)h[5] << 16,
+                               h[6] | (uint32_t)h[7] << 16);
+            }
+            *reinterpret_cast<uint4*>(sX + tc_off(e / 12, (e % 12) * 8, kTile)) = x;
         }
     };
     auto pack8 = [](const float* v) {
@@ -675,37 +758,32 @@ __global__ void __launch_bounds__(kTrThreads, 1)
         for (int q = 0; q < 4; q++) {
             float a[8];
 #pragma unroll
-            for (int i = 0; i < 8; i += 2) {
+            for (int i = 0; i < 8; i++) {
                 float* x = v + 8 * q + i;
-                float2 y2, d2;
-                gelu_both(__fadd2_rn(make_float2(x[0], x[1]), *reinterpret_cast<const float2*>(bias + c0 + 8 * q + i)),
-                          &y2, &d2);
-                a[i] = y2.x;
-                a[i + 1] = y2.y;
-                x[0] = d2.x;
-                x[1] = d2.y;
+                gelu_both(*x + bias[c0 + 8 * q + i], &a[i], x);
             }
             *reinterpret_cast<uint4*>(t + tc_off(row, c0 + 8 * q, kTile)) = pack8(a);
         }
     };
 
-    const int ntiles = (B + kTile - 1) / kTile;
-    /* 1 / B where that is exact: a product with it is the quotient */
-    const float inv_b = (B & (B - 1)) == 0 ? 1.0f / (float)B : 0.0f;
+    const float fb = (float)B, rfb = 1.0f / fb;
     float db1 = 0.0f, db2 = 0.0f, db3 = 0.0f, db3b = 0.0f, loss = 0.0f;
     int right = 0;
     bool add = false;
-    int tile = (int)blockIdx.x;
-    load_x(tile);
-    for (; tile < ntiles; tile += (int)gridDim.x) {
-        const int r = tile * kTile + row;
-        store_x();
+    int tile = (int)blockIdx.x, buf = 0;
+    load_x(0);
+    asm volatile("cp.async.wait_all;" ::: "memory"); /* the weights */
+    for (; tile < ntiles; tile += (int)gridDim.x, buf ^= 1) {
+        store_x(buf);
         float g1[32], g2[32];
         if (ready()) {
             tc_chain(tmem, aX, kTile, 0, aW1, HID, 0, HID, IN / 16, false);
             tc_commit(mb);
         }
-        const int yy = r < B ? (int)y[train_row(r, n, seed, draw)] : 0;
+        const int xrow = s_row[buf * kTile + row];
+        const bool valid = xrow >= 0;
+        const int yy = (int)y[max(xrow, 0)];
+        set_rows(tile + (int)gridDim.x, buf ^ 1);
         if (!wait()) break;
         tmem_ld32(lane_base + c0, g1);
         activate(g1, sb, sA1);
@@ -721,8 +799,9 @@ __global__ void __launch_bounds__(kTrThreads, 1)
             tc_commit(mb);
         }
         if (!wait()) break;
+        /* the outputs of a thread: columns 32 g + 8 cg + 0..7, g = 0..4 */
         float z[32], zb[8];
-        tmem_ld32(lane_base + c0, z);
+        tmem_ld8x4(lane_base + cg * 8, z);
         if (ready()) { /* outputs 128..159, eight per column group */
             tc_chain(tmem, aA2, kTile, 0, aW3 + (uint32_t)(kOutA / 8) * 128u, OUT, 0, OUT - kOutA, HID / 16, false);
             tc_commit(mb);
@@ -734,20 +813,22 @@ __global__ void __launch_bounds__(kTrThreads, 1)
         float* sx = reinterpret_cast<float*>(sZ);
         int* sxi = reinterpret_cast<int*>(sx + 4 * kTile);
         float mx = -INFINITY, zt = 0.0f;
-        int am = 0;
+        int am = -1;
+        const int yl = yy < OUT && ((yy >> 3) & 3) == cg ? (yy >> 5) * 8 + (yy & 7) : -1;
+        const float* b3 = sb + 2 * HID + 8 * cg;
 #pragma unroll
         for (int i = 0; i < 32; i++) {
-            z[i] += sb[2 * HID + c0 + i];
-            if (z[i] > mx) { mx = z[i]; am = c0 + i; }
-            if (c0 + i == yy) zt = z[i];
+            z[i] += b3[(i >> 3) * 32 + (i & 7)];
+            if (z[i] > mx) { mx = z[i]; am = i; }
+            if (i == yl) zt = z[i];
         }
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const int c = kOutA + cg * 8 + i;
-            zb[i] += sb[2 * HID + c];
-            if (zb[i] > mx) { mx = zb[i]; am = c; }
-            if (c == yy) zt = zb[i];
+            zb[i] += b3[kOutA + i];
+            if (zb[i] > mx) { mx = zb[i]; am = 32 + i; }
+            if (32 + i == yl) zt = zb[i];
         }
+        am = am < 0 ? 0 : (am >> 3) * 32 + 8 * cg + (am & 7);
         sx[cg * kTile + row] = mx;
         sxi[cg * kTile + row] = am;
         group_sync(1 + quad);
@@ -757,97 +838,110 @@ __global__ void __launch_bounds__(kTrThreads, 1)
             const int a = sxi[q * kTile + row];
             if (m > mx || (m == mx && a < am)) { mx = m; am = a; }
         }
-        float se = 0.0f;
+        /* the sum of the exponentials as a warp with one output in 32 per lane
+           takes it: five outputs in order, then halves of the lanes added */
+        float4* ss = reinterpret_cast<float4*>(sxi + 4 * kTile);
+        float p8[8];
 #pragma unroll
-        for (int i = 0; i < 32; i++) se += z[i] = expf(z[i] - mx);
-#pragma unroll
-        for (int i = 0; i < 8; i++) se += zb[i] = expf(zb[i] - mx);
-        float* sxs = reinterpret_cast<float*>(sxi + 4 * kTile);
-        sxs[cg * kTile + row] = se;
-        group_sync(1 + quad);
-        se = (sxs[row] + sxs[kTile + row]) + (sxs[2 * kTile + row] + sxs[3 * kTile + row]);
-        /* the column group that holds the label counts the row */
-        const int own = yy < kOutA ? yy >> 5 : (yy - kOutA) >> 3;
-        if (r < B && own == cg) loss += -(zt - mx - logf(se));
-        if (r < B && cg == 0 && am == yy) right++;
-        /* e / se, correctly rounded from the row's reciprocal by one residual
-           step (Markstein): the divisor is shared, 1 <= se <= 160 */
-        const float rse = 1.0f / se;
-        auto dz = [&](float e, int c) {
-            const float q0 = e * rse, quo = __fmaf_rn(__fmaf_rn(-q0, se, e), rse, q0);
-            const float d = quo - (c == yy ? 1.0f : 0.0f);
-            return r < B ? (inv_b != 0.0f ? d * inv_b : d / (float)B) : 0.0f;
-        };
-#pragma unroll
-        for (int i = 0; i < 32; i++) z[i] = dz(z[i], c0 + i);
-#pragma unroll
-        for (int i = 0; i < 8; i++) zb[i] = dz(zb[i], kOutA + cg * 8 + i);
-        group_sync(1 + quad); /* the quarter's exchange has been read */
-        __syncthreads();      /* and the other quarters': the tile may be written */
-        store32(sZ, z);
-        *reinterpret_cast<uint4*>(sZ + tc_off(row, kOutA + cg * 8, kTile)) = pack8(zb);
-        if (ready()) {
-            tc_chain(tmem + kTrW3, aA2, kTile, 1, aZ, kTile, 1, OUT, kTile / 16, add);
-            tc_chain(tmem, aZ, kTile, 0, aW3, OUT, 1, HID, OUT / 16, false);
-            tc_commit(mb);
-        }
-        db3 += warp_colsum(z);
+        for (int i = 0; i < 32; i++) z[i] = expf(z[i] - mx);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-#pragma unroll
-            for (int o = 16; o; o >>= 1) zb[i] += __shfl_xor_sync(0xffffffffu, zb[i], o);
-            if (lane == i) db3b += zb[i];
+            zb[i] = expf(zb[i] - mx);
+            p8[i] = (((z[i] + z[i + 8]) + z[i + 16]) + z[i + 24]) + zb[i];
         }
+        ss[2 * cg * kTile + row] = make_float4(p8[0], p8[1], p8[2], p8[3]);
+        ss[(2 * cg + 1) * kTile + row] = make_float4(p8[4], p8[5], p8[6], p8[7]);
+        group_sync(1 + quad);
+        float4 h[2];
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const float4 a0 = ss[q * kTile + row], a1 = ss[(2 + q) * kTile + row], a2 = ss[(4 + q) * kTile + row],
+                         a3 = ss[(6 + q) * kTile + row];
+            h[q] = make_float4((a0.x + a2.x) + (a1.x + a3.x), (a0.y + a2.y) + (a1.y + a3.y),
+                               (a0.z + a2.z) + (a1.z + a3.z), (a0.w + a2.w) + (a1.w + a3.w));
+        }
+        const float se = ((h[0].x + h[1].x) + (h[0].z + h[1].z)) + ((h[0].y + h[1].y) + (h[0].w + h[1].w));
+        /* the column group that holds the label counts the row */
+        if (valid && yl >= 0) loss += -(zt - mx - logf(se));
+        if (valid && cg == 0 && am == yy) right++;
+        /* (e / se - [label]) / B, each quotient correctly rounded from the
+           divisor's reciprocal by one residual step (Markstein; 1 <= se <=
+           160); a row beyond the batch counts nothing */
+        const float rse = 1.0f / se, rb = valid ? rfb : 0.0f;
+        auto quotient = [](float x, float d, float rd) {
+            const float q = x * rd;
+            return __fmaf_rn(__fmaf_rn(-q, d, x), rd, q);
+        };
+        auto dz = [&](float e, int i) { return quotient(quotient(e, se, rse) - (i == yl ? 1.0f : 0.0f), fb, rb); };
+#pragma unroll
+        for (int i = 0; i < 32; i++) z[i] = dz(z[i], i);
+#pragma unroll
+        for (int i = 0; i < 8; i++) zb[i] = dz(zb[i], 32 + i);
+        group_sync(1 + quad); /* the quarter's exchange has been read */
+        __syncthreads();      /* and the other quarters': the tile may be written */
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            *reinterpret_cast<uint4*>(sZ + tc_off(row, 32 * q + 8 * cg, kTile)) = pack8(z + 8 * q);
+        *reinterpret_cast<uint4*>(sZ + tc_off(row, kOutA + cg * 8, kTile)) = pack8(zb);
+        if (ready()) {
+            tc_chain(tmem, aZ, kTile, 0, aW3, OUT, 1, HID, OUT / 16, false);
+            tc_commit(mb);
+            tc_chain(tmem + kTrW3, aA2, kTile, 1, aZ, kTile, 1, OUT, kTile / 16, add);
+            tc_commit(mbw);
+        }
+        pending_w = true;
+        db3 += warp_colsum(z);
+        db3b += warp_colsum8(zb);
         if (!wait()) break;
         float d[32];
         tmem_ld32(lane_base + c0, d);
 #pragma unroll
         for (int i = 0; i < 32; i++) d[i] *= g2[i];
+        wait_w(); /* A2 is read by dW3 */
         store32(sA2, d);
         if (ready()) {
-            tc_chain(tmem + kTrW2, aA1, kTile, 1, aA2, kTile, 1, HID, kTile / 16, add);
             tc_chain(tmem, aA2, kTile, 0, aW2, HID, 1, HID, HID / 16, false);
             tc_commit(mb);
+            tc_chain(tmem + kTrW2, aA1, kTile, 1, aA2, kTile, 1, HID, kTile / 16, add);
+            tc_commit(mbw);
         }
+        pending_w = true;
         db2 += warp_colsum(d);
-        load_x(tile + (int)gridDim.x); /* rows beyond the batch: zeros, not used */
         if (!wait()) break;
         tmem_ld32(lane_base + c0, d);
 #pragma unroll
         for (int i = 0; i < 32; i++) d[i] *= g1[i];
+        wait_w(); /* A1 is read by dW2 */
         store32(sA1, d);
         if (ready()) {
             tc_chain(tmem + kTrW1, aA1, kTile, 1, aX, kTile, 1, IN, kTile / 16, add);
             tc_commit(mb);
         }
+        load_x(buf ^ 1);
         db1 += warp_colsum(d);
         if (!wait()) break;
         add = true;
     }
     if (fail && tid == 0) atomicOr(err, 1);
     if (pending) (void)mbar_wait(mb, ph);
+    if (pending_w) (void)mbar_wait(mbw, phw);
     if (!fail) {
-        /* the CTA's partial gradient: dW3 and dW2 by rows of the lane's input
-           unit, dW1^T by the lane's output unit */
+        /* the CTA's partial gradient, in the order of part_param: a warp's
+           stores are contiguous */
         float* G = part + (size_t)blockIdx.x * NPARAM;
         float v[32];
         for (int b = cg; b < (OUT + HID + IN) / 32; b += 4) {
             tmem_ld32(lane_base + kTrW3 + b * 32, v);
-            if (b < OUT / 32 + HID / 32) {
-                float* o = b < OUT / 32 ? G + OW3 + row * OUT + b * 32 : G + OW2 + row * HID + (b - OUT / 32) * 32;
 #pragma unroll
-                for (int i = 0; i < 32; i += 4)
-                    *reinterpret_cast<float4*>(o + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-            } else {
-#pragma unroll
-                for (int i = 0; i < 32; i++) G[OW1 + ((b - (OUT + HID) / 32) * 32 + i) * HID + row] = v[i];
-            }
+            for (int i = 0; i < 32; i += 4)
+                *reinterpret_cast<float4*>(G + ((b * 8 + i / 4) * kTile + row) * 4) =
+                    make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
         }
         /* bias gradients: the four row quarters in order, through the dZ3 tile */
         float* sg = reinterpret_cast<float*>(sZ) + quad * (2 * HID + OUT);
         sg[c0 + lane] = db1;
         sg[HID + c0 + lane] = db2;
-        sg[2 * HID + c0 + lane] = db3;
+        sg[2 * HID + (lane >> 3) * 32 + 8 * cg + (lane & 7)] = db3;
         if (lane < 8) sg[2 * HID + kOutA + cg * 8 + lane] = db3b;
         float* sl = reinterpret_cast<float*>(sA1);
         int* sr = reinterpret_cast<int*>(sA2);
@@ -862,8 +956,7 @@ __global__ void __launch_bounds__(kTrThreads, 1)
         const float* s4 = reinterpret_cast<const float*>(sZ);
         constexpr int NB = 2 * HID + OUT;
         for (int i = tid; i < NB; i += kTrThreads)
-            G[i < HID ? OB1 + i : (i < 2 * HID ? OB2 + i - HID : OB3 + i - 2 * HID)] =
-                (s4[i] + s4[NB + i]) + (s4[2 * NB + i] + s4[3 * NB + i]);
+            G[NWEIGHT + i] = (s4[i] + s4[NB + i]) + (s4[2 * NB + i] + s4[3 * NB + i]);
         if (tid == 0) {
             float l = 0.0f;
             int k = 0;
@@ -880,6 +973,22 @@ __global__ void __launch_bounds__(kTrThreads, 1)
     tc_fence_after();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTrCols) : "memory");
+}
+
+/* the parameter that entry j of a partial gradient belongs to.  The weights'
+   entries are tensor-memory columns dW3 | dW2 | dW1^T in fours, by lanes: a
+   lane is the input unit of W3 and W2 and the output unit of W1; then the
+   biases b1 | b2 | b3. */
+__device__ __forceinline__ int part_param(int j)
+{
+    if (j >= NWEIGHT) {
+        const int i = j - NWEIGHT;
+        return i < HID ? OB1 + i : (i < 2 * HID ? OB2 + i - HID : OB3 + i - 2 * HID);
+    }
+    const int c = j / (4 * kTile) * 4 + (j & 3), l = (j >> 2) & (kTile - 1);
+    if (c < OUT) return OW3 + l * OUT + c;
+    if (c < OUT + HID) return OW2 + l * HID + c - OUT;
+    return OW1 + (c - OUT - HID) * HID + l;
 }
 
 /* place of parameter i of the flat array in the packed weights (-1: a bias) */
@@ -911,11 +1020,11 @@ __global__ void __launch_bounds__(256) k_reduce_adam(const float* part, int npar
 {
     __shared__ float s[8][33];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int i = blockIdx.x * 32 + lane;
+    const int j = blockIdx.x * 32 + lane;
     float a = 0.0f;
-    if (i < NPARAM) {
+    if (j < NPARAM) {
 #pragma unroll 10
-        for (int q = w; q < nparts; q += 8) a += part[(size_t)q * NPARAM + i];
+        for (int q = w; q < nparts; q += 8) a += part[(size_t)q * NPARAM + j];
     }
     s[w][lane] = a;
     __syncthreads();
@@ -934,7 +1043,8 @@ __global__ void __launch_bounds__(256) k_reduce_adam(const float* part, int npar
             *right = k;
         }
     }
-    if (w != 0 || i >= NPARAM) return;
+    if (w != 0 || j >= NPARAM) return;
+    const int i = part_param(j);
     float gi = s[0][lane];
 #pragma unroll
     for (int q = 1; q < 8; q++) gi += s[q][lane];
@@ -1185,8 +1295,11 @@ static ecmg_status ensure_train(ecmg_mlp* mm, int steps)
 static cudaError_t train_step(ecmg_mlp* mm, const void* X, const unsigned char* y, int n, int B,
                               unsigned long long seed, int draw, int at, float lr, float c1, float c2)
 {
-    const int grid = std::min(mm->parts, (B + kTile - 1) / kTile);
-    k_train<<<grid, kTrThreads, kTrainSmem, mm->s>>>((const __nv_bfloat16*)X, y, n, B, seed, draw, mm->tpack, mm->p,
+    /* as few CTAs as give every one the same number of tiles: each writes a
+       partial gradient of 213 KB */
+    const int tiles = (B + kTile - 1) / kTile, rounds = (tiles + mm->parts - 1) / mm->parts;
+    const int grid = (tiles + rounds - 1) / rounds;
+    k_train<<<grid, kTrThreads, kTrainSmem, mm->s>>>((const __nv_bfloat16*)X, y, n, B, ~0ull / (unsigned)n, seed, draw, mm->tpack, mm->p,
                                                      mm->part, mm->part_loss, mm->part_ok, mm->gerr, mm->spin);
     k_reduce_adam<<<(NPARAM + 31) / 32, 256, 0, mm->s>>>(mm->part, grid, mm->g, mm->p, mm->m, mm->v, mm->tpack, lr,
                                                          kBeta1, kBeta2, 1e-8f, c1, c2, mm->part_loss, mm->part_ok,
