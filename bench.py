@@ -439,23 +439,15 @@ def run_ours(args):
     # velocity, active flag, slot, neighbour count and k indices, and writes
     # pos and vel
     kern = {"k_neighbors": (main_t.tot["neighbors_ms"], 8 + 4 * k), "k_agents": (main_t.tot["orca_ms"], 57 + 4 * k)}
-    fused = launch.get("lp_mode") == "fused" and args.neighbors != "kdtree"
-    if fused:
-        # the search inside the per-agent kernel: the agent's state in and
-        # out (snapshot pos, vel, radius, speed, preferred velocity, active
-        # flag, slot in; pos, vel out); the lists it writes and reads back
-        # are intermediate
-        kern = {"k_agents_knn": (main_t.tot["orca_ms"], 53)}
     if args.neighbors == "kdtree":
         # the kd-tree pipeline (build, query, cache composition) in place of
-        # k_neighbors; its algorithmic bytes per agent are derived in DESIGN
+        # k_neighbors (KD_BYTES_PER_AGENT)
         kern = {"kd-tree pipeline": (main_t.tot["neighbors_ms"], KD_BYTES_PER_AGENT(k, (n + spawn_slots).bit_length())),
                 "k_agents": (main_t.tot["orca_ms"], 57 + 4 * k)}
-    kernel_ms = {"k_attract": main_t.tot["attract_ms"] / args.steps}
-    if not fused:
-        kernel_ms["k_neighbors"] = main_t.tot["neighbors_ms"] / args.steps
+    kernel_ms = {"k_attract": main_t.tot["attract_ms"] / args.steps,
+                 "k_neighbors": main_t.tot["neighbors_ms"] / args.steps}
     kernel_ms["features+k_mlp_infer"] = main_t.tot["proposal_ms"] / args.steps
-    kernel_ms["k_agents_knn" if fused else "k_agents"] = main_t.tot["orca_ms"] / args.steps
+    kernel_ms["k_agents"] = main_t.tot["orca_ms"] / args.steps
     kname = max(kern, key=lambda q: kern[q][0])
     kern_ms = kern[kname][0] / max(args.steps, 1)
     alg_bytes = kern[kname][1]

@@ -61,9 +61,11 @@ __global__ void k_bin(BinArgs a)
    Three launches bin a tick: k_bin, k_scan (every block scans its 4,096
    counts in place; the last block to finish scans the block sums) and
    k_scatter (adds the block sums while it places the agents, and writes the
-   final bucket starts).  The launches bound it, not the work: with a scan of
-   three launches and a clearing of the counts in front (now k_attract's) the
-   binning of 1,000 agents took 25 us of the tick, this takes 12. */
+   final bucket starts).  The launches bound small crowds: with a scan of
+   three launches and a clearing of the counts in front (now k_attract's) a
+   tick of 1,000 agents took 95 us of device time, with this and the 64-byte
+   edge records 72.  At a million 14.8, 8.1 and 36.1 us: k_scatter is bound by
+   its scattered sectors (four slots in flight per thread: 37 -> 42). */
 constexpr int kScanBlock = 1024, kScanPer = 4, kScanTile = kScanBlock * kScanPer;
 
 __device__ __forceinline__ int block_exclusive_scan(int v, int* sh, int* total)
@@ -151,7 +153,9 @@ __global__ void k_scatter(BinArgs a)
 
 /* the whole binning of up to kSmallSlots slots by one block, the counts in
    shared memory: below that size the three launches' latency is all there is
-   (1,000 agents: three launches 12 us of the tick, this 5) */
+   (1,000 agents: with three launches the tick's device time 72 us, with this
+   65; the kernel 8.3 us under ncu).  The line is what a block's shared memory
+   and registers hold. */
 constexpr int kSmallSlots = 8192, kSmallCells = 11264, kSmallBlock = 1024;
 __global__ void __launch_bounds__(kSmallBlock) k_bin_small(BinArgs a)
 {
@@ -596,7 +600,11 @@ __device__ void orca_tick(const TickArgs& a, int t)
 /* neighbour lists of every grid-order agent of the tick (knn_rows.cuh).
    Persistent: a warp takes 32 consecutive grid-order agents per work grab
    (neighbouring agents: their candidates share L1), so that warps whose
-   agents have more candidates do not leave the SMs' last wave ragged */
+   agents have more candidates do not leave the SMs' last wave ragged.  Bound
+   by instruction issue: 156 warp instructions per agent at 29.9 of 32 threads
+   (250,000 of the crossing); a million 302 us beside k_attract (416 with one
+   insertion per candidate and cells in distance order), 25,000 26 (86-105,
+   where a cell of more than 32 agents sent its lanes to the 64-bit search) */
 constexpr int kNbrWarps = 4; /* per block */
 template <int K>
 __global__ void __launch_bounds__(32 * kNbrWarps, K <= 16 ? 8 : 4) k_neighbors(TickArgs a)
@@ -855,7 +863,8 @@ __global__ void __launch_bounds__(256, (K <= 16) ? 4 : 1) k_agents(TickArgs a)
 }
 
 /* G lanes per agent (orca_group.cuh): a warp steps 32 / G consecutive
-   grid-order agents */
+   grid-order agents.  Bound by an agent's chain of half-planes and LP steps;
+   the figures by G and agent count are at lanes_of in ctx.cu */
 template <int K, int G, bool FULL>
 __global__ void __launch_bounds__(32 * kGroupWarps, K <= 16 ? 7 : 4) k_agents_group(TickArgs a)
 {

@@ -489,15 +489,16 @@ __global__ void __launch_bounds__(kInferThreads, 1)
  * (accurate tanh, exp and quotients of 416 activations per row) at the four
  * warps per scheduler that the registers leave: of a tile's 35,000 cycles the
  * two activations take 8,700, the softmax 8,500, waiting for chains and
- * barriers 9,000; the scheduler issues in 44 % of them.  65,536 rows: 85 us
- * (107 us with a 64-bit remainder per loaded chunk, a divide per output and
- * weights loaded through registers) and 14 us for k_reduce_adam; a step took
- * 722 us as 24 launches that passed every activation, its transpose and its
- * BF16 copy through memory, with a two-block column sum for each bias
- * gradient.
+ * barriers 9,000; the scheduler issues in 44 % of them.  Four steps of 65,536
+ * rows take 417 us (4 x 14 of it k_reduce_adam); 505 with a 64-bit remainder
+ * per loaded chunk (5,400 cycles a tile), a divide per output (5,300) and the
+ * weights loaded through registers; 2,890 as 4 x 24 launches that passed
+ * every activation, its transpose and its BF16 copy through memory, with a
+ * two-block column sum for each bias gradient.
  * ---------------------------------------------------------------------- */
 constexpr int OW1 = 0, OB1 = OW1 + IN * HID, OW2 = OB1 + HID, OB2 = OW2 + HID * HID, OW3 = OB2 + HID,
-              OB3 = OW3 + HID * OUT, NPARAM = OB3 + OUT, NWEIGHT = HID * (IN + HID + OUT); /* W1 [IN x HID], b1, W2 [HID x HID], b2, W3 [HID x OUT], b3 */
+              OB3 = OW3 + HID * OUT, NPARAM = OB3 + OUT; /* W1 [IN x HID], b1, W2 [HID x HID], b2, W3 [HID x OUT], b3 */
+constexpr int NWEIGHT = HID * (IN + HID + OUT);
 constexpr int kTrThreads = 512, kTrCols = 512; /* tensor memory: all of it */
 constexpr int kTrW3 = 128, kTrW2 = kTrW3 + OUT, kTrW1 = kTrW2 + HID; /* first columns of dW3, dW2, dW1^T */
 static_assert(kTrW1 + IN == kTrCols, "the weight gradients fill the tensor memory");
@@ -1012,7 +1013,9 @@ __global__ void k_pack_all(const float* p, unsigned char* pack)
 
 /* gradient = sum of the partial gradients (the same order on every run), then
    the Adam step on it (lr > 0) with the BF16 copy of the new weights.  A warp
-   sums an eighth of the partials of 32 parameters; block 0 adds up the loss. */
+   sums an eighth of the partials of 32 parameters; block 0 adds up the loss.
+   Bound by reading the partials: 128 of 198 KB, 14 us from DRAM, less from L2,
+   where k_train has just written them. */
 __global__ void __launch_bounds__(256) k_reduce_adam(const float* part, int nparts, float* g, float* p, float* m,
                                                      float* v, unsigned char* pack, float lr, float b1, float b2,
                                                      float eps, float c1, float c2, const float* part_loss,
@@ -1296,7 +1299,7 @@ static cudaError_t train_step(ecmg_mlp* mm, const void* X, const unsigned char* 
                               unsigned long long seed, int draw, int at, float lr, float c1, float c2)
 {
     /* as few CTAs as give every one the same number of tiles: each writes a
-       partial gradient of 213 KB */
+       partial gradient of 198 KB (65,536 rows: 128 CTAs, not 152) */
     const int tiles = (B + kTile - 1) / kTile, rounds = (tiles + mm->parts - 1) / mm->parts;
     const int grid = (tiles + rounds - 1) / rounds;
     k_train<<<grid, kTrThreads, kTrainSmem, mm->s>>>((const __nv_bfloat16*)X, y, n, B, ~0ull / (unsigned)n, seed, draw, mm->tpack, mm->p,

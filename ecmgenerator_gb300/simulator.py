@@ -508,9 +508,10 @@ def set_launch(sim: Simulator, block_size: int, agents_per_warp_grab: int, grid_
 
 
 def set_lp_mode(sim: Simulator, mode: str = "warp", agents_per_warp_grab: int = 4):
-    """per-agent kernel layout: "thread" (one thread per agent), "warp"
-    (one warp per agent) or "fused" (one thread per agent, the neighbour
-    search in the same kernel); results are identical"""
+    """per-agent kernel layout: "thread" (one thread per agent), "warp" (a
+    warp takes agents_per_warp_grab agents side by side: 32 lanes per agent
+    for 1, 16 for 2, 8 for 4, 4 for 8) or "fused" (runs as "thread"); unless
+    called, the tick chooses by the agent count; results are identical"""
     m = {"thread": 0, "warp": 1, "fused": 2}[mode]
     sim._ck(sim.L.ecmg_set_lp_mode(sim.h, m, int(agents_per_warp_grab)))
 

@@ -355,24 +355,24 @@ typedef struct {
     int trials;
     int lp_mode;             /* ECMG_LP_THREAD, ECMG_LP_WARP or ECMG_LP_THREAD_FUSED */
     int occupancy_divisor;   /* per-thread layout: resident blocks per SM divided by this */
-    int neighbor_blocks_per_sm; /* exact-kNN kernel (k <= 16): 8 resident blocks at 64 registers or 6 at 80 */
+    int neighbor_blocks_per_sm; /* exact-kNN kernel: blocks of its grid per SM */
 } ecmg_tune_result;
 ecmg_status ecmg_set_launch(ecmg_ctx* ctx, int block_size, int agents_per_warp_grab, float grid_cell_scale);
-/* Per-agent kernel layout.  ECMG_LP_THREAD: one thread per agent (work
-   grabs of agents_per_warp_grab from ecmg_set_launch).  ECMG_LP_WARP: one
-   warp per agent -- the lanes build the constraints in parallel and share
-   the inner loops of the LPs -- taking agents_per_warp_grab agents per work
-   grab (1..64).  ECMG_LP_THREAD_FUSED: the per-thread layout with the
-   neighbour search in the same kernel (each thread finds its agent's k
-   nearest, then steps it; the separate search kernel is skipped; with a
-   learned proposal or the kd-tree neighbour mode the per-thread layout runs
-   instead).  All give identical results. */
+/* Per-agent kernel layout.  Unless set, the tick chooses by the agent count:
+   8 lanes per agent to 8,000 agents, 4 to 160,000 (and always in the kd-tree
+   neighbour mode), one thread per agent above.  ECMG_LP_THREAD: one thread
+   per agent (work grabs of agents_per_warp_grab from ecmg_set_launch).
+   ECMG_LP_WARP: a warp takes agents_per_warp_grab agents (1..64) side by
+   side -- 32 lanes per agent for 1, 16 for 2 or 3, 8 for 4 to 7, 4 for 8 and
+   more -- whose lanes build the constraints in parallel and share the inner
+   loops of the LPs.  ECMG_LP_THREAD_FUSED: runs as ECMG_LP_THREAD.  All give
+   identical results. */
 /* per-thread layout: run the persistent per-agent kernel with the resident
    blocks per SM divided by `divisor` (1..8; fewer resident warps leave more
    L1 to each thread's local constraint arrays) */
 ecmg_status ecmg_set_occupancy(ecmg_ctx* ctx, int divisor);
-/* exact-kNN kernel for k <= 16: 8 resident blocks of 128 threads per SM
-   (64 registers) or 6 (80 registers, no spills); the autotuner picks one */
+/* exact-kNN kernel: at most this many blocks of 128 threads per SM (its
+   grid; 6 or 8); the autotuner picks one */
 ecmg_status ecmg_set_neighbor_blocks(ecmg_ctx* ctx, int blocks_per_sm);
 #define ECMG_LP_THREAD 0
 #define ECMG_LP_WARP 1
@@ -386,9 +386,8 @@ ecmg_status ecmg_set_lp_mode(ecmg_ctx* ctx, int mode, int agents_per_warp_grab);
    (ORCA.h:87,100) -- i.e. the neighbour lists of the unmodified
    Simulator::Update; agents whose x (or y) coordinates are equal keep the
    order of the level above (std::sort agrees on subtrees of up to 16 agents).
-   neighbor_dist is not used.  Runs the per-agent kernel one thread per agent,
-   without the learned proposal or the trace; single-scene contexts, up to
-   2^24 slots. */
+   neighbor_dist is not used.  Runs without the learned proposal or the trace;
+   single-scene contexts, up to 2^24 slots. */
 #define ECMG_NEIGHBORS_EXACT 0
 #define ECMG_NEIGHBORS_KDTREE 1
 ecmg_status ecmg_set_neighbor_mode(ecmg_ctx* ctx, int mode);
