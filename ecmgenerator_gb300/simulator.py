@@ -341,9 +341,10 @@ class Simulator:
                 arr = np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_float)), shape=(n,))
             else:
                 arr = np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_float)), shape=(n, 2))
-            arr.flags.writeable = False
             kept = self._views[field] = (p.value, arr)
-        return kept[1].view()
+        arr = kept[1].view()
+        arr.flags.writeable = False
+        return arr
 
     def get_num_agents(self) -> int:
         n = C.c_int()
