@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
  * warps per scheduler that the registers leave: of a tile's 35,000 cycles the
  * two activations take 8,700, the softmax 8,500, waiting for chains and
  * barriers 9,000; the scheduler issues in 44 % of them.  Four steps of 65,536
- * rows take 417 us (4 x 14 of it k_reduce_adam); 505 with a 64-bit remainder
+ * rows take 403 us; 505 with a 64-bit remainder
  * per loaded chunk (5,400 cycles a tile), a divide per output (5,300) and the
  * weights loaded through registers; 2,890 as 4 x 24 launches that passed
  * every activation, its transpose and its BF16 copy through memory, with a
@@ -1013,25 +1013,44 @@ __global__ void k_pack_all(const float* p, unsigned char* pack)
 
 /* gradient = sum of the partial gradients (the same order on every run), then
    the Adam step on it (lr > 0) with the BF16 copy of the new weights.  A warp
-   sums an eighth of the partials of 32 parameters; block 0 adds up the loss.
-   Bound by reading the partials: 128 of 198 KB, 14 us from DRAM, less from L2,
-   where k_train has just written them. */
+   sums an eighth of the partials of 128 parameters, four per lane; block 0 adds
+   up the loss.  Bound by reading the partials (128 of 198 KB) out of L2, where
+   k_train has just written them: 16-byte loads and 388 blocks, one wave, in
+   place of 4-byte loads and 1,549 blocks, and the weights and moments loaded
+   ahead of the sum (four training steps 417 -> 403 us). */
+constexpr int kRedParams = 128;
+static_assert(NPARAM % 4 == 0, "a partial gradient is read in fours");
 __global__ void __launch_bounds__(256) k_reduce_adam(const float* part, int nparts, float* g, float* p, float* m,
                                                      float* v, unsigned char* pack, float lr, float b1, float b2,
                                                      float eps, float c1, float c2, const float* part_loss,
                                                      const int* part_ok, float* loss, int* right)
 {
-    __shared__ float s[8][33];
+    __shared__ float s[8][kRedParams];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int j = blockIdx.x * 32 + lane;
-    float a = 0.0f;
-    if (j < NPARAM) {
-#pragma unroll 10
-        for (int q = w; q < nparts; q += 8) a += part[(size_t)q * NPARAM + j];
+    const int j = blockIdx.x * kRedParams + (int)threadIdx.x;
+    const bool mine = threadIdx.x < kRedParams && j < NPARAM;
+    const int i = mine ? part_param(j) : 0;
+    float p0 = 0.0f, m0 = 0.0f, v0 = 0.0f;
+    if (mine && lr > 0.0f) {
+        p0 = p[i];
+        m0 = m[i];
+        v0 = v[i];
     }
-    s[w][lane] = a;
+    const int j4 = blockIdx.x * kRedParams + 4 * lane;
+    float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (j4 < NPARAM) {
+#pragma unroll 8
+        for (int q = w; q < nparts; q += 8) {
+            const float4 x = *reinterpret_cast<const float4*>(part + (size_t)q * NPARAM + j4);
+            a.x += x.x;
+            a.y += x.y;
+            a.z += x.z;
+            a.w += x.w;
+        }
+    }
+    *reinterpret_cast<float4*>(&s[w][4 * lane]) = a;
     __syncthreads();
-    if (blockIdx.x == 0 && w == 1) {
+    if (blockIdx.x == 0 && w == 7) {
         float l = 0.0f;
         int k = 0;
         for (int q = lane; q < nparts; q += 32) {
@@ -1046,18 +1065,17 @@ __global__ void __launch_bounds__(256) k_reduce_adam(const float* part, int npar
             *right = k;
         }
     }
-    if (w != 0 || j >= NPARAM) return;
-    const int i = part_param(j);
-    float gi = s[0][lane];
+    if (!mine) return;
+    float gi = s[0][threadIdx.x];
 #pragma unroll
-    for (int q = 1; q < 8; q++) gi += s[q][lane];
+    for (int q = 1; q < 8; q++) gi += s[q][threadIdx.x];
     g[i] = gi;
     if (!(lr > 0.0f)) return;
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+    const float mi = b1 * m0 + (1.0f - b1) * gi;
+    const float vi = b2 * v0 + (1.0f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    const float pn = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    const float pn = p0 - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     p[i] = pn;
     const int o = pack_off(i);
     if (o >= 0) *reinterpret_cast<__nv_bfloat16*>(pack + o) = __float2bfloat16_rn(pn);
@@ -1304,7 +1322,7 @@ static cudaError_t train_step(ecmg_mlp* mm, const void* X, const unsigned char* 
     const int grid = (tiles + rounds - 1) / rounds;
     k_train<<<grid, kTrThreads, kTrainSmem, mm->s>>>((const __nv_bfloat16*)X, y, n, B, ~0ull / (unsigned)n, seed, draw, mm->tpack, mm->p,
                                                      mm->part, mm->part_loss, mm->part_ok, mm->gerr, mm->spin);
-    k_reduce_adam<<<(NPARAM + 31) / 32, 256, 0, mm->s>>>(mm->part, grid, mm->g, mm->p, mm->m, mm->v, mm->tpack, lr,
+    k_reduce_adam<<<(NPARAM + kRedParams - 1) / kRedParams, 256, 0, mm->s>>>(mm->part, grid, mm->g, mm->p, mm->m, mm->v, mm->tpack, lr,
                                                          kBeta1, kBeta2, 1e-8f, c1, c2, mm->part_loss, mm->part_ok,
                                                          mm->hist_loss + at, mm->hist_ok + at);
     return cudaGetLastError();
