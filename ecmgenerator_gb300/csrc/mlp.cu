@@ -490,9 +490,9 @@ __global__ void __launch_bounds__(kInferThreads, 1)
  * warps per scheduler that the registers leave: of a tile's 35,000 cycles the
  * two activations take 8,700, the softmax 8,500, waiting for chains and
  * barriers 9,000; the scheduler issues in 44 % of them.  Four steps of 65,536
- * rows take 403 us; 505 with a 64-bit remainder
- * per loaded chunk (5,400 cycles a tile), a divide per output (5,300) and the
- * weights loaded through registers; 2,890 as 4 x 24 launches that passed
+ * rows take 393 us; 505 with a 64-bit remainder per loaded chunk (5,400
+ * cycles a tile), a divide per output (5,300), the weights loaded through
+ * registers and a start that waits for the step before; 2,890 as 4 x 24 launches that passed
  * every activation, its transpose and its BF16 copy through memory, with a
  * two-block column sum for each bias gradient.
  * ---------------------------------------------------------------------- */
@@ -639,14 +639,6 @@ __global__ void __launch_bounds__(kTrThreads, 1)
     const int quad = warp & 3, cg = warp >> 2; /* tensor-memory lane quarter, column group */
     const int row = quad * 32 + lane, c0 = cg * 32;
 
-    static_assert(kWB % (16 * kTrThreads) == 0, "whole 16-byte pieces per thread");
-#pragma unroll
-    for (int i = 0; i < kWB / (16 * kTrThreads); i++) {
-        const int o = (i * kTrThreads + tid) * 16;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(sm + o)),
-                     "l"(wpack + o)
-                     : "memory");
-    }
     /* the rows of a tile, by the last four warps (-1: beyond the batch) */
     const int ntiles = (B + kTile - 1) / kTile;
     auto set_rows = [&](int tile, int buf) {
@@ -657,8 +649,6 @@ __global__ void __launch_bounds__(kTrThreads, 1)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(y + max(x, 0)));
     };
     set_rows((int)blockIdx.x, 0);
-    for (int i = tid; i < 2 * HID + OUT; i += kTrThreads)
-        sb[i] = i < HID ? P[OB1 + i] : (i < 2 * HID ? P[OB2 + i - HID] : P[OB3 + i - 2 * HID]);
     const uint32_t mb = (uint32_t)__cvta_generic_to_shared(s_mbar), mbw = mb + 8;
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
@@ -773,7 +763,20 @@ __global__ void __launch_bounds__(kTrThreads, 1)
     bool add = false;
     int tile = (int)blockIdx.x, buf = 0;
     load_x(0);
-    asm volatile("cp.async.wait_all;" ::: "memory"); /* the weights */
+    /* everything above reads the minibatch only; from here on the weights that
+       the kernel before writes, and the partial gradients that it reads */
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    static_assert(kWB % (16 * kTrThreads) == 0, "whole 16-byte pieces per thread");
+#pragma unroll
+    for (int i = 0; i < kWB / (16 * kTrThreads); i++) {
+        const int o = (i * kTrThreads + tid) * 16;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(sm + o)),
+                     "l"(wpack + o)
+                     : "memory");
+    }
+    for (int i = tid; i < 2 * HID + OUT; i += kTrThreads)
+        sb[i] = i < HID ? P[OB1 + i] : (i < 2 * HID ? P[OB2 + i - HID] : P[OB3 + i - 2 * HID]);
+    asm volatile("cp.async.wait_all;" ::: "memory");
     for (; tile < ntiles; tile += (int)gridDim.x, buf ^= 1) {
         store_x(buf);
         float g1[32], g2[32];
@@ -1005,6 +1008,7 @@ __device__ __forceinline__ int pack_off(int i)
 
 __global__ void k_pack_all(const float* p, unsigned char* pack)
 {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); /* k_train's start */
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= NPARAM) return;
     const int o = pack_off(i);
@@ -1025,6 +1029,7 @@ __global__ void __launch_bounds__(256) k_reduce_adam(const float* part, int npar
                                                      float eps, float c1, float c2, const float* part_loss,
                                                      const int* part_ok, float* loss, int* right)
 {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); /* the next step's k_train */
     __shared__ float s[8][kRedParams];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int j = blockIdx.x * kRedParams + (int)threadIdx.x;
@@ -1320,8 +1325,24 @@ static cudaError_t train_step(ecmg_mlp* mm, const void* X, const unsigned char* 
        partial gradient of 198 KB (65,536 rows: 128 CTAs, not 152) */
     const int tiles = (B + kTile - 1) / kTile, rounds = (tiles + mm->parts - 1) / mm->parts;
     const int grid = (tiles + rounds - 1) / rounds;
-    k_train<<<grid, kTrThreads, kTrainSmem, mm->s>>>((const __nv_bfloat16*)X, y, n, B, ~0ull / (unsigned)n, seed, draw, mm->tpack, mm->p,
-                                                     mm->part, mm->part_loss, mm->part_ok, mm->gerr, mm->spin);
+    /* its start -- tensor memory, row indices, the first rows -- runs beside the
+       end of the kernel before, whose weights it waits for (four steps 402 ->
+       393 us, 3,001 rows 65 -> 62) */
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kTrThreads);
+    cfg.dynamicSmemBytes = kTrainSmem;
+    cfg.stream = mm->s;
+    cudaLaunchAttribute pdl{};
+    pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &pdl;
+    cfg.numAttrs = 1;
+    const cudaError_t e =
+        cudaLaunchKernelEx(&cfg, k_train, (const __nv_bfloat16*)X, y, n, B, ~0ull / (unsigned)n, seed, draw,
+                           (const unsigned char*)mm->tpack, (const float*)mm->p, mm->part, mm->part_loss, mm->part_ok,
+                           mm->gerr, mm->spin);
+    if (e != cudaSuccess) return e;
     k_reduce_adam<<<(NPARAM + kRedParams - 1) / kRedParams, 256, 0, mm->s>>>(mm->part, grid, mm->g, mm->p, mm->m, mm->v, mm->tpack, lr,
                                                          kBeta1, kBeta2, 1e-8f, c1, c2, mm->part_loss, mm->part_ok,
                                                          mm->hist_loss + at, mm->hist_ok + at);
