@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(kInferThreads, 1)
  * warps per scheduler that the registers leave: of a tile's 35,000 cycles the
  * two activations take 8,700, the softmax 8,500, waiting for chains and
  * barriers 9,000; the scheduler issues in 44 % of them.  Four steps of 65,536
- * rows take 393 us; 505 with a 64-bit remainder per loaded chunk (5,400
+ * rows take 381 us; 505 with a 64-bit remainder per loaded chunk (5,400
  * cycles a tile), a divide per output (5,300), the weights loaded through
  * registers and a start that waits for the step before; 2,890 as 4 x 24 launches that passed
  * every activation, its transpose and its BF16 copy through memory, with a
@@ -972,6 +972,7 @@ __global__ void __launch_bounds__(kTrThreads, 1)
             part_ok[blockIdx.x] = k;
         }
     }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); /* k_reduce_adam */
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1035,6 +1036,9 @@ __global__ void __launch_bounds__(256) k_reduce_adam(const float* part, int npar
     const int j = blockIdx.x * kRedParams + (int)threadIdx.x;
     const bool mine = threadIdx.x < kRedParams && j < NPARAM;
     const int i = mine ? part_param(j) : 0;
+    /* after k_train's end, which comes after the last step's (the parameters
+       and moments below) */
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     float p0 = 0.0f, m0 = 0.0f, v0 = 0.0f;
     if (mine && lr > 0.0f) {
         p0 = p[i];
@@ -1327,7 +1331,10 @@ static cudaError_t train_step(ecmg_mlp* mm, const void* X, const unsigned char* 
     const int grid = (tiles + rounds - 1) / rounds;
     /* its start -- tensor memory, row indices, the first rows -- runs beside the
        end of the kernel before, whose weights it waits for (four steps 402 ->
-       393 us, 3,001 rows 65 -> 62) */
+       393 us, 3,001 rows 65 -> 62).  The reduction is launched the same way: its
+       blocks are let in as the CTAs end, not before, where they would crowd on
+       the SMs that have no tile (393 -> 381; let in before the partial gradients
+       are written: 398) */
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kTrThreads);
@@ -1343,10 +1350,12 @@ static cudaError_t train_step(ecmg_mlp* mm, const void* X, const unsigned char* 
                            (const unsigned char*)mm->tpack, (const float*)mm->p, mm->part, mm->part_loss, mm->part_ok,
                            mm->gerr, mm->spin);
     if (e != cudaSuccess) return e;
-    k_reduce_adam<<<(NPARAM + kRedParams - 1) / kRedParams, 256, 0, mm->s>>>(mm->part, grid, mm->g, mm->p, mm->m, mm->v, mm->tpack, lr,
-                                                         kBeta1, kBeta2, 1e-8f, c1, c2, mm->part_loss, mm->part_ok,
-                                                         mm->hist_loss + at, mm->hist_ok + at);
-    return cudaGetLastError();
+    cfg.gridDim = dim3((NPARAM + kRedParams - 1) / kRedParams);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = 0;
+    return cudaLaunchKernelEx(&cfg, k_reduce_adam, (const float*)mm->part, grid, mm->g, mm->p, mm->m, mm->v, mm->tpack, lr,
+                              kBeta1, kBeta2, 1e-8f, c1, c2, (const float*)mm->part_loss, (const int*)mm->part_ok,
+                              mm->hist_loss + at, mm->hist_ok + at);
 }
 
 ecmg_status ecmg_mlp_loss_grad(ecmg_mlp* mm, const void* dev_x, const unsigned char* dev_y, int n, float* loss,
