@@ -30,6 +30,7 @@
  * the cache the next tick starts from.
  */
 #include "ecmg_internal.h"
+#include "launch_ahead.cuh"
 
 #include <cfloat>
 
@@ -79,8 +80,9 @@ __device__ T block_excl_scan(T v, T* total)
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* __restrict__ in, int n, T* __restrict__ sums)
+__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* in, int n, T* sums)
 {
+    wait_for_previous();
     const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     T s = 0;
 #pragma unroll
@@ -95,6 +97,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* __restric
 template <typename T>
 __global__ void __launch_bounds__(1024) k_scan_top(T* sums, int nb)
 {
+    wait_for_previous();
     __shared__ T ws[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     T v[8];
@@ -133,8 +136,9 @@ __global__ void __launch_bounds__(1024) k_scan_top(T* sums, int nb)
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kScanThreads) k_scan_down(T* __restrict__ data, int n, const T* __restrict__ sums)
+__global__ void __launch_bounds__(kScanThreads) k_scan_down(T* data, int n, const T* sums)
 {
+    wait_for_previous();
     const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     T v[kScanItems];
     T s = 0;
@@ -157,18 +161,19 @@ cudaError_t scan_excl(T* data, int n, T* tmp, cudaStream_t s)
     const int nb = (n + kScanTile - 1) / kScanTile;
     if (nb < 1) return cudaSuccess;
     if (nb > 8192) return cudaErrorInvalidValue;
-    k_scan_reduce<T><<<nb, kScanThreads, 0, s>>>(data, n, tmp);
-    k_scan_top<T><<<1, 1024, 0, s>>>(tmp, nb);
-    k_scan_down<T><<<nb, kScanThreads, 0, s>>>(data, n, tmp);
+    launch_ahead(k_scan_reduce<T>, nb, kScanThreads, 0, s, data, n, tmp);
+    launch_ahead(k_scan_top<T>, 1, 1024, 0, s, tmp, nb);
+    launch_ahead(k_scan_down<T>, nb, kScanThreads, 0, s, data, n, tmp);
     return cudaGetLastError();
 }
 
 /* ---- stable LSD radix sort of (key, value) pairs, 8-bit digits ----------
    Tiles of 2,048 keys: a quarter of a million agents fill the GPU (with 4,096
    they were 62 blocks). */
-__global__ void __launch_bounds__(kRsThreads) k_rs_hist(const unsigned* __restrict__ keys, const int* __restrict__ n_ptr,
-                                                        int shift, int* __restrict__ hist)
+__global__ void __launch_bounds__(kRsThreads) k_rs_hist(const unsigned* keys, const int* n_ptr,
+                                                        int shift, int* hist)
 {
+    wait_for_previous();
     __shared__ int h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
@@ -186,8 +191,9 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_hist(const unsigned* __restri
 /* hist [nblk][256] -> the keys of each digit in the tiles before each tile, in
    place, and the digits' totals: a warp per digit.  (One block over all
    digits took 9.6 us a pass at 123 tiles, as long as the scatter.) */
-__global__ void __launch_bounds__(256) k_rs_scan(int* __restrict__ hist, int nblk, int* __restrict__ total)
+__global__ void __launch_bounds__(256) k_rs_scan(int* hist, int nblk, int* total)
 {
+    wait_for_previous();
     const int lane = threadIdx.x & 31, d = blockIdx.x * 8 + (threadIdx.x >> 5);
     int carry = 0;
     for (int b0 = 0; b0 < nblk; b0 += 128) {
@@ -216,12 +222,13 @@ __global__ void __launch_bounds__(256) k_rs_scan(int* __restrict__ hist, int nbl
 /* elements of a tile are placed in tile order, round by round (256 per
    round, in thread order): rank among equal digits = warps before + lanes
    before, so the pass is stable */
-__global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const unsigned* __restrict__ kin, const int* __restrict__ vin,
-                                                           unsigned* __restrict__ kout, int* __restrict__ vout,
-                                                           const int* __restrict__ n_ptr, int shift,
-                                                           const int* __restrict__ offs,
-                                                           const int* __restrict__ total)
+__global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const unsigned* kin, const int* vin,
+                                                           unsigned* kout, int* vout,
+                                                           const int* n_ptr, int shift,
+                                                           const int* offs,
+                                                           const int* total)
 {
+    wait_for_previous();
     __shared__ int base[256];
     __shared__ int wc[kRsThreads / 32][256];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -280,9 +287,9 @@ cudaError_t radix_sort(unsigned* keys, int* vals, unsigned* ktmp, int* vtmp, con
     unsigned* kb = ktmp;
     int* vb = vtmp;
     for (int shift = 0; shift < 32; shift += 8) {
-        k_rs_hist<<<nblk, kRsThreads, 0, s>>>(ka, n_ptr, shift, hist);
-        k_rs_scan<<<32, 256, 0, s>>>(hist, nblk, hist + nblk * 256);
-        k_rs_scatter<<<nblk, kRsThreads, 0, s>>>(ka, va, kb, vb, n_ptr, shift, hist, hist + nblk * 256);
+        launch_ahead(k_rs_hist, nblk, kRsThreads, 0, s, ka, n_ptr, shift, hist);
+        launch_ahead(k_rs_scan, 32, 256, 0, s, hist, nblk, hist + nblk * 256);
+        launch_ahead(k_rs_scatter, nblk, kRsThreads, 0, s, ka, va, kb, vb, n_ptr, shift, hist, hist + nblk * 256);
         unsigned* tk = ka; ka = kb; kb = tk;
         int* tv = va; va = vb; vb = tv;
     }
@@ -292,6 +299,7 @@ cudaError_t radix_sort(unsigned* keys, int* vals, unsigned* ktmp, int* vtmp, con
 /* ---- members, keys and lists ------------------------------------------- */
 __global__ void k_kd_mark(KdArgs a)
 {
+    wait_for_previous();
     const int n = a.counters[C_NSORTED];
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const int slot = a.s_slot[t];
@@ -307,18 +315,21 @@ __global__ void k_kd_mark(KdArgs a)
 
 __global__ void k_kd_flag(KdArgs a, int* flags)
 {
+    wait_for_previous();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.max_slots; i += gridDim.x * blockDim.x)
         flags[i] = a.mark[i];
 }
 
 __global__ void k_kd_compact(KdArgs a, const int* flags, int* ids)
 {
+    wait_for_previous();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.max_slots; i += gridDim.x * blockDim.x)
         if (a.mark[i]) ids[flags[i]] = i;
 }
 
 __global__ void k_kd_keys(KdArgs a, const int* ids, int axis, unsigned* keys, int* vals)
 {
+    wait_for_previous();
     const int n = a.n_dev[0];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int id = ids[i];
@@ -330,6 +341,7 @@ __global__ void k_kd_keys(KdArgs a, const int* ids, int axis, unsigned* keys, in
 
 __global__ void k_kd_seg_init(KdArgs a)
 {
+    wait_for_previous();
     const int n = a.n_dev[0];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.cap; i += gridDim.x * blockDim.x) {
         a.seg_lo[i] = 0;
@@ -341,6 +353,7 @@ __global__ void k_kd_seg_init(KdArgs a)
 /* ---- one level of ConstructRecursive over the whole lists ---------------- */
 __global__ void k_kd_side(KdArgs a, const int* A)
 {
+    wait_for_previous();
     const int n = a.n_dev[0];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int lo = a.seg_lo[i], hi = a.seg_hi[i];
@@ -376,6 +389,7 @@ __device__ __forceinline__ void kd_flags(const KdArgs& a, const int* B, int firs
 
 __global__ void __launch_bounds__(kScanThreads) k_kd_count(KdArgs a, const int* B)
 {
+    wait_for_previous();
     const int n = a.n_dev[0];
     const int base = blockIdx.x * kScanTile + threadIdx.x;
     unsigned long long f[kScanItems], s = 0;
@@ -390,6 +404,7 @@ __global__ void __launch_bounds__(kScanThreads) k_kd_count(KdArgs a, const int* 
 /* exclusive left / right counts of every position (the tiles' sums scanned) */
 __global__ void __launch_bounds__(kScanThreads) k_kd_prefix(KdArgs a, const int* B)
 {
+    wait_for_previous();
     const int n = a.n_dev[0];
     const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     unsigned long long v[kScanItems], s = 0;
@@ -409,6 +424,7 @@ __global__ void __launch_bounds__(kScanThreads) k_kd_prefix(KdArgs a, const int*
    the level's segments) */
 __global__ void k_kd_partition(KdArgs a, const int* B, int* Bout, int update_seg)
 {
+    wait_for_previous();
     const int n = a.n_dev[0];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int lo = a.seg_lo[i], hi = a.seg_hi[i];
@@ -443,10 +459,10 @@ cudaError_t kd_partition(const KdArgs& a, const int* B, int* Bout, int update_se
 {
     const int nb = (a.cap + kScanTile - 1) / kScanTile;
     if (nb > 8192) return cudaErrorInvalidValue;
-    k_kd_count<<<nb, kScanThreads, 0, s>>>(a, B);
-    k_scan_top<unsigned long long><<<1, 1024, 0, s>>>(a.scan_tmp64, nb);
-    k_kd_prefix<<<nb, kScanThreads, 0, s>>>(a, B);
-    k_kd_partition<<<gc, 256, 0, s>>>(a, B, Bout, update_seg);
+    launch_ahead(k_kd_count, nb, kScanThreads, 0, s, a, B);
+    launch_ahead(k_scan_top<unsigned long long>, 1, 1024, 0, s, a.scan_tmp64, nb);
+    launch_ahead(k_kd_prefix, nb, kScanThreads, 0, s, a, B);
+    launch_ahead(k_kd_partition, gc, 256, 0, s, a, B, Bout, update_seg);
     return cudaGetLastError();
 }
 
@@ -468,6 +484,7 @@ struct KdSmallSm {
 
 __global__ void __launch_bounds__(kSmallThreads) k_kd_small(KdArgs a, const int* X, const int* Y, int top, int* place)
 {
+    wait_for_previous();
     extern __shared__ __align__(16) unsigned char raw[];
     KdSmallSm& m = *reinterpret_cast<KdSmallSm*>(raw);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -584,6 +601,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_kd_small(KdArgs a, const int*
    load per visit in the query */
 __global__ void k_kd_tree_pos(KdArgs a)
 {
+    wait_for_previous();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.tree_cap; i += gridDim.x * blockDim.x) {
         const int id = a.tree[i];
         const V2 p = id >= 0 ? a.pos[id] : mk(0.0f, 0.0f);
@@ -603,6 +621,7 @@ constexpr int kQueryWarps = 4;
 template <int K>
 __global__ void __launch_bounds__(32 * kQueryWarps, K <= 16 ? 8 : 4) k_kd_query(KdArgs a, const int* members)
 {
+    wait_for_previous();
     __shared__ float s_nd[kQueryWarps][K][33];
     __shared__ int s_ni[kQueryWarps][K][33];
     extern __shared__ float2 s_far[]; /* [warp][depth][lane]: distance to the split line, bounds (two upper halves) */
@@ -758,6 +777,7 @@ __device__ __forceinline__ int fold_rows(const KdArgs& a, int level)
 constexpr int kFoldWarps = 4;
 __global__ void __launch_bounds__(32 * kFoldWarps) k_kd_fold(KdArgs a, int level, int* rows, int* out)
 {
+    wait_for_previous();
     __shared__ int sm[kFoldWarps][32 * kMaxK];
     const int q = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int k = a.k, n = fold_rows(a, level);
@@ -853,6 +873,7 @@ __device__ __forceinline__ int fold_resolve(const KdArgs& a, int v, int b)
    on this tick's */
 __global__ void k_kd_cache(KdArgs a, const int* total)
 {
+    wait_for_previous();
     const int q = threadIdx.x;
     if (q >= a.k || a.counters[C_LAST] < 0) return;
     const int v = total[q];
@@ -866,6 +887,7 @@ __global__ void k_kd_cache(KdArgs a, const int* total)
    -(slot + 1)) */
 __global__ void k_kd_emit(KdArgs a)
 {
+    wait_for_previous();
     const int k = a.k, n = a.counters[C_NSORTED];
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         if (!a.open[t]) continue;
@@ -925,29 +947,29 @@ cudaError_t kd_build_and_query(const KdArgs& a, cudaStream_t s, int sms)
     const int gs = grid_n(a.max_slots, 256, sms), gc = grid_n(a.cap, 256, sms);
     k_kd_mark<<<gc, 256, 0, s>>>(a);
     /* members in slot order */
-    k_kd_flag<<<gs, 256, 0, s>>>(a, a.iscan);
+    launch_ahead(k_kd_flag, gs, 256, 0, s, a, a.iscan);
     e = scan_excl<int>(a.iscan, a.max_slots, a.scan_tmp32, s);
     if (e != cudaSuccess) return e;
-    k_kd_compact<<<gs, 256, 0, s>>>(a, a.iscan, a.ids0);
+    launch_ahead(k_kd_compact, gs, 256, 0, s, a, a.iscan, a.ids0);
     /* X0 = (x, index); Y = (y, x, index) sorted from X0; X = (x, y, index)
        sorted from Y (equal x keep Y's order, and equal x and y the index's) */
-    k_kd_keys<<<gc, 256, 0, s>>>(a, a.ids0, 0, a.keys, a.X0);
+    launch_ahead(k_kd_keys, gc, 256, 0, s, a, a.ids0, 0, a.keys, a.X0);
     e = radix_sort(a.keys, a.X0, a.ktmp, a.vtmp, a.n_dev, a.cap, a.hist, s);
     if (e != cudaSuccess) return e;
-    k_kd_keys<<<gc, 256, 0, s>>>(a, a.X0, 1, a.keys, a.Y[0]);
+    launch_ahead(k_kd_keys, gc, 256, 0, s, a, a.X0, 1, a.keys, a.Y[0]);
     e = radix_sort(a.keys, a.Y[0], a.ktmp, a.vtmp, a.n_dev, a.cap, a.hist, s);
     if (e != cudaSuccess) return e;
-    k_kd_keys<<<gc, 256, 0, s>>>(a, a.Y[0], 0, a.keys, a.X[0]);
+    launch_ahead(k_kd_keys, gc, 256, 0, s, a, a.Y[0], 0, a.keys, a.X[0]);
     e = radix_sort(a.keys, a.X[0], a.ktmp, a.vtmp, a.n_dev, a.cap, a.hist, s);
     if (e != cudaSuccess) return e;
-    k_kd_seg_init<<<gc, 256, 0, s>>>(a);
+    launch_ahead(k_kd_seg_init, gc, 256, 0, s, a);
     /* level 0 splits on X0 and partitions X and Y; then Y / X alternate; from
        level `top` on a segment is one block's */
     int xi = 0, yi = 0;
     const int top = kd_top(a.cap);
     for (int lv = 0; lv < top; lv++) {
         const bool on_y = (lv & 1) != 0;
-        k_kd_side<<<gc, 256, 0, s>>>(a, lv == 0 ? a.X0 : (on_y ? a.Y[yi] : a.X[xi]));
+        launch_ahead(k_kd_side, gc, 256, 0, s, a, lv == 0 ? a.X0 : (on_y ? a.Y[yi] : a.X[xi]));
         if (lv == 0 || on_y) {
             e = kd_partition(a, a.X[xi], a.X[xi ^ 1], lv == 0 ? 0 : 1, gc, s);
             xi ^= 1;
@@ -960,20 +982,20 @@ cudaError_t kd_build_and_query(const KdArgs& a, cudaStream_t s, int sms)
     }
     e = cudaFuncSetAttribute(k_kd_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KdSmallSm));
     if (e != cudaSuccess) return e;
-    k_kd_small<<<1 << top, kSmallThreads, sizeof(KdSmallSm), s>>>(a, a.X[xi], a.Y[yi], top, a.iscan);
+    launch_ahead(k_kd_small, 1 << top, kSmallThreads, sizeof(KdSmallSm), s, a, a.X[xi], a.Y[yi], top, a.iscan);
     /* queries in grid order: the agents of a warp are neighbours, so their
        traversals share nodes in cache */
-    k_kd_tree_pos<<<grid_n(a.tree_cap, 256, sms), 256, 0, s>>>(a);
+    launch_ahead(k_kd_tree_pos, grid_n(a.tree_cap, 256, sms), 256, 0, s, a);
     const int gq = grid_n(a.cap, 128, sms);
     /* at most 25 levels (2^24 slots): 25.6 KB beside the lists' 33.8 KB at
        K = 32, above the default limit of 48 KB only there */
     const size_t far = sizeof(float2) * 32 * kQueryWarps * (size_t)a.levels;
-    if (a.k <= 8) k_kd_query<8><<<gq, 32 * kQueryWarps, far, s>>>(a, a.s_slot);
-    else if (a.k <= 16) k_kd_query<16><<<gq, 32 * kQueryWarps, far, s>>>(a, a.s_slot);
+    if (a.k <= 8) launch_ahead(k_kd_query<8>, gq, 32 * kQueryWarps, far, s, a, a.s_slot);
+    else if (a.k <= 16) launch_ahead(k_kd_query<16>, gq, 32 * kQueryWarps, far, s, a, a.s_slot);
     else {
         e = cudaFuncSetAttribute(k_kd_query<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * 1024);
         if (e != cudaSuccess) return e;
-        k_kd_query<32><<<gq, 32 * kQueryWarps, far, s>>>(a, a.s_slot);
+        launch_ahead(k_kd_query<32>, gq, 32 * kQueryWarps, far, s, a, a.s_slot);
     }
     return cudaGetLastError();
 }
@@ -987,14 +1009,16 @@ cudaError_t kd_finish(const KdArgs& a, cudaStream_t s, int sms)
     int n = a.max_slots, level = 0;
     do {
         const int m = (n + kFold - 1) / kFold;
-        k_kd_fold<<<grid_n(m, kFoldWarps, sms), 32 * kFoldWarps, 0, s>>>(a, level, rows, out);
+        const int gf = grid_n(m, kFoldWarps, sms);
+        if (level == 0) k_kd_fold<<<gf, 32 * kFoldWarps, 0, s>>>(a, level, rows, out); /* after the join */
+        else launch_ahead(k_kd_fold, gf, 32 * kFoldWarps, 0, s, a, level, rows, out);
         rows = out;
         out += (size_t)m * a.k;
         n = m;
         level++;
     } while (n > 1);
-    k_kd_emit<<<grid_n(a.cap, 256, sms), 256, 0, s>>>(a);
-    k_kd_cache<<<1, 32, 0, s>>>(a, rows);
+    launch_ahead(k_kd_emit, grid_n(a.cap, 256, sms), 256, 0, s, a);
+    launch_ahead(k_kd_cache, 1, 32, 0, s, a, rows);
     return cudaGetLastError();
 }
 

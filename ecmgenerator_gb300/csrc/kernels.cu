@@ -20,6 +20,7 @@
  */
 #include "ecmg_internal.h"
 #include "knn_rows.cuh"
+#include "launch_ahead.cuh"
 
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -27,27 +28,6 @@
 #include <type_traits>
 
 namespace ecmg {
-
-/* Kernels that follow one another without an event between them (the binning
-   and the stand-alone query) are launched ahead: the next kernel's blocks take
-   the room that the last blocks of the one before leave, and wait there for its
-   end and its writes before they touch memory. */
-__device__ __forceinline__ void let_next_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-template <class... P, class... A>
-static cudaError_t launch_ahead(void (*kern)(P...), int blocks, int threads, cudaStream_t s, A... args)
-{
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.stream = s;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
-}
 
 /* the counters of a tick: zero but for the last slot (the other kernels of
    the tick start after the binning) */
@@ -60,7 +40,6 @@ __device__ __forceinline__ int start_counters(const BinArgs& a)
 
 __global__ void k_bin(BinArgs a)
 {
-    let_next_in();
     const int last = start_counters(a);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= last; i += gridDim.x * blockDim.x) {
         if (!a.active[i]) {
@@ -121,7 +100,6 @@ __global__ void __launch_bounds__(kScanBlock) k_scan(int* counts, int n, int* bl
 {
     __shared__ int sh[32];
     __shared__ bool last;
-    let_next_in();
     wait_for_previous();
     const int i0 = blockIdx.x * kScanTile + threadIdx.x * kScanPer;
     int v[kScanPer], sum = 0, tot;
@@ -161,7 +139,6 @@ int scan_tmp_ints(int n) { return (n + 1023) / 1024 + 32; }
 /* tick-start snapshot in grid order, and the final bucket starts */
 __global__ void k_scatter(BinArgs a)
 {
-    let_next_in();
     wait_for_previous();
     const int last = a.counters[C_LAST];
     const int t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
@@ -188,7 +165,6 @@ __global__ void __launch_bounds__(kSmallBlock) k_bin_small(BinArgs a)
     constexpr int R = kSmallSlots / kSmallBlock, C = kSmallCells / kSmallBlock;
     __shared__ int count[kSmallCells];
     __shared__ int sh[32];
-    let_next_in();
     const int last = start_counters(a);
     for (int c = threadIdx.x; c < kSmallCells; c += kSmallBlock) count[c] = 0;
     __syncthreads();
@@ -263,9 +239,9 @@ static cudaError_t launch_bin(const BinArgs& b, int slots, int blocks, cudaStrea
     k_bin<<<blocks, 256, 0, s>>>(b);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess)
-        e = launch_ahead(k_scan, (b.total_buckets + kScanTile - 1) / kScanTile, kScanBlock, s, b.cell_count,
+        e = launch_ahead(k_scan, (b.total_buckets + kScanTile - 1) / kScanTile, kScanBlock, 0, s, b.cell_count,
                          b.total_buckets, b.block_sums, b.counters);
-    if (e == cudaSuccess) e = launch_ahead(k_scatter, blocks, 256, s, b);
+    if (e == cudaSuccess) e = launch_ahead(k_scatter, blocks, 256, 0, s, b);
     return e;
 }
 
@@ -1150,7 +1126,7 @@ cudaError_t launch_knn(const V2* pos, const unsigned char* active, int n, int k,
     const int ga = (n + 32 * kNbrWarps - 1) / (32 * kNbrWarps);
     const float r2 = r * r;
     auto query = [&](auto kern) {
-        return launch_ahead(kern, ga, 32 * kNbrWarps, s, s_pos, s_slot, cell_start, g, k, r2, counters, out_ids, out_cnt);
+        return launch_ahead(kern, ga, 32 * kNbrWarps, 0, s, s_pos, s_slot, cell_start, g, k, r2, counters, out_ids, out_cnt);
     };
     return k <= 8 ? query(k_knn<8>) : (k <= 16 ? query(k_knn<16>) : query(k_knn<32>));
 }
