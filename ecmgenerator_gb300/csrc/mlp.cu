@@ -683,22 +683,28 @@ __global__ void __launch_bounds__(kTrThreads, 1)
         pending = true;
         return tid == 0;
     };
-    /* the weight-gradient chain: its operands may be overwritten.  A wait that
-       runs out is reported by the next wait() */
-    bool late = false;
-    auto wait_w = [&] {
-        if (!pending_w) return;
-        if (mbar_wait(mbw, phw, spin)) {
+    /* the weight-gradient chain has read this operand: a tile of the thread's
+       own goes over it.  A thread whose wait runs out leaves the tile as it is
+       and keeps the chain pending; the barrier before the next chain then
+       stops the CTA, so that never more than one chain is outstanding on mbw
+       and the drain below waits for that one.  False: stop. */
+    auto over_tile = [&](unsigned char* t, const float (&v)[32], auto&& store) {
+        const bool ok = mbar_wait(mbw, phw, spin);
+        tc_fence_after();
+        if (ok) {
             phw ^= 1u;
             pending_w = false;
-        } else {
-            late = true;
+            store(t, v);
         }
+        fence_async_smem();
+        tc_fence_before();
+        fail = __syncthreads_or(!ok) != 0;
         tc_fence_after();
+        return !fail;
     };
     auto wait = [&] {
         const bool ok = mbar_wait(mb, ph, spin);
-        fail = __syncthreads_or(!ok || late) != 0;
+        fail = __syncthreads_or(!ok) != 0;
         if (!fail) {
             ph ^= 1u;
             pending = false;
@@ -901,9 +907,9 @@ __global__ void __launch_bounds__(kTrThreads, 1)
         tmem_ld32(lane_base + c0, d);
 #pragma unroll
         for (int i = 0; i < 32; i++) d[i] *= g2[i];
-        wait_w(); /* A2 is read by dW3 */
-        store32(sA2, d);
-        if (ready()) {
+        if (!over_tile(sA2, d, store32)) break; /* A2 is read by dW3 */
+        pending = true;
+        if (tid == 0) {
             tc_chain(tmem, aA2, kTile, 0, aW2, HID, 1, HID, HID / 16, false);
             tc_commit(mb);
             tc_chain(tmem + kTrW2, aA1, kTile, 1, aA2, kTile, 1, HID, kTile / 16, add);
@@ -915,9 +921,9 @@ __global__ void __launch_bounds__(kTrThreads, 1)
         tmem_ld32(lane_base + c0, d);
 #pragma unroll
         for (int i = 0; i < 32; i++) d[i] *= g1[i];
-        wait_w(); /* A1 is read by dW2 */
-        store32(sA1, d);
-        if (ready()) {
+        if (!over_tile(sA1, d, store32)) break; /* A1 is read by dW2 */
+        pending = true;
+        if (tid == 0) {
             tc_chain(tmem + kTrW1, aA1, kTile, 1, aX, kTile, 1, IN, kTile / 16, add);
             tc_commit(mb);
         }
