@@ -1023,18 +1023,22 @@ __global__ void k_pack_all(const float* p, unsigned char* pack)
 }
 
 /* gradient = sum of the partial gradients (the same order on every run), then
-   the Adam step on it (lr > 0) with the BF16 copy of the new weights.  A warp
+   the Adam step on it (lr > 0) with the BF16 copy of the new weights.  Once a
+   wait of k_train has run out (*err, until the host clears it) there is no
+   whole gradient: this step and the ones queued behind it change nothing, and
+   their loss and hits say so.  A warp
    sums an eighth of the partials of 128 parameters, four per lane; block 0 adds
    up the loss.  Bound by reading the partials (128 of 198 KB) out of L2, where
    k_train has just written them: 16-byte loads and 388 blocks, one wave, in
    place of 4-byte loads and 1,549 blocks, and the weights and moments loaded
    ahead of the sum (four training steps 417 -> 403 us). */
 constexpr int kRedParams = 128;
+constexpr int kNoStep = -1; /* hits of a step that was not taken */
 static_assert(NPARAM % 4 == 0, "a partial gradient is read in fours");
 __global__ void __launch_bounds__(256) k_reduce_adam(const float* part, int nparts, float* g, float* p, float* m,
                                                      float* v, unsigned char* pack, float lr, float b1, float b2,
                                                      float eps, float c1, float c2, const float* part_loss,
-                                                     const int* part_ok, float* loss, int* right)
+                                                     const int* part_ok, const int* err, float* loss, int* right)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); /* the next step's k_train */
     __shared__ float s[8][kRedParams];
@@ -1045,6 +1049,13 @@ __global__ void __launch_bounds__(256) k_reduce_adam(const float* part, int npar
     /* after k_train's end, which comes after the last step's (the parameters
        and moments below) */
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (*err) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            *loss = __int_as_float(0x7fffffff); /* NaN */
+            *right = kNoStep;
+        }
+        return;
+    }
     float p0 = 0.0f, m0 = 0.0f, v0 = 0.0f;
     if (mine && lr > 0.0f) {
         p0 = p[i];
@@ -1361,7 +1372,7 @@ static cudaError_t train_step(ecmg_mlp* mm, const void* X, const unsigned char* 
     cfg.dynamicSmemBytes = 0;
     return cudaLaunchKernelEx(&cfg, k_reduce_adam, (const float*)mm->part, grid, mm->g, mm->p, mm->m, mm->v, mm->tpack, lr,
                               kBeta1, kBeta2, 1e-8f, c1, c2, (const float*)mm->part_loss, (const int*)mm->part_ok,
-                              mm->hist_loss + at, mm->hist_ok + at);
+                              (const int*)mm->gerr, mm->hist_loss + at, mm->hist_ok + at);
 }
 
 ecmg_status ecmg_mlp_loss_grad(ecmg_mlp* mm, const void* dev_x, const unsigned char* dev_y, int n, float* loss,
@@ -1415,11 +1426,19 @@ ecmg_status ecmg_mlp_train(ecmg_mlp* mm, const void* dev_x, const unsigned char*
     if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, mm->gerr, sizeof(int), cudaMemcpyDeviceToHost, mm->s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(mm->s);
     if (e != cudaSuccess) return ECMG_ERR_CUDA;
+    if (herr) { /* the model has taken the steps before the wait that ran out */
+        ok.resize((size_t)steps);
+        cudaMemsetAsync(mm->gerr, 0, sizeof(int), mm->s);
+        if (steps && (cudaMemcpyAsync(ok.data(), mm->hist_ok, sizeof(int) * (size_t)steps, cudaMemcpyDeviceToHost,
+                                      mm->s) != cudaSuccess ||
+                      cudaStreamSynchronize(mm->s) != cudaSuccess))
+            return ECMG_ERR_CUDA;
+        mm->step -= (int)std::count(ok.begin(), ok.end(), kNoStep);
+    }
     for (int it = 0; it < steps; it++) {
         if (host_loss) host_loss[it] /= (float)batch;
-        if (host_acc) host_acc[it] = (float)ok[it] / (float)batch;
+        if (host_acc) host_acc[it] = herr && ok[it] == kNoStep ? NAN : (float)ok[it] / (float)batch;
     }
-    if (herr) cudaMemsetAsync(mm->gerr, 0, sizeof(int), mm->s);
     return herr ? ECMG_ERR_BOUND : ECMG_OK;
 }
 

@@ -457,21 +457,26 @@ int ecmg_mlp_param_count(void);
 ecmg_status ecmg_mlp_get_params(ecmg_mlp* model, float* host_out);
 ecmg_status ecmg_mlp_set_params(ecmg_mlp* model, const float* host_in);
 /* mean softmax cross-entropy and its gradient (host float[param_count]) over
-   all n rows; dev_x: bf16 [n x 96], dev_y: class per row (device memory) */
+   all n rows; dev_x: bf16 [n x 96], dev_y: class per row (device memory).
+   ECMG_ERR_BOUND when a bounded wait of the training kernel gave up (the
+   outputs are not written) */
 ecmg_status ecmg_mlp_loss_grad(ecmg_mlp* model, const void* dev_x, const unsigned char* dev_y, int n,
                                float* loss, float* host_grad);
 /* `steps` Adam steps on minibatches of `batch` rows drawn with replacement
-   from the n rows (seeded); per-step loss / accuracy to host arrays if given */
+   from the n rows (seeded); per-step loss / accuracy to host arrays if given.
+   ECMG_ERR_BOUND when a bounded wait of the training kernel gave up: the model
+   has taken the steps before that one and none after, and the loss and the
+   accuracy of those not taken are NaN */
 ecmg_status ecmg_mlp_train(ecmg_mlp* model, const void* dev_x, const unsigned char* dev_y, int n, int steps,
                            int batch, float lr, unsigned long long seed, float* host_loss, float* host_acc);
 /* class of every row (argmax of the BF16 tensor-core forward); returns
    ECMG_ERR_BOUND when a bounded wait of the inference kernel gave up (the
    kernel drains its copies and MMAs, frees its tensor memory and returns) */
 ecmg_status ecmg_mlp_predict(ecmg_mlp* model, const void* dev_x, int n, unsigned char* dev_cls);
-/* how many times the inference kernel polls an mbarrier (a feature-tile copy
-   or an MMA chain) before it gives up with ECMG_ERR_BOUND; 0 restores the
-   default (2^22).  A diagnostic of the device-side timeout path: a tiny
-   limit makes the first wait run out. */
+/* how many times the inference and training kernels poll an mbarrier (a
+   feature-tile copy or an MMA chain) before they give up with ECMG_ERR_BOUND;
+   0 restores the default (2^22).  A diagnostic of the device-side timeout
+   path: a tiny limit makes the first wait run out. */
 ecmg_status ecmg_mlp_set_wait_limit(ecmg_mlp* model, int polls);
 
 /* Learned mode for a context: model != NULL turns it on (the context does

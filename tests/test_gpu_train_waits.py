@@ -42,3 +42,38 @@ def test_gradient_with_short_waits(lib):
         assert got[0] == loss and np.array_equal(got[1], grad), limit
     assert ran_out > 0
     m.close()
+
+
+def test_training_takes_whole_steps_only(lib):
+    """a step whose gradient is not whole changes neither the weights nor Adam's
+    state or step count, and neither do the steps queued behind it: what is left
+    to do, done afterwards, ends in the bits of an undisturbed run"""
+    import ctypes
+
+    from ecmgenerator_gb300.proposal import ProposalModel
+
+    steps, batch, lr, seed = 6, 700, 1e-3, 8
+    x, y = _rows(5000)
+    m = ProposalModel(seed=3)
+    start = m.get_params()
+    want_loss, want_acc = m.train(x, y, steps=steps, batch=batch, lr=lr, seed=seed)
+    want = m.get_params()
+    m.close()
+    for limit in LIMITS:
+        m = ProposalModel(seed=3)
+        assert lib.ecmg_mlp_set_wait_limit(m.h, limit) == 0
+        loss, acc = np.zeros(steps, np.float32), np.zeros(steps, np.float32)
+        rc = lib.ecmg_mlp_train(m.h, x.data_ptr(), y.data_ptr(), 5000, steps, batch, lr, ctypes.c_ulonglong(seed),
+                                loss.ctypes.data, acc.ctypes.data)
+        done = int(np.sum(~np.isnan(loss)))
+        assert rc == (0 if done == steps else 3), limit
+        assert np.array_equal(loss[:done], want_loss[:done]) and np.array_equal(acc[:done], want_acc[:done])
+        assert np.isnan(loss[done:]).all() and np.isnan(acc[done:]).all()
+        if limit == 1:
+            assert done == 0
+        if done == 0:
+            assert np.array_equal(m.get_params(), start)
+        assert lib.ecmg_mlp_set_wait_limit(m.h, 0) == 0
+        m.train(x, y, steps=steps - done, batch=batch, lr=lr, seed=seed)
+        assert np.array_equal(m.get_params(), want), limit
+        m.close()
