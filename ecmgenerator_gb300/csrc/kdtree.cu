@@ -870,16 +870,20 @@ __device__ __forceinline__ int fold_resolve(const KdArgs& a, int v, int b)
 }
 
 /* the cache the next tick starts from: the composition of all rows (`total`)
-   on this tick's */
-__global__ void k_kd_cache(KdArgs a, const int* total)
+   on this tick's.  One warp: every lane comes to the barrier between the
+   reads, which go to other lanes' entries, and the writes. */
+__global__ void __launch_bounds__(32) k_kd_cache(KdArgs a, const int* total)
 {
     wait_for_previous();
     const int q = threadIdx.x;
-    if (q >= a.k || a.counters[C_LAST] < 0) return;
-    const int v = total[q];
-    const int c = v < 0 ? a.cache[-v - 1] : a.s_slot[v];
-    __syncwarp(__activemask());
-    a.cache[q] = c;
+    const bool mine = q < a.k && a.counters[C_LAST] >= 0;
+    int c = 0;
+    if (mine) {
+        const int v = total[q];
+        c = v < 0 ? a.cache[-v - 1] : a.s_slot[v];
+    }
+    __syncwarp();
+    if (mine) a.cache[q] = c;
 }
 
 /* the open rows' references, looked up: the per-agent kernel's inputs (grid
