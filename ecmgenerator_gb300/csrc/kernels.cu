@@ -229,6 +229,16 @@ int bin_kernels(int total_buckets, int slots)
     return bins_small(b, slots) ? 1 : 3;
 }
 
+/* blocks for work on every bucket, four buckets a thread to 8 blocks an SM:
+   where the agents alone give the grid, a few of them in a large one leave the
+   buckets to a few threads (300 agents in 25 million cells: query 18,450 us,
+   with these 206; in 3 million cells of 0.3 m: tick 1,572 and 120) */
+static int blocks_of_buckets(int buckets, int threads)
+{
+    const int per = 4 * threads;
+    return std::min((buckets + per - 1) / per, 152 * 8);
+}
+
 /* counts (zero) -> bins, starts and snapshot */
 static cudaError_t launch_bin(const BinArgs& b, int slots, int blocks, cudaStream_t s)
 {
@@ -241,7 +251,10 @@ static cudaError_t launch_bin(const BinArgs& b, int slots, int blocks, cudaStrea
     if (e == cudaSuccess)
         e = launch_ahead(k_scan, (b.total_buckets + kScanTile - 1) / kScanTile, kScanBlock, 0, s, b.cell_count,
                          b.total_buckets, b.block_sums, b.counters);
-    if (e == cudaSuccess) e = launch_ahead(k_scatter, blocks, 256, 0, s, b);
+    /* k_scatter writes every bucket's start too: enough blocks for those of a
+       few agents in a large grid */
+    if (e == cudaSuccess)
+        e = launch_ahead(k_scatter, std::max(blocks, blocks_of_buckets(b.total_buckets, 256)), 256, 0, s, b);
     return e;
 }
 
@@ -967,9 +980,12 @@ cudaError_t launch_tick(const BinArgs& b, const TickArgs& t, int max_slots, int 
     const int split = max_slots <= sms * 2048 ? 50 : 75;
     int ao = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ao, k_attract, 128, 0);
-    const int ga = ao > 0 && gk > sms * ao ? sms * ao : gk; /* one wave, grid-stride */
-    if (t.attract_lanes) e = launch_split(k_attract_group, grid_for(max_slots, 128 / kAttractLanes, sms, 32), 128, split, s2, t);
-    else e = launch_split(k_attract, ga, 128, split, s2, t);
+    /* blocks for the agents and for the bucket counts that these kernels clear */
+    const int gc = blocks_of_buckets(t.total_buckets, 128);
+    const int ga = std::max(gk, gc);
+    if (t.attract_lanes)
+        e = launch_split(k_attract_group, std::max(grid_for(max_slots, 128 / kAttractLanes, sms, 32), gc), 128, split, s2, t);
+    else e = launch_split(k_attract, ao > 0 ? std::min(ga, sms * ao) : ga, 128, split, s2, t); /* one wave, grid-stride */
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecordWithFlags(ev[1], s2, evflags);
     /* the per-agent kernel waits for the attraction kernel, not for the

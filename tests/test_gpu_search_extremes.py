@@ -1,0 +1,70 @@
+"""Neighbour searches whose grid does not fit their crowd: the lists (against
+brute force in the same 32-bit arithmetic; ids and counts are whole numbers, no
+tolerance) and the time beside that of a crowd that fits, with room to spare
+for another clock or another box."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _query(L, pos, k, r, box, cell, repeats=1):
+    """ids, counts and the least time (us)"""
+    import torch
+
+    n = len(pos)
+    b = tuple(map(ctypes.c_float, (*box, cell)))
+    p = torch.from_numpy(np.ascontiguousarray(pos, np.float32)).cuda()
+    a = torch.ones(n, dtype=torch.uint8, device="cuda")
+    scratch = torch.empty(L.ecmg_knn_scratch_bytes(n, *b), dtype=torch.uint8, device="cuda")
+    ids = torch.full((n, k), -7, dtype=torch.int32, device="cuda")
+    cnt = torch.full((n,), -7, dtype=torch.int32, device="cuda")
+    best = float("inf")
+    for _ in range(repeats):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        e[0].record()
+        assert L.ecmg_knn(p.data_ptr(), a.data_ptr(), n, k, r, *b, ids.data_ptr(), cnt.data_ptr(), scratch.data_ptr(),
+                          scratch.numel(), torch.cuda.current_stream().cuda_stream) == 0
+        e[1].record()
+        torch.cuda.synchronize()
+        best = min(best, 1e3 * e[0].elapsed_time(e[1]))
+    return ids.cpu().numpy(), cnt.cpu().numpy(), best
+
+
+def _check(pos, k, r, ids, cnt, rows):
+    """the lists of the agents `rows`"""
+    pos = np.ascontiguousarray(pos, np.float32)
+    r2 = np.float32(r) * np.float32(r)
+    for i in rows:
+        d = pos - pos[i]
+        d2 = d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1]
+        near = np.nonzero((d2 > np.float32(1e-4)) & (d2 < r2))[0]
+        near = near[np.argsort(d2[near], kind="stable")][:k]  # slots ascend among equal distances
+        assert cnt[i] == near.size and np.array_equal(ids[i, : near.size], near), i
+        assert (ids[i, near.size:] == -1).all()
+
+
+def test_few_agents_in_many_cells(lib):
+    rng = np.random.default_rng(1)
+    box = (0, 0, 5000, 5000)
+    few, many = rng.uniform(0, 5000, (300, 2)), rng.uniform(0, 5000, (20000, 2))
+    ids, cnt, _ = _query(lib, few, 8, 500.0, box, 1.0)
+    _check(few, 8, 500.0, ids, cnt, range(300))
+    assert _query(lib, few, 8, 5.0, box, 1.0, 5)[2] < 3.0 * _query(lib, many, 8, 5.0, box, 1.0, 5)[2]
+
+
+def test_tick_of_few_agents_in_many_cells(lib, c1_small):
+    """2 M cells (binning by several blocks) and the usual ones: the same bits"""
+    from ecmgenerator_gb300.simulator import Simulator
+
+    scene, st, paths = c1_small
+    n, out = st.num_agents, []
+    for cell in (0.0, 0.08):
+        sim = Simulator(scene, n, 1.0 / 60.0, max_neighbors=10, tau_agent=2.0, tau_obst=2.0, grid_cell=cell)
+        sim.add_agents(st.pos[:n], st.clear[:n], st.pref_speed[:n], paths[:n])
+        sim.update(ticks=5)
+        out.append((sim.get_position_data(), sim.get_velocity_data()))
+        sim.close()
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
