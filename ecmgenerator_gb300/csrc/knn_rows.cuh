@@ -43,8 +43,10 @@ __device__ __forceinline__ int bucket_of(const AgentGrid& g, V2 p)
  * of the lane's index column that holds the candidate's grid index: one float
  * min / max pair per comparator, and the lists come out sorted by d2 except
  * for keys within 2^-17 of each other ("near ties"), which are re-sorted by
- * the exact (d2, slot); a near tie that may reach past the list (`rej` is the
- * smallest key dropped) sends the lane to the 64-bit search.
+ * the exact (d2, slot).  A near tie that may reach past the list (`rej` is the
+ * smallest key dropped) is settled among the entries of the index column: a
+ * crowd on a lattice has one nearly everywhere (100,000 points, k = 16: 101 us;
+ * 508 when such lanes went to the 64-bit search).
  * ---------------------------------------------------------------------- */
 constexpr unsigned kKnnCode = 63u; /* low key bits: entry of the index column */
 /* list capacity K: the k nearest in key[K-k .. K-1]; entries below hold 0.
@@ -140,11 +142,13 @@ __device__ __forceinline__ float dist2(V2 q, float2 np)
 /* The k nearest of the agents at p (one per lane; `valid` false: none) into
    the lanes' lists.  All 32 lanes must call.  Returns 1 when key[K-k .. K-1]
    (INFINITY beyond the count) is the answer in order, 2 when it holds near
-   ties that must be re-sorted by the exact key, 0 when a near tie may reach
-   past the list.  cs: the scene's cell starts. */
+   ties that must be re-sorted by the exact key, 3 when a near tie may reach
+   past the list (whoever it may mean was accepted and is among the first
+   *column entries of the lane's index column), 0 when the index column was too
+   short for the search.  cs: the scene's cell starts. */
 template <int K>
 __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, float r2, const V2* s_pos,
-                                        const int* cs, const AgentGrid& g, float (&key)[K])
+                                        const int* cs, const AgentGrid& g, float (&key)[K], int* column)
 {
     constexpr int B = kKnnBuf<K>;
     constexpr unsigned kAll = 0xffffffffu;
@@ -262,7 +266,9 @@ __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, f
 #pragma unroll
     for (int q = 0; q + 1 < K; q++)
         if (q >= K - k && key[q + 1] < INFINITY && knn_hi(key[q]) == knn_hi(key[q + 1])) tie = true;
-    if (over || (key[K - 1] < INFINITY && knn_hi(rej) == knn_hi(key[K - 1]))) return 0;
+    *column = ord;
+    if (over) return 0;
+    if (key[K - 1] < INFINITY && knn_hi(rej) == knn_hi(key[K - 1])) return 3;
     return tie ? 2 : 1;
 }
 
@@ -296,9 +302,40 @@ __device__ __noinline__ void knn_resort(int n, V2 p, const V2* s_pos, const int*
     for (int q = 0; q < n; q++) o[q] = id[q];
 }
 
-/* the search by 64-bit (d2, slot) keys (rare: a near tie at the k-th
-   distance that the list cannot settle, a full index column; out of line): the rows of the disc of
-   squared radius `lim`, which holds at least k agents or is r^2; o[q] gets
+/* a near tie across the k-th place (a lattice crowd has one nearly everywhere;
+   out of line): o[0 .. k) in key order; its entries with the leading bits `hi`
+   of the k-th key are replaced by those of the n column entries with these
+   bits that come first by the exact (d2, slot).  `before`: entries in front of
+   them */
+template <int K>
+__device__ __noinline__ void knn_tied(const int* column, int n, int k, int before, unsigned hi, V2 p, const V2* s_pos,
+                                      const int* s_slot, int* o)
+{
+    unsigned long long key[K];
+    int id[K];
+    const int room = k - before;
+    int have = 0;
+    for (int i = 0; i < n; i++) {
+        const int j = column[i * 32];
+        const V2 c = s_pos[j];
+        const float dx = c.x - p.x, dy = c.y - p.y;
+        const unsigned d2 = __float_as_uint(dx * dx + dy * dy);
+        if ((d2 & ~kKnnCode) != hi) continue;
+        const unsigned long long kk = ((unsigned long long)d2 << 32) | (unsigned)s_slot[j];
+        if (have == room && kk >= key[room - 1]) continue;
+        int q = have < room ? have++ : room - 1;
+        for (; q > 0 && key[q - 1] > kk; q--) {
+            key[q] = key[q - 1];
+            id[q] = id[q - 1];
+        }
+        key[q] = kk;
+        id[q] = j;
+    }
+    for (int q = 0; q < have; q++) o[before + q] = id[q];
+}
+
+/* the search by 64-bit (d2, slot) keys (rare: a full index column; out of
+   line): the rows of the disc of squared radius `lim`, which holds at least k agents or is r^2; o[q] gets
    the grid indices, the return value is the count */
 template <int K>
 __device__ __noinline__ int knn_exact(int k, V2 p, float lim, float r2, const V2* s_pos, const int* s_slot,
@@ -340,16 +377,18 @@ __device__ __forceinline__ int knn_list(KnnSm<K>& sm, bool valid, int k, V2 p, f
                                         const int* s_slot, const int* cs, const AgentGrid& g, int* o)
 {
     float key[K];
-    const int st = knn_rows<K>(sm, valid, k, p, r2, s_pos, cs, g, key);
+    int column;
+    const int st = knn_rows<K>(sm, valid, k, p, r2, s_pos, cs, g, key, &column);
     if (!valid) return 0;
     const int lane = threadIdx.x & 31;
-    int n = 0;
+    int n = 0, before = 0; /* before: keys below the k-th's leading bits */
     int id[K];
 #pragma unroll
     for (int q = 0; q < K; q++) {
         const bool in = q >= K - k && key[q] < INFINITY;
         id[q] = in ? sm.idx[__float_as_uint(key[q]) & kKnnCode][lane] : -1;
         n += in ? 1 : 0;
+        before += in && knn_hi(key[q]) < knn_hi(key[K - 1]) ? 1 : 0;
     }
     if (SLOTS && st == 1) {
 #pragma unroll
@@ -365,7 +404,9 @@ __device__ __forceinline__ int knn_list(KnnSm<K>& sm, bool valid, int k, V2 p, f
         for (int q = 0; q < K; q++)
             if (q >= K - k) o[q - (K - k)] = id[q];
     }
-    if (st == 2) knn_resort<K>(n, p, s_pos, s_slot, o);
+    if (st == 3)
+        knn_tied<K>(&sm.idx[0][lane], column, k, before, __float_as_uint(key[K - 1]) & ~kKnnCode, p, s_pos, s_slot, o);
+    if (st >= 2) knn_resort<K>(n, p, s_pos, s_slot, o);
     else if (st == 0)
         n = knn_exact<K>(k, p, fminf(r2, __uint_as_float(__float_as_uint(key[K - 1]) | kKnnCode)), r2, s_pos, s_slot,
                          cs, g, o);

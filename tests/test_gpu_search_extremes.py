@@ -68,3 +68,15 @@ def test_tick_of_few_agents_in_many_cells(lib, c1_small):
         out.append((sim.get_position_data(), sim.get_velocity_data()))
         sim.close()
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("k", [5, 8, 14, 16, 27, 32])
+def test_lattice(lib, k):
+    """a crowd on a lattice: distances tie across the k-th place"""
+    rng = np.random.default_rng(2)
+    pos = 0.4 * np.stack(np.meshgrid(np.arange(317), np.arange(316)), -1).reshape(-1, 2)
+    pos = pos[rng.permutation(len(pos))]
+    box, cell = (0, 0, 127, 127), max(0.3, 0.5 * (k / 6.25) ** 0.5)
+    ids, cnt, t = _query(lib, pos, k, 5.0, box, cell, 5)
+    _check(pos, k, 5.0, ids, cnt, rng.integers(0, len(pos), 300))
+    assert t < 3.0 * _query(lib, rng.uniform(0, 126.6, pos.shape), k, 5.0, box, cell, 5)[2]
