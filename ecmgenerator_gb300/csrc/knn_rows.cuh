@@ -62,6 +62,17 @@ constexpr int kKnnBuf = K <= 16 ? 8 : 16;
 template <int K>
 constexpr int kKnnIdx = K <= 8 ? 32 : (K <= 16 ? 46 : 64);
 
+/* agents of the 3 x 3 cells around an agent from which its warp takes the
+   search for crowded cells (CROWD).  There most of a row lies outside the disc
+   that is wanted, whose first estimate is unreliable, and a column that is full
+   would begin the search again and again: rows are tested eight at a time, and
+   a full column is renumbered.  20,000 points in one cell of 4 m take 3,400 us
+   so, 17,900 with the ordinary search; 20,000 outside the grid 3,480 and
+   13,000.  Evenly spread crowds do not care which (100,000 points, k = 16: 61
+   and 63 us with 121 agents in the 3 x 3 cells, 238 and 242 with 1,944); at
+   256 the ticks of the measured crowds all take the ordinary one. */
+constexpr int kKnnDense = 256;
+
 template <int K>
 struct KnnSm { /* of one warp */
     float key[kKnnBuf<K>][32];
@@ -130,6 +141,20 @@ __device__ __forceinline__ void knn_flush(const KnnSm<K>& sm, int lane, int cnt,
     bitonic_net<K>(key);
 }
 
+/* the column's entries that the (full) list refers to become its first K */
+template <int K>
+__device__ __forceinline__ void knn_renumber(int* column, float (&key)[K])
+{
+    int id[K];
+#pragma unroll
+    for (int q = 0; q < K; q++) id[q] = column[(__float_as_uint(key[q]) & kKnnCode) * 32];
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+        column[q * 32] = id[q];
+        if (key[q] > 0.0f) key[q] = __uint_as_float((__float_as_uint(key[q]) & ~kKnnCode) | (unsigned)q);
+    }
+}
+
 /* dx*dx + dy*dy of KDTree.cpp:107-108 (np: the negated centre; adding it is
    the subtraction), two components per instruction */
 __device__ __forceinline__ float dist2(V2 q, float2 np)
@@ -145,9 +170,11 @@ __device__ __forceinline__ float dist2(V2 q, float2 np)
    ties that must be re-sorted by the exact key, 3 when a near tie may reach
    past the list (whoever it may mean was accepted and is among the first
    *column entries of the lane's index column), 0 when the index column was too
-   short for the search.  cs: the scene's cell starts. */
-template <int K>
-__device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, float r2, const V2* s_pos,
+   short for the search (CROWD: for such a tie, the list itself is right but
+   for it).  n9: the agents of the 3 x 3 cells around p; cs: the scene's cell
+   starts. */
+template <int K, bool CROWD>
+__device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, float r2, int n9, const V2* s_pos,
                                         const int* cs, const AgentGrid& g, float (&key)[K], int* column)
 {
     constexpr int B = kKnnBuf<K>;
@@ -157,9 +184,8 @@ __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, f
     for (int q = 0; q < K; q++) key[q] = q < K - k ? 0.0f : INFINITY;
     float rej = INFINITY;
     int ord = 0, ord0 = 0; /* next entry of the index column; that of the buffer's first candidate */
-    bool over = false;     /* the index column is full */
+    bool over = false;     /* the index column is full (CROWD: has been renumbered) */
     int tries = 0;         /* searches begun again for that */
-    valid = valid && p.x - p.x == 0.0f && p.y - p.y == 0.0f; /* no distance to a non-finite position is finite */
     const float fy = (p.y - g.y0) * g.inv;
     const int cx = cell_clamp((p.x - g.x0) * g.inv, g.gw), cy = cell_clamp(fy, g.gh);
     /* distance to the nearer end of the own row (0 outside the grid) and the
@@ -171,11 +197,11 @@ __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, f
     float lim = 0.0f, lo = kEps, disc = 0.0f, more_area = 3.0f;
     if (valid) {
         const int xa = max(cx - 1, 0), xb = min(cx + 1, g.gw - 1), ya = max(cy - 1, 0), yb = min(cy + 1, g.gh - 1);
-        int n9 = 0;
-        for (int y = ya; y <= yb; y++) n9 += cs[y * g.gw + xb + 1] - cs[y * g.gw + xa];
         const float area = (float)((xb - xa + 1) * (yb - ya + 1)) * g.cell * g.cell;
         /* pi disc n9 / area = 1.8 (k + 2) */
         disc = fminf(r2, 0.573f * (float)(k + 2) * area / (float)max(n9, 1));
+        /* a border cell is endless: the agents outside the grid are in it */
+        if (CROWD && (cx == 0 || cx == g.gw - 1 || cy == 0 || cy == g.gh - 1)) disc = r2;
         lim = disc;
     }
     while (true) {
@@ -203,31 +229,75 @@ __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, f
                 }
             }
             const int longest = __reduce_max_sync(kAll, left);
-            /* the next candidate's position is loaded while this one is used */
             const int end = j + left;
-            V2 q = mk(0.0f, 0.0f);
-            if (left > 0) q = s_pos[j];
-            for (int it = longest; it > 0; it--) {
-                const float d2 = dist2(q, np);
-                const bool in = j < end && d2 > lo && d2 < lim;
-                if (j + 1 < end) q = s_pos[j + 1];
-                if (in) {
-                    sm.key[ord - ord0][lane] = __uint_as_float((__float_as_uint(d2) & ~kKnnCode) | (unsigned)ord);
-                    sm.idx[ord][lane] = j;
-                    ord++;
+            /* candidates beyond the k-th key (its code bits taken as ones)
+               cannot enter any more; equal leading bits still count as near
+               ties */
+            auto shrink = [&] {
+                if (key[K - 1] < INFINITY)
+                    lim = fminf(lim, __uint_as_float((__float_as_uint(key[K - 1]) | kKnnCode) + 1u));
+            };
+            auto push = [&](float d2, int at) {
+                sm.key[ord - ord0][lane] = __uint_as_float((__float_as_uint(d2) & ~kKnnCode) | (unsigned)ord);
+                sm.idx[ord][lane] = at;
+                ord++;
+            };
+            if (CROWD) {
+                /* a long row: eight at a time while no lane wants one, else
+                   four, with room for them made before */
+                auto at = [&](int q) { return dist2(s_pos[max(min(j + q, end - 1), 0)], np); };
+                for (int todo = longest; todo > 0;) {
+                    if (todo >= 8) {
+                        float d[8];
+                        bool want = false;
+#pragma unroll
+                        for (int q = 0; q < 8; q++) d[q] = at(q);
+#pragma unroll
+                        for (int q = 0; q < 8; q++) want |= j + q < end && d[q] > lo && d[q] < lim;
+                        if (!__any_sync(kAll, want)) {
+                            j += 8;
+                            todo -= 8;
+                            continue;
+                        }
+                    }
+                    const bool full = ord + 4 > kKnnIdx<K>; /* more than K accepted */
+                    if (__any_sync(kAll, full || ord - ord0 > B - 4)) {
+                        knn_flush<K>(sm, lane, ord - ord0, key, &rej);
+                        if (full) {
+                            knn_renumber<K>(&sm.idx[0][lane], key);
+                            ord = K;
+                            over = true;
+                        }
+                        ord0 = ord;
+                        shrink();
+                    }
+                    float d[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) d[q] = at(q);
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        if (j + q < end && d[q] > lo && d[q] < lim) push(d[q], j + q);
+                    j += 4;
+                    todo -= 4;
                 }
-                j++;
-                if (__any_sync(kAll, ord == ord0 + B)) {
-                    knn_flush<K>(sm, lane, ord - ord0, key, &rej);
-                    ord0 = ord;
-                    /* candidates beyond the k-th key (its code bits taken as
-                       ones) cannot enter any more; equal leading bits still
-                       count as near ties */
-                    if (key[K - 1] < INFINITY)
-                        lim = fminf(lim, __uint_as_float((__float_as_uint(key[K - 1]) | kKnnCode) + 1u));
-                    if (ord > kKnnIdx<K> - B) { /* no room for another buffer */
-                        over = true;
-                        lim = 0.0f;
+            } else {
+                /* the next candidate's position is loaded while this one is used */
+                V2 q = mk(0.0f, 0.0f);
+                if (left > 0) q = s_pos[j];
+                for (int it = longest; it > 0; it--) {
+                    const float d2 = dist2(q, np);
+                    const bool in = j < end && d2 > lo && d2 < lim;
+                    if (j + 1 < end) q = s_pos[j + 1];
+                    if (in) push(d2, j);
+                    j++;
+                    if (__any_sync(kAll, ord == ord0 + B)) {
+                        knn_flush<K>(sm, lane, ord - ord0, key, &rej);
+                        ord0 = ord;
+                        shrink();
+                        if (ord > kKnnIdx<K> - B) { /* no room for another buffer */
+                            over = true;
+                            lim = 0.0f;
+                        }
                     }
                 }
             }
@@ -241,13 +311,17 @@ __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, f
         const bool grow = valid && !(key[K - 1] < INFINITY) && disc < r2;
         /* a full index column: once more from the start, with the k-th
            distance known by now (a disc of little more than k agents) */
-        const bool again = over && tries < 2;
+        const bool again = !CROWD && over && tries < 2;
         if (!__any_sync(kAll, grow || again)) break;
         lim = 0.0f;
         if (grow) {
             lo = fmaxf(kEps, __uint_as_float(__float_as_uint(disc) - 1u));
-            disc = fminf(r2, more_area * disc);
-            more_area *= more_area;
+            if (CROWD) { /* by the density that the disc has shown, or all */
+                disc = ord > 0 ? fminf(r2, fmaxf(3.0f, 1.8f * (float)(k + 2) / (float)ord) * disc) : r2;
+            } else {
+                disc = fminf(r2, more_area * disc);
+                more_area *= more_area;
+            }
             lim = disc;
         }
         if (again) {
@@ -267,9 +341,9 @@ __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, f
     for (int q = 0; q + 1 < K; q++)
         if (q >= K - k && key[q + 1] < INFINITY && knn_hi(key[q]) == knn_hi(key[q + 1])) tie = true;
     *column = ord;
-    if (over) return 0;
-    if (key[K - 1] < INFINITY && knn_hi(rej) == knn_hi(key[K - 1])) return 3;
-    return tie ? 2 : 1;
+    const bool past = key[K - 1] < INFINITY && knn_hi(rej) == knn_hi(key[K - 1]);
+    if (over && (past || !CROWD)) return 0;
+    return past ? 3 : (tie ? 2 : 1);
 }
 
 /* near ties in the list (rare; out of line): the n indices in o[0 .. n)
@@ -334,8 +408,9 @@ __device__ __noinline__ void knn_tied(const int* column, int n, int k, int befor
     for (int q = 0; q < have; q++) o[before + q] = id[q];
 }
 
-/* the search by 64-bit (d2, slot) keys (rare: a full index column; out of
-   line): the rows of the disc of squared radius `lim`, which holds at least k agents or is r^2; o[q] gets
+/* the search by 64-bit (d2, slot) keys (rare: a near tie across the k-th place
+   after the column was renumbered; out of line): the rows of the disc of
+   squared radius `lim`, which holds at least k agents or is r^2; o[q] gets
    the grid indices, the return value is the count */
 template <int K>
 __device__ __noinline__ int knn_exact(int k, V2 p, float lim, float r2, const V2* s_pos, const int* s_slot,
@@ -353,7 +428,7 @@ __device__ __noinline__ int knn_exact(int k, V2 p, float lim, float r2, const V2
             const V2 c = s_pos[j];
             const float dx = c.x - p.x, dy = c.y - p.y;
             const float d2 = dx * dx + dy * dy;
-            if (!(d2 > kEps) || !(d2 < r2)) continue;
+            if (!(d2 > kEps) || !(d2 < r2) || d2 > lim) continue;
             const unsigned long long kk = ((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)s_slot[j];
             if (n == k && kk >= key[k - 1]) continue;
             int q = n < k ? n++ : k - 1;
@@ -363,23 +438,20 @@ __device__ __noinline__ int knn_exact(int k, V2 p, float lim, float r2, const V2
             }
             key[q] = kk;
             id[q] = j;
+            if (n == k) lim = __uint_as_float((unsigned)(key[k - 1] >> 32));
         }
     }
     for (int q = 0; q < n; q++) o[q] = id[q];
     return n;
 }
 
-/* the neighbour list of the agent at p: grid indices (SLOTS: slots) in
-   o[0 .. k), -1 beyond the count, which is returned.  All 32 lanes must call;
-   lanes with valid false write nothing. */
+/* o[0 .. k) of one lane from its list and column (knn_rows' answer st, not 0
+   unless CROWD); returns the count */
 template <int K, bool SLOTS>
-__device__ __forceinline__ int knn_list(KnnSm<K>& sm, bool valid, int k, V2 p, float r2, const V2* s_pos,
-                                        const int* s_slot, const int* cs, const AgentGrid& g, int* o)
+__device__ __forceinline__ int knn_write(const KnnSm<K>& sm, int st, int k, V2 p, float r2, const float (&key)[K],
+                                         int column, const V2* s_pos, const int* s_slot, const int* cs,
+                                         const AgentGrid& g, int* o)
 {
-    float key[K];
-    int column;
-    const int st = knn_rows<K>(sm, valid, k, p, r2, s_pos, cs, g, key, &column);
-    if (!valid) return 0;
     const int lane = threadIdx.x & 31;
     int n = 0, before = 0; /* before: keys below the k-th's leading bits */
     int id[K];
@@ -412,6 +484,51 @@ __device__ __forceinline__ int knn_list(KnnSm<K>& sm, bool valid, int k, V2 p, f
                          cs, g, o);
     if (SLOTS && st != 1)
         for (int q = 0; q < n; q++) o[q] = s_slot[o[q]];
+    return n;
+}
+
+/* knn_list where the cells hold far more agents than a search wants (out of
+   line, so that the ordinary search keeps its registers and instructions) */
+template <int K, bool SLOTS>
+__device__ __noinline__ int knn_list_crowd(KnnSm<K>* sm, bool valid, int k, V2 p, float r2, int n9, const V2* s_pos,
+                                           const int* s_slot, const int* cs, const AgentGrid* g, int* o)
+{
+    float key[K];
+    int column;
+    const bool finite = p.x - p.x == 0.0f && p.y - p.y == 0.0f;
+    const int st = knn_rows<K, true>(*sm, valid && finite, k, p, r2, n9, s_pos, cs, *g, key, &column);
+    return valid ? knn_write<K, SLOTS>(*sm, st, k, p, r2, key, column, s_pos, s_slot, cs, *g, o) : 0;
+}
+
+/* the neighbour list of the agent at p: grid indices (SLOTS: slots) in
+   o[0 .. k), -1 beyond the count, which is returned.  All 32 lanes must call;
+   lanes with valid false write nothing. */
+template <int K, bool SLOTS>
+__device__ __forceinline__ int knn_list(KnnSm<K>& sm, bool valid, int k, V2 p, float r2, const V2* s_pos,
+                                        const int* s_slot, const int* cs, const AgentGrid& g, int* o)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    const bool finite = p.x - p.x == 0.0f && p.y - p.y == 0.0f; /* no distance to another position is finite */
+    int n9 = 0;                                                  /* agents of the 3 x 3 cells around p */
+    if (valid && finite) {
+        const int cx = cell_clamp((p.x - g.x0) * g.inv, g.gw), cy = cell_clamp((p.y - g.y0) * g.inv, g.gh);
+        const int xa = max(cx - 1, 0), xb = min(cx + 1, g.gw - 1), ya = max(cy - 1, 0), yb = min(cy + 1, g.gh - 1);
+        for (int y = ya; y <= yb; y++) n9 += cs[y * g.gw + xb + 1] - cs[y * g.gw + xa];
+    }
+    const bool dense = __any_sync(kAll, n9 > kKnnDense);
+    int n = 0;
+    bool left = valid && dense;
+    if (!dense) {
+        float key[K];
+        int column;
+        const int st = knn_rows<K, false>(sm, valid && finite, k, p, r2, n9, s_pos, cs, g, key, &column);
+        left = valid && st == 0;
+        if (valid && !left) n = knn_write<K, SLOTS>(sm, st, k, p, r2, key, column, s_pos, s_slot, cs, g, o);
+    }
+    if (__any_sync(kAll, left)) {
+        const int c = knn_list_crowd<K, SLOTS>(&sm, left, k, p, r2, n9, s_pos, s_slot, cs, &g, o);
+        if (left) n = c;
+    }
     return n;
 }
 

@@ -80,3 +80,64 @@ def test_lattice(lib, k):
     ids, cnt, t = _query(lib, pos, k, 5.0, box, cell, 5)
     _check(pos, k, 5.0, ids, cnt, rng.integers(0, len(pos), 300))
     assert t < 3.0 * _query(lib, rng.uniform(0, 126.6, pos.shape), k, 5.0, box, cell, 5)[2]
+
+
+def _crowded(name, rng):
+    """crowds far denser than their cells: positions, radius, box, cell"""
+    if name == "cluster":
+        return rng.normal(50, 0.5, (4000, 2)), 5.0, (0, 0, 100, 100), 4.0
+    if name == "cluster and strays":
+        return np.concatenate([rng.normal(50, 0.1, (1500, 2)), rng.uniform(0, 100, (500, 2))]), 30.0, \
+            (0, 0, 100, 100), 4.0
+    if name == "lattice in a cell":  # ties in a column that has been renumbered
+        g = np.stack(np.meshgrid(np.arange(40), np.arange(40)), -1).reshape(-1, 2)
+        return 48.5 + 0.06 * g[rng.permutation(len(g))], 5.0, (0, 0, 100, 100), 4.0
+    if name == "coincident":  # more agents at one distance than a column holds
+        return np.repeat(rng.uniform(48.1, 51.9, (12, 2)), 100, 0), 5.0, (0, 0, 100, 100), 4.0
+    if name == "outside":  # one corner cell holds everybody
+        return rng.uniform(0, 60, (4000, 2)) + 500, 5.0, (0, 0, 100, 100), 1.0
+    p = rng.uniform(48, 52, (1000, 2))  # "not finite"
+    p[::7] = np.nan
+    p[::11, 0] = np.inf
+    return p, 5.0, (0, 0, 100, 100), 4.0
+
+
+@pytest.mark.parametrize("k", [1, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("name", ["cluster", "cluster and strays", "lattice in a cell", "coincident", "outside",
+                                  "not finite"])
+def test_crowded_cells(lib, name, k):
+    rng = np.random.default_rng(4)
+    pos, r, box, cell = _crowded(name, rng)
+    ids, cnt, _ = _query(lib, pos, k, r, box, cell)
+    with np.errstate(invalid="ignore", over="ignore"):
+        _check(pos, k, r, ids, cnt, rng.integers(0, len(pos), 400))
+
+
+def test_crowded_cell_in_time(lib):
+    """every agent has to look at all 4,000: beside a crowd in cells that fit"""
+    rng = np.random.default_rng(4)
+    pos, r, box, cell = _crowded("cluster", rng)
+    fit = _query(lib, rng.uniform(0, 26, pos.shape), 16, 5.0, (0, 0, 26, 26), 0.8, 5)[2]
+    assert _query(lib, pos, 16, r, box, cell, 5)[2] < 60.0 * fit
+
+
+def test_tick_with_crowded_cells(lib, c1_small):
+    """cells of 40 m (everybody in the 3 x 3 around an agent) and the usual
+    ones: the same bits"""
+    from ecmgenerator_gb300.simulator import Simulator
+
+    scene, st, paths = c1_small
+    n = st.num_agents
+    for k in (7, 16, 25):
+        out = []
+        for cell in (0.0, 40.0):
+            sim = Simulator(scene, n, 1.0 / 60.0, max_neighbors=k, tau_agent=2.0, tau_obst=2.0, grid_cell=cell,
+                            neighbor_dist=15.0)
+            sim.set_record(True)
+            sim.add_agents(st.pos[:n], st.clear[:n], st.pref_speed[:n], paths[:n])
+            sim.update(ticks=5)
+            rec = sim.get_record()
+            out.append((sim.get_position_data(), sim.get_velocity_data(), rec["nbr_ids"], rec["nbr_count"]))
+            sim.close()
+        for a, b in zip(*out):
+            assert np.array_equal(a, b)
