@@ -322,7 +322,7 @@ def run_ours(args):
             set_neighbor_mode(s_, "kdtree")
         args.plain_only = True
         if args.lp_mode == "warp":
-            args.lp_mode = "thread"
+            args.lp_mode = "auto"
     flush = torch.empty(512 * 1024 * 1024, dtype=torch.uint8, device="cuda")
     plain.update()
     learned.update()

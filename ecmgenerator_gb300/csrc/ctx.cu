@@ -138,9 +138,7 @@ struct ecmg_ctx {
        25,000 to a million agents (neighbour kernel 56 us at 0.25 against 70 at
        0.4 with 25,000 agents in 500 m, 324 against 330 at a million) */
     float cell_scale = 0.25f;
-    /* ECMG_LP_THREAD, ECMG_LP_WARP, ECMG_LP_THREAD_FUSED, or by the agent count */
-    static constexpr int kLpAuto = -1;
-    int lp_mode = kLpAuto;
+    int lp_mode = ECMG_LP_AUTO;
     int lanes_agents = 0; /* the agent count the automatic layouts were chosen for */
     int occ_div = 1; /* per-thread layout: resident blocks per SM divided by this */
     int knn_wide = 0; /* neighbour kernel: 8 resident blocks per SM at most, or 6 */
@@ -1852,7 +1850,7 @@ static int lanes_of(ecmg_ctx* c)
 {
     if (c->lp_mode == ECMG_LP_WARP)
         return c->wgrab >= 8 ? 4 : (c->wgrab >= 4 ? 8 : (c->wgrab >= 2 ? 16 : 32));
-    if (c->lp_mode != ecmg_ctx::kLpAuto) return 1;
+    if (c->lp_mode != ECMG_LP_AUTO) return 1;
     if (c->lanes_agents <= 8000) return 8;
     return c->lanes_agents <= 160000 || c->nbr_mode == ECMG_NEIGHBORS_KDTREE ? 4 : 1;
 }
@@ -2434,21 +2432,23 @@ ecmg_status ecmg_autotune(ecmg_ctx* c, int ticks_per_trial, ecmg_tune_result* ou
     const int divs[] = {1, 2, 3};
     const int wgrabs[] = {1, 2, 4, 8};
     const bool fixed_cell = c->prm.grid_cell > 0.0f;
+    /* the kd-tree mode steps agents by several lanes, which read the cell only:
+       neither the search kernel's blocks nor the per-thread layout's launch */
     const bool kdtree = c->nbr_mode == ECMG_NEIGHBORS_KDTREE;
-    const int base = kdtree ? ecmg_ctx::kLpAuto : ECMG_LP_THREAD;
+    const int base = kdtree ? ECMG_LP_AUTO : ECMG_LP_THREAD;
     const int def_block = c->prm.block_size ? c->prm.block_size : 128;
     bool better = false;
     ecmg_status st = ECMG_OK;
     for (float sc : scales) {
         if (fixed_cell && sc != scales[0]) break;
-        for (int kw = 0; kw < 2 && st == ECMG_OK; kw++)
+        for (int kw = 0; kw < (kdtree ? 1 : 2) && st == ECMG_OK; kw++)
             st = trial(Launch{sc, base, def_block, 32, 1, c->wgrab, kw}, &better);
         if (st != ECMG_OK) break;
     }
     const float cell = bestL.scale;
     const int kw = bestL.knn_wide;
     for (int b : blocks) {
-        if (st != ECMG_OK) break;
+        if (st != ECMG_OK || kdtree) break;
         if (c->prm.block_size && b != c->prm.block_size) continue;
         for (int tl : tiles)
             for (int dv : divs) {
@@ -2458,7 +2458,7 @@ ecmg_status ecmg_autotune(ecmg_ctx* c, int ticks_per_trial, ecmg_tune_result* ou
     }
     const Launch thr = bestL;
     for (int w : wgrabs) {
-        if (st != ECMG_OK || kdtree) break; /* the layout goes by the agent count there */
+        if (st != ECMG_OK || kdtree) break;
         st = trial(Launch{cell, ECMG_LP_WARP, thr.block, thr.tile, 1, w, kw}, &better);
     }
     if (st != ECMG_OK) {
@@ -2483,7 +2483,7 @@ ecmg_status ecmg_autotune(ecmg_ctx* c, int ticks_per_trial, ecmg_tune_result* ou
     if (out) {
         out->block_size = bb;
         out->agents_per_warp_grab = bmode == ECMG_LP_WARP ? bw : bt;
-        out->lp_mode = bmode == ecmg_ctx::kLpAuto ? ECMG_LP_THREAD : bmode;
+        out->lp_mode = bmode;
         out->grid_cell_scale = bs;
         out->best_tick_ms = best;
         out->trials = trials;
@@ -2524,7 +2524,7 @@ ecmg_status ecmg_set_neighbor_mode(ecmg_ctx* c, int mode)
         CK(K.keys.alloc(N)); CK(K.ktmp.alloc(N)); CK(K.flags.alloc(N));
         /* ORCA::m_NeighborCache starts as std::vector<Entity>(k): zeros */
         CK(cudaMemset(K.cache.p, 0, sizeof(int) * (size_t)k));
-        c->lp_mode = ecmg_ctx::kLpAuto;
+        c->lp_mode = ECMG_LP_AUTO;
     } else {
         c->kd.free_all();
     }
@@ -2535,10 +2535,10 @@ ecmg_status ecmg_set_neighbor_mode(ecmg_ctx* c, int mode)
 
 ecmg_status ecmg_set_lp_mode(ecmg_ctx* c, int mode, int agents_per_warp_grab)
 {
-    if (!c || (mode != ECMG_LP_THREAD && mode != ECMG_LP_WARP && mode != ECMG_LP_THREAD_FUSED))
+    if (!c || (mode != ECMG_LP_THREAD && mode != ECMG_LP_WARP && mode != ECMG_LP_THREAD_FUSED && mode != ECMG_LP_AUTO))
         return ECMG_ERR_INVALID_ARG;
     if (mode == ECMG_LP_WARP && c->nbr_mode == ECMG_NEIGHBORS_KDTREE)
-        return fail(c, ECMG_ERR_STATE, "the kd-tree neighbour mode runs one thread per agent");
+        return fail(c, ECMG_ERR_STATE, "the kd-tree neighbour mode takes ECMG_LP_AUTO or one thread per agent");
     if (mode == ECMG_LP_WARP && (agents_per_warp_grab < 1 || agents_per_warp_grab > 64)) return ECMG_ERR_INVALID_ARG;
     c->lp_mode = mode;
     if (mode == ECMG_LP_WARP) c->wgrab = agents_per_warp_grab;

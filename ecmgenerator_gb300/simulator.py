@@ -496,7 +496,7 @@ def autotune(sim: Simulator, ticks_per_trial: int = 2) -> dict:
     sim._ck(sim.L.ecmg_autotune(sim.h, int(ticks_per_trial), C.byref(r)))
     return dict(block_size=r.block_size, agents_per_warp_grab=r.agents_per_warp_grab,
                 grid_cell_scale=r.grid_cell_scale, best_tick_ms=r.best_tick_ms, trials=r.trials,
-                lp_mode={0: "thread", 1: "warp", 2: "fused"}[r.lp_mode], occupancy_divisor=r.occupancy_divisor,
+                lp_mode={0: "thread", 1: "warp", 2: "fused", 3: "auto"}[r.lp_mode], occupancy_divisor=r.occupancy_divisor,
                 neighbor_blocks_per_sm=r.neighbor_blocks_per_sm)
 
 
@@ -511,9 +511,9 @@ def set_launch(sim: Simulator, block_size: int, agents_per_warp_grab: int, grid_
 def set_lp_mode(sim: Simulator, mode: str = "warp", agents_per_warp_grab: int = 4):
     """per-agent kernel layout: "thread" (one thread per agent), "warp" (a
     warp takes agents_per_warp_grab agents side by side: 32 lanes per agent
-    for 1, 16 for 2, 8 for 4, 4 for 8) or "fused" (runs as "thread"); unless
-    called, the tick chooses by the agent count; results are identical"""
-    m = {"thread": 0, "warp": 1, "fused": 2}[mode]
+    for 1, 16 for 2, 8 for 4, 4 for 8), "fused" (runs as "thread") or "auto"
+    (the default: by the agent count); results are identical"""
+    m = {"thread": 0, "warp": 1, "fused": 2, "auto": 3}[mode]
     sim._ck(sim.L.ecmg_set_lp_mode(sim.h, m, int(agents_per_warp_grab)))
 
 

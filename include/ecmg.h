@@ -353,20 +353,21 @@ typedef struct {
     float grid_cell_scale;
     float best_tick_ms;
     int trials;
-    int lp_mode;             /* ECMG_LP_THREAD, ECMG_LP_WARP or ECMG_LP_THREAD_FUSED */
+    int lp_mode;             /* ECMG_LP_THREAD or ECMG_LP_WARP; ECMG_LP_AUTO in the kd-tree neighbour mode */
     int occupancy_divisor;   /* per-thread layout: resident blocks per SM divided by this */
     int neighbor_blocks_per_sm; /* exact-kNN kernel: blocks of its grid per SM */
 } ecmg_tune_result;
 ecmg_status ecmg_set_launch(ecmg_ctx* ctx, int block_size, int agents_per_warp_grab, float grid_cell_scale);
-/* Per-agent kernel layout.  Unless set, the tick chooses by the agent count:
-   8 lanes per agent to 8,000 agents, 4 to 160,000 (and always in the kd-tree
-   neighbour mode), one thread per agent above.  ECMG_LP_THREAD: one thread
-   per agent (work grabs of agents_per_warp_grab from ecmg_set_launch).
+/* Per-agent kernel layout.  ECMG_LP_AUTO (the default, and set by the change
+   to the kd-tree neighbour mode): by the agent count, 8 lanes per agent to
+   8,000 agents, 4 to 160,000 (in the kd-tree mode above that as well), one
+   thread per agent above.  ECMG_LP_THREAD: one thread per agent (work grabs of
+   agents_per_warp_grab from ecmg_set_launch).
    ECMG_LP_WARP: a warp takes agents_per_warp_grab agents (1..64) side by
    side -- 32 lanes per agent for 1, 16 for 2 or 3, 8 for 4 to 7, 4 for 8 and
    more -- whose lanes build the constraints in parallel and share the inner
-   loops of the LPs.  ECMG_LP_THREAD_FUSED: runs as ECMG_LP_THREAD.  All give
-   identical results. */
+   loops of the LPs (not in the kd-tree mode: ECMG_ERR_STATE).
+   ECMG_LP_THREAD_FUSED: runs as ECMG_LP_THREAD.  All give identical results. */
 /* per-thread layout: run the persistent per-agent kernel with the resident
    blocks per SM divided by `divisor` (1..8; fewer resident warps leave more
    L1 to each thread's local constraint arrays) */
@@ -377,6 +378,7 @@ ecmg_status ecmg_set_neighbor_blocks(ecmg_ctx* ctx, int blocks_per_sm);
 #define ECMG_LP_THREAD 0
 #define ECMG_LP_WARP 1
 #define ECMG_LP_THREAD_FUSED 2
+#define ECMG_LP_AUTO 3
 ecmg_status ecmg_set_lp_mode(ecmg_ctx* ctx, int mode, int agents_per_warp_grab);
 /* Neighbour query of the tick.  ECMG_NEIGHBORS_EXACT (default): the exact k
    nearest within neighbor_dist, ordered by (d^2, index).
@@ -393,8 +395,10 @@ ecmg_status ecmg_set_lp_mode(ecmg_ctx* ctx, int mode, int agents_per_warp_grab);
 ecmg_status ecmg_set_neighbor_mode(ecmg_ctx* ctx, int mode);
 /* times ticks_per_trial ticks per configuration -- first the grid cell with
    the default launch, then, at the best cell, the per-agent kernel's layout,
-   block size, work grab and occupancy -- on a copy of the current state, restores the state after each
-   trial (no re-plans are served during trials) and keeps the fastest */
+   block size, work grab and occupancy (in the kd-tree neighbour mode the cell
+   only, with ECMG_LP_AUTO) -- on a copy of the current state, restores the
+   state after each trial (no re-plans are served during trials) and keeps the
+   fastest */
 ecmg_status ecmg_autotune(ecmg_ctx* ctx, int ticks_per_trial, ecmg_tune_result* out);
 
 /* the cudaStream_t the context launches on (for callers that record CUDA

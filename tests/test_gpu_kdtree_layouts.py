@@ -77,3 +77,46 @@ def test_entries_outside_the_grid(port, n, k, layout):
     agent that leaves) is carried through every list"""
     done, outside = _run(port, *_crowd(n, n + 3, True), 40, k, layout)
     assert done == 40 and outside > 0
+
+
+def test_tuner_reports_the_layout_it_timed(lib, c1_small):
+    """in the kd-tree mode the tuner times the automatic layout, one trial per
+    cell size (nothing else is read there), and what it reports can be set"""
+    from ecmgenerator_gb300._lib import EcmgError
+    from ecmgenerator_gb300.simulator import Simulator, autotune, set_lp_mode, set_neighbor_mode
+
+    scene, st, paths = c1_small
+    n = st.num_agents
+    out = []
+    for tuned in (False, True):
+        sim = Simulator(scene, n, 1.0 / 60.0, max_neighbors=10, **ORCA)
+        set_neighbor_mode(sim, "kdtree")
+        sim.add_agents(st.pos[:n], st.clear[:n], st.pref_speed[:n], paths[:n])
+        if tuned:
+            set_lp_mode(sim, "thread", 1)
+            r = autotune(sim, ticks_per_trial=1)
+            assert r["lp_mode"] == "auto" and r["trials"] == 7
+            set_lp_mode(sim, r["lp_mode"])
+            with pytest.raises(EcmgError):
+                set_lp_mode(sim, "warp")
+        sim.update(ticks=5)
+        out.append((sim.get_position_data(), sim.get_velocity_data()))
+        sim.close()
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+def test_back_to_the_automatic_layout(lib, c1_small):
+    from ecmgenerator_gb300.simulator import Simulator, set_lp_mode
+
+    scene, st, paths = c1_small
+    n = st.num_agents
+    out = []
+    for switch in (False, True):
+        sim = Simulator(scene, n, 1.0 / 60.0, max_neighbors=10, **ORCA)
+        sim.add_agents(st.pos[:n], st.clear[:n], st.pref_speed[:n], paths[:n])
+        for mode in ("thread", "auto", "warp", "auto") if switch else ("auto",) * 4:
+            set_lp_mode(sim, mode)
+            sim.update(ticks=3)
+        out.append((sim.get_position_data(), sim.get_velocity_data()))
+        sim.close()
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
