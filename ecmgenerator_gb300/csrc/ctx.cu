@@ -2067,7 +2067,10 @@ int ecmg_kernels_per_tick(const ecmg_ctx* c)
        k_neighbors, k_agents (or k_agents_group); k_features with a proposal
        model or a trace; k_mlp_infer with a proposal model */
     if (!c) return 6;
-    int n = bin_kernels(c->total_buckets, c->max_agents) + 3 + ((c->model || c->trace) ? 1 : 0) + (c->model ? 1 : 0);
+    /* the graph is captured for every slot; without it a tick is launched for
+       those up to the last in use */
+    const int slots = c->prm.use_graph || c->dev_last < 0 ? c->max_agents : c->dev_last + 1;
+    int n = bin_kernels(c->total_buckets, slots) + 3 + ((c->model || c->trace) ? 1 : 0) + (c->model ? 1 : 0);
     /* kd-tree mode, instead of k_neighbors */
     if (c->nbr_mode == ECMG_NEIGHBORS_KDTREE) n += -1 + kd_kernels(c->max_agents);
     return n;
