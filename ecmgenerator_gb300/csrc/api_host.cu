@@ -122,8 +122,8 @@ ecmg_status ecmg_planner_locate(ecmg_planner* pl, int n, const float* xy, int* o
 
 /* ---------------------------------------------------------------------- */
 /* The grid of the stand-alone kNN: cells of `cell` metres over the box with
-   one spare ring and one overflow bucket.  Sizes are computed in double and
-   refused (false) when the box or the cell is not finite or the grid would
+   one spare ring; agents beyond it belong to the border cells.  Sizes are
+   computed in double and refused (false) when the box or the cell is not finite or the grid would
    exceed kKnnMaxCells cells, so that no int below overflows. */
 bool ecmg::knn_grid_of(float x0, float y0, float x1, float y1, float cell, AgentGrid* out)
 {
@@ -185,7 +185,7 @@ ecmg_status ecmg_knn(const float* dev_pos, const unsigned char* dev_active, int 
     int* cell_start = (int*)take(sizeof(int) * (nb + 1));
     int* scan_tmp = (int*)take(sizeof(int) * (size_t)scan_tmp_ints((int)nb));
     cudaError_t e = launch_knn((const V2*)dev_pos, dev_active, n, k, radius, g, key, rank, cell_count, cell_start,
-                               s_slot, s_pos, scan_tmp, 0, dev_out_ids, dev_out_count, (cudaStream_t)stream);
+                               s_slot, s_pos, scan_tmp, dev_out_ids, dev_out_count, (cudaStream_t)stream);
     return e == cudaSuccess ? ECMG_OK : ECMG_ERR_CUDA;
 }
 

@@ -228,7 +228,7 @@ struct ecmg_ctx {
     int trace_rows = 0;
     DBuf<unsigned char> feat, cls, label;
     /* pinned staging */
-    int* h_counters = nullptr; /* [3 * kCounters]: (unused), out, after k_attract */
+    int* h_counters = nullptr; /* [2 * kCounters]: after the tick, after k_attract */
     DBuf<int> d_last;          /* the last slot index of the tick's binning, uploaded when it changes */
     int dev_last = -1;
     void* hview[4] = {nullptr, nullptr, nullptr, nullptr}; /* ecmg_host_view of the float2 fields */
@@ -431,7 +431,7 @@ ecmg_status ecmg_create_batch(const ecmg_params* p, int n_scenes, const int* max
     CKC(cudaMemset(c->path_off.p, 0, sizeof(int) * N));
     CKC(cudaMemset(c->d_clear.p, 0, sizeof(float) * N)); CKC(cudaMemset(c->d_speed.p, 0, sizeof(float) * N));
     CKC(c->d_last.alloc(1));
-    CKC(cudaHostAlloc((void**)&c->h_counters, sizeof(int) * 3 * kCounters, cudaHostAllocDefault));
+    CKC(cudaHostAlloc((void**)&c->h_counters, sizeof(int) * 2 * kCounters, cudaHostAllocDefault));
     CKC(cudaHostAlloc((void**)&c->h_lists, sizeof(int) * 4 * ecmg_ctx::kListStage, cudaHostAllocDefault));
     c->active.assign(N, 0);
     c->clear.assign(N, 0.0f);
@@ -1840,10 +1840,12 @@ static ecmg_status ensure_grids(ecmg_ctx* c)
    Measured (per-agent kernel, us; 1 / 4 / 8 / 16 / 32 lanes): 1,000 agents of
    the box scene 42 / 23 / 20 / 19 / 18; 25,000 there 59 / 33 / 32 / 38 / 51;
    crossing 30,000 93 / 45 / 45 / 50 / 64; 100,000 174 / 121 / 138 / 174 / 243;
-   300,000 249 / 264 / 322 / 434 / 672; 1,000,000 385 / 599 / ... .  The line
-   between 1 and 4 lies at 230,000 agents in the 400 m crossing (200,000: 227
-   and 218) and at 160,000 at the density of its million (125,000 in 200 m: 176
-   and 156; 180,000: 173 and 192).  The kd-tree mode's lists are not in order
+   300,000 249 / 264 / 322 / 434 / 672; 1,000,000 350 / 599 / ... .  Where 1
+   and 4 cross depends on density: at 230,000 agents in the 400 m crossing
+   (200,000: 227 and 218), at 160,000 at the density of its million (125,000 in
+   200 m: 176 and 156; 180,000: 173 and 192).  The rule goes by the count alone
+   and takes the dense crowd's line, where a wrong choice costs 11 % against 4 %
+   between the two.  The kd-tree mode's lists are not in order
    of distance, which costs a thread's constraint loop its coherence: 4 lanes
    there (250,000 agents: 422 and 347). */
 static int lanes_of(ecmg_ctx* c)
@@ -1986,7 +1988,7 @@ static cudaError_t propose_cb(void* user, cudaStream_t s)
 static cudaError_t after_attract_cb(void* user, cudaStream_t s, unsigned evflags)
 {
     ecmg_ctx* c = (ecmg_ctx*)user;
-    cudaError_t e = cudaMemcpyAsync(c->h_counters + 2 * kCounters, c->counters.p, sizeof(int) * kCounters,
+    cudaError_t e = cudaMemcpyAsync(c->h_counters + kCounters, c->counters.p, sizeof(int) * kCounters,
                                     cudaMemcpyDeviceToHost, s);
     const size_t ls = (size_t)std::min(ecmg_ctx::kListStage, c->max_agents);
     int* hl = c->h_lists;
@@ -2055,7 +2057,7 @@ static cudaError_t enqueue_tick(ecmg_ctx* c, int launch_slots, bool use_model)
                     c->ev_join, c->ev_k,
                     use_model ? propose_cb : nullptr, &pc, after_attract_cb, c, c->nbr_mode == 1 ? &kd : nullptr);
     if (e != cudaSuccess) return e;
-    return cudaMemcpyAsync(c->h_counters + kCounters, c->counters.p, sizeof(int) * kCounters, cudaMemcpyDeviceToHost,
+    return cudaMemcpyAsync(c->h_counters, c->counters.p, sizeof(int) * kCounters, cudaMemcpyDeviceToHost,
                            c->stream);
 }
 
@@ -2168,7 +2170,7 @@ static ecmg_status run_ticks(ecmg_ctx* c, int n_ticks, ecmg_tick_stats* stats)
            device; path uploads are queued behind the tick */
         CK(cudaEventSynchronize(c->ev_mid));
         auto h0 = std::chrono::steady_clock::now();
-        const int* mid = c->h_counters + 2 * kCounters;
+        const int* mid = c->h_counters + kCounters;
         const int nd_mid = mid[C_DESTROYED], nr = mid[C_REPLAN];
         st.replans_host += nr;
         /* the destroys of a tick with a fix-up are known only after it */
@@ -2243,8 +2245,8 @@ static ecmg_status run_ticks(ecmg_ctx* c, int n_ticks, ecmg_tick_stats* stats)
             TickArgs tf;
             fill_args(c, bf, tf, use_model);
             CK(launch_fixup(tf, c->d_pend.p, npend, c->stream));
-            CK(cudaMemcpyAsync(c->h_counters + kCounters, c->counters.p, sizeof(int) * kCounters,
-                               cudaMemcpyDeviceToHost, c->stream));
+            CK(cudaMemcpyAsync(c->h_counters, c->counters.p, sizeof(int) * kCounters, cudaMemcpyDeviceToHost,
+                               c->stream));
         }
         /* the getters' host arrays: slots [0, last] are all this tick can
            have moved (spawns included); the copy runs while the host does
@@ -2254,7 +2256,7 @@ static ecmg_status run_ticks(ecmg_ctx* c, int n_ticks, ecmg_tick_stats* stats)
         st.host_ms += std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - h0).count();
         CK(cudaStreamSynchronize(c->stream));
         c->h_up_used = 0; /* every queued upload has been applied */
-        const int* fin = c->h_counters + kCounters;
+        const int* fin = c->h_counters;
         if (npend > 0) {
             /* the fix-up's destroys join the tick's; its re-plans (an agent whose
                new path already fails) are served now */
@@ -2302,7 +2304,7 @@ static ecmg_status run_ticks(ecmg_ctx* c, int n_ticks, ecmg_tick_stats* stats)
         st.neighbors_ms += nbr;
         st.proposal_ms += prop;
         st.orca_ms += orca;
-        const int* out = c->h_counters + kCounters;
+        const int* out = c->h_counters;
         st.agent_steps += out[C_NSORTED];
         st.lp3d += out[C_LP3D];
         st.proposed += out[C_PROPOSED];

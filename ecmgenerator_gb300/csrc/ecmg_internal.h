@@ -41,7 +41,6 @@ enum {
     C_REPLAN = 1,
     C_LP3D = 2,
     C_ERROR = 3,       /* bitmask of ECMG_DEV_ERR_* */
-    C_PROCESSED = 4,   /* agents processed by the per-agent kernel */
     C_WORK = 5,        /* work counter of the persistent agent kernel */
     C_LAST = 6,        /* last slot index of the tick */
     C_NSORTED = 7,     /* agents in the neighbour grid */
@@ -190,7 +189,7 @@ constexpr double kKnnMaxCells = 32.0e6;
 bool knn_grid_of(float x0, float y0, float x1, float y1, float cell, AgentGrid* out);
 cudaError_t launch_knn(const V2* pos, const unsigned char* active, int n, int k, float r, AgentGrid g,
                        int* key, int* rank, int* cell_count, int* cell_start, int* s_slot, V2* s_pos,
-                       int* scan_tmp, int scan_blocks, int* out_ids, int* out_cnt, cudaStream_t s);
+                       int* scan_tmp, int* out_ids, int* out_cnt, cudaStream_t s);
 int scan_tmp_ints(int n);
 int bin_kernels(int total_buckets, int slots); /* launches of the binning */
 /* kernels.cu: mark the agents of `list` pending (before the tick's graph);
@@ -236,7 +235,8 @@ cudaError_t launch_spawn_place(const SpawnRec* rec, int n, const SpawnTargets& t
 
 /* kdtree.cu: the reference's kd-tree neighbour query (neighbour mode
    ECMG_NEIGHBORS_KDTREE).  Members = agents in this tick's grid (active at
-   the start of the tick); lists hold slots. */
+   the start of the tick).  The build's lists hold slots; the query's lists and
+   their composition hold grid indices, the cache between ticks slots again. */
 struct KdArgs {
     int max_slots, cap, k, levels, tree_cap;
     const V2* pos;              /* slot-indexed positions at the start of the tick */
@@ -262,7 +262,7 @@ struct KdArgs {
     unsigned long long* scan_tmp64;
     int* hist;                  /* [kd_hist_ints(cap)] */
     int* tree;                  /* [tree_cap] KDTree::m_Tree */
-    float4* tree_pos;           /* [tree_cap] position and slot (bits) of each node's agent */
+    float4* tree_pos;           /* [tree_cap] position and grid index (bits) of each node's agent */
     int* gidx;                  /* [max_slots] members' grid indices */
     unsigned char* open;        /* [cap] by grid index: the row refers to the list before it */
     int* agg;                   /* [kd_compose_rows * k] */

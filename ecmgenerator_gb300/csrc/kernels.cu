@@ -1113,9 +1113,8 @@ cudaError_t launch_fixup(const TickArgs& t, const int* list, int n, cudaStream_t
 
 cudaError_t launch_knn(const V2* pos, const unsigned char* active, int n, int k, float r, AgentGrid g,
                        int* key, int* rank, int* cell_count, int* cell_start, int* s_slot, V2* s_pos,
-                       int* scan_tmp, int scan_blocks, int* out_ids, int* out_cnt, cudaStream_t s)
+                       int* scan_tmp, int* out_ids, int* out_cnt, cudaStream_t s)
 {
-    (void)scan_blocks;
     /* the counters live behind the bucket counts: [nb+1 .. nb+1+kCounters) */
     int nb = g.ncells + 1;
     int* counters = cell_count + nb + 1;

@@ -53,8 +53,10 @@ constexpr unsigned kKnnCode = 63u; /* low key bits: entry of the index column */
    Buffer entries: 8 merge into 16 at the cost per candidate of 16, with less
    of the buffers empty (a flush takes the whole warp); for K = 32 the merge
    weighs more.  Index column: every candidate accepted (24 on average at
-   k = 16); 46 entries keep eight blocks on an SM, a lane that needs more (9 %
-   of the warps have one in the 1M crossing) searches again (renumbering the
+   k = 16); with 46 entries eight blocks of the stand-alone query fit an SM's
+   shared memory (the tick's, beside the attraction kernel, gets half or three
+   quarters of it: four or six).  A lane that needs more (9 % of the warps have
+   one in the 1M crossing) searches again, twice at most (renumbering the
    column instead cost every warp 15 % of its instructions, run or not; sent to
    the 64-bit search these lanes took the kernel from 318 to 369 us). */
 template <int K>

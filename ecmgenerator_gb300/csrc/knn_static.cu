@@ -77,6 +77,6 @@ extern "C" ecmg_status ecmg_knn_noalloc(const float* dev_pos, const unsigned cha
     int* cell_start = (int*)take(sizeof(int) * (nb + 1));
     int* scan_tmp = (int*)take(sizeof(int) * (size_t)scan_tmp_ints((int)nb));
     cudaError_t e = launch_knn((const V2*)dev_pos, dev_active, n, k, radius, g, key, rank, cell_count, cell_start,
-                               s_slot, s_pos, scan_tmp, 0, dev_out_ids, dev_out_count, (cudaStream_t)stream);
+                               s_slot, s_pos, scan_tmp, dev_out_ids, dev_out_count, (cudaStream_t)stream);
     return e == cudaSuccess ? ECMG_OK : ECMG_ERR_CUDA;
 }

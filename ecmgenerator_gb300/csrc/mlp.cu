@@ -286,7 +286,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v)
     for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
-/* barrier of one 4-warp group (ids 1 and 2; 0 is the CTA barrier) */
+/* barrier of one 4-warp group (ids 1 to 4; 0 is the CTA barrier) */
 __device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
 /* barrier of one group that also ORs a flag over its threads */
 __device__ __forceinline__ bool group_any(bool v, int id)
@@ -874,9 +874,11 @@ __global__ void __launch_bounds__(kTrThreads, 1)
         /* the column group that holds the label counts the row */
         if (valid && yl >= 0) loss += -(zt - mx - logf(se));
         if (valid && cg == 0 && am == yy) right++;
-        /* (e / se - [label]) / B, each quotient correctly rounded from the
-           divisor's reciprocal by one residual step (Markstein; 1 <= se <=
-           160); a row beyond the batch counts nothing */
+        /* (e / se - [label]) / B, each quotient from the divisor's reciprocal
+           and one residual step (Markstein; 1 <= se <= 160): correctly rounded
+           while the residual is a normal number, down to some 1e-30, and off by
+           a unit of the smallest number below; a row beyond the batch counts
+           nothing */
         const float rse = 1.0f / se, rb = valid ? rfb : 0.0f;
         auto quotient = [](float x, float d, float rd) {
             const float q = x * rd;

@@ -3,8 +3,9 @@ counterpart; the LP it short-cuts is ``ORCA::RandomizedLP``, ORCA.cpp:428-587).
 
 ``ProposalModel`` wraps ``ecmg_mlp``: a 96 -> 128 -> 128 -> 160 MLP whose
 inference runs in BF16 on the tensor cores inside the tick and whose training
-(FP32 forward/backward, softmax cross-entropy, Adam) runs in this library's own
-CUDA kernels.  ``collect_traces`` runs a simulator in trace mode and gathers
+(matrix products of BF16 operands accumulated in FP32; activations, softmax
+cross-entropy, master weights and Adam in FP32) runs in this library's own CUDA
+kernels.  ``collect_traces`` runs a simulator in trace mode and gathers
 (features, class of the plain LP result) rows on the device.
 
 Class encoding (neighbour q is the q-th nearest, constraint index nObst + q):
