@@ -45,7 +45,7 @@ __device__ __forceinline__ int bucket_of(const AgentGrid& g, V2 p)
  * for keys within 2^-17 of each other ("near ties"), which are re-sorted by
  * the exact (d2, slot).  A near tie that may reach past the list (`rej` is the
  * smallest key dropped) is settled among the entries of the index column: a
- * crowd on a lattice has one nearly everywhere (100,000 points, k = 16: 101 us;
+ * crowd on a lattice has one nearly everywhere (100,000 points, k = 16: 88 us;
  * 508 when such lanes went to the 64-bit search).
  * ---------------------------------------------------------------------- */
 constexpr unsigned kKnnCode = 63u; /* low key bits: entry of the index column */
@@ -69,8 +69,8 @@ constexpr int kKnnIdx = K <= 8 ? 32 : (K <= 16 ? 46 : 64);
    that is wanted, whose first estimate is unreliable, and a column that is full
    would begin the search again and again: rows are tested eight at a time, and
    a full column is renumbered.  20,000 points in one cell of 4 m take 3,400 us
-   so, 17,900 with the ordinary search; 20,000 outside the grid 3,480 and
-   13,000.  Evenly spread crowds do not care which (100,000 points, k = 16: 61
+   so, 17,900 with the ordinary search; 20,000 outside the grid 1,350 to
+   1,940 and 13,000.  Evenly spread crowds do not care which (100,000 points, k = 16: 61
    and 63 us with 121 agents in the 3 x 3 cells, 238 and 242 with 1,944); at
    256 the ticks of the measured crowds all take the ordinary one. */
 constexpr int kKnnDense = 256;
@@ -391,21 +391,27 @@ __device__ __noinline__ void knn_tied(const int* column, int n, int k, int befor
     int id[K];
     const int room = k - before;
     int have = 0;
-    for (int i = 0; i < n; i++) {
-        const int j = column[i * 32];
-        const V2 c = s_pos[j];
-        const float dx = c.x - p.x, dy = c.y - p.y;
-        const unsigned d2 = __float_as_uint(dx * dx + dy * dy);
-        if ((d2 & ~kKnnCode) != hi) continue;
-        const unsigned long long kk = ((unsigned long long)d2 << 32) | (unsigned)s_slot[j];
-        if (have == room && kk >= key[room - 1]) continue;
-        int q = have < room ? have++ : room - 1;
-        for (; q > 0 && key[q - 1] > kk; q--) {
-            key[q] = key[q - 1];
-            id[q] = id[q - 1];
+    const float2 np = make_float2(-p.x, -p.y);
+    for (int i0 = 0; i0 < n; i0 += 4) {
+        unsigned d2[4];
+        int j[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) j[u] = column[min(i0 + u, n - 1) * 32];
+#pragma unroll
+        for (int u = 0; u < 4; u++) d2[u] = __float_as_uint(dist2(s_pos[j[u]], np));
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (i0 + u >= n || (d2[u] & ~kKnnCode) != hi) continue;
+            const unsigned long long kk = ((unsigned long long)d2[u] << 32) | (unsigned)s_slot[j[u]];
+            if (have == room && kk >= key[room - 1]) continue;
+            int q = have < room ? have++ : room - 1;
+            for (; q > 0 && key[q - 1] > kk; q--) {
+                key[q] = key[q - 1];
+                id[q] = id[q - 1];
+            }
+            key[q] = kk;
+            id[q] = j[u];
         }
-        key[q] = kk;
-        id[q] = j;
     }
     for (int q = 0; q < have; q++) o[before + q] = id[q];
 }
@@ -425,8 +431,23 @@ __device__ __noinline__ int knn_exact(int k, V2 p, float lim, float r2, const V2
     const float w = sqrtf(lim) * 1.000001f + g.slack;
     const int xa = cell_clamp((p.x - w - g.x0) * g.inv, g.gw), xb = cell_clamp((p.x + w - g.x0) * g.inv, g.gw);
     const int ya = cell_clamp((p.y - w - g.y0) * g.inv, g.gh), yb = cell_clamp((p.y + w - g.y0) * g.inv, g.gh);
+    const float2 np = make_float2(-p.x, -p.y);
     for (int y = ya; y <= yb; y++) {
-        for (int j = cs[y * g.gw + xa], e = cs[y * g.gw + xb + 1]; j < e; j++) {
+        const int e = cs[y * g.gw + xb + 1];
+        for (int j = cs[y * g.gw + xa], next = j; j < e; j++) {
+            if (j == next) { /* eight at a time while none can enter: a lone lane waits for every load */
+                float d[8];
+                bool want = false;
+#pragma unroll
+                for (int q = 0; q < 8; q++) d[q] = dist2(s_pos[min(j + q, e - 1)], np);
+#pragma unroll
+                for (int q = 0; q < 8; q++) want |= !(d[q] > lim);
+                next += 8;
+                if (!want) {
+                    j += 7;
+                    continue;
+                }
+            }
             const V2 c = s_pos[j];
             const float dx = c.x - p.x, dy = c.y - p.y;
             const float d2 = dx * dx + dy * dy;
