@@ -420,11 +420,12 @@ def run_ours(args):
         e2e[name] = e2e_steps * max(world, 1) / (t1 - t0)
     gc.enable()
     e2e_main = {"value": e2e["learned" if model is not None else "plain"], "unit": "agent-steps/s",
-                "h2d_bytes_per_step": 64, "d2h_bytes_per_step": 16 * n + 64,
+                "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 16 * n + 2 * 64 + 16 * min(n, 1024),
                 "plain": e2e["plain"], "note": "wall clock of Simulator.update() + the position and velocity getters "
                 "(ecmg_host_view) per tick; each tick ends with a device copy of the positions and velocities "
-                "into the page-locked host arrays the getters return (ecmg_set_host_mirror); h2d = counters, d2h = positions and velocities + "
-                "counters"}
+                "into the page-locked host arrays the getters return (ecmg_set_host_mirror); a tick takes no input from the host (its state stays "
+                "on the device, its counters start there); d2h = positions and velocities + the counters, twice, and the "
+                "first 1,024 places of the lists of removed and re-planned agents"}
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(HERE, "MEASURED_PEAKS.json")))

@@ -2002,7 +2002,7 @@ static cudaError_t after_attract_cb(void* user, cudaStream_t s, unsigned evflags
     return e;
 }
 
-/* the device work of one tick: counters in, kernels, counters out */
+/* the device work of one tick: kernels, counters out */
 static cudaError_t enqueue_tick(ecmg_ctx* c, int launch_slots, bool use_model)
 {
     BinArgs b;

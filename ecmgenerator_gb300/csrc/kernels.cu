@@ -619,9 +619,9 @@ __device__ void orca_tick(const TickArgs& a, int t)
    Persistent: a warp takes 32 consecutive grid-order agents per work grab
    (neighbouring agents: their candidates share L1), so that warps whose
    agents have more candidates do not leave the SMs' last wave ragged.  Bound
-   by instruction issue: 156 warp instructions per agent at 29.9 of 32 threads
-   (250,000 of the crossing); a million 302 us beside k_attract (416 with one
-   insertion per candidate and cells in distance order), 25,000 26 (86-105,
+   by instruction issue: 158 warp instructions per agent at 30.2 of 32 threads
+   (250,000 of the crossing); a million 287 us beside k_attract (416 with one
+   insertion per candidate and cells in distance order), 25,000 23 (86-105,
    where a cell of more than 32 agents sent its lanes to the 64-bit search) */
 constexpr int kNbrWarps = 4; /* per block */
 template <int K>
