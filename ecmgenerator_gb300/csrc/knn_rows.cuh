@@ -172,11 +172,11 @@ __device__ __forceinline__ float dist2(V2 q, float2 np)
    ties that must be re-sorted by the exact key, 3 when a near tie may reach
    past the list (whoever it may mean was accepted and is among the first
    *column entries of the lane's index column), 0 when the index column was too
-   short for the search (CROWD: for such a tie, the list itself is right but
-   for it).  n9: the agents of the 3 x 3 cells around p; cs: the scene's cell
+   short for the search or the warp is one for the other variant (CROWD: for
+   such a tie, the list itself is right but for it).  cs: the scene's cell
    starts. */
 template <int K, bool CROWD>
-__device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, float r2, int n9, const V2* s_pos,
+__device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, float r2, const V2* s_pos,
                                         const int* cs, const AgentGrid& g, float (&key)[K], int* column)
 {
     constexpr int B = kKnnBuf<K>;
@@ -188,6 +188,7 @@ __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, f
     int ord = 0, ord0 = 0; /* next entry of the index column; that of the buffer's first candidate */
     bool over = false;     /* the index column is full (CROWD: has been renumbered) */
     int tries = 0;         /* searches begun again for that */
+    valid = valid && p.x - p.x == 0.0f && p.y - p.y == 0.0f; /* no distance to a non-finite position is finite */
     const float fy = (p.y - g.y0) * g.inv;
     const int cx = cell_clamp((p.x - g.x0) * g.inv, g.gw), cy = cell_clamp(fy, g.gh);
     /* distance to the nearer end of the own row (0 outside the grid) and the
@@ -197,14 +198,22 @@ __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, f
     const float edge = fmaxf(fminf(ry, g.cell - ry), 0.0f) - g.slack;
     const float2 np = make_float2(-p.x, -p.y);
     float lim = 0.0f, lo = kEps, disc = 0.0f, more_area = 3.0f;
+    int n9 = 0; /* agents of the 3 x 3 cells around p */
     if (valid) {
         const int xa = max(cx - 1, 0), xb = min(cx + 1, g.gw - 1), ya = max(cy - 1, 0), yb = min(cy + 1, g.gh - 1);
+        for (int y = ya; y <= yb; y++) n9 += cs[y * g.gw + xb + 1] - cs[y * g.gw + xa];
         const float area = (float)((xb - xa + 1) * (yb - ya + 1)) * g.cell * g.cell;
         /* pi disc n9 / area = 1.8 (k + 2) */
         disc = fminf(r2, 0.573f * (float)(k + 2) * area / (float)max(n9, 1));
         /* a border cell is endless: the agents outside the grid are in it */
         if (CROWD && (cx == 0 || cx == g.gw - 1 || cy == 0 || cy == g.gh - 1)) disc = r2;
         lim = disc;
+    }
+    if (!CROWD && __any_sync(kAll, n9 > kKnnDense)) { /* not a search for this variant */
+        over = valid;
+        tries = 2;
+        lim = 0.0f;
+        disc = r2;
     }
     while (true) {
         const int far_row = max(cy, g.gh - 1 - cy);
@@ -513,13 +522,12 @@ __device__ __forceinline__ int knn_write(const KnnSm<K>& sm, int st, int k, V2 p
 /* knn_list where the cells hold far more agents than a search wants (out of
    line, so that the ordinary search keeps its registers and instructions) */
 template <int K, bool SLOTS>
-__device__ __noinline__ int knn_list_crowd(KnnSm<K>* sm, bool valid, int k, V2 p, float r2, int n9, const V2* s_pos,
+__device__ __noinline__ int knn_list_crowd(KnnSm<K>* sm, bool valid, int k, V2 p, float r2, const V2* s_pos,
                                            const int* s_slot, const int* cs, const AgentGrid* g, int* o)
 {
     float key[K];
     int column;
-    const bool finite = p.x - p.x == 0.0f && p.y - p.y == 0.0f;
-    const int st = knn_rows<K, true>(*sm, valid && finite, k, p, r2, n9, s_pos, cs, *g, key, &column);
+    const int st = knn_rows<K, true>(*sm, valid, k, p, r2, s_pos, cs, *g, key, &column);
     return valid ? knn_write<K, SLOTS>(*sm, st, k, p, r2, key, column, s_pos, s_slot, cs, *g, o) : 0;
 }
 
@@ -530,26 +538,14 @@ template <int K, bool SLOTS>
 __device__ __forceinline__ int knn_list(KnnSm<K>& sm, bool valid, int k, V2 p, float r2, const V2* s_pos,
                                         const int* s_slot, const int* cs, const AgentGrid& g, int* o)
 {
-    constexpr unsigned kAll = 0xffffffffu;
-    const bool finite = p.x - p.x == 0.0f && p.y - p.y == 0.0f; /* no distance to another position is finite */
-    int n9 = 0;                                                  /* agents of the 3 x 3 cells around p */
-    if (valid && finite) {
-        const int cx = cell_clamp((p.x - g.x0) * g.inv, g.gw), cy = cell_clamp((p.y - g.y0) * g.inv, g.gh);
-        const int xa = max(cx - 1, 0), xb = min(cx + 1, g.gw - 1), ya = max(cy - 1, 0), yb = min(cy + 1, g.gh - 1);
-        for (int y = ya; y <= yb; y++) n9 += cs[y * g.gw + xb + 1] - cs[y * g.gw + xa];
-    }
-    const bool dense = __any_sync(kAll, n9 > kKnnDense);
+    float key[K];
+    int column;
+    const int st = knn_rows<K, false>(sm, valid, k, p, r2, s_pos, cs, g, key, &column);
+    const bool left = valid && st == 0;
     int n = 0;
-    bool left = valid && dense;
-    if (!dense) {
-        float key[K];
-        int column;
-        const int st = knn_rows<K, false>(sm, valid && finite, k, p, r2, n9, s_pos, cs, g, key, &column);
-        left = valid && st == 0;
-        if (valid && !left) n = knn_write<K, SLOTS>(sm, st, k, p, r2, key, column, s_pos, s_slot, cs, g, o);
-    }
-    if (__any_sync(kAll, left)) {
-        const int c = knn_list_crowd<K, SLOTS>(&sm, left, k, p, r2, n9, s_pos, s_slot, cs, &g, o);
+    if (valid && !left) n = knn_write<K, SLOTS>(sm, st, k, p, r2, key, column, s_pos, s_slot, cs, g, o);
+    if (__any_sync(0xffffffffu, left)) {
+        const int c = knn_list_crowd<K, SLOTS>(&sm, left, k, p, r2, s_pos, s_slot, cs, &g, o);
         if (left) n = c;
     }
     return n;
