@@ -624,7 +624,13 @@ __device__ void orca_tick(const TickArgs& a, int t)
    insertion per candidate and cells in distance order), 25,000 23 (86-105,
    where a cell of more than 32 agents sent its lanes to the 64-bit search) */
 constexpr int kNbrWarps = 4; /* per block */
-template <int K>
+/* The variant for crowded cells (CROWDS) costs the ordinary search registers
+   wherever it stands in the kernel: a tick of 100 agents 55.7 -> 56.7 us, of
+   1,000 60.3 -> 60.9, a query of 100 points 16.5 -> 17.4, of 3,000 26.6 -> 27.4.
+   Crowds that are small leave a lane's 64-bit search little to do: ticks to
+   8,192 slots and queries to 2,048 points do without. */
+constexpr int kCrowdSlots = 8192, kCrowdPoints = 2048;
+template <int K, bool CROWDS>
 __global__ void __launch_bounds__(32 * kNbrWarps, K <= 16 ? 8 : 4) k_neighbors(TickArgs a)
 {
     __shared__ KnnSm<K> sm[kNbrWarps];
@@ -638,8 +644,8 @@ __global__ void __launch_bounds__(32 * kNbrWarps, K <= 16 ? 8 : 4) k_neighbors(T
         const int t = min(base + lane, n - 1);
         const bool in = base + lane < n;
         const SceneDev& sc = a.scenes[a.slot_scene ? a.slot_scene[a.s_slot[t]] : 0];
-        const int c = knn_list<K, false>(sm[threadIdx.x >> 5], in, a.k, a.s_pos[t], a.rnb2, a.s_pos, a.s_slot,
-                                  a.cell_start + sc.bucket_base, sc.grid, a.nbr + (size_t)t * a.k);
+        const int c = knn_list<K, false, CROWDS>(sm[threadIdx.x >> 5], in, a.k, a.s_pos[t], a.rnb2, a.s_pos, a.s_slot,
+                                                 a.cell_start + sc.bucket_base, sc.grid, a.nbr + (size_t)t * a.k);
         if (in) a.ncnt[t] = c;
     }
 }
@@ -905,7 +911,7 @@ __global__ void __launch_bounds__(32 * kGroupWarps, K <= 16 ? 7 : 4) k_agents_gr
 }
 
 /* the stand-alone query: lists of slots by slot */
-template <int K>
+template <int K, bool CROWDS>
 __global__ void __launch_bounds__(32 * kNbrWarps, K <= 16 ? 8 : 4)
     k_knn(const V2* s_pos, const int* s_slot, const int* cell_start, AgentGrid g, int k, float r2, const int* counters,
           int* out_ids, int* out_cnt)
@@ -919,7 +925,7 @@ __global__ void __launch_bounds__(32 * kNbrWarps, K <= 16 ? 8 : 4)
         const bool in = base + lane < n;
         const int slot = s_slot[t];
         int* o = out_ids + (size_t)slot * k;
-        const int c = knn_list<K, true>(sm[threadIdx.x >> 5], in, k, s_pos[t], r2, s_pos, s_slot, cell_start, g, o);
+        const int c = knn_list<K, true, CROWDS>(sm[threadIdx.x >> 5], in, k, s_pos[t], r2, s_pos, s_slot, cell_start, g, o);
         if (in) out_cnt[slot] = c;
     }
 }
@@ -1009,9 +1015,10 @@ cudaError_t launch_tick(const BinArgs& b, const TickArgs& t, int max_slots, int 
             e = launch_split(kern, grid_for(max_slots, 32 * kNbrWarps, sms, std::max(1, std::min(pn, t.knn_blocks))),
                              32 * kNbrWarps, split, s, t);
         };
-        if (t.k <= 8) go(k_neighbors<8>);
-        else if (t.k <= 16) go(k_neighbors<16>);
-        else go(k_neighbors<32>);
+        const bool crowds = max_slots > kCrowdSlots;
+        if (t.k <= 8) crowds ? go(k_neighbors<8, true>) : go(k_neighbors<8, false>);
+        else if (t.k <= 16) crowds ? go(k_neighbors<16, true>) : go(k_neighbors<16, false>);
+        else crowds ? go(k_neighbors<32, true>) : go(k_neighbors<32, false>);
         if (e != cudaSuccess) return e;
     }
     if (ev && !kd) cudaEventRecordWithFlags(ev[2], s, evflags);
@@ -1143,7 +1150,8 @@ cudaError_t launch_knn(const V2* pos, const unsigned char* active, int n, int k,
     auto query = [&](auto kern) {
         return launch_ahead(kern, ga, 32 * kNbrWarps, 0, s, s_pos, s_slot, cell_start, g, k, r2, counters, out_ids, out_cnt);
     };
-    return k <= 8 ? query(k_knn<8>) : (k <= 16 ? query(k_knn<16>) : query(k_knn<32>));
+    if (n > kCrowdPoints) return k <= 8 ? query(k_knn<8, true>) : (k <= 16 ? query(k_knn<16, true>) : query(k_knn<32, true>));
+    return k <= 8 ? query(k_knn<8, false>) : (k <= 16 ? query(k_knn<16, false>) : query(k_knn<32, false>));
 }
 
 }  // namespace ecmg

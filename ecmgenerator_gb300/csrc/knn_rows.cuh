@@ -68,12 +68,12 @@ constexpr int kKnnIdx = K <= 8 ? 32 : (K <= 16 ? 46 : 64);
    search for crowded cells (CROWD).  There most of a row lies outside the disc
    that is wanted, whose first estimate is unreliable, and a column that is full
    would begin the search again and again: rows are tested eight at a time, and
-   a full column is renumbered.  20,000 points in one cell of 4 m take 3,400 us
-   so, 17,900 with the ordinary search; 20,000 outside the grid 1,350 to
-   1,940 and 13,000.  Evenly spread crowds do not care which (100,000 points, k = 16: 61
-   and 63 us with 121 agents in the 3 x 3 cells, 238 and 242 with 1,944); at
-   256 the ticks of the measured crowds all take the ordinary one. */
-constexpr int kKnnDense = 256;
+   a full column is renumbered.  20,000 points in one cell of 4 m take 2,470 to
+   3,400 us so, 17,900 with the ordinary search; 20,000 outside the grid 1,890
+   and 13,000.  Evenly spread crowds set the line (100,000 points, ordinary /
+   crowded; k = 16: 337 in the 3 x 3 89 / 102 us, 864 141 / 150, 1,944 279 / 233,
+   3,456 437 / 330; k = 3: 740 66 / 117). */
+constexpr int kKnnDense = 1024;
 
 template <int K>
 struct KnnSm { /* of one warp */
@@ -172,10 +172,10 @@ __device__ __forceinline__ float dist2(V2 q, float2 np)
    ties that must be re-sorted by the exact key, 3 when a near tie may reach
    past the list (whoever it may mean was accepted and is among the first
    *column entries of the lane's index column), 0 when the index column was too
-   short for the search or the warp is one for the other variant (CROWD: for
-   such a tie, the list itself is right but for it).  cs: the scene's cell
+   short for the search or (CHECK) the warp is one for the other variant (CROWD:
+   for such a tie, the list itself is right but for it).  cs: the scene's cell
    starts. */
-template <int K, bool CROWD>
+template <int K, bool CROWD, bool CHECK>
 __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, float r2, const V2* s_pos,
                                         const int* cs, const AgentGrid& g, float (&key)[K], int* column)
 {
@@ -209,7 +209,7 @@ __device__ __forceinline__ int knn_rows(KnnSm<K>& sm, bool valid, int k, V2 p, f
         if (CROWD && (cx == 0 || cx == g.gw - 1 || cy == 0 || cy == g.gh - 1)) disc = r2;
         lim = disc;
     }
-    if (!CROWD && __any_sync(kAll, n9 > kKnnDense)) { /* not a search for this variant */
+    if (CHECK && __any_sync(kAll, n9 > kKnnDense)) { /* not a search for this variant */
         over = valid;
         tries = 2;
         lim = 0.0f;
@@ -426,7 +426,8 @@ __device__ __noinline__ void knn_tied(const int* column, int n, int k, int befor
 }
 
 /* the search by 64-bit (d2, slot) keys (rare: a near tie across the k-th place
-   after the column was renumbered; out of line): the rows of the disc of
+   after the column was renumbered, or a column full for the third time where
+   there is no variant for crowded cells; out of line): the rows of the disc of
    squared radius `lim`, which holds at least k agents or is r^2; o[q] gets
    the grid indices, the return value is the count */
 template <int K>
@@ -477,8 +478,8 @@ __device__ __noinline__ int knn_exact(int k, V2 p, float lim, float r2, const V2
     return n;
 }
 
-/* o[0 .. k) of one lane from its list and column (knn_rows' answer st, not 0
-   unless CROWD); returns the count */
+/* o[0 .. k) of one lane from its list and column (knn_rows' answer st); returns
+   the count */
 template <int K, bool SLOTS>
 __device__ __forceinline__ int knn_write(const KnnSm<K>& sm, int st, int k, V2 p, float r2, const float (&key)[K],
                                          int column, const V2* s_pos, const int* s_slot, const int* cs,
@@ -523,29 +524,30 @@ __device__ __forceinline__ int knn_write(const KnnSm<K>& sm, int st, int k, V2 p
    line, so that the ordinary search keeps its registers and instructions) */
 template <int K, bool SLOTS>
 __device__ __noinline__ int knn_list_crowd(KnnSm<K>* sm, bool valid, int k, V2 p, float r2, const V2* s_pos,
-                                           const int* s_slot, const int* cs, const AgentGrid* g, int* o)
+                                           const int* s_slot, const int* cs, AgentGrid g, int* o)
 {
     float key[K];
     int column;
-    const int st = knn_rows<K, true>(*sm, valid, k, p, r2, s_pos, cs, *g, key, &column);
-    return valid ? knn_write<K, SLOTS>(*sm, st, k, p, r2, key, column, s_pos, s_slot, cs, *g, o) : 0;
+    const int st = knn_rows<K, true, false>(*sm, valid, k, p, r2, s_pos, cs, g, key, &column);
+    return valid ? knn_write<K, SLOTS>(*sm, st, k, p, r2, key, column, s_pos, s_slot, cs, g, o) : 0;
 }
 
 /* the neighbour list of the agent at p: grid indices (SLOTS: slots) in
-   o[0 .. k), -1 beyond the count, which is returned.  All 32 lanes must call;
-   lanes with valid false write nothing. */
-template <int K, bool SLOTS>
+   o[0 .. k), -1 beyond the count, which is returned.  CROWDS: with the variant
+   for crowded cells.  All 32 lanes must call; lanes with valid false write
+   nothing. */
+template <int K, bool SLOTS, bool CROWDS>
 __device__ __forceinline__ int knn_list(KnnSm<K>& sm, bool valid, int k, V2 p, float r2, const V2* s_pos,
                                         const int* s_slot, const int* cs, const AgentGrid& g, int* o)
 {
     float key[K];
     int column;
-    const int st = knn_rows<K, false>(sm, valid, k, p, r2, s_pos, cs, g, key, &column);
-    const bool left = valid && st == 0;
+    const int st = knn_rows<K, false, CROWDS>(sm, valid, k, p, r2, s_pos, cs, g, key, &column);
+    const bool left = CROWDS && valid && st == 0;
     int n = 0;
     if (valid && !left) n = knn_write<K, SLOTS>(sm, st, k, p, r2, key, column, s_pos, s_slot, cs, g, o);
-    if (__any_sync(0xffffffffu, left)) {
-        const int c = knn_list_crowd<K, SLOTS>(&sm, left, k, p, r2, s_pos, s_slot, cs, &g, o);
+    if (CROWDS && __any_sync(0xffffffffu, left)) {
+        const int c = knn_list_crowd<K, SLOTS>(&sm, left, k, p, r2, s_pos, s_slot, cs, g, o);
         if (left) n = c;
     }
     return n;

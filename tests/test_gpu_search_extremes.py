@@ -82,62 +82,71 @@ def test_lattice(lib, k):
     assert t < 3.0 * _query(lib, rng.uniform(0, 126.6, pos.shape), k, 5.0, box, cell, 5)[2]
 
 
-def _crowded(name, rng):
-    """crowds far denser than their cells: positions, radius, box, cell"""
+def _crowded(name, rng, m):
+    """crowds far denser than their cells, about m agents: positions, radius,
+    box, cell"""
+    box, cell = (0, 0, 100, 100), 4.0
     if name == "cluster":
-        return rng.normal(50, 0.5, (4000, 2)), 5.0, (0, 0, 100, 100), 4.0
+        return rng.normal(50, 0.5, (m, 2)), 5.0, box, cell
     if name == "cluster and strays":
-        return np.concatenate([rng.normal(50, 0.1, (1500, 2)), rng.uniform(0, 100, (500, 2))]), 30.0, \
-            (0, 0, 100, 100), 4.0
-    if name == "lattice in a cell":  # ties in a column that has been renumbered
-        g = np.stack(np.meshgrid(np.arange(40), np.arange(40)), -1).reshape(-1, 2)
-        return 48.5 + 0.06 * g[rng.permutation(len(g))], 5.0, (0, 0, 100, 100), 4.0
-    if name == "coincident":  # more agents at one distance than a column holds
-        return np.repeat(rng.uniform(48.1, 51.9, (12, 2)), 100, 0), 5.0, (0, 0, 100, 100), 4.0
+        return np.concatenate([rng.normal(50, 0.1, (m, 2)), rng.uniform(0, 100, (1500, 2))]), 30.0, box, cell
+    if name == "lattice in a cell":  # ties across every k-th place
+        side = int(m**0.5)
+        g = np.stack(np.meshgrid(np.arange(side), np.arange(side)), -1).reshape(-1, 2)
+        return 48.5 + 0.04 * g[rng.permutation(len(g))], 5.0, box, cell
+    if name == "coincident":  # more agents at one distance than a list, a column or a warp holds
+        return np.repeat(rng.uniform(48.1, 51.9, (m // 100, 2)), 100, 0), 5.0, box, cell
+    if name == "few in reach":  # fewer than k within the radius
+        return rng.uniform(48, 52, (m, 2)), 0.05, box, cell
     if name == "outside":  # one corner cell holds everybody
-        return rng.uniform(0, 60, (4000, 2)) + 500, 5.0, (0, 0, 100, 100), 1.0
-    p = rng.uniform(48, 52, (1000, 2))  # "not finite"
+        return rng.uniform(0, 60, (m, 2)) + 500, 5.0, box, 1.0
+    p = rng.uniform(48, 52, (m, 2))  # "not finite"
     p[::7] = np.nan
     p[::11, 0] = np.inf
-    return p, 5.0, (0, 0, 100, 100), 4.0
+    return p, 5.0, box, cell
 
 
 @pytest.mark.parametrize("k", [1, 8, 9, 16, 17, 32])
-@pytest.mark.parametrize("name", ["cluster", "cluster and strays", "lattice in a cell", "coincident", "outside",
-                                  "not finite"])
-def test_crowded_cells(lib, name, k):
+@pytest.mark.parametrize("m", [900, 4000])  # on both sides of the sizes at which another variant is taken
+@pytest.mark.parametrize("name", ["cluster", "cluster and strays", "lattice in a cell", "coincident", "few in reach",
+                                  "outside", "not finite"])
+def test_crowded_cells(lib, name, m, k):
     rng = np.random.default_rng(4)
-    pos, r, box, cell = _crowded(name, rng)
+    pos, r, box, cell = _crowded(name, rng, m)
     ids, cnt, _ = _query(lib, pos, k, r, box, cell)
     with np.errstate(invalid="ignore", over="ignore"):
-        _check(pos, k, r, ids, cnt, rng.integers(0, len(pos), 400))
+        _check(pos, k, r, ids, cnt, rng.integers(0, len(pos), 300))
 
 
 def test_crowded_cell_in_time(lib):
     """every agent has to look at all 4,000: beside a crowd in cells that fit"""
     rng = np.random.default_rng(4)
-    pos, r, box, cell = _crowded("cluster", rng)
+    pos, r, box, cell = _crowded("cluster", rng, 4000)
     fit = _query(lib, rng.uniform(0, 26, pos.shape), 16, 5.0, (0, 0, 26, 26), 0.8, 5)[2]
     assert _query(lib, pos, 16, r, box, cell, 5)[2] < 60.0 * fit
 
 
-def test_tick_with_crowded_cells(lib, c1_small):
-    """cells of 40 m (everybody in the 3 x 3 around an agent) and the usual
-    ones: the same bits"""
+@pytest.mark.parametrize("n,slots,cell", [(300, 300, 40.0), (300, 8193, 40.0), (4000, 4000, 60.0), (4000, 8193, 60.0)])
+def test_tick_with_crowded_cells(lib, c1_small, n, slots, cell):
+    """cells with hundreds or thousands of agents in the 3 x 3 around one, and
+    the usual ones: the same lists and the same bits"""
     from ecmgenerator_gb300.simulator import Simulator
 
     scene, st, paths = c1_small
-    n = st.num_agents
+    rng = np.random.default_rng(6)
+    pos, goal = (st.pos[:n], None) if n <= 300 else (rng.uniform(5, 95, (n, 2)).astype(np.float32),
+                                                     rng.uniform(5, 95, (n, 2)).astype(np.float32))
+    ways = paths[:n] if n <= 300 else [np.stack([p, g]) for p, g in zip(pos, goal)]
     for k in (7, 16, 25):
         out = []
-        for cell in (0.0, 40.0):
-            sim = Simulator(scene, n, 1.0 / 60.0, max_neighbors=k, tau_agent=2.0, tau_obst=2.0, grid_cell=cell,
+        for c in (0.0, cell):
+            sim = Simulator(scene, slots, 1.0 / 60.0, max_neighbors=k, tau_agent=2.0, tau_obst=2.0, grid_cell=c,
                             neighbor_dist=15.0)
             sim.set_record(True)
-            sim.add_agents(st.pos[:n], st.clear[:n], st.pref_speed[:n], paths[:n])
-            sim.update(ticks=5)
+            sim.add_agents(pos, np.full(n, 0.25, np.float32), np.full(n, 1.3, np.float32), ways)
+            sim.update(ticks=3)
             rec = sim.get_record()
-            out.append((sim.get_position_data(), sim.get_velocity_data(), rec["nbr_ids"], rec["nbr_count"]))
+            out.append((sim.get_position_data(), sim.get_velocity_data(), rec["nbr_ids"][:n], rec["nbr_count"][:n]))
             sim.close()
         for a, b in zip(*out):
-            assert np.array_equal(a, b)
+            assert np.array_equal(a, b, equal_nan=True)
